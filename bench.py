@@ -420,9 +420,9 @@ def main():
     frac_view = rays_per_launch / R
     alg_fwd = 300.0 * args.gaussians + 16.0 * rays_per_launch
     alg_bwd = 536.0 * args.gaussians + 28.0 * rays_per_launch
-    # the forward's recording for the backward: per slab with hits a 528-byte head with the per-sample sums and
-    # 4 bytes per hit; written once by the forward, read once by the backward
-    tape_bytes = (528.0 * Sh + 4.0 * P) * frac_view
+    # the forward's recording for the backward: 140 ints per ray and slab with hits, nearly all of it the per-sample sums (the
+    # list of hits is shared by the rays of a patch); written once by the forward, read once by the backward
+    tape_bytes = 560.0 * Sh * frac_view
     # DRAM traffic of one forward launch = what it records + the Gaussian records and lists it streams once;
     # ratio taken from ncu captures of smaller cases on both sides of the L2 size (profiles/)
     traffic = TRAFFIC_PER_RECORDED_BYTE * tape_bytes
@@ -442,17 +442,17 @@ def main():
     view_ms = ms_per_step / max(1, len(blocks0))
     step_fp32 = (f_fwd + f_bwd) / (view_ms * 1e-3) / fp32_peak
     step_mufu = (mufu_fwd + mufu_bwd) / (view_ms * 1e-3) / mufu_peak
-    roofline = {"kernel": "march_forward_lists_kernel<false,true,2> (forward march, recording for the backward, over lists that stop at a horizon)",
+    roofline = {"kernel": "march_forward_patches_kernel<2,false,true,2> (forward march, recording for the backward, over lists that stop at a horizon)",
                 "bound": "fp32-issue", "achieved": achieved, "peak": hbm_peak,
                 "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_src, "traffic": traffic,
-                "traffic_note": "DRAM bytes of one launch: the recording (528 B per slab with hits + 4 B per hit) "
+                "traffic_note": "DRAM bytes of one launch: the recording (560 B per ray and slab with hits) "
                                 "times the ratio ncu measured on smaller cases; not part of the algorithmic bytes",
                 "ms_per_launch": fwd_ms, "launches_timed": ktimes["forward_launches"],
                 "algorithmic_bytes_per_launch": alg_fwd, "recorded_bytes_per_launch": tape_bytes,
                 "fp32_frac": f_fwd / (fwd_ms * 1e-3) / fp32_peak, "mufu_frac": mufu_fwd / (fwd_ms * 1e-3) / mufu_peak,
                 "achieved_step": max(step_fp32, step_mufu), "step_fp32_frac": step_fp32, "step_mufu_frac": step_mufu,
                 "step_ms_per_launch_of_rays": view_ms,
-                "backward": {"kernel": "march_backward_replay_kernel + march_backward_lists_kernel",
+                "backward": {"kernel": "march_backward_patches_kernel + march_backward_lists_kernel",
                              "ms_per_launch": bwd_ms, "launches_timed": ktimes["backward_launches"],
                              "algorithmic_bytes_per_launch": alg_bwd,
                              "achieved": alg_bwd / (bwd_ms * 1e-3) / 1e9,

@@ -1,5 +1,6 @@
 // C ABI of librgx.so: context, workspace and the entry points of include/rgx.h.
 #include "rgx_internal.cuh"
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -46,6 +47,7 @@ struct rgx_ctx {
     int* bounds = nullptr;
     SceneBox* box = nullptr;
     DeviceCounters* counters = nullptr;
+    unsigned int* next_unit = nullptr;
     // state of the last build
     bool built = false;
     int n = 0, n_pad = 0;
@@ -109,7 +111,7 @@ struct rgx_ctx {
     long long tape_cap = 0;
     unsigned long long* tape_used = nullptr;
     unsigned long long* tape_used_host = nullptr;   // pinned; refreshed asynchronously after every recording forward
-    long long* ray_head = nullptr;
+    long long* ray_head = nullptr;                  // first chunk of every patch, then a byte per ray: not recorded
     long long ray_head_cap = 0;
     bool tape_valid = false;
     unsigned long long rgba_serial = 0, tape_rgba_serial = 0;   // which evaluation of the per-view colours is in rgba / was recorded with
@@ -183,7 +185,7 @@ void release_workspace(rgx_ctx* ctx) {
                      (void**)&ctx->bx, (void**)&ctx->by, (void**)&ctx->bz, (void**)&ctx->g0, (void**)&ctx->g1,
                      (void**)&ctx->g2, (void**)&ctx->quat, (void**)&ctx->sdens, (void**)&ctx->rgba,
                      (void**)&ctx->grad_rows, (void**)&ctx->hk, (void**)&ctx->refit_counters, (void**)&ctx->cub_temp,
-                     (void**)&ctx->bounds, (void**)&ctx->box, (void**)&ctx->counters, (void**)&ctx->bin_keys_in,
+                     (void**)&ctx->bounds, (void**)&ctx->box, (void**)&ctx->counters, (void**)&ctx->next_unit, (void**)&ctx->bin_keys_in,
                      (void**)&ctx->bin_keys_out, (void**)&ctx->bin_vals_in, (void**)&ctx->bin_vals_out,
                      (void**)&ctx->tile_first, (void**)&ctx->tile_last, (void**)&ctx->tile_cnt, (void**)&ctx->tile_pcnt,
                      (void**)&ctx->tile_pbegin, (void**)&ctx->ent_id, (void**)&ctx->ent_range, (void**)&ctx->ent_blk,
@@ -252,6 +254,7 @@ int ensure_workspace(rgx_ctx* ctx, int n_pad, int boxes) {
         if ((e = regrow(ctx, ctx->bounds, 12)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
         if ((e = regrow(ctx, ctx->box, 1)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
         if ((e = regrow(ctx, ctx->counters, 1)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
+        if ((e = regrow(ctx, ctx->next_unit, 2)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
         cudaMemset(ctx->counters, 0, sizeof(DeviceCounters));
         cudaMemset(ctx->box, 0, sizeof(SceneBox));
     }
@@ -424,6 +427,8 @@ int rgx_create(int device, rgx_ctx** out) {
     rgx_ctx* ctx = new (std::nothrow) rgx_ctx();
     if (!ctx) return RGX_E_INVALID;
     ctx->device = device;
+    if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || ctx->sm_count <= 0)
+        ctx->sm_count = 148;
     *out = ctx;
     return RGX_OK;
 }
@@ -546,17 +551,16 @@ struct Cull {
 
 static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, BinLaunch& b, int& ntiles, const Cull* cull = nullptr) {
     cudaError_t e = cudaSuccess;
-    const int tiles_x = (cam->width + kBinTile - 1) / kBinTile;
+    const int tile = bin_tile_size(*cam);
+    const int tiles_x = (cam->width + tile - 1) / tile;
     if (tiles_x > 65535) return fail(ctx, RGX_E_TOO_LARGE, "image wider than 65535 tiles");
-    const int ty_first = m->row_begin / kBinTile, ty_last = (m->row_end - 1) / kBinTile;
+    const int ty_first = m->row_begin / tile, ty_last = (m->row_end - 1) / tile;
     const int tiles_y = ty_last - ty_first + 1;
     ntiles = tiles_x * tiles_y;
     if (!ctx->bin_total_dev) {
         RGB_(bin_total_dev, 4);
         if (!ctx->bin_total_host && (e = cudaMallocHost((void**)&ctx->bin_total_host, 4 * sizeof(unsigned long long))) != cudaSuccess)
             return cuda_fail(ctx, e, "pinned scalar");
-        if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || ctx->sm_count <= 0)
-            ctx->sm_count = 148;
     }
     if (ctx->n_pad > ctx->big_cap) {
         RGB_(big_slot, (size_t)ctx->n_pad); RGB_(big_rect, (size_t)ctx->n_pad);
@@ -579,7 +583,7 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     b.tile_dir = ctx->tile_dir;
     b.cam = *cam;
     if (!camera_dual(*cam, b.dual)) return fail(ctx, RGX_E_INVALID, "camera axes are not linearly independent");
-    b.row_begin = m->row_begin; b.row_end = m->row_end; b.tile = kBinTile;
+    b.row_begin = m->row_begin; b.row_end = m->row_end; b.tile = tile;
     b.tiles_x = tiles_x; b.tiles_y = tiles_y; b.ty_first = ty_first;
     b.total_dev = ctx->bin_total_dev;
     b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID;
@@ -678,6 +682,7 @@ static int fill_lists(rgx_ctx* ctx, BinLaunch& b, uint64_t* keys, uint32_t* vals
     ctx->lists.ent_id = ctx->ent_id; ctx->lists.ent_range = ctx->ent_range; ctx->lists.blk = ctx->ent_blk;
     ctx->lists.tile_pbegin = ctx->tile_pbegin; ctx->lists.tile_cnt = ctx->tile_cnt; ctx->lists.tile_order = ctx->tile_order;
     ctx->lists.tiles_x = b.tiles_x; ctx->lists.tiles_y = b.tiles_y; ctx->lists.ty_first = b.ty_first;
+    ctx->lists.tile = b.tile;
     return RGX_OK;
 }
 
@@ -767,8 +772,8 @@ static void lists_ahead_begin(rgx_ctx* ctx, cudaStream_t s, ListsAhead& a) {
     const rgx_march* m = &ctx->hint_march;
     if ((m->flags & (RGX_FLAG_BRUTE_FORCE | RGX_FLAG_PER_RAY_SEARCH)) || ctx->n == 0 || m->row_end <= m->row_begin) return;
     if (lists_cached(ctx, cam, m)) return;
-    const int tiles_x = (cam->width + kBinTile - 1) / kBinTile;
-    const int ntiles = tiles_x * ((m->row_end - 1) / kBinTile - m->row_begin / kBinTile + 1);
+    const int tile = bin_tile_size(*cam), tiles_x = (cam->width + tile - 1) / tile;
+    const int ntiles = tiles_x * ((m->row_end - 1) / tile - m->row_begin / tile + 1);
     if (!ctx->bin_total_dev || ctx->bin_pair_cap == 0 || ctx->n_pad > ctx->big_cap || ntiles + 1 > ctx->bin_tiles_cap) return;
     if (!ctx->side) {
         int lo = 0, hi = 0;
@@ -892,6 +897,8 @@ static int prepare_march(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera*
     L.cam = *cam;
     L.m = *march;
     L.box = ctx->box;
+    L.next_unit = ctx->next_unit;
+    L.sm_count = ctx->sm_count;
     L.counters = (march->flags & RGX_FLAG_COUNT_WORK) ? ctx->counters : nullptr;
     return RGX_OK;
 }
@@ -944,18 +951,19 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
                     return cuda_fail(ctx, e, "tape");
                 for (int i = 0; i < 4; ++i) ctx->tape_used_host[i] = 0;
             }
-            if (rays > ctx->ray_head_cap) {
-                if ((e = regrow(ctx, ctx->ray_head, (size_t)rays)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
-                ctx->ray_head_cap = rays;
-            }
             const int ntiles = L.lists.tiles_x * L.lists.tiles_y;
+            const long long heads = (long long)ntiles * kMaxPatchesPerTile, head_words = heads + (rays + 7) / 8;
+            if (head_words > ctx->ray_head_cap) {
+                if ((e = regrow(ctx, ctx->ray_head, (size_t)head_words)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
+                ctx->ray_head_cap = head_words;
+            }
             if (ntiles > ctx->tape_order_cap) {
                 if ((e = regrow(ctx, ctx->tape_tile_order, (size_t)ntiles + 64)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
                 ctx->tape_order_cap = ntiles + 64;
             }
             // room: 1024 ints per ray to begin with; what the previous recording asked for and half as much again when
             // that came close to the end (the counter keeps counting past the end), within half of the free memory
-            long long want = rows_rays * 1024 + 4096;
+            long long want = rows_rays * 1024 + std::min(heads, (long long)ctx->sm_count * 16) * kTapeBlockInts;
             const long long seen = (long long)*ctx->tape_used_host;
             if (seen > (ctx->tape_cap / 8) * 7) want = want > seen + seen / 2 ? want : seen + seen / 2;
             if (want > ctx->tape_cap) {
@@ -981,7 +989,8 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
                 (e = cudaMemcpyAsync(ctx->tape_tile_order, L.lists.tile_order, sizeof(int) * (size_t)ntiles, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
                 return cuda_fail(ctx, e, "tape");
             if (ctx->tape) {
-                L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap; L.ray_head = ctx->ray_head;
+                L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
+                L.patch_head = ctx->ray_head; L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + heads);
                 L.tile_unrecorded = ctx->tile_unrecorded;
                 if (ctx->tape_limit >= 0 && ctx->tape_limit < L.tape_cap) L.tape_cap = ctx->tape_limit;
             }
@@ -1029,7 +1038,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         return cuda_fail(ctx, e, "horizon counter");
     if ((rc = march_once())) return rc;
     if ((rc = run_colors_if_beyond(ctx, scene, cam->eye, L.hz_count, s))) return rc;
-    if ((e = launch_march_forward_listed_rays(L, (ctx->sm_count > 0 ? ctx->sm_count : 148) * 4, s)) != cudaSuccess ||
+    if ((e = launch_march_forward_listed_rays(L, ctx->sm_count * 4, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(ctx->beyond_host, ctx->hz_scalars + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaEventRecord(ctx->ev_beyond, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "rays beyond the horizon");
@@ -1097,13 +1106,11 @@ int rgx_backward(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* cam, co
         L.lists = ctx->lists;
     }
     if (L.lists.ent_id && tape_matches) {
-        L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap; L.ray_head = ctx->ray_head;
+        L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
+        L.patch_head = ctx->ray_head;
+        L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + (long long)L.lists.tiles_x * L.lists.tiles_y * kMaxPatchesPerTile);
         L.tile_unrecorded = ctx->tile_unrecorded;
         L.replay_order = ctx->tape_tile_order;
-        // Slabs with few hits are worked off several at a time.  The statistics are those of the latest recording
-        // whose read-back has arrived (this view's, or an earlier one's: a hint, either kernel gives the same result).
-        const unsigned long long slabs = ctx->tape_used_host[1], nhits = ctx->tape_used_host[2];
-        L.replay_batched = slabs == 0 || nhits < 24ull * slabs;
     }
     L.rgb_in = rgb; L.dl_drgb = dL_drgb; L.grad_rows = ctx->grad_rows; L.grad_copies = ctx->grad_copies;
     // rays without a recording first: theirs is the last launch that reads the view's lists, so the lists of an

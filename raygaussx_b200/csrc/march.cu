@@ -50,7 +50,7 @@ __device__ __forceinline__ void march_ray_by_search(const MarchLaunch& L, int px
             const float tau = __fmul_rn((float)lane + 0.5f, p.dt);            // sample offset from tbuffer
             float s, cr, cg, cb;
             bool overflow;
-            int nhit = slab_sums<COUNT, false>(L, L.m, tbuffer, tau, ray_id, slab_index, make_float3(0.f, 0.f, 0.f),
+            int nhit = slab_sums<COUNT, false>(L, L.m, tbuffer, p.dt, ray_id, slab_index, make_float3(0.f, 0.f, 0.f),
                                                ws, lane, tl, [&](auto&& leaf) {
                 search_all<COUNT, BRUTE>(L, r, p.tmin, p.tmax, ws, lane, tl, leaf);
             }, s, cr, cg, cb, overflow);
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kWarps * 32) march_backward_kernel(const __gri
             // pass 1: per-sample sigma and delta.colour sums, same arithmetic as the forward
             float s, dc, u0, u1;
             bool overflow;
-            int nhit = slab_sums<false, true>(L, L.m, tbuffer, tau, ray_id, slab_index, dl, ws, lane, tl, enumerate, s,
+            int nhit = slab_sums<false, true>(L, L.m, tbuffer, p.dt, ray_id, slab_index, dl, ws, lane, tl, enumerate, s,
                                               dc, u0, u1, overflow);
             if (nhit == 0) {
                 tbuffer = __fadd_rn(tbuffer, p.slab);

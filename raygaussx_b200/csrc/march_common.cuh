@@ -22,9 +22,6 @@ constexpr int kTile = 8;   // per-ray variant (march.cu): a CTA marches 8x8 pixe
 #endif
 constexpr int kEvalUnroll = RGX_EVAL_UNROLL;
 constexpr int kMaxSlabs = 1 << 22;   // hard bound on slab iterations per ray
-#ifndef RGX_PACKED_FMA
-#define RGX_PACKED_FMA 1
-#endif
 
 struct WarpStage {      // staged hit records of one warp
     float4 recA[kStage];
@@ -67,17 +64,20 @@ __device__ __forceinline__ float exp_neg(float x) {   // exp(-x), x >= 0
     return ex2_approx(__fmul_rn(x, -1.4426950408889634f));
 }
 
-// cuda_train/forward/gaussians_aabb.cu:95-110
-__device__ __forceinline__ void make_ray(const rgx_camera& c, int px, int py, Ray& r) {
-    float ix = __fdiv_rn((float)px + 0.5f, (float)c.width);
-    float iy = __fdiv_rn((float)py + 0.5f, (float)c.height);
+// Direction of the ray through image position (fx, fy), in pixels: cuda_train/forward/gaussians_aabb.cu:95-110
+__device__ __forceinline__ void make_ray_dir(const rgx_camera& c, float fx, float fy, float3& out) {
+    float ix = __fdiv_rn(fx, (float)c.width);
+    float iy = __fdiv_rn(fy, (float)c.height);
     float a = __fmul_rn(__fmul_rn(2.0f, ix - c.pp[0]), c.tan_half_fov[0]);
     float b = __fmul_rn(__fmul_rn(2.0f, iy - c.pp[1]), c.tan_half_fov[1]);
     float3 d = make_float3(__fadd_rn(__fadd_rn(__fmul_rn(a, c.u[0]), __fmul_rn(b, c.v[0])), c.w[0]),
                            __fadd_rn(__fadd_rn(__fmul_rn(a, c.u[1]), __fmul_rn(b, c.v[1])), c.w[1]),
                            __fadd_rn(__fadd_rn(__fmul_rn(a, c.u[2]), __fmul_rn(b, c.v[2])), c.w[2]));
     float inv_len = __fdiv_rn(1.0f, __fsqrt_rn(dot3(d, d)));
-    r.d = make_float3(__fmul_rn(d.x, inv_len), __fmul_rn(d.y, inv_len), __fmul_rn(d.z, inv_len));
+    out = make_float3(__fmul_rn(d.x, inv_len), __fmul_rn(d.y, inv_len), __fmul_rn(d.z, inv_len));
+}
+__device__ __forceinline__ void make_ray(const rgx_camera& c, int px, int py, Ray& r) {
+    make_ray_dir(c, (float)px + 0.5f, (float)py + 0.5f, r.d);
     r.o = make_float3(c.eye[0], c.eye[1], c.eye[2]);
     r.inv = make_float3(__frcp_rn(r.d.x), __frcp_rn(r.d.y), __frcp_rn(r.d.z));
 }
@@ -110,32 +110,47 @@ __device__ __forceinline__ void whiten_ray(const Ray& r, float4 g0, float4 g1, f
     de.z = fmaf(g2.y, r.d.x, fmaf(g2.z, r.d.y, __fmul_rn(g2.w, r.d.z)));
 }
 
-// Interval of the ray inside the truncation ellipsoid
-// (square root and the division for the first root are the approximate instructions, good to 2 ulp: the roots
-// only decide whether and where the interval meets a slab; forward 10.2 -> 10.0 ms)
-// (cuda_train/forward/gaussians_aabb.cu:43-91 with M = S^-1 R^T / k folded into g0..g2).
-__device__ __forceinline__ bool ellipsoid_interval(const Ray& r, float4 g0, float4 g1, float4 g2, float3& Oe,
-                                                   float3& de, float& r1, float& r2) {
-    whiten_ray(r, g0, g1, g2, Oe, de);
-    float a = dot3(de, de);
-    float b = -dot3(Oe, de);
-    float c = fmaf(Oe.x, Oe.x, fmaf(Oe.y, Oe.y, fmaf(Oe.z, Oe.z, -1.0f)));
-    float inv_a = __fdividef(1.0f, a);
-    float bia = __fmul_rn(b, inv_a);
-    float3 P = make_float3(fmaf(bia, de.x, Oe.x), fmaf(bia, de.y, Oe.y), fmaf(bia, de.z, Oe.z));
-    float disc = 1.0f - dot3(P, P);
-    if (!(disc > 1e-7f)) return false;
-    float sd = sqrt_approx(__fmul_rn(disc, a));
-    float q = b + copysignf(sd, b);
-    r1 = __fdividef(c, q);
-    r2 = __fmul_rn(q, inv_a);
-    return true;
+// What a ray is to a Gaussian, in the Gaussian's whitened frame: along the ray the squared distance from the centre is
+// a (t - t0)^2 + q.  t0, the closest approach, is b / a after one correction step (the residual of the approximate
+// quotient is exact in an FMA), good to an ulp: the response is evaluated as a parabola about it.
+struct RayParabola {
+    float a, inv_a, t0, q, disc, w2, hw;      // disc = 1 - q; w2 = disc / a, hw its root: the ray is inside for |t - t0| < hw
+};
+
+// The stretch of the ray Oe + t de inside the truncation ellipsoid (the unit sphere of the whitened frame), t0 - hw .. t0 + hw
+// (cuda_train/forward/gaussians_aabb.cu:43-91 with M = S^-1 R^T / k folded into g0..g2).  No early return: hw of a miss is NaN.
+// A ray whose closest approach lies behind the eye misses, even from inside: the reference's two roots are then out of order.
+__device__ __forceinline__ bool ellipsoid_stretch(float3 Oe, float3 de, RayParabola& p) {
+    p.a = dot3(de, de);
+    const float b = -dot3(Oe, de);
+    p.inv_a = __fdividef(1.0f, p.a);
+    const float t = __fmul_rn(b, p.inv_a);
+    p.t0 = fmaf(fmaf(-t, p.a, b), p.inv_a, t);
+    float3 P = make_float3(fmaf(p.t0, de.x, Oe.x), fmaf(p.t0, de.y, Oe.y), fmaf(p.t0, de.z, Oe.z));
+    p.q = dot3(P, P);
+    p.disc = 1.0f - p.q;
+    p.w2 = __fmul_rn(p.disc, p.inv_a);
+    p.hw = sqrt_approx(p.w2);
+    return p.disc > 1e-7f && p.t0 >= 0.f;
+}
+// Where the ray enters: the smaller root, from the form that does not cancel (c / q).  c = |Oe|^2 - 1.
+__device__ __forceinline__ float whitened_c(float3 Oe) {
+    return fmaf(Oe.x, Oe.x, fmaf(Oe.y, Oe.y, fmaf(Oe.z, Oe.z, -1.0f)));
+}
+__device__ __forceinline__ float entry_root(float3 Oe, float3 de, float c, const RayParabola& p) {
+    const float b = -dot3(Oe, de);
+    return __fdividef(c, b + copysignf(sqrt_approx(__fmul_rn(p.disc, p.a)), b));
+}
+// Whether the stretch meets [tmin, tmax].
+__device__ __forceinline__ bool stretch_meets(const RayParabola& p, float tmin, float tmax) {
+    return __fadd_rn(p.t0, -p.hw) <= tmax && __fadd_rn(p.t0, p.hw) >= tmin;
 }
 
 struct LeafTest {
     bool hit;
     float t_hit;     // max(tmin, root1) when hit
     float3 Oe, de;
+    RayParabola p;
 };
 
 // The per-ray test that decides a hit: the reference's interval test on the truncation ellipsoid, nothing else
@@ -156,11 +171,10 @@ __device__ __forceinline__ LeafTest test_gaussian(const MarchLaunch& L, const Ra
     }
     if (bh) {
         float4 g0 = __ldg(&L.g.g0[j]), g1 = __ldg(&L.g.g1[j]), g2 = __ldg(&L.g.g2[j]);
-        float r1, r2;
-        if (ellipsoid_interval(r, g0, g1, g2, out.Oe, out.de, r1, r2)) {
-            float lo = fmaxf(tmin, r1), hi = fminf(tmax, r2);
-            out.hit = lo <= hi;
-            out.t_hit = lo;
+        whiten_ray(r, g0, g1, g2, out.Oe, out.de);
+        if (ellipsoid_stretch(out.Oe, out.de, out.p) && tmin <= tmax && stretch_meets(out.p, tmin, tmax)) {
+            out.hit = true;
+            out.t_hit = fmaxf(tmin, entry_root(out.Oe, out.de, whitened_c(out.Oe), out.p));
         }
     }
     if (count) {
@@ -340,19 +354,21 @@ __device__ __forceinline__ void clip_scene(const SceneBox& b, const Ray& r, floa
 // (payload)*g, payload being rgb*sigma in the forward (cuda_train/forward/gaussians_aabb.cu:166-178).
 // Along a ray the whitened squared distance is a parabola in the sample position, q(tau) = q_min +
 // |de|^2 (tau - tau*)^2 about the closest approach tau* (a sum of two non-negative terms: no cancellation), so a
-// staged record is (tau*, (1 - q_min)/|de|^2, -hk |de|^2, -hk q_min) and (payload, sigma): the truncation
+// staged record is (tau*, (1 - q_min)/|de|^2, -hk |de|^2, hk (1 - q_min) - hk) and (payload, sigma): the truncation
 // test q < 1 is d^2 < (1 - q_min)/|de|^2 and the exponent one fused multiply-add of d^2.
 // The four sums advance with two packed fp32x2 fused multiply-adds per hit (sm_100's FFMA2: two IEEE fp32 FMAs in
 // one instruction, same bits as two scalar ones): the loop is bound by instruction issue, not by the FMA pipe.
+// Sample s = 2k + h lies at (s + 1/2) dt; its distance from tau* is formed as 2k dt + ((h + 1/2) dt - tau*) with two FMAs,
+// here and in the march over tile lists.
 template <bool COUNT>
-__device__ __forceinline__ void eval_forward(const WarpStage& ws, int count, float tau, float& s, float& cr,
+__device__ __forceinline__ void eval_forward(const WarpStage& ws, int count, float dt, int lane, float& s, float& cr,
                                              float& cg, float& cb, Tally& tl) {
-#if RGX_PACKED_FMA
+    const float k2 = (float)(lane & ~1), h2 = (float)(lane & 1) + 0.5f;
     float2 rg = make_float2(cr, cg), bs = make_float2(cb, s);
 #pragma unroll kEvalUnroll
     for (int j = 0; j < count; ++j) {
         const float4 A = ws.recA[j], C = ws.recB[j];
-        const float d = __fadd_rn(tau, -A.x);
+        const float d = fmaf(k2, dt, fmaf(h2, dt, -A.x));
         const float d2 = __fmul_rn(d, d);
         const bool in = d2 < A.y;
         const float e = in ? ex2_approx(fmaf(A.z, d2, A.w)) : 0.0f;
@@ -362,31 +378,12 @@ __device__ __forceinline__ void eval_forward(const WarpStage& ws, int count, flo
         if (COUNT) tl.v[C_PAIRS] += __popc(__ballot_sync(kFull, in));
     }
     cr = rg.x; cg = rg.y; cb = bs.x; s = bs.y;
-#else
-#pragma unroll kEvalUnroll
-    for (int j = 0; j < count; ++j) {
-        const float4 A = ws.recA[j], C = ws.recB[j];
-        const float d = __fadd_rn(tau, -A.x);
-        const float d2 = __fmul_rn(d, d);
-        const bool in = d2 < A.y;
-        const float e = in ? ex2_approx(fmaf(A.z, d2, A.w)) : 0.0f;
-        s = fmaf(C.w, e, s);
-        cr = fmaf(C.x, e, cr);
-        cg = fmaf(C.y, e, cg);
-        cb = fmaf(C.z, e, cb);
-        if (COUNT) tl.v[C_PAIRS] += __popc(__ballot_sync(kFull, in));
-    }
-#endif
 }
 
-// The record of eval_forward for a hit with whitened ray origin Oe and direction de, sample positions counted
-// from tbuffer; hk is the exponent scale of ex2 (response = ex2(-hk q)).
-__device__ __forceinline__ float4 parabola_record(float3 Oe, float3 de, float tbuffer, float hk) {
-    const float a = dot3(de, de);
-    const float tstar = __fdiv_rn(-dot3(Oe, de), a);
-    const float3 P = make_float3(fmaf(tstar, de.x, Oe.x), fmaf(tstar, de.y, Oe.y), fmaf(tstar, de.z, Oe.z));
-    const float qmin = dot3(P, P);
-    return make_float4(__fadd_rn(tstar, -tbuffer), __fdividef(1.0f - qmin, a), __fmul_rn(-hk, a), __fmul_rn(-hk, qmin));
+// The record of eval_forward for a hit, sample positions counted from tbuffer; hk is the exponent scale of ex2
+// (response = ex2(-hk q)).
+__device__ __forceinline__ float4 parabola_record(const RayParabola& p, float tbuffer, float hk) {
+    return make_float4(__fadd_rn(p.t0, -tbuffer), p.w2, __fmul_rn(-hk, p.a), fmaf(hk, p.disc, -hk));
 }
 
 __device__ __forceinline__ void flush_tally(const MarchLaunch& L, const Tally& tl, int lane) {
@@ -471,7 +468,7 @@ __device__ __forceinline__ void eval_backward(const WarpStage& ws, int count, fl
 // Per-sample sums of sigma*g (s) and payload*g (c0..c2); payload is rgb*sigma in
 // the forward and (dl . rgb*sigma, 0, 0) in the backward.  Returns the hit count.
 template <bool COUNT, bool BWD, class Enum>
-__device__ __forceinline__ int slab_sums(const MarchLaunch& L, const rgx_march& m, float tbuffer, float tau,
+__device__ __forceinline__ int slab_sums(const MarchLaunch& L, const rgx_march& m, float tbuffer, float dt,
                                          int ray_id, int slab_index, float3 dl, WarpStage& ws, int lane, Tally& tl,
                                          Enum&& enumerate, float& s, float& c0, float& c1, float& c2,
                                          bool& overflow, int* const* hit_list = nullptr, int hit_cap = 0) {
@@ -496,7 +493,7 @@ __device__ __forceinline__ int slab_sums(const MarchLaunch& L, const rgx_march& 
                 if (list && nhit + rank < hit_cap) list[nhit + rank] = j;
             }
             const float4 c = __ldg(&L.g.rgba[j]);       // (rgb sigma, sigma)
-            ws.recA[slot] = parabola_record(t.Oe, t.de, tbuffer, __ldg(&L.g.hk[j]));
+            ws.recA[slot] = parabola_record(t.p, tbuffer, __ldg(&L.g.hk[j]));
             ws.recB[slot] = BWD ? make_float4(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), 0.f, 0.f, c.w) : c;
         }
         if (COUNT) {
@@ -513,7 +510,7 @@ __device__ __forceinline__ int slab_sums(const MarchLaunch& L, const rgx_march& 
         if (COUNT) tl.v[C_CYC_WINDOW] += clock64() - c_s;       // staging of the hits
         if (nstage > kStage - kFan) {
             long long c_a = COUNT ? clock64() : 0;
-            eval_forward<COUNT>(ws, nstage, tau, s, c0, c1, c2, tl);
+            eval_forward<COUNT>(ws, nstage, dt, lane, s, c0, c1, c2, tl);
             nstage = 0;
             __syncwarp();
             if (COUNT) tl.v[C_CYC_EVAL] += clock64() - c_a;
@@ -522,7 +519,7 @@ __device__ __forceinline__ int slab_sums(const MarchLaunch& L, const rgx_march& 
     });
     if (nstage > 0) {
         long long c_a = COUNT ? clock64() : 0;
-        eval_forward<COUNT>(ws, nstage, tau, s, c0, c1, c2, tl);
+        eval_forward<COUNT>(ws, nstage, dt, lane, s, c0, c1, c2, tl);
         __syncwarp();
         if (COUNT) tl.v[C_CYC_EVAL] += clock64() - c_a;
     }
@@ -544,7 +541,7 @@ __device__ __forceinline__ SlabTrans slab_transmittance(float s, float dt, float
     float excl = __fadd_rn(o.incl, -o.x);
     o.w = exp_neg(o.x);
     o.Ts = __fmul_rn(T, exp_neg(excl));
-    o.T16 = __shfl_sync(kFull, o.Ts, kChunk);
+    o.T16 = __fmul_rn(T, exp_neg(__shfl_sync(kFull, o.incl, kChunk - 1)));
     o.live = lane < kChunk || o.T16 > eps;
     o.T32 = __fmul_rn(T, exp_neg(__shfl_sync(kFull, o.incl, 31)));
     return o;
@@ -569,27 +566,6 @@ __device__ __forceinline__ void composite_forward(const SlabPlan& p, float tbuff
         st.depth = __fadd_rn(st.depth, warp_sum(tr.live ? __fmul_rn(__fmul_rn(tr.Ts, one_m_w), ts) : 0.f));
     }
     st.T = slab_exit_T(tr, eps);
-}
-
-// The same with the ray's colour and depth kept in shared memory (x, y, z = colour, w = depth; lane 0 owns
-// them): they are touched once per slab, and the registers are wanted elsewhere all the time.
-__device__ __forceinline__ void composite_forward_shared(const SlabPlan& p, float tbuffer, float tau, float eps, int lane,
-                                                         float s, float cr, float cg, float cb, bool want_depth,
-                                                         float& T, float4* acc) {
-    SlabTrans tr = slab_transmittance(s, p.dt, T, eps, lane);
-    float one_m_w = 1.0f - tr.w;
-    float f = tr.live ? __fmul_rn(tr.Ts, __fmul_rn(p.dt, __fdividef(one_m_w, fmaxf(tr.x, 1e-6f)))) : 0.f;
-    const float sr = warp_sum(__fmul_rn(f, cr)), sg = warp_sum(__fmul_rn(f, cg)), sb = warp_sum(__fmul_rn(f, cb));
-    float sd = 0.f;
-    if (want_depth) {
-        float ts = __fadd_rn(tbuffer, tau);
-        sd = warp_sum(tr.live ? __fmul_rn(__fmul_rn(tr.Ts, one_m_w), ts) : 0.f);
-    }
-    if (lane == 0) {
-        float4 a = *acc;
-        *acc = make_float4(__fadd_rn(a.x, sr), __fadd_rn(a.y, sg), __fadd_rn(a.z, sb), __fadd_rn(a.w, sd));
-    }
-    T = slab_exit_T(tr, eps);
 }
 
 // 8-bit colour of the reference's viewer (cuda_gui/helpers.h:45-58): clamp to [0,1], times 256,

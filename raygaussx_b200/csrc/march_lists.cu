@@ -1,20 +1,19 @@
 // Forward and backward ray march over per-view tile lists: the default path.
 //
-// binning.cu leaves, for every 16x16-pixel tile of the view, a front-to-back list
+// binning.cu leaves, for every tile of the view (16x16 pixels; 8x8 or 4x4 of small images), a front-to-back list
 // of the Gaussians that any ray of the tile can meet, each with the range of
 // distances from the eye that its box spans, plus a (nearest near, farthest far)
-// summary per 32 entries.  A CTA owns a tile; its eight warps take the tile's
-// rays one at a time (one warp marches one ray, lanes = samples of a slab, as in
-// march.cu).  A query over [tmin,tmax] looks at 32 block summaries per step, opens
-// only the blocks whose range overlaps the query, filters their entries by range,
-// compacts the survivors into full groups of 32 and runs the exact per-ray test
-// on those.  A per-ray cursor skips the blocks the ray has left behind for good.
-// There is no hierarchy search, no CTA-wide barrier and no waiting between rays.
+// summary per 32 entries.
 //
-// The list is a superset of every hit set and the deciding test is the per-ray one
-// of march_common.cuh, so hit sets equal those of the per-ray and exhaustive
-// variants; hits are met in list order (near distance, then sorted slot), the same
-// in the forward and in both passes of the backward.
+// A warp marches a patch of neighbouring pixels (4x4; less of a small image): its rays go through the list
+// together.  Neighbouring rays begin and end their slabs within a fraction of a slab of each
+// other and meet the same Gaussians (measured: 15 of 16 rays of a patch share a hit on
+// the 3 M-Gaussian scene, 10 of 16 on the 300 k object), so a list entry is fetched,
+// whitened and culled once per patch instead of once per ray, and everything a ray does by
+// itself -- planning a slab, compositing, bookkeeping -- costs a lane or two of a warp
+// instruction, not a whole one.  The deciding test of a hit is the per-ray one of
+// march_common.cuh, so hit sets equal those of the per-ray and exhaustive variants; hits are
+// met in list order (near distance, then sorted slot), the same in the forward and the backward.
 //
 // Reference semantics: cuda_train/forward/gaussians_aabb.cu:205-340 and
 // cuda_train/backward/gaussians_aabb.cu:209-497 (see march_common.cuh).
@@ -24,66 +23,57 @@ namespace rgx {
 
 namespace {
 
-constexpr int kRaysPerTile = kBinTile * kBinTile;
 constexpr int kThreads = kWarps * 32;
-// CTAs per tile in the forward march and in the replay: each takes an equal share of the tile's rays.  The work
-// of a tile is only loosely predicted by the length of its list, so the kernels used to end with a few long
-// tiles on otherwise idle SMs (6 % of their time on the 3 M-Gaussian view); smaller units shorten that tail.
-#ifndef RGX_TILE_SPLIT
-#define RGX_TILE_SPLIT 8          // 3 M-Gaussian step: 1: 440.3 ms, 2: 432.2, 4: 428.5, 8: 427.6 (later: 4: 358.5, 8: 357.5)
-#endif
-#ifndef RGX_REPLAY_SPLIT
-#define RGX_REPLAY_SPLIT 4        // 2: 361.2 ms, 4: 358.5, 8: 358.5
-#endif
-constexpr int kTileSplit = RGX_TILE_SPLIT;
-constexpr int kRaysPerCta = kRaysPerTile / kTileSplit;
-constexpr int kReplaySplit = RGX_REPLAY_SPLIT;
-constexpr int kRaysPerReplayCta = kRaysPerTile / kReplaySplit;
 
-constexpr int kHitList = 256;      // hits of a slab remembered between the two passes of the backward
+// Shape of a patch.  P lanes carry a ray; the 32 / P rays of a warp lie in a block of W x H pixels.
+template <int P>
+struct Patch {
+    static constexpr int kLanes = P, kRays = 32 / P;
+    static constexpr int kW = P == 8 ? 2 : 4, kH = kRays / kW;
+    static constexpr unsigned kRayBits = (1u << kRays) - 1u;          // the lanes of one list entry in a ballot
+    static constexpr unsigned kSameRay = P == 2 ? 0x10001u : P == 4 ? 0x01010101u : 0x11111111u;   // the lanes of ray 0
+    static constexpr int kSamples = kSlab / P;                        // samples of a lane
+    static constexpr int kParts = P == 8 ? 2 : 4;                     // a slab is evaluated in this many parts
+    static constexpr int kPairs = kSamples / 2, kPairsPerPart = kPairs / kParts;
+    // recording, in ints: header, tbuffer and sample spacing per ray, sums, list
+    static constexpr int kTapeDt = 8 + kRays, kTapeSums = 8 + 2 * kRays, kTapeList = kTapeSums + 4 * kSamples * 32;
+};
+constexpr int kPatchWarps = 4;                              // warps per CTA of the patch kernels; they share nothing
 
-// Recording of a forward slab for the backward ("tape"), in ints, 16-byte aligned:
-//   [0] tbuffer bits  [1] hit count  [2,3] offset of the ray's next chunk (-1: last)
-//   [4, 132) per sample (lane) the sums (sigma, r sigma, g sigma, b sigma) weighted by the Gaussians' responses
-//   [132, 132 + hits) sorted slots of the hits in the order they were met
-constexpr int kTapeHead = 4 + 4 * kSlab;
-constexpr int kTapeBlock = 4096;   // ints a warp reserves at a time; slabs are recorded if kTapeHead + hit cap fits
+constexpr int kHitList = 256;      // hits of a slab remembered between the two passes of the backward search
 
-struct ListShared {
+// Recording of the forward for the backward ("tape"), in ints, everything 16-byte aligned.  A patch has a chain of chunks,
+// one per slab step in which some of its rays had hits:
+//   [0] entries in this piece   [1] rays (bits) the step belongs to   [2,3] offset of the next piece of the list (-1: none)
+//   [4,5] offset of the patch's next chunk (-1: last)                 [6,7] -
+//   tbuffer, then sample spacing, of the patch's rays
+//   the per-sample sums (sigma, r sigma, g sigma, b sigma): float4 [samples of a lane][lane]
+//   list: (sorted slot, rays that hit it as bits) in the order met
+// A list that outgrows the block goes on in a piece elsewhere: [0] entries, [2,3] next piece, [4, ...) list.
+// 140 ints per ray and slab on the 3 M-Gaussian scene: sharing the list among the rays makes the hits nearly free.
+constexpr int kTapeBlock = kTapeBlockInts;
+constexpr int kTapePiece = 4;
+
+struct ListShared {                // backward search: per warp and ray
     int next_ray;
-    float4 color[kWarps];      // forward: the ray's colour and depth so far (lane 0 of the warp owns it)
     int pend[kWarps][2 * kFan];
     int prim_of[kWarps][kFan];
     WarpStage ws[kWarps];
 };
 
-// Where a warp stands on the tape.  Kept in shared memory, not in registers: it is touched once per slab,
-// the registers it would take are wanted all the time by the search and the evaluation.
-struct TapeState {
-    long long off;      // next free int of the warp's current block
-    long long head;     // first chunk of the current ray (-1: none yet)
-    long long prev;     // latest chunk of the current ray
-    int* hits;          // where the current slab's hits go (null: the slab is not recorded)
-    int left;           // ints left in the block
-    int ok;             // 0: the current ray cannot be recorded (no room)
-    unsigned int slabs, nhits;   // recorded by this warp so far (for the backward's choice of kernel)
-};
-
-struct TileView {      // one tile's list
-    const int* id;
-    const float2* range;
-    const float2* blk;
-    int nblk;
+struct TileView {      // one tile's list: entries begin, begin + 1, ... of the view's
+    int begin, nblk;
 };
 
 __device__ __forceinline__ TileView tile_view(const TileLists& l, int tile) {
-    TileView v;
-    const int begin = __ldg(&l.tile_pbegin[tile]);
-    v.id = l.ent_id + begin;
-    v.range = l.ent_range + begin;
-    v.blk = l.blk + begin / 32;
-    v.nblk = (__ldg(&l.tile_cnt[tile]) + 31) / 32;
-    return v;
+    return {__ldg(&l.tile_pbegin[tile]), (__ldg(&l.tile_cnt[tile]) + 31) / 32};
+}
+__device__ __forceinline__ int entry_id(const MarchLaunch& L, const TileView& tv, int k) { return __ldg(&L.lists.ent_id[tv.begin + k]); }
+__device__ __forceinline__ float2 entry_range(const MarchLaunch& L, const TileView& tv, int k) {
+    return __ldg(&L.lists.ent_range[tv.begin + k]);
+}
+__device__ __forceinline__ float2 block_range(const MarchLaunch& L, const TileView& tv, int b) {
+    return b < tv.nblk ? __ldg(&L.lists.blk[tv.begin / 32 + b]) : make_float2(INFINITY, -INFINITY);
 }
 
 // Runs the exact test on the first min(npend, 32) pending candidates and hands them to leaf.
@@ -113,7 +103,7 @@ __device__ __forceinline__ void search_tile(const MarchLaunch& L, const Ray& r, 
     for (int b0 = cursor; b0 < tv.nblk; b0 += kFan) {
         const int bi = b0 + lane;
         const bool valid = bi < tv.nblk;
-        const float2 s = valid ? __ldg(&tv.blk[bi]) : make_float2(INFINITY, -INFINITY);
+        const float2 s = block_range(L, tv, bi);
         const bool reaches = valid && s.y >= tmin;          // something in the block extends to tmin or beyond
         const bool beyond = valid && s.x > tmax;            // the block, and every later one, starts after tmax
         unsigned live = __ballot_sync(kFull, reaches && !beyond);
@@ -127,10 +117,10 @@ __device__ __forceinline__ void search_tile(const MarchLaunch& L, const Ray& r, 
             const int bb = b0 + __ffs(live) - 1;
             live &= live - 1;
             const int k = bb * kFan + lane;
-            const float2 rg = __ldg(&tv.range[k]);
+            const float2 rg = entry_range(L, tv, k);
             const bool pass = rg.x <= tmax && rg.y >= tmin;
             const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) pend[npend + __popc(m & ((1u << lane) - 1u))] = __ldg(&tv.id[k]);
+            if (pass) pend[npend + __popc(m & ((1u << lane) - 1u))] = entry_id(L, tv, k);
             npend += __popc(m);
             if (COUNT) tl.v[C_CANDS] += 32;
             __syncwarp();
@@ -168,7 +158,7 @@ __device__ __forceinline__ float closest_in_tile(const MarchLaunch& L, const Ray
     for (int b0 = cursor; b0 < tv.nblk && !done; b0 += kFan) {
         const int bi = b0 + lane;
         const bool valid = bi < tv.nblk;
-        const float2 s = valid ? __ldg(&tv.blk[bi]) : make_float2(INFINITY, -INFINITY);
+        const float2 s = block_range(L, tv, bi);
         const bool reaches = valid && s.y >= tmin;
         unsigned live = __ballot_sync(kFull, reaches && s.x <= tmax);
         const unsigned any_beyond = __ballot_sync(kFull, valid && s.x > tmax);
@@ -183,10 +173,10 @@ __device__ __forceinline__ float closest_in_tile(const MarchLaunch& L, const Ray
             // entries are sorted by near distance: nothing from here on can start before `best`
             if (__shfl_sync(kFull, s.x, src) > best) { done = true; break; }
             const int k = (b0 + src) * kFan + lane;
-            const float2 rg = __ldg(&tv.range[k]);
+            const float2 rg = entry_range(L, tv, k);
             const bool pass = rg.x <= fminf(tmax, best) && rg.y >= tmin;
             const unsigned m = __ballot_sync(kFull, pass);
-            if (pass) pend[npend + __popc(m & ((1u << lane) - 1u))] = __ldg(&tv.id[k]);
+            if (pass) pend[npend + __popc(m & ((1u << lane) - 1u))] = entry_id(L, tv, k);
             npend += __popc(m);
             if (COUNT) tl.v[C_CANDS] += 32;
             __syncwarp();
@@ -201,8 +191,8 @@ __device__ __forceinline__ float closest_in_tile(const MarchLaunch& L, const Ray
 
 // pixel of the tile's ray number `ray` (row-major inside the tile)
 __device__ __forceinline__ bool ray_pixel(const MarchLaunch& L, int tile_x, int tile_y, int ray, int& px, int& py) {
-    px = tile_x * kBinTile + ray % kBinTile;
-    py = (L.lists.ty_first + tile_y) * kBinTile + ray / kBinTile;
+    px = tile_x * L.lists.tile + ray % L.lists.tile;
+    py = (L.lists.ty_first + tile_y) * L.lists.tile + ray / L.lists.tile;
     return px < L.cam.width && py >= L.m.row_begin && py < L.m.row_end;
 }
 
@@ -214,7 +204,236 @@ __device__ __forceinline__ void hz_note(const MarchLaunch& L, int ray_id) {
     if (HZ == 2) L.hz_rays[at] = ray_id;
 }
 
+// ---------------------------------------------------------------- what the sixteen rays of a patch share
+constexpr int kGroup = 8;          // entries that are tested before their hits are evaluated
+constexpr int kStaged = 64;        // ring of list entries that passed the patch's filters
+
+struct PatchStage {                // per warp
+    float4 m0[kStaged];            // rows of M = S^-1 R^T / k, and the eye in the whitened frame:
+    float4 m1[kStaged];            // (m00, m01, m02, Oe.x), (m10, ...), (m20, ...)
+    float4 m2[kStaged];
+    float4 ex[kStaged];            // hk, |Oe|^2 - 1, sorted slot (bits), -
+    float4 rgba[kStaged];          // (r sigma, g sigma, b sigma, sigma)
+    unsigned mask[kStaged];        // rays that hit it
+};
+
+// smallest / largest of non-negative floats over the warp (they order like their bits)
+__device__ __forceinline__ float warp_min_pos(float v) { return __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(v))); }
+__device__ __forceinline__ float warp_max_pos(float v) { return __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(v))); }
+
+// One Gaussian's record, as the sorted arrays hold it, into slot `q` (by one lane).
+__device__ __forceinline__ void stage_record(PatchStage& st, int q, int j, float4 g0, float4 g1, float4 g2, float3 Oe, float hk, float4 rgba) {
+    st.m0[q] = make_float4(g0.w, g1.x, g1.y, Oe.x);
+    st.m1[q] = make_float4(g1.z, g1.w, g2.x, Oe.y);
+    st.m2[q] = make_float4(g2.y, g2.z, g2.w, Oe.z);
+    st.ex[q] = make_float4(hk, whitened_c(Oe), __int_as_float(j), 0.f);
+    st.rgba[q] = rgba;
+}
+__device__ __forceinline__ float3 whiten_eye(const MarchLaunch& L, float4 g0, float4 g1, float4 g2) {
+    const float3 O = make_float3(L.cam.eye[0] - g0.x, L.cam.eye[1] - g0.y, L.cam.eye[2] - g0.z);
+    float3 Oe;
+    Oe.x = fmaf(g0.w, O.x, fmaf(g1.x, O.y, __fmul_rn(g1.y, O.z)));
+    Oe.y = fmaf(g1.z, O.x, fmaf(g1.w, O.y, __fmul_rn(g2.x, O.z)));
+    Oe.z = fmaf(g2.y, O.x, fmaf(g2.z, O.y, __fmul_rn(g2.w, O.z)));
+    return Oe;
+}
+__device__ __forceinline__ float3 whiten_dir(float4 m0, float4 m1, float4 m2, float3 d) {
+    return make_float3(fmaf(m0.x, d.x, fmaf(m0.y, d.y, __fmul_rn(m0.z, d.z))),
+                       fmaf(m1.x, d.x, fmaf(m1.y, d.y, __fmul_rn(m1.z, d.z))),
+                       fmaf(m2.x, d.x, fmaf(m2.y, d.y, __fmul_rn(m2.z, d.z))));
+}
+
+// No ray of the patch can meet the Gaussian.  The rays' directions lie in the parallelogram mid +- e1 +- e2 (cone[0..2], the
+// directions scaled to the middle one's projection; what the normalisation of each ray takes off only shortens its reach), so at
+// parameter t <= far a ray is within far |M (e1 +- e2)| of the middle ray in the whitened frame, the longer of the two diagonals:
+// the middle ray would have to come that close to the unit sphere.  With a slack well above the rounding.
+__device__ __forceinline__ bool cone_misses(const float4* cone, float4 g0, float4 g1, float4 g2, float3 Oe, float far) {
+    const float4 m0 = make_float4(g0.w, g1.x, g1.y, 0.f), m1 = make_float4(g1.z, g1.w, g2.x, 0.f), m2 = make_float4(g2.y, g2.z, g2.w, 0.f);
+    const float4 c = cone[0], p = cone[1], q = cone[2];
+    const float3 de = whiten_dir(m0, m1, m2, make_float3(c.x, c.y, c.z));
+    const float3 dp = whiten_dir(m0, m1, m2, make_float3(p.x, p.y, p.z)), dq = whiten_dir(m0, m1, m2, make_float3(q.x, q.y, q.z));
+    const float t = __fdividef(-dot3(Oe, de), dot3(de, de));
+    const float3 P = make_float3(fmaf(t, de.x, Oe.x), fmaf(t, de.y, Oe.y), fmaf(t, de.z, Oe.z));
+    const float rho = fmaf(__fmul_rn(far, c.w), sqrt_approx(fmaxf(dot3(dp, dp), dot3(dq, dq))), 1.0f);
+    return dot3(P, P) > fmaf(__fmul_rn(rho, rho), 1.0005f, 1e-5f);       // false for NaN: kept
+}
+
+// The cone of a patch: the unit direction of its middle ray with the scale of the diagonals, and the two half diagonals.
+__device__ __forceinline__ void patch_cone(const rgx_camera& c, int x0, int y0, int w, int h, float4* cone) {
+    float3 mid;
+    make_ray_dir(c, (float)x0 + 0.5f * (float)w, (float)y0 + 0.5f * (float)h, mid);
+    // a pixel to the right adds su u to the unnormalised direction, a row down adds sv v; rays reach (w - 1) / 2 and (h - 1) / 2
+    // pixels from the middle.  |unnormalised direction| of the middle one and of any ray of the patch: at least the shortest of
+    // the patch's, which the corner below bounds from below.
+    const float su = 2.0f * c.tan_half_fov[0] / (float)c.width * 0.5f * (float)(w - 1), sv = 2.0f * c.tan_half_fov[1] / (float)c.height * 0.5f * (float)(h - 1);
+    const float3 e1 = make_float3(su * c.u[0], su * c.u[1], su * c.u[2]), e2 = make_float3(sv * c.v[0], sv * c.v[1], sv * c.v[2]);
+    const float a = 2.0f * (((float)x0 + 0.5f * (float)w) / (float)c.width - c.pp[0]) * c.tan_half_fov[0];
+    const float b = 2.0f * (((float)y0 + 0.5f * (float)h) / (float)c.height - c.pp[1]) * c.tan_half_fov[1];
+    const float3 d = make_float3(a * c.u[0] + b * c.v[0] + c.w[0], a * c.u[1] + b * c.v[1] + c.w[1], a * c.u[2] + b * c.v[2] + c.w[2]);
+    const float len = sqrtf(dot3(d, d)), reach = sqrtf(dot3(e1, e1)) + sqrtf(dot3(e2, e2));
+    // a ray d + e, |e| <= reach: its point at parameter t is t (d + e) / |d + e|; the middle ray passes t / |d + e| d, so the
+    // distance between the two is t |e| / |d + e| <= t |e| / (len - reach)
+    const float scale = reach < 0.5f * len ? 1.001f / (len - reach) : INFINITY;
+    cone[0] = make_float4(mid.x, mid.y, mid.z, scale);
+    cone[1] = make_float4(e1.x + e2.x, e1.y + e2.y, e1.z + e2.z, 0.f);
+    cone[2] = make_float4(e1.x - e2.x, e1.y - e2.y, e1.z - e2.z, 0.f);
+}
+
+// Walks the entries of the list that can matter to rays whose windows lie within [wlo, whi]: 32 block summaries per step,
+// the blocks that overlap, their entries filtered by range and by the patch's cone; what is left is staged, and handed to
+// process(first, count) in list order, three groups or more at a time and whatever remains at the end.  `cursor`: first block that
+// may still matter to a ray of the patch that has got as far as `wall`; it only moves forward.  whi may shrink while walking (closest hit).
+// One loop with one place that processes: the code that follows is long, and a second copy of it did not fit the instruction
+// cache beside the first (a third of all stalls on the 300 k object).  Fetching a block ahead with asynchronous copies was no
+// faster: the registers it takes cost what it hides.
+template <bool COUNT, class Process>
+__device__ __forceinline__ void walk_list(const MarchLaunch& L, const TileView& tv, const float4* cone_at, float wall, float wlo,
+                                          float& whi, int& cursor, PatchStage& st, int batch, int lane, Tally& tl,
+                                          Process&& process) {
+    int head = 0, n = 0, b0 = cursor - kFan;
+    bool advancing = true, more = true;
+    unsigned live = 0u;
+    float near_of = 0.f;                                              // smallest near distance of this lane's block
+    while (true) {
+        while (more && n < batch) {
+            if (live == 0u) {
+                b0 += kFan;
+                if (b0 >= tv.nblk) { more = false; break; }
+                const float2 s = block_range(L, tv, b0 + lane);        // (inf, -inf) past the last block
+                near_of = s.x;
+                live = __ballot_sync(kFull, s.y >= wlo && s.x <= whi);
+                if (advancing) {
+                    const unsigned alive = __ballot_sync(kFull, s.y >= wall);
+                    if (alive == 0u) cursor = min(b0 + kFan, tv.nblk);
+                    else { cursor = b0 + __ffs(alive) - 1; advancing = false; }
+                }
+                if (live == 0u) {
+                    if (__any_sync(kFull, s.x > whi)) more = false;
+                    continue;
+                }
+            }
+            const int src = __ffs(live) - 1;
+            live &= live - 1;
+            // sorted by near: once a block begins beyond whi, nothing further on can matter
+            if (__shfl_sync(kFull, near_of, src) > whi) { more = false; break; }
+            const int k = (b0 + src) * kFan + lane;
+            const float2 rg = entry_range(L, tv, k);
+            bool keep = rg.x <= whi && rg.y >= wlo;
+            int j = 0;
+            float4 g0, g1, g2;
+            float3 Oe;
+            if (keep) {
+                j = entry_id(L, tv, k);
+                g0 = __ldg(&L.g.g0[j]); g1 = __ldg(&L.g.g1[j]); g2 = __ldg(&L.g.g2[j]);
+                Oe = whiten_eye(L, g0, g1, g2);
+                keep = !cone_misses(cone_at, g0, g1, g2, Oe, rg.y);
+            }
+            const unsigned m = __ballot_sync(kFull, keep);
+            if (keep)
+                stage_record(st, (head + n + __popc(m & ((1u << lane) - 1u))) & (kStaged - 1), j, g0, g1, g2, Oe, __ldg(&L.g.hk[j]),
+                             __ldg(&L.g.rgba[j]));
+            n += __popc(m);
+            if (COUNT && lane == 0) tl.v[C_CANDS] += 32;
+        }
+        __syncwarp();
+        const int take = more ? n & ~(kGroup - 1) : n;
+        if (take > 0) process(head, take);
+        __syncwarp();
+        head = (head + take) & (kStaged - 1);
+        n -= take;
+        if (!more) break;
+    }
+}
+
+// Where a warp stands on the tape (lane 0 writes, all lanes read).
+struct TapeState {
+    long long off;      // next free int of the warp's current block
+    long long head;     // first chunk of the patch (-1: none yet)
+    long long prev;     // latest chunk of the patch
+    long long chunk;    // chunk of the current step (-1: the step is not recorded)
+    long long piece;    // piece the list is being written to (the chunk itself, or a later piece)
+    int left;           // ints left in the block
+    int ok;             // 0: the patch cannot be recorded (no room)
+    int n;              // entries in the current piece
+};
+
+template <int P>
+struct PatchShared {
+    static constexpr int kPatchRays = Patch<P>::kRays;
+    PatchStage st;
+    float4 cone[3];                   // see cone_misses
+    float2 clip[kPatchRays];          // tenter, texit
+    int slabs[kPatchRays];            // slabs begun so far
+    float4 rec[kGroup][kPatchRays];   // what eval_forward's record is in march_common.cuh, per entry and ray (y = -1: no hit)
+    float4 color[kPatchRays];      // colour and depth of the patch's rays so far
+    TapeState tq;
+};
+
+// Room for `need` ints at tq.off, from the warp's block or a new one.  Lane 0 only.
+__device__ __forceinline__ bool tape_room(const MarchLaunch& L, TapeState& tq, int need) {
+    if (need > tq.left) {
+        const unsigned long long o = atomicAdd(L.tape_used, (unsigned long long)kTapeBlock);
+        if ((long long)(o + kTapeBlock) > L.tape_cap) return false;
+        tq.off = (long long)o;
+        tq.left = kTapeBlock;
+    }
+    return true;
+}
+__device__ __forceinline__ void put_offset(int* at, long long off) {
+    *reinterpret_cast<int2*>(at) = make_int2((int)(off & 0xffffffffll), (int)(off >> 32));
+}
+__device__ __forceinline__ long long get_offset(int lo, int hi) { return ((long long)hi << 32) | (unsigned int)lo; }
+
+// Appends the staged entries [first, first + count) that some ray hit to the list of the current step.
+__device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq, const PatchStage& st, int first, int count, int lane) {
+    if (tq.chunk < 0) return;
+    for (int base = 0; base < count; base += 32) {
+        const int q = (first + base + lane) & (kStaged - 1);
+        const unsigned mask = base + lane < count ? st.mask[q] : 0u;
+        const unsigned m = __ballot_sync(kFull, mask != 0u);
+        const int n = __popc(m);
+        if (n == 0) continue;
+        if (lane == 0 && tq.left < 2 * n) {                          // the block is full: the list goes on elsewhere
+            const long long old = tq.piece;
+            L.tape[old] = tq.n;
+            if (tape_room(L, tq, kTapePiece + 64)) {
+                put_offset(L.tape + old + 2, tq.off);
+                put_offset(L.tape + tq.off + 2, -1);
+                tq.piece = tq.off;
+                tq.n = 0;
+                tq.off += kTapePiece;
+                tq.left -= kTapePiece;
+            } else {
+                tq.chunk = -1;
+                tq.ok = 0;
+            }
+        }
+        __syncwarp();
+        if (tq.chunk < 0) return;
+        if (mask != 0u)
+            reinterpret_cast<int2*>(L.tape + tq.off)[__popc(m & ((1u << lane) - 1u))] =
+                make_int2(__float_as_int(st.ex[q].z), (int)mask);
+        __syncwarp();
+        if (lane == 0) { tq.off += 2 * n; tq.left -= 2 * n; tq.n += n; }
+        __syncwarp();
+    }
+}
+
 // ---------------------------------------------------------------- forward
+// One warp per patch of 32 / P rays.  Lane r + h (32 / P) belongs to ray r; the P lanes of a ray carry the same state.  While list
+// entries are tested, lane group h tests entry e + h for all the rays; while hits are evaluated, lane h of a ray holds the samples
+// P i + h of its slab, 32 / P samples times four sums in registers.  Hits are evaluated only in the parts of the slab that some ray's
+// stretch inside the Gaussian reaches.
+//   What bounds it: instruction issue (66 % of the slots on the 300 k object, 2,376 M warp instructions; a warp per ray took
+// 7,800 M) and, recording, the 512 bytes of sums per ray and slab.  With P = 1 the sums of a slab would be 128 registers and eight
+// warps would fill an SM; P = 2 halves them at the price of one exchange per sample in the compositing.
+//   Tests of a group of entries come before their evaluation, through shared memory: the loops are short (a unit of tests and the
+// evaluation of both halves in one body missed the instruction cache) and the evaluation runs over entries that were hit only.
+//   Slabs of the rays are taken in steps: the ray that is furthest behind leads, and every ray whose slab begins before the
+// leader's ends marches with it.  The list is walked once per step over the union of the windows.
+//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.1 -> 4.3, 300 k object 9.25 -> 3.75 (7.8 -> 2.95
+// without recording), 7 M needles 11.6 -> 4.6 (two depths), 1 M at 640x360 1.67 -> 0.79.
+//
 // HZ: the two-depth variant for forward-only views whose rays end early (binning.cu).  In its first phase
 // (L.hz_phase == 1) the tile lists hold only the pairs that begin before L.horizon; a ray that would need more
 // -- its next slab reaches past the horizon, or a closest-hit query finds nothing before it, in a tile that has
@@ -225,439 +444,606 @@ __device__ __forceinline__ void hz_note(const MarchLaunch& L, int ray_id) {
 // are expected to end before the horizon): a ray that would need more is counted and listed (L.hz_rays), marked as
 // not recorded, and finished by march_forward_listed_rays_kernel, which the caller launches next.
 // HZ = 1: the two phases (L.hz_phase 1 or 2); HZ = 2: counting only (L.hz_phase 3), nothing is put aside.
-template <bool COUNT, bool SAVE, int HZ = 0>
-__global__ void __launch_bounds__(kThreads, COUNT ? 1 : 4) march_forward_lists_kernel(const __grid_constant__ MarchLaunch L) {
-    __shared__ ListShared sh;
-    __shared__ TapeState tape_state[SAVE ? kWarps : 1];
-    constexpr bool save = SAVE;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    WarpStage& ws = sh.ws[warp];
-    int* pend = sh.pend[warp];
-    const int unit = blockIdx.x / kTileSplit, part = blockIdx.x % kTileSplit;
-    const int tile = L.lists.tile_order ? __ldg(&L.lists.tile_order[unit]) : unit;   // longest lists first
-    if (HZ == 1 && L.hz_phase == 2 && !L.tile_resume[tile]) return;      // no ray of this tile stopped at the horizon
-    // the tile has pairs beyond the horizon that its lists do not hold
-    const bool hz_more = HZ != 0 && (HZ == 2 || L.hz_phase == 1) && L.tile_more[tile] != 0;
-    const int tile_x = tile % L.lists.tiles_x, tile_y = tile / L.lists.tiles_x;
+enum RayMode { kSeekFirst, kSeekNext, kInSlab, kDone };
+
+// Sum of one value over the P lanes of a ray (P consecutive samples), as a balanced tree; `before`: over the lanes before this one.
+template <int P>
+__device__ __forceinline__ float across_ray(float x, int sub, float& before) {
+    before = 0.f;
+#pragma unroll
+    for (int o = 1; o < P; o <<= 1) {
+        const float other = __shfl_xor_sync(kFull, x, o * Patch<P>::kRays);
+        if (sub & o) before = __fadd_rn(before, other);
+        x = __fadd_rn(x, other);
+    }
+    return x;
+}
+// Balanced sum of the values of sixteen consecutive samples, fed P at a time (indices known at compile time): what decides
+// the course of a ray is summed in the order of warp_scan in march_common.cuh, whichever way samples are dealt out to lanes.
+template <int P>
+struct SampleTree {
+    static constexpr int kLeaves = 16 / P;
+    float part[4];
+    float half;                        // complete after kLeaves values, again after twice as many
+    __device__ __forceinline__ void add(int i, float v) {
+        int k = i % kLeaves, level = 0;
+        while (k & 1) { v = __fadd_rn(part[level], v); k >>= 1; ++level; }
+        if ((1 << level) == kLeaves) half = v;
+        else part[level] = v;
+    }
+};
+// CTAs per SM that a forward kernel is compiled for.  With the recording 168 registers and twelve warps are faster than 128 and
+// sixteen: what spills at 128 is read back in the inner loops (300 k object 3.75 against 4.28 ms, 3 M-Gaussian view 4.30 against 4.60).
+template <int P, bool SAVE>
+__host__ __device__ constexpr int patch_ctas_per_sm() { return SAVE ? 3 : 4; }
+
+template <int P, bool COUNT, bool SAVE, int HZ>
+__global__ void __launch_bounds__(kPatchWarps * 32, COUNT ? 1 : patch_ctas_per_sm<P, SAVE>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+    using Pt = Patch<P>;
+    __shared__ PatchShared<P> shared[kPatchWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
+    PatchShared<P>& sh = shared[warp];
+    PatchStage& st = sh.st;
+    TapeState& tq = sh.tq;
     const float eps = L.m.transmittance_eps;
-    const float bg = L.m.white_background ? 1.0f : 0.0f;
-    const SceneBox box = *L.box;
-    const TileView tv = tile_view(L.lists, tile);
+    const float sub_even = (float)(sub & ~1), sub_off = (float)(sub & 1) + 0.5f;       // see eval_forward
+    const int cap = L.m.max_prim_slice;
+    const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
+    const unsigned units = (unsigned)(L.lists.tiles_x * L.lists.tiles_y) * per_tile;
     Tally tl;
 #pragma unroll
     for (int i = 0; i < C_NUM; ++i) tl.v[i] = 0;
-    TapeState& tq = tape_state[SAVE ? warp : 0];
-    if (tid == 0) sh.next_ray = 0;
-    if (save && lane == 0) { tq.off = 0; tq.left = 0; tq.hits = nullptr; tq.slabs = 0u; tq.nhits = 0u; }
-    __syncthreads();
+    if (SAVE && lane == 0) { tq.off = 0; tq.left = 0; }
 
     while (true) {
-        int ray = 0;
-        if (lane == 0) ray = atomicAdd(&sh.next_ray, 1);
-        ray = __shfl_sync(kFull, ray, 0);
-        if (ray >= kRaysPerCta) break;
-        ray += part * kRaysPerCta;
-        int px, py;
-        if (!ray_pixel(L, tile_x, tile_y, ray, px, py)) continue;
+        unsigned unit = 0;
+        if (lane == 0) unit = atomicAdd(L.next_unit, 1u);
+        unit = __shfl_sync(kFull, unit, 0);
+        if (unit >= units) break;
+        const int tile = __ldg(&L.lists.tile_order[unit / per_tile]), patch = (int)(unit % per_tile);   // longest lists first
+        if (HZ == 1 && L.hz_phase == 2 && !L.tile_resume[tile]) continue;    // no ray of this tile stopped at the horizon
+        const int x0 = (tile % L.lists.tiles_x) * L.lists.tile + (patch % (int)per_row) * Pt::kW;
+        const int y0 = (L.lists.ty_first + tile / L.lists.tiles_x) * L.lists.tile + (patch / (int)per_row) * Pt::kH;
+        if (x0 >= L.cam.width || y0 >= L.m.row_end || y0 + Pt::kH <= L.m.row_begin) continue;
+        // the tile has pairs beyond the horizon that its lists do not hold
+        const bool hz_more = HZ != 0 && (HZ == 2 || L.hz_phase == 1) && L.tile_more[tile] != 0;
+        const int px = x0 + r % Pt::kW, py = y0 + r / Pt::kW;
+        const bool in_image = px < L.cam.width && py >= L.m.row_begin && py < L.m.row_end;
         const int ray_id = py * L.cam.width + px;
-        Ray r;
-        make_ray(L.cam, px, py, r);
-        float tenter, texit;
-        clip_scene(box, r, tenter, texit);
-        float T = 1.0f;
-        if (lane == 0) sh.color[warp] = make_float4(0.f, 0.f, 0.f, 0.f);
-        int cursor = 0;
-        if (save) {
-            if (lane == 0) { tq.head = -1; tq.prev = -1; tq.ok = 1; }
-            __syncwarp();
-        }
-        if (COUNT) tl.v[C_RAYS] += 1;
-        // cycle counters of the counting variant: whole ray, closest-hit queries, slab queries (the
-        // evaluation of the staged hits is timed inside slab_sums), compositing
-        const long long c_ray = COUNT ? clock64() : 0;
-        // two-depth variant: 0 = march from the start, 1 = resume at a slab, 2 = resume at the first query,
-        // 3 = resume at a query after an empty slab; what was put aside is (tbuffer, T, tenter, mode) + colour
-        int hz_mode = 0;
-        bool hz_susp = false;
-        float4 hz_a = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (HZ == 1) {
-            if (L.hz_phase == 2) {
-                hz_a = L.hz_state[2 * (size_t)ray_id];
-                hz_mode = (int)hz_a.w;
-                if (hz_mode == 0) continue;                                       // finished in the first phase
-                if (hz_mode != 2) {
-                    T = hz_a.y;
-                    if (lane == 0) sh.color[warp] = L.hz_state[2 * (size_t)ray_id + 1];
-                }
+        const TileView tv = tile_view(L.lists, tile);
+        float3 dir;
+        float t;                           // where the ray stands: start of its next slab, or of its next query
+        {
+            Ray ray;
+            float tenter, texit;
+            make_ray(L.cam, px, py, ray);                                    // rays outside the image or the rows stay idle
+            clip_scene(*L.box, ray, tenter, texit);
+            dir = ray.d;
+            t = tenter;
+            // what a ray needs now and then lives in shared memory: its registers are wanted by the sums of the slab
+            if (lane == 0) patch_cone(L.cam, x0, y0, Pt::kW, Pt::kH, sh.cone);
+            if (sub == 0) {
+                sh.clip[r] = make_float2(tenter, texit);
+                sh.color[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                sh.slabs[r] = 0;
             }
         }
-        float first;
-        if (HZ == 1 && (hz_mode == 1 || hz_mode == 3)) first = hz_a.z;                  // the first hit is known
-        else first = closest_in_tile<COUNT>(L, r, tenter, texit, tv, cursor, pend, lane, tl);
-        if (COUNT) tl.v[C_CYC_SEEK] += clock64() - c_ray;
-        if (HZ && hz_more && !(first < L.horizon)) {                             // nothing before the horizon: ask again later
-            hz_susp = true;
-            if (lane == 0) {
+        int mode = in_image ? kSeekFirst : kDone;
+        float T = 1.0f;
+        bool suspended = false;
+        int cursor = 0;
+        if (HZ == 1 && L.hz_phase == 2 && in_image) {
+            // what was put aside is (t, T, tenter, mode) + colour; mode 1: at a slab, 2: before the first query, 3: at a query
+            // after an empty slab, 0: finished
+            const float4 a = L.hz_state[2 * (size_t)ray_id];
+            const int was = (int)a.w;
+            if (was == 0) { mode = kDone; suspended = true; }                // nothing to do, nothing to write
+            else if (was != 2) {
+                mode = was == 1 ? kInSlab : kSeekNext;
+                t = a.x; T = a.y;
+                if (sub == 0) sh.clip[r].x = a.z;
+                if (sub == 0) sh.color[r] = L.hz_state[2 * (size_t)ray_id + 1];
+            }
+        }
+        if (SAVE && lane == 0) { tq.head = -1; tq.prev = -1; tq.chunk = -1; tq.ok = 1; }
+        if (COUNT && in_image && sub == 0) tl.v[C_RAYS] += 1;
+        __syncwarp();
+        const long long c_patch = COUNT ? clock64() : 0;
+        // a ray that would need pairs from beyond the horizon: put aside (HZ = 1, first phase), counted and listed
+        auto suspend = [&](float at, float how) {
+            suspended = true;
+            mode = kDone;
+            if (sub == 0) {
                 if (HZ == 1 && L.hz_phase == 1) {
-                    L.hz_state[2 * (size_t)ray_id] = make_float4(tenter, 1.0f, tenter, 2.0f);
+                    L.hz_state[2 * (size_t)ray_id] = make_float4(at, T, sh.clip[r].x, how);
+                    L.hz_state[2 * (size_t)ray_id + 1] = sh.color[r];
                     L.tile_resume[tile] = 1;
                 }
                 hz_note<HZ>(L, ray_id);
             }
-        } else if (first < INFINITY && first < texit) {                           // :249-260
-            tenter = first;
-            float tbuffer = tenter;
-            int slab_index = 0;
-            if (HZ == 1 && hz_mode == 1) tbuffer = hz_a.x;
-            if (HZ == 1 && hz_mode == 3) {                                             // the query after an empty slab, again
-                const float nxt = closest_in_tile<COUNT>(L, r, hz_a.x, texit, tv, cursor, pend, lane, tl);
-                tbuffer = nxt < INFINITY ? nxt : texit;                           // nothing further: the loop below does not start
+        };
+
+        while (__any_sync(kFull, mode != kDone)) {
+            const float wall = warp_min_pos(mode != kDone ? t : INFINITY);
+            // ---- closest-hit queries (:249-260, :297-319)
+            if (__any_sync(kFull, mode == kSeekFirst || mode == kSeekNext)) {
+                const long long c_t = COUNT ? clock64() : 0;
+                const bool seeking = mode == kSeekFirst || mode == kSeekNext;
+                if (COUNT && seeking && sub == 0) tl.v[C_CLOSEST] += 1;
+                const float from = seeking ? t : INFINITY, texit = sh.clip[r].y;
+                float best = seeking && t <= texit ? texit : -INFINITY;     // nothing from here on can matter
+                bool found = false;
+                float whi = warp_max_pos(fmaxf(best, 0.0f));
+                walk_list<COUNT>(L, tv, sh.cone, wall, warp_min_pos(from), whi, cursor, st, kGroup, lane, tl, [&](int first, int count) {
+#pragma unroll 1
+                    for (int e = 0; e < count; e += P) {
+                        const int q = (first + e + sub) & (kStaged - 1);
+                        const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
+                        RayParabola pb;
+                        const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
+                        if (ellipsoid_stretch(Oe, de, pb) && e + sub < count && from <= best && stretch_meets(pb, from, best)) {
+                            const float at = fmaxf(from, entry_root(Oe, de, st.ex[q].y, pb));
+                            if (at <= best) { best = at; found = true; }
+                        }
+                        if (COUNT && seeking && e + sub < count) { tl.v[C_PRIM_TESTS] += 1; tl.v[C_ELL_TESTS] += 1; }
+                    }
+                    whi = warp_max_pos(fmaxf(best, 0.0f));                  // each lane prunes by what it has found itself
+                });
+                if (!found) best = INFINITY;
+                for (int o = Pt::kRays; o < 32; o <<= 1) best = fminf(best, __shfl_xor_sync(kFull, best, o));
+                if (seeking) {
+                    if (HZ && hz_more && !(best < L.horizon)) {                      // nothing before the horizon: ask again later
+                        suspend(t, mode == kSeekFirst ? 2.0f : 3.0f);
+                    } else if (mode == kSeekFirst) {
+                        if (best < INFINITY && best < texit) { t = best; if (sub == 0) sh.clip[r].x = best; mode = kInSlab; }
+                        else mode = kDone;
+                    } else {
+                        if (best < INFINITY) { t = best; mode = kInSlab; }
+                        else mode = kDone;
+                    }
+                }
+                if (COUNT && lane == 0) tl.v[C_CYC_SEEK] += clock64() - c_t;
             }
-            while (tbuffer < texit && T > eps && slab_index < kMaxSlabs) {        // :266
-                SlabPlan p = plan_slab(L.m, tbuffer, T, tenter, texit);
-                if (HZ && hz_more && !(p.tmax < L.horizon)) {                        // this slab needs pairs from beyond
-                    hz_susp = true;
-                    if (lane == 0) {
-                        if (HZ == 1 && L.hz_phase == 1) {
-                            L.hz_state[2 * (size_t)ray_id] = make_float4(tbuffer, T, tenter, 1.0f);
-                            L.hz_state[2 * (size_t)ray_id + 1] = sh.color[warp];
-                            L.tile_resume[tile] = 1;
-                        }
-                        hz_note<HZ>(L, ray_id);
+            __syncwarp();
+            const float2 clip = sh.clip[r];
+            if (mode == kInSlab && !(t < clip.y && T > eps && sh.slabs[r] < kMaxSlabs)) mode = kDone;   // :266
+
+            // ---- one slab of every ray that is near the one furthest behind
+            SlabPlan p = plan_slab(L.m, t, T, clip.x, clip.y);
+            const bool ready = mode == kInSlab;
+            const float lead = warp_min_pos(ready ? t : INFINITY);
+            const float lead_end = warp_min_pos(ready && t == lead ? p.tmax : INFINITY);
+            bool act = ready && (t < lead_end || t == lead);
+            if (HZ && hz_more && act && !(p.tmax < L.horizon)) { suspend(t, 1.0f); act = false; }   // this slab needs pairs from beyond
+            if (act) {
+                if (COUNT && sub == 0) tl.v[C_SLABS] += 1;
+                if (sub == 0) sh.slabs[r] += 1;
+                if (!p.traced) { t = __fadd_rn(t, p.slab); act = false; }
+            }
+            if (!__any_sync(kFull, act)) continue;
+            const long long c_q = COUNT ? clock64() : 0;
+            const float tmin = act ? p.tmin : INFINITY, tmax = act ? p.tmax : -INFINITY;
+            const float dt = p.dt, inv_part = __fdividef((float)Pt::kParts / (float)kSlab, p.dt);
+            float2 S[Pt::kPairs], R[Pt::kPairs], G[Pt::kPairs], B[Pt::kPairs];
+#pragma unroll
+            for (int i = 0; i < Pt::kPairs; ++i) S[i] = R[i] = G[i] = B[i] = make_float2(0.f, 0.f);
+            int nhit = 0, most = 0;                     // hits of this ray; bound on the hits of any ray of the patch
+            bool overflow = false;
+            if (SAVE) {
+                if (lane == 0 && tq.ok) {
+                    if (tape_room(L, tq, Pt::kTapeList + 64)) {
+                        tq.chunk = tq.piece = tq.off;
+                        tq.n = 0;
+                        tq.off += Pt::kTapeList;
+                        tq.left -= Pt::kTapeList;
+                        put_offset(L.tape + tq.chunk + 2, -1);
+                        put_offset(L.tape + tq.chunk + 4, -1);
+                    } else {
+                        tq.chunk = -1;
+                        tq.ok = 0;                     // no room: the backward will search these rays
                     }
-                    break;
                 }
-                if (COUNT) tl.v[C_SLABS] += 1;
-                ++slab_index;
-                if (!p.traced) { tbuffer = __fadd_rn(tbuffer, p.slab); continue; }
-                const float tau = __fmul_rn((float)lane + 0.5f, p.dt);
-                float s, cr, cg, cb;
-                bool overflow;
-                // room on the tape for the largest chunk this slab can make; the hits are written there as they
-                // are met and the unused rest is handed back
-                if (save) {
-                    if (lane == 0) {
-                        tq.hits = nullptr;
-                        if (tq.ok) {
-                            const int worst = (kTapeHead + L.m.max_prim_slice + 3) & ~3;
-                            if (worst > tq.left && worst <= kTapeBlock) {
-                                const unsigned long long o = atomicAdd(L.tape_used, (unsigned long long)kTapeBlock);
-                                if ((long long)(o + kTapeBlock) <= L.tape_cap) { tq.off = (long long)o; tq.left = kTapeBlock; }
+                __syncwarp();
+            }
+            float whi = warp_max_pos(fmaxf(tmax, 0.0f));
+            walk_list<COUNT>(L, tv, sh.cone, wall, warp_min_pos(tmin), whi, cursor, st, 3 * kGroup, lane, tl, [&](int first, int count) {
+#pragma unroll 1
+                for (int base = 0; base < count; base += kGroup) {
+                    const int f = first + base, n = min(count - base, kGroup), nhit0 = nhit;
+                    // test: lane group h of the warp takes entry e + h; no branches, so that the tests of two steps overlap
+                    unsigned reach = 0u;               // kParts bits per entry: parts of the slab that some ray's stretch inside reaches
+#pragma unroll 1
+                    for (int e = 0; e < n; e += P) {
+                        const int q = (f + e + sub) & (kStaged - 1);
+                        const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
+                        RayParabola pb;
+                        bool hit = ellipsoid_stretch(make_float3(m0.w, m1.w, m2.w), whiten_dir(m0, m1, m2, dir), pb);
+                        hit = hit && e + sub < n && stretch_meets(pb, tmin, tmax);
+                        if (COUNT && act && e + sub < n) { tl.v[C_PRIM_TESTS] += 1; tl.v[C_ELL_TESTS] += 1; }
+                        const unsigned m = __ballot_sync(kFull, hit);
+                        nhit += __popc(m & (Pt::kSameRay << r));
+                        if (r == 0) st.mask[q] = (m >> (Pt::kRays * sub)) & Pt::kRayBits;
+                        float4 A = parabola_record(pb, t, st.ex[q].x);
+                        // parts of the slab that the ray's stretch inside reaches, with a fiftieth of one on either side against
+                        // rounding (the test of each sample decides)
+                        const int lo = max(__float2int_rd(fmaf(A.x - pb.hw, inv_part, -0.5f * Pt::kParts / kSlab - 0.02f)), 0);
+                        const int hi = min(__float2int_rd(fmaf(A.x + pb.hw, inv_part, -0.5f * Pt::kParts / kSlab + 0.02f)), Pt::kParts - 1);
+                        const unsigned groups = hit && lo <= hi ? (2u << hi) - (1u << lo) : 0u;
+                        if (!hit) A.y = -1.0f;
+                        sh.rec[e + sub][r] = A;
+                        reach |= __reduce_or_sync(kFull, groups << (Pt::kParts * sub)) << (Pt::kParts * e);
+                    }
+                    __syncwarp();
+                    most += n;
+                    if (most > cap) {                   // cuda_train/forward/gaussians_aabb.cu:352-356: hits past the cap are dropped
+                        int seen = nhit0;
+                        for (int e = 0; e < n; ++e) {
+                            const int q = (f + e) & (kStaged - 1);
+                            bool hit = (st.mask[q] >> r) & 1u;
+                            if (hit && seen >= cap) { hit = false; overflow = true; if (sub == 0) sh.rec[e][r].y = -1.0f; }
+                            seen += hit ? 1 : 0;
+                            const unsigned m = __ballot_sync(kFull, hit) & Pt::kRayBits;
+                            if (lane == 0) st.mask[q] = m;
+                            __syncwarp();
+                        }
+                        nhit = seen;
+                    }
+                    if (COUNT)
+                        for (int e = 0; e < n; ++e) {
+                            const int q = (f + e) & (kStaged - 1);
+                            if (sub == 0 && ((st.mask[q] >> r) & 1u))
+                                tl.v[C_HASH] += mix64(((unsigned long long)ray_id << 40) ^ ((unsigned long long)sh.slabs[r] << 24) ^
+                                                      (unsigned long long)__ldg(&L.g.perm[__float_as_int(st.ex[q].z)]));
+                        }
+                    // evaluate
+#pragma unroll 1
+                    while (reach) {
+                        const int e = (__ffs(reach) - 1) / Pt::kParts;
+                        constexpr unsigned kPartBits = (1u << Pt::kParts) - 1u;
+                        const unsigned here = (reach >> (Pt::kParts * e)) & kPartBits;
+                        reach &= ~(kPartBits << (Pt::kParts * e));
+                        const float4 A = sh.rec[e][r];
+                        const float4 c = st.rgba[(f + e) & (kStaged - 1)];
+                        const float off = fmaf(sub_off, dt, -A.x);
+#pragma unroll
+                        for (int g = 0; g < Pt::kParts; ++g) {
+                            if (!((here >> g) & 1u)) continue;
+#pragma unroll
+                            for (int i = Pt::kPairsPerPart * g; i < Pt::kPairsPerPart * (g + 1); ++i) {
+                                const float2 s2 = P == 2 ? make_float2((float)(4 * i), (float)(4 * i + 2))
+                                                         : make_float2((float)(2 * P * i) + sub_even, (float)(2 * P * i + P) + sub_even);
+                                const float2 d = __ffma2_rn(s2, make_float2(dt, dt), make_float2(off, off));
+                                const float2 d2 = __fmul2_rn(d, d);
+                                const float2 arg = __ffma2_rn(make_float2(A.z, A.z), d2, make_float2(A.w, A.w));
+                                const float2 ee = make_float2(d2.x < A.y ? ex2_approx(arg.x) : 0.0f, d2.y < A.y ? ex2_approx(arg.y) : 0.0f);
+                                R[i] = __ffma2_rn(make_float2(c.x, c.x), ee, R[i]);
+                                G[i] = __ffma2_rn(make_float2(c.y, c.y), ee, G[i]);
+                                B[i] = __ffma2_rn(make_float2(c.z, c.z), ee, B[i]);
+                                S[i] = __ffma2_rn(make_float2(c.w, c.w), ee, S[i]);
+                                if (COUNT) tl.v[C_PAIRS] += (d2.x < A.y ? 1 : 0) + (d2.y < A.y ? 1 : 0);
                             }
-                            if (worst <= tq.left) tq.hits = L.tape + tq.off + kTapeHead;
-                            else tq.ok = 0;                // no room: the backward will search this ray
                         }
                     }
                     __syncwarp();
                 }
-                const long long c_q = COUNT ? clock64() : 0;
-                int nhit = slab_sums<COUNT, false>(L, L.m, tbuffer, tau, ray_id, slab_index, make_float3(0.f, 0.f, 0.f),
-                                                   ws, lane, tl, [&](auto&& leaf) {
-                    search_tile<COUNT>(L, r, p.tmin, p.tmax, tv, cursor, pend, lane, tl, leaf);
-                }, s, cr, cg, cb, overflow, save ? &tq.hits : nullptr, L.m.max_prim_slice);
-                if (COUNT) { tl.v[C_HITS] += nhit; tl.v[C_OVF] += overflow ? 1 : 0; tl.v[C_CYC_SEARCH] += clock64() - c_q; }
-                if (save && nhit > 0 && tq.hits) {
-                    int* chunk = tq.hits - kTapeHead;
-                    reinterpret_cast<float4*>(chunk + 4)[lane] = make_float4(s, cr, cg, cb);
-                    __syncwarp();
-                    if (lane == 0) {
-                        const int need = (kTapeHead + nhit + 3) & ~3;
-                        *reinterpret_cast<int4*>(chunk) = make_int4(__float_as_int(tbuffer), nhit, -1, -1);
-                        if (tq.prev >= 0)
-                            *reinterpret_cast<int2*>(L.tape + tq.prev + 2) = make_int2((int)(tq.off & 0xffffffffll), (int)(tq.off >> 32));
-                        if (tq.head < 0) tq.head = tq.off;
-                        tq.prev = tq.off;
-                        tq.off += need;
-                        tq.left -= need;
-                        tq.slabs += 1u;
-                        tq.nhits += (unsigned int)nhit;
-                    }
-                    __syncwarp();
+                if (SAVE) tape_append(L, tq, st, first, count, lane);
+            });
+            const bool hits = act && nhit > 0;
+            if (COUNT) {
+                if (lane == 0) tl.v[C_CYC_SEARCH] += clock64() - c_q;
+                if (act && sub == 0) { tl.v[C_HITS] += nhit; tl.v[C_OVF] += overflow ? 1 : 0; tl.v[C_SLABS_HIT] += hits ? 1 : 0; }
+            }
+            const unsigned with_hits = __ballot_sync(kFull, hits) & Pt::kRayBits;
+            if (SAVE && with_hits && tq.chunk >= 0) {
+                int* chunk = L.tape + tq.chunk;
+                if (lane == 0) {
+                    L.tape[tq.piece] = tq.n;
+                    chunk[1] = (int)with_hits;
+                    if (tq.prev >= 0) put_offset(L.tape + tq.prev + 4, tq.chunk);
+                    if (tq.head < 0) tq.head = tq.chunk;
+                    tq.prev = tq.chunk;
+                    const int pad = (int)(-tq.off & 3);                  // the next chunk starts on 16 bytes again
+                    tq.off += pad;
+                    tq.left -= pad;
                 }
-                if (nhit == 0) {                                                  // :297-319
-                    tbuffer = __fadd_rn(tbuffer, p.slab);
-                    const long long c_s = COUNT ? clock64() : 0;
-                    float nxt = closest_in_tile<COUNT>(L, r, tbuffer, texit, tv, cursor, pend, lane, tl);
-                    if (COUNT) tl.v[C_CYC_SEEK] += clock64() - c_s;
-                    if (HZ && hz_more && !(nxt < L.horizon)) {                   // the next hit, if any, is beyond the horizon
-                        hz_susp = true;
-                        if (lane == 0) {
-                            if (HZ == 1 && L.hz_phase == 1) {
-                                L.hz_state[2 * (size_t)ray_id] = make_float4(tbuffer, T, tenter, 3.0f);
-                                L.hz_state[2 * (size_t)ray_id + 1] = sh.color[warp];
-                                L.tile_resume[tile] = 1;
-                            }
-                            hz_note<HZ>(L, ray_id);
-                        }
-                        break;
-                    }
-                    if (!(nxt < INFINITY)) break;
-                    tbuffer = nxt;
-                    continue;
+                if (lane < 2 * Pt::kRays) chunk[8 + lane] = __float_as_int(sub == 0 ? t : dt);
+                float4* sums = reinterpret_cast<float4*>(chunk + Pt::kTapeSums) + lane;
+#pragma unroll
+                for (int i = 0; i < Pt::kPairs; ++i) {
+                    __stcs(sums + 64 * i, make_float4(S[i].x, R[i].x, G[i].x, B[i].x));
+                    __stcs(sums + 64 * i + 32, make_float4(S[i].y, R[i].y, G[i].y, B[i].y));
                 }
-                if (COUNT) tl.v[C_SLABS_HIT] += 1;
+                __syncwarp();
+            } else if (SAVE && !with_hits && tq.chunk >= 0) {
+                __syncwarp();
+                if (lane == 0) { tq.off -= Pt::kTapeList; tq.left += Pt::kTapeList; tq.chunk = -1; }    // nothing met: the room is handed back
+                __syncwarp();
+            }
+            // ---- compositing (march_common.cuh, composite_forward): transmittance before sample s = T exp(-sum of the x before it);
+            // what decides the ray's course -- T after 16 and after 32 samples -- is summed in the same order there and here
+            if (with_hits) {
                 const long long c_c = COUNT ? clock64() : 0;
-                composite_forward_shared(p, tbuffer, tau, eps, lane, s, cr, cg, cb, L.depth != nullptr, T, &sh.color[warp]);
-                if (COUNT) tl.v[C_CYC_COMP] += clock64() - c_c;
-                tbuffer = __fadd_rn(tbuffer, p.slab);                             // :324
+                float run = 0.f, cr = 0.f, cg = 0.f, cb = 0.f, cd = 0.f, T16 = T, x16 = 0.f;
+                bool live = true;
+                SampleTree<P> tree;
+#pragma unroll
+                for (int i = 0; i < Pt::kSamples; ++i) {
+                    const float x = __fmul_rn(i & 1 ? S[i / 2].y : S[i / 2].x, dt);
+                    float before;
+                    const float all = across_ray<P>(x, sub, before);
+                    if (i == Pt::kSamples / 2) {
+                        x16 = tree.half;
+                        T16 = __fmul_rn(T, exp_neg(x16));
+                        live = T16 > eps;                                // :190-201: the second chunk only counts while T is above the threshold
+                    }
+                    const float excl = __fadd_rn(run, before);
+                    run = __fadd_rn(run, all);
+                    const float one_m_w = 1.0f - exp_neg(x);
+                    const float Ts = live ? __fmul_rn(T, exp_neg(excl)) : 0.f;
+                    const float f = __fmul_rn(Ts, __fmul_rn(dt, __fdividef(one_m_w, fmaxf(x, 1e-6f))));
+                    cr = fmaf(f, i & 1 ? R[i / 2].y : R[i / 2].x, cr);
+                    cg = fmaf(f, i & 1 ? G[i / 2].y : G[i / 2].x, cg);
+                    cb = fmaf(f, i & 1 ? B[i / 2].y : B[i / 2].x, cb);
+                    if (L.depth) cd = fmaf(__fmul_rn(Ts, one_m_w), __fadd_rn(t, __fmul_rn((float)(P * i) + (float)sub + 0.5f, dt)), cd);
+                    tree.add(i, all);
+                }
+                for (int o = Pt::kRays; o < 32; o <<= 1) {
+                    cr = __fadd_rn(cr, __shfl_xor_sync(kFull, cr, o));
+                    cg = __fadd_rn(cg, __shfl_xor_sync(kFull, cg, o));
+                    cb = __fadd_rn(cb, __shfl_xor_sync(kFull, cb, o));
+                    if (L.depth) cd = __fadd_rn(cd, __shfl_xor_sync(kFull, cd, o));
+                }
+                if (hits) {
+                    if (sub == 0) {
+                        const float4 a = sh.color[r];
+                        sh.color[r] = make_float4(__fadd_rn(a.x, cr), __fadd_rn(a.y, cg), __fadd_rn(a.z, cb), __fadd_rn(a.w, cd));
+                    }
+                    T = live ? __fmul_rn(T, exp_neg(__fadd_rn(x16, tree.half))) : T16;
+                }
+                if (COUNT && lane == 0) tl.v[C_CYC_COMP] += clock64() - c_c;
+            }
+            if (act) {
+                t = __fadd_rn(t, p.slab);                                // :324
+                if (!hits) mode = kSeekNext;                             // :297-319
             }
         }
-        if (HZ == 2 && hz_susp && save && lane == 0) {             // the backward searches this ray again
-            L.ray_head[ray_id] = -2;
-            L.tile_unrecorded[tile] = 1;
-        }
-        if (lane == 0 && !(HZ && hz_susp)) {                                       // :326-339
-            const float4 acc = sh.color[warp];
-            const RayColor st = {T, acc.x, acc.y, acc.z, acc.w};
-            write_ray(L, ray_id, st, bg);
-            if (HZ == 1 && L.hz_phase == 1) L.hz_state[2 * (size_t)ray_id] = make_float4(0.f, 0.f, 0.f, 0.f);   // done
-            if (save) {
-                L.ray_head[ray_id] = tq.ok ? tq.head : -2;
-                if (!tq.ok) L.tile_unrecorded[tile] = 1;
+        __syncwarp();
+        if (in_image && sub == 0) {                                     // :326-339
+            if (!suspended) {
+                const float4 acc = sh.color[r];
+                const RayColor out = {T, acc.x, acc.y, acc.z, acc.w};
+                write_ray(L, ray_id, out, L.m.white_background ? 1.0f : 0.0f);
+                if (HZ == 1 && L.hz_phase == 1) L.hz_state[2 * (size_t)ray_id] = make_float4(0.f, 0.f, 0.f, 0.f);   // done
+            }
+            if (SAVE) {
+                const bool unrecorded = !tq.ok || (HZ == 2 && suspended);   // the backward searches this ray again
+                L.ray_unrecorded[ray_id] = unrecorded ? 1 : 0;
+                if (unrecorded) L.tile_unrecorded[tile] = 1;
             }
         }
-        if (COUNT) tl.v[C_CYC_TOTAL] += clock64() - c_ray;
+        if (SAVE && lane == 0) L.patch_head[tile * (int)per_tile + patch] = tq.ok ? tq.head : -1;
+        __syncwarp();
+        if (COUNT && lane == 0) tl.v[C_CYC_TOTAL] += clock64() - c_patch;
     }
-    if (COUNT) flush_tally(L, tl, lane);
-    if (save && lane == 0 && tq.slabs) {
-        atomicAdd(L.tape_used + 1, (unsigned long long)tq.slabs);
-        atomicAdd(L.tape_used + 2, (unsigned long long)tq.nhits);
+    if (COUNT) {
+#pragma unroll
+        for (int i = 0; i < C_NUM; ++i)
+            if (tl.v[i]) atomicAdd(&L.counters->v[i], tl.v[i]);
     }
 }
 
 // ---------------------------------------------------------------- backward, by replaying the forward's recording
 //
-// For rays whose forward was recorded.  Per slab the recording holds the hits and the
-// per-sample sums, so what is left is the second pass of the reference's backward
-// (cuda_train/backward/gaussians_aabb.cu:354-470): the gradient of every (slab,
-// Gaussian) pair.  Here lanes are Gaussians, not samples: a lane takes one hit of the
-// slab, walks only the samples that lie inside that Gaussian's truncation ellipsoid
-// (a handful of the 32 on average) and keeps the four moment sums in registers -- no
-// staging in shared memory and no reduction across lanes.
-constexpr int kRun = 4;     // samples per work item of the replay (2: 12.9 ms, 4: 11.1 ms, 8: 11.1 / 7.8 ms on the two test scenes)
-
-constexpr int kBatch = 8;   // slabs of a ray whose hits are worked off together
-
-struct ReplayStage {        // per warp: one group of up to 32 hits
-    float4 a[kFan];         // whitened ray point at the reference parameter of the moments, sigma
-    float4 b[kFan];         // whitened direction, -
-    float4 c[kFan];         // chat_i, tbuffer - reference parameter, first and last sample (as int bits)
-    float4 d[kFan];         // the response along the ray as a parabola about the closest approach (march_common.cuh,
-                            // eval_forward): -hk q_min, -hk |de|^2, (1 - q_min)/|de|^2, tbuffer - closest approach
-    int slot[kFan];
-    int upto[kFan];         // inclusive prefix of the number of runs
-    int slab[kFan];         // which slab of the batch the hit belongs to
+// For rays whose forward was recorded.  Per slab step the recording holds the per-sample sums of the patch's rays and the list of
+// Gaussians they hit, so what is left is the second pass of the reference's backward
+// (cuda_train/backward/gaussians_aabb.cu:354-470): the gradient of every (slab, Gaussian) pair.
+// One warp per patch.  First the step's per-sample terms beta and gamma, P lanes per ray as in the forward (same arithmetic:
+// T comes out bit for bit), into shared memory.  Then the listed Gaussians, P at a time: lane group h takes entry e + h for the
+// patch's rays; a lane walks the samples that lie inside that Gaussian on its ray (a handful of the 32) and keeps the four
+// moment sums in registers.  The thirteen sums of the Gaussian's gradient row are then added up over the rays in shared memory and
+// leave the SM as one coalesced reduction of 52 bytes, where a reduction per ray and hit kept the L2 and the L1 data pipe busy.
+// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 3.2 ms, 300 k object 4.7 -> 2.6 ms.
+template <int P>
+struct ReplayShared {              // per warp
+    PatchStage st;
+    float2 bg[kSlab][Patch<P>::kRays];  // beta, gamma of every sample
+    float red[13][36];             // one row per component, 32 lanes (+4: rows start in other banks)
 };
 
-template <int NB>
-struct ReplayBatchT {       // per warp: up to NB consecutive slabs of the ray
-    float2 bg[NB][kSlab];    // per sample: beta, gamma (slab_back_terms)
-    float tbuffer[NB];
-    float dt[NB];
-    long long hits[NB];      // where the slab's hit list starts on the tape
-    int upto[NB];            // inclusive prefix of the hit counts
-};
-
-template <int NB>
-struct ReplayShared {
-    int next_ray;
-    ReplayBatchT<NB> batch[kWarps];
-    ReplayStage stage[kWarps];
-};
-
-// Second pass of the backward for the hits of a batch of slabs (see the kernel's comment).
-// SINGLE: the batch is one slab (the common case where a slab fills the lanes by itself).
-template <bool SINGLE, int NB>
-__device__ __forceinline__ void replay_batch(const MarchLaunch& L, const Ray& r, float3 dl, const ReplayBatchT<NB>& bt,
-                                             ReplayStage& sp, int nslab, int lane, float tbuffer1, float dt1,
-                                             long long hits1, int nhit1) {
-    // a single slab's values come in registers (tbuffer1 ...), those of a batch from shared memory
-    const int total_hits = SINGLE ? nhit1 : bt.upto[nslab - 1];
-    for (int base = 0; base < total_hits; base += kFan) {
-        // step 1, one hit per lane: where the ray is inside the Gaussian, cut into runs of kRun samples
-        int nitem = 0;
-        const int g = base + lane;
-        if (g < total_hits) {
-            int k = 0;
-            if (!SINGLE) {
-#pragma unroll
-                for (int t = 0; t < NB - 1; ++t) k += (t < nslab - 1 && bt.upto[t] <= g) ? 1 : 0;
-            }
-            const int j = SINGLE ? L.tape[hits1 + g] : L.tape[bt.hits[k] + (g - (k > 0 ? bt.upto[k - 1] : 0))];
-            const float tbuffer = SINGLE ? tbuffer1 : bt.tbuffer[k], dt = SINGLE ? dt1 : bt.dt[k];
-            const float inv_dt = __fdividef(1.0f, dt);
-            const float tend = __fadd_rn(tbuffer, __fmul_rn(dt, (float)kSlab));
-            float3 Oe, de;
-            whiten_ray(r, __ldg(&L.g.g0[j]), __ldg(&L.g.g1[j]), __ldg(&L.g.g2[j]), Oe, de);
-            const float hk = __ldg(&L.g.hk[j]);
-            const float4 c = __ldg(&L.g.rgba[j]);
-            const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
-            // closest approach and half width of the stretch inside the ellipsoid |Oe + t de| < 1
-            const float aa = dot3(de, de);
-            const float inv_a = __fdividef(1.0f, aa);
-            // correctly rounded: the response is evaluated as a parabola about this point, and what the point is
-            // off the true closest approach comes back as an unmodelled linear term 2 |de|^2 (tau - tau*) error
-            const float tca = __fdiv_rn(-dot3(Oe, de), aa);
-            const float3 P = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
-            const float qmin = dot3(P, P);
-            const float hw = sqrt_approx(__fmul_rn(fmaxf(1.0f - qmin, 0.f), inv_a));      // only sizes the window of samples
-            // samples (s + 1/2) dt inside it, one more on each side against rounding; the test q < 1 decides
-            const float x_lo = fmaf(__fadd_rn(__fadd_rn(tca, -hw), -tbuffer), inv_dt, -0.5f);
-            const float x_hi = fmaf(__fadd_rn(__fadd_rn(tca, hw), -tbuffer), inv_dt, -0.5f);
-            const int s_lo = (int)fminf(fmaxf(ceilf(x_lo) - 1.0f, 0.f), (float)kSlab);
-            const int s_hi = (int)fmaxf(fminf(floorf(x_hi) + 1.0f, (float)(kSlab - 1)), -1.f);
-            // moments about the closest approach clamped to the slab, so that they stay small
-            const float tcr = fminf(fmaxf(tca, tbuffer), tend);
-            sp.a[lane] = make_float4(fmaf(tcr, de.x, Oe.x), fmaf(tcr, de.y, Oe.y), fmaf(tcr, de.z, Oe.z), c.w);
-            sp.b[lane] = make_float4(de.x, de.y, de.z, 0.f);
-            sp.c[lane] = make_float4(ci, __fadd_rn(tbuffer, -tcr), __int_as_float(s_lo), __int_as_float(s_hi));
-            sp.d[lane] = make_float4(__fmul_rn(-hk, qmin), __fmul_rn(-hk, aa), __fmul_rn(1.0f - qmin, inv_a),
-                                     __fadd_rn(tbuffer, -tca));
-            sp.slot[lane] = j;
-            if (!SINGLE) sp.slab[lane] = k;
-            nitem = s_hi >= s_lo ? (s_hi - s_lo + kRun) / kRun : 0;
-        }
-        int incl = nitem;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int total = __shfl_sync(kFull, incl, 31);
-        sp.upto[lane] = incl;
-        __syncwarp();
-        // step 2, one run per lane, whichever hit it belongs to: the four moment sums of the run,
-        // which share the reference point with the other runs of the hit and so simply add up
-        for (int i0 = 0; i0 < total; i0 += kFan) {
-            const int i = i0 + lane;
-            const bool active = i < total;
-            int h = 0;
-            float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
-            if (active) {
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (sp.upto[h + step - 1] <= i) h += step;          // first hit whose runs end after i
-                const float4 C = sp.c[h], D = sp.d[h];
-                const int k = SINGLE ? 0 : sp.slab[h];
-                const float dt = SINGLE ? dt1 : bt.dt[k];
-                const float2* sbg = bt.bg[k];
-                const int s_hi = __float_as_int(C.w);
-                const int nrun = (s_hi - __float_as_int(C.z) + kRun) / kRun;
-                const int s0 = __float_as_int(C.z) + kRun * (i - (sp.upto[h] - nrun));
-                // sample position counted from the closest approach (d: the response) and from the reference
-                // point of the moments (tc); both advance by dt
-                const float x0 = __fmul_rn((float)s0 + 0.5f, dt);
-                float d = __fadd_rn(x0, D.w), tc = __fadd_rn(x0, C.y);
-#pragma unroll
-                for (int q4 = 0; q4 < kRun; ++q4) {
-                    const int s = s0 + q4;
-                    const float d2 = __fmul_rn(d, d);
-                    if (s <= s_hi && d2 < D.z) {
-                        const float ex = ex2_approx(fmaf(D.y, d2, D.x));
-                        const float2 bg = sbg[s];
-                        const float be = bg.x;
-                        const float ga = __fmul_rn(ex, fmaf(C.x, be, bg.y));   // g * (alpha + beta*(chat_i - chat_s))
-                        const float g1 = __fmul_rn(ga, tc);
-                        sb = fmaf(ex, be, sb);
-                        n0 = __fadd_rn(n0, ga);
-                        n1 = __fadd_rn(n1, g1);
-                        n2 = fmaf(g1, tc, n2);
-                    }
-                    d = __fadd_rn(d, dt);
-                    tc = __fadd_rn(tc, dt);
-                }
-            }
-            // runs of one hit sit in neighbouring lanes (at most 32 / kRun of them): add them up so that
-            // the Gaussian's row gets one update per hit, not one per run
-            const int seg = active ? h : -1 - lane;
-#pragma unroll
-            for (int d = 1; d < kSlab / kRun; d <<= 1) {
-                const int seg_o = __shfl_down_sync(kFull, seg, d);
-                const float o_sb = __shfl_down_sync(kFull, sb, d), o_n0 = __shfl_down_sync(kFull, n0, d),
-                            o_n1 = __shfl_down_sync(kFull, n1, d), o_n2 = __shfl_down_sync(kFull, n2, d);
-                if (lane + d < 32 && seg_o == seg) {
-                    sb = __fadd_rn(sb, o_sb); n0 = __fadd_rn(n0, o_n0); n1 = __fadd_rn(n1, o_n1); n2 = __fadd_rn(n2, o_n2);
-                }
-            }
-            const int seg_prev = __shfl_up_sync(kFull, seg, 1);
-            const bool first = lane == 0 || seg_prev != seg;
-            if (active && first && (sb != 0.f || n0 != 0.f || n1 != 0.f || n2 != 0.f)) {
-                const float4 A = sp.a[h];
-                emit_global(L, dl, sp.slot[h], expand_gradient(A.w, A, sp.b[h], sb, n0, n1, n2), blockIdx.x / kReplaySplit);
-            }
-        }
-        __syncwarp();                      // the next group reuses the staging arrays
-    }
-}
-
-// NB: slabs batched.  1 where slabs fill the lanes by themselves (fewer registers, one more CTA per SM).
-template <int NB>
-__global__ void __launch_bounds__(kThreads) march_backward_replay_kernel(const __grid_constant__ MarchLaunch L) {
-    __shared__ ReplayShared<NB> sh;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int unit = blockIdx.x / kReplaySplit, part = blockIdx.x % kReplaySplit;
-    const int tile = L.replay_order ? __ldg(&L.replay_order[unit]) : unit;
-    const int tile_x = tile % L.lists.tiles_x, tile_y = tile / L.lists.tiles_x;
+template <int P>
+__global__ void __launch_bounds__(kPatchWarps * 32, 4) march_backward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+    using Pt = Patch<P>;
+    extern __shared__ __align__(16) unsigned char replay_smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
+    ReplayShared<P>& sh = reinterpret_cast<ReplayShared<P>*>(replay_smem)[warp];
+    PatchStage& st = sh.st;
     const float eps = L.m.transmittance_eps;
-    const SceneBox box = *L.box;
-    ReplayBatchT<NB>& bt = sh.batch[warp];
-    ReplayStage& sp = sh.stage[warp];
-    if (tid == 0) sh.next_ray = 0;
-    __syncthreads();
+    const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
+    const unsigned units = (unsigned)(L.lists.tiles_x * L.lists.tiles_y) * per_tile;
 
     while (true) {
-        int ray = 0;
-        if (lane == 0) ray = atomicAdd(&sh.next_ray, 1);
-        ray = __shfl_sync(kFull, ray, 0);
-        if (ray >= kRaysPerReplayCta) break;
-        ray += part * kRaysPerReplayCta;
-        int px, py;
-        if (!ray_pixel(L, tile_x, tile_y, ray, px, py)) continue;
+        unsigned unit = 0;
+        if (lane == 0) unit = atomicAdd(L.next_unit, 1u);
+        unit = __shfl_sync(kFull, unit, 0);
+        if (unit >= units) break;
+        const int tile = __ldg(&L.replay_order[unit / per_tile]), patch = (int)(unit % per_tile);
+        const int x0 = (tile % L.lists.tiles_x) * L.lists.tile + (patch % (int)per_row) * Pt::kW;
+        const int y0 = (L.lists.ty_first + tile / L.lists.tiles_x) * L.lists.tile + (patch / (int)per_row) * Pt::kH;
+        if (x0 >= L.cam.width || y0 >= L.m.row_end || y0 + Pt::kH <= L.m.row_begin) continue;
+        long long off = L.patch_head[tile * (int)per_tile + patch];
+        if (off < 0) continue;                     // the patch met nothing, or is left to the search kernel
+        const int px = x0 + r % Pt::kW, py = y0 + r / Pt::kW;
         const int ray_id = py * L.cam.width + px;
-        long long off = L.ray_head[ray_id];
-        if (off < 0) continue;                     // -1: the ray met nothing; -2: not recorded, left to the search kernel
-        Ray r;
-        make_ray(L.cam, px, py, r);
-        float tenter, texit;
-        clip_scene(box, r, tenter, texit);
-        const float3 dl = make_float3(L.dl_drgb[3 * (size_t)ray_id], L.dl_drgb[3 * (size_t)ray_id + 1],
-                                      L.dl_drgb[3 * (size_t)ray_id + 2]);
-        float D = fmaf(dl.x, L.rgb_in[3 * (size_t)ray_id],
-                       fmaf(dl.y, L.rgb_in[3 * (size_t)ray_id + 1], __fmul_rn(dl.z, L.rgb_in[3 * (size_t)ray_id + 2])));
-        float T = 1.0f;
-        int nslab = 0, nhits = 0;
+        const bool mine = px < L.cam.width && py >= L.m.row_begin && py < L.m.row_end && !L.ray_unrecorded[ray_id];
+        const unsigned recorded = __ballot_sync(kFull, mine) & Pt::kRayBits;
+        float3 dir, dl = make_float3(0.f, 0.f, 0.f);
+        float D = 0.f, T = 1.0f;
+        {
+            Ray ray;
+            make_ray(L.cam, px, py, ray);
+            dir = ray.d;
+        }
+        if (mine) {
+            const float* g = L.dl_drgb + 3 * (size_t)ray_id;
+            const float* c = L.rgb_in + 3 * (size_t)ray_id;
+            dl = make_float3(g[0], g[1], g[2]);
+            D = fmaf(dl.x, c[0], fmaf(dl.y, c[1], __fmul_rn(dl.z, c[2])));
+        }
         while (off >= 0) {
-            // first pass of a slab, from the recording: transmittance and the per-sample terms
-            const int4 hd = *reinterpret_cast<const int4*>(L.tape + off);
-            const float tbuffer = __int_as_float(hd.x);
-            const int nhit = hd.y;
-            const float4 sums = reinterpret_cast<const float4*>(L.tape + off + 4)[lane];
-            const long long hits_at = off + kTapeHead;
-            off = ((long long)hd.w << 32) | (unsigned int)hd.z;
-            // same step size as the forward: T is rebuilt from the recorded sums bit for bit
-            const SlabPlan p = plan_slab(L.m, tbuffer, T, tbuffer, texit);
-            const float dc = fmaf(dl.x, sums.y, fmaf(dl.y, sums.z, __fmul_rn(dl.z, sums.w)));
-            const SlabBackTerms terms = slab_back_terms(sums.x, dc, p.dt, T, D, eps, lane);
-            D = __fadd_rn(D, -terms.d_total);
-            T = slab_exit_T(terms.tr, eps);
-            bt.bg[nslab][lane] = make_float2(terms.beta, terms.gamma);
-            nhits += nhit;
-            if (lane == 0) { bt.tbuffer[nslab] = tbuffer; bt.dt[nslab] = p.dt; bt.hits[nslab] = hits_at; bt.upto[nslab] = nhits; }
-            ++nslab;
-            if (NB == 1 || nhits >= kFan || nslab == NB || off < 0) {   // enough hits to fill the lanes, or nothing more to wait for
-                __syncwarp();
-                if (NB == 1 || nslab == 1) replay_batch<true>(L, r, dl, bt, sp, 1, lane, tbuffer, p.dt, hits_at, nhit);
-                else replay_batch<false>(L, r, dl, bt, sp, nslab, lane, 0.f, 0.f, 0, 0);
-                nslab = 0;
-                nhits = 0;
+            const int* chunk = L.tape + off;
+            const int4 h0 = __ldcs(reinterpret_cast<const int4*>(chunk)), h1 = __ldcs(reinterpret_cast<const int4*>(chunk) + 1);
+            const unsigned rays = (unsigned)h0.y & recorded;
+            const bool act = (rays >> r) & 1u;
+            const float tbuffer = __int_as_float(chunk[8 + r]), dt = __int_as_float(chunk[Pt::kTapeDt + r]);
+            // ---- first pass: transmittance and the per-sample terms (slab_back_terms of march_common.cuh)
+            {
+                const float4* sums = reinterpret_cast<const float4*>(chunk + Pt::kTapeSums) + lane;
+                float run = 0.f, back = 0.f, T16 = T, x16 = 0.f;
+                bool live = true;
+                SampleTree<P> tree;
+                constexpr int kAhead = Pt::kSamples < 4 ? Pt::kSamples : 4;
+                float4 ahead[kAhead];
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) ahead[i] = __ldcs(sums + 32 * i);
+#pragma unroll
+                for (int i = 0; i < Pt::kSamples; ++i) {
+                    const float4 c = ahead[i % kAhead];
+                    if (i + kAhead < Pt::kSamples) ahead[i % kAhead] = __ldcs(sums + 32 * (i + kAhead));
+                    const float x = __fmul_rn(c.x, dt);
+                    float before, earlier;
+                    const float all = across_ray<P>(x, sub, before);
+                    if (i == Pt::kSamples / 2) {
+                        x16 = tree.half;
+                        T16 = __fmul_rn(T, exp_neg(x16));
+                        live = T16 > eps;
+                    }
+                    const float excl = __fadd_rn(run, before);
+                    run = __fadd_rn(run, all);
+                    const float one_m_w = 1.0f - exp_neg(x);
+                    const float Ts = __fmul_rn(T, exp_neg(excl));
+                    const float inv_s = c.x > 0.f ? __fdividef(1.0f, c.x) : 0.f;
+                    const float chat = __fmul_rn(fmaf(dl.x, c.y, fmaf(dl.y, c.z, __fmul_rn(dl.z, c.w))), inv_s);
+                    const float tw = __fmul_rn(Ts, one_m_w);
+                    const float step = __fmul_rn(tw, chat);                       // T_s (1 - w_s) chat_s
+                    const float steps = across_ray<P>(step, sub, earlier);
+                    const float Ds = __fadd_rn(D, -__fadd_rn(back, earlier));
+                    back = __fadd_rn(back, steps);
+                    const float beta = live ? __fmul_rn(tw, inv_s) : 0.f;
+                    const float alpha = __fmul_rn(fmaf(Ts, chat, -Ds), dt);
+                    sh.bg[P * i + sub][r] = make_float2(beta, live ? fmaf(-beta, chat, alpha) : 0.f);
+                    tree.add(i, all);
+                }
+                if (act) {
+                    D = __fadd_rn(D, -back);
+                    T = live ? __fmul_rn(T, exp_neg(__fadd_rn(x16, tree.half))) : T16;
+                }
             }
+            __syncwarp();
+            // ---- second pass: the Gaussians of the step
+            const float inv_dt = __fdividef(1.0f, dt);
+            const float tend = __fadd_rn(tbuffer, __fmul_rn(dt, (float)kSlab));
+            const float2* bg = &sh.bg[0][r];
+            const int2* list = reinterpret_cast<const int2*>(chunk + Pt::kTapeList);
+            int n = h0.x;
+            long long piece = get_offset(h0.z, h0.w);
+            while (true) {
+                for (int base = 0; base < n; base += 32) {
+                    const int cnt = min(n - base, 32);
+                    if (lane < cnt) {
+                        const int2 en = __ldcs(list + base + lane);
+                        const int j = en.x;
+                        const float4 g0 = __ldg(&L.g.g0[j]), g1 = __ldg(&L.g.g1[j]), g2 = __ldg(&L.g.g2[j]);
+                        stage_record(st, lane, j, g0, g1, g2, whiten_eye(L, g0, g1, g2), __ldg(&L.g.hk[j]), __ldg(&L.g.rgba[j]));
+                        st.mask[lane] = (unsigned)en.y & rays;
+                    } else {
+                        st.mask[lane] = 0u;
+                    }
+                    __syncwarp();
+                    for (int e = 0; e < cnt; e += P) {
+                        const int q = e + sub;
+                        const bool hit = (st.mask[q] >> r) & 1u;
+                        const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
+                        const float2 ex = make_float2(st.ex[q].x, st.ex[q].z);
+                        const float4 c = st.rgba[q];
+                        const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
+                        const float a = dot3(de, de), inv_a = __fdividef(1.0f, a), b = -dot3(Oe, de);
+                        float tca = __fmul_rn(b, inv_a);
+                        tca = fmaf(fmaf(-tca, a, b), inv_a, tca);
+                        const float3 P = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
+                        const float disc = 1.0f - dot3(P, P);
+                        const float ay = __fmul_rn(disc, inv_a), az = __fmul_rn(-ex.x, a), aw = fmaf(ex.x, disc, -ex.x);
+                        // samples (s + 1/2) dt inside the ellipsoid, one more on each side against rounding; d^2 < ay decides
+                        const float hw = sqrt_approx(fmaxf(ay, 0.f));
+                        const float rel = __fadd_rn(tca, -tbuffer);
+                        const int s_lo = max(__float2int_ru(fmaf(rel - hw, inv_dt, -0.5f)) - 1, 0);
+                        const int s_hi = min(__float2int_rd(fmaf(rel + hw, inv_dt, -0.5f)) + 1, kSlab - 1);
+                        const int len = hit ? s_hi - s_lo + 1 : 0;
+                        // moments about the closest approach clamped to the slab, so that they stay small
+                        const float tcr = fminf(fmaxf(tca, tbuffer), tend);
+                        const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
+                        const float off_d = __fadd_rn(tbuffer, -tca), off_c = __fadd_rn(tbuffer, -tcr);
+                        float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
+                        float x = (float)s_lo + 0.5f;
+                        const float2* at = bg + s_lo * Pt::kRays;
+                        for (int i = 0; i < len; ++i) {
+                            const float d = fmaf(x, dt, off_d);
+                            const float d2 = __fmul_rn(d, d);
+                            const float2 w = *at;
+                            const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
+                            const float tc = fmaf(x, dt, off_c);
+                            const float ga = __fmul_rn(g, fmaf(ci, w.x, w.y));        // g * (alpha + beta*(chat_i - chat_s))
+                            const float g1 = __fmul_rn(ga, tc);
+                            sb = fmaf(g, w.x, sb);
+                            n0 = __fadd_rn(n0, ga);
+                            n1 = __fadd_rn(n1, g1);
+                            n2 = fmaf(g1, tc, n2);
+                            x += 1.0f;
+                            at += Pt::kRays;
+                        }
+                        const float4 A = make_float4(fmaf(tcr, de.x, Oe.x), fmaf(tcr, de.y, Oe.y), fmaf(tcr, de.z, Oe.z), 0.f);
+                        GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sb, n0, n1, n2);
+                        if (!hit) gg = GaussGrad{};
+                        sh.red[0][lane] = gg.mu.x; sh.red[1][lane] = gg.mu.y; sh.red[2][lane] = gg.mu.z;
+                        sh.red[3][lane] = gg.y00; sh.red[4][lane] = gg.y11; sh.red[5][lane] = gg.y22;
+                        sh.red[6][lane] = gg.y01; sh.red[7][lane] = gg.y02; sh.red[8][lane] = gg.y12;
+                        sh.red[9][lane] = gg.dsigma;
+                        sh.red[10][lane] = __fmul_rn(dl.x, gg.drgb_scale);
+                        sh.red[11][lane] = __fmul_rn(dl.y, gg.drgb_scale);
+                        sh.red[12][lane] = __fmul_rn(dl.z, gg.drgb_scale);
+                        __syncwarp();
+                        // the lanes of entry e + h add its components over the rays (row layout: emit_global)
+                        if (q < cnt) {
+                            float* row = reinterpret_cast<float*>(L.grad_rows) +
+                                         16 * ((size_t)((unsigned)tile & (unsigned)(L.grad_copies - 1)) * (size_t)L.g.n_pad + (size_t)__float_as_int(ex.y));
+#pragma unroll
+                            for (int k0 = 0; k0 < 13; k0 += Pt::kRays) {
+                                const int k = k0 + r;
+                                if (k < 13) {
+                                    const float4* v = reinterpret_cast<const float4*>(&sh.red[k][Pt::kRays * sub]);
+                                    float sum = 0.f;
+#pragma unroll
+                                    for (int i = 0; i < Pt::kRays / 4; ++i) { const float4 a4 = v[i]; sum += (a4.x + a4.y) + (a4.z + a4.w); }
+                                    atomicAdd(row + k, sum);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (piece < 0) break;
+                const int4 h = *reinterpret_cast<const int4*>(L.tape + piece);
+                list = reinterpret_cast<const int2*>(L.tape + piece + kTapePiece);
+                n = h.x;
+                piece = get_offset(h.z, h.w);
+            }
+            off = get_offset(h1.x, h1.y);
         }
     }
 }
 
 // ---------------------------------------------------------------- backward, by searching again
 // For rays without a recording: all of them when the forward did not record, else only those
-// it could not record (ray_head == -2).
+// it could not record (ray_unrecorded).
 __global__ void __launch_bounds__(kThreads) march_backward_lists_kernel(const __grid_constant__ MarchLaunch L) {
     __shared__ ListShared sh;
     __shared__ int hit_lists[kWarps][kHitList];
@@ -680,11 +1066,11 @@ __global__ void __launch_bounds__(kThreads) march_backward_lists_kernel(const __
         int ray = 0;
         if (lane == 0) ray = atomicAdd(&sh.next_ray, 1);
         ray = __shfl_sync(kFull, ray, 0);
-        if (ray >= kRaysPerTile) break;
+        if (ray >= L.lists.tile * L.lists.tile) break;
         int px, py;
         if (!ray_pixel(L, tile_x, tile_y, ray, px, py)) continue;
         const int ray_id = py * L.cam.width + px;
-        if (L.tape && L.ray_head[ray_id] != -2) continue;       // recorded: the replay kernel's
+        if (L.tape && !L.ray_unrecorded[ray_id]) continue;      // recorded: the replay kernel's
         Ray r;
         make_ray(L.cam, px, py, r);
         float tenter, texit;
@@ -709,7 +1095,7 @@ __global__ void __launch_bounds__(kThreads) march_backward_lists_kernel(const __
             float s, dc, u0, u1;
             bool overflow;
             int* hits = hit_lists[warp];
-            int nhit = slab_sums<false, true>(L, L.m, tbuffer, tau, ray_id, slab_index, dl, ws, lane, tl, enumerate, s, dc,
+            int nhit = slab_sums<false, true>(L, L.m, tbuffer, p.dt, ray_id, slab_index, dl, ws, lane, tl, enumerate, s, dc,
                                               u0, u1, overflow, &hits, kHitList);
             if (nhit == 0) {
                 tbuffer = __fadd_rn(tbuffer, p.slab);
@@ -751,26 +1137,52 @@ static bool use_lists(const MarchLaunch& m) {
     return !(m.m.flags & (RGX_FLAG_BRUTE_FORCE | RGX_FLAG_PER_RAY_SEARCH)) && m.lists.ent_id != nullptr && m.g.n > 0;
 }
 
+// Lanes per ray.  Two where the image gives every warp the device can hold a patch of sixteen rays (28,000 rays and more); with
+// fewer rays, smaller patches: more warps, and fewer Gaussians per patch, the longest patch being all there is to wait for.
+// Forward + backward in ms with 2 / 4 / 8 lanes per ray, 100 k object: 64x64 7.7 / 6.3 / 5.6, 128x128 1.94 / 1.47 / 1.27, 160x160
+// 1.37 / 1.01 / 1.15, 256x256 1.13 / 1.26 / 1.73 (tiles of 16 pixels).  The choice depends on the image alone, so that every march of
+// a view -- whole or a row range, recording or not -- adds up a ray's colour in the same order.
+static int patch_lanes(const MarchLaunch& m) {
+    const long long rays = (long long)m.cam.width * m.cam.height;
+    return rays <= 128 * 128 ? 8 : rays <= 200 * 200 ? 4 : 2;
+}
+
+// CTAs of a patch kernel: as many as fit the device at once (their warps fetch patches until there are none left).
+template <int P>
+static int patch_ctas(const MarchLaunch& m, int ctas_per_sm) {
+    const long long warps = (long long)m.lists.tiles_x * m.lists.tiles_y * (m.lists.tile * m.lists.tile / Patch<P>::kRays);
+    const long long want = (warps + kPatchWarps - 1) / kPatchWarps, fit = (long long)m.sm_count * ctas_per_sm;
+    return (int)(want < fit ? want : fit);
+}
+
+template <int P, bool COUNT, bool SAVE, int HZ>
+static void launch_patches(const MarchLaunch& m, cudaStream_t s) {
+    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, COUNT ? 1 : patch_ctas_per_sm<P, SAVE>()), kPatchWarps * 32, 0, s>>>(m);
+}
+
+template <int P>
+static void launch_forward_lanes(const MarchLaunch& m, cudaStream_t s) {
+    const bool count = (m.m.flags & RGX_FLAG_COUNT_WORK) != 0, save = m.tape != nullptr;
+    if (m.hz_phase == 3) {
+        if (save) launch_patches<P, false, true, 2>(m, s);
+        else launch_patches<P, false, false, 2>(m, s);
+    } else if (m.hz_phase != 0) launch_patches<P, false, false, 1>(m, s);
+    else if (count && save) launch_patches<P, true, true, 0>(m, s);
+    else if (count) launch_patches<P, true, false, 0>(m, s);
+    else if (save) launch_patches<P, false, true, 0>(m, s);
+    else launch_patches<P, false, false, 0>(m, s);
+}
+
 cudaError_t launch_march_forward(const MarchLaunch& m, cudaStream_t s) {
     if (!use_lists(m)) return launch_march_forward_per_ray(m, s);
-    const int grid = m.lists.tiles_x * m.lists.tiles_y;
-    if (grid <= 0) return cudaSuccess;
-    const bool count = (m.m.flags & RGX_FLAG_COUNT_WORK) != 0, save = m.tape != nullptr;
-    const int ctas = grid * kTileSplit;
-    if (m.hz_phase == 3) {
-        if (save) note_launch(), march_forward_lists_kernel<false, true, 2><<<ctas, kThreads, 0, s>>>(m);
-        else note_launch(), march_forward_lists_kernel<false, false, 2><<<ctas, kThreads, 0, s>>>(m);
-        return cudaGetLastError();
+    if (m.lists.tiles_x * m.lists.tiles_y <= 0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(m.next_unit, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess) return e;
+    switch (patch_lanes(m)) {
+        case 2: launch_forward_lanes<2>(m, s); break;
+        case 4: launch_forward_lanes<4>(m, s); break;
+        default: launch_forward_lanes<8>(m, s);
     }
-    if (m.hz_phase != 0) {
-        if (save) note_launch(), march_forward_lists_kernel<false, true, 1><<<ctas, kThreads, 0, s>>>(m);
-        else note_launch(), march_forward_lists_kernel<false, false, 1><<<ctas, kThreads, 0, s>>>(m);
-        return cudaGetLastError();
-    }
-    if (count && save) note_launch(), march_forward_lists_kernel<true, true><<<ctas, kThreads, 0, s>>>(m);
-    else if (count) note_launch(), march_forward_lists_kernel<true, false><<<ctas, kThreads, 0, s>>>(m);
-    else if (save) note_launch(), march_forward_lists_kernel<false, true><<<ctas, kThreads, 0, s>>>(m);
-    else note_launch(), march_forward_lists_kernel<false, false><<<ctas, kThreads, 0, s>>>(m);
     return cudaGetLastError();
 }
 
@@ -782,13 +1194,25 @@ cudaError_t launch_march_backward_search(const MarchLaunch& m, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <int P>
+static cudaError_t launch_replay(const MarchLaunch& m, cudaStream_t s) {
+    const int bytes = (int)sizeof(ReplayShared<P>) * kPatchWarps;
+    cudaError_t e = cudaFuncSetAttribute(march_backward_patches_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    note_launch(), march_backward_patches_kernel<P><<<patch_ctas<P>(m, 4), kPatchWarps * 32, bytes, s>>>(m);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_march_backward_replay(const MarchLaunch& m, cudaStream_t s) {
     if (!use_lists(m) || !m.tape) return cudaSuccess;
-    const int grid = m.lists.tiles_x * m.lists.tiles_y;
-    if (grid <= 0) return cudaSuccess;
-    if (m.replay_batched) note_launch(), march_backward_replay_kernel<kBatch><<<grid * kReplaySplit, kThreads, 0, s>>>(m);
-    else note_launch(), march_backward_replay_kernel<1><<<grid * kReplaySplit, kThreads, 0, s>>>(m);
-    return cudaGetLastError();
+    if (m.lists.tiles_x * m.lists.tiles_y <= 0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(m.next_unit, 0, sizeof(unsigned int), s);
+    if (e != cudaSuccess) return e;
+    switch (patch_lanes(m)) {
+        case 2: return launch_replay<2>(m, s);
+        case 4: return launch_replay<4>(m, s);
+        default: return launch_replay<8>(m, s);
+    }
 }
 
 }  // namespace rgx

@@ -70,7 +70,18 @@ struct SceneBox {         // written by the build, read by the march kernels
     float hi[3];
 };
 
-constexpr int kBinTile = 16;      // pixels per side of a binning tile
+// Pixels per side of a binning tile.  16 for images of ordinary size; a small image has few tiles of that size, each as wide as
+// a large part of the scene and with a list as long, and walking it by the warps of a few SMs is then all the time there is.
+// Forward march with tiles of 16 / 8 / 4 pixels: 600 k object at 64x64 28.0 / 0.87 / 0.86 ms, at 128x128 4.3 / 1.0 / 0.5, at
+// 256x256 1.65 / 0.99 / 0.78; but smaller tiles mean more pairs, and from 256x256 on (8) and 128x128 on (4) the lists of
+// scenes with large Gaussians cost more than the march gains.  Depends on the image alone, so that a row range of it meets
+// its Gaussians in the same order.
+inline int bin_tile_size(const rgx_camera& c) {
+    const long long rays = (long long)c.width * c.height;
+    return rays <= 128 * 128 ? 4 : rays <= 256 * 256 ? 8 : 16;
+}
+constexpr int kMaxPatchesPerTile = 64;  // patches of rays that a warp marches together: 4 rays at least (march_lists.cu)
+constexpr int kTapeBlockInts = 16384;   // ints of the recording that a warp reserves at a time
 
 // Per-view, per-tile candidate lists (binning.cu).  Tile t owns entries
 // [tile_pbegin[t], tile_pbegin[t] + roundup32(tile_cnt[t])), sorted by near distance;
@@ -83,6 +94,7 @@ struct TileLists {
     const int* tile_cnt;
     const int* tile_order;     // tiles by falling list length: CTA b marches tile tile_order[b] (null: tile b)
     int tiles_x, tiles_y, ty_first;
+    int tile;                  // pixels per side
 };
 
 // Horizon of a culled emission (binning.cu): picked on the device from a histogram of the Gaussians' nearest
@@ -143,16 +155,16 @@ struct MarchLaunch {
     uchar4* frame;        // [R] 8-bit colour (cuda_gui/helpers.h:45-58), or null
     const float* rgb_in;
     const float* dl_drgb;
-    // "tape": what the forward met, kept for the backward (RGX_FLAG_SAVE_HITS).  Per slab with hits a chunk
-    // [tbuffer bits, hit count, next chunk offset lo, hi, sorted slots...]; ray_head[ray] = first chunk,
-    // -1 = no slab with hits, -2 = not recorded (the backward searches again).
+    // "tape": what the forward met, kept for the backward (RGX_FLAG_SAVE_HITS); layout in march_lists.cu.
     int* tape;
-    unsigned long long* tape_used;   // [3]: ints reserved, slabs recorded, hits recorded
-    int replay_batched;              // backward: work several slabs of a ray off together (few hits per slab)
+    unsigned long long* tape_used;   // ints reserved so far
     long long tape_cap;
-    long long* ray_head;
-    int* tile_unrecorded;   // per tile (of the lists): set by the forward when a ray of the tile got ray_head = -2
-    const int* replay_order;  // backward replay: tiles in the order of the recording forward's CTAs (own copy: the lists may be remade meanwhile)
+    long long* patch_head;           // [tiles * patches per tile] first chunk of every patch of rays, -1: nothing to replay
+    unsigned char* ray_unrecorded;   // [R] the ray could not be recorded: the backward searches it again
+    int* tile_unrecorded;            // per tile (of the lists): set by the forward when a ray of the tile is unrecorded
+    const int* replay_order;  // backward replay: tiles in the order of the recording forward (own copy: the lists may be remade meanwhile)
+    unsigned int* next_unit;  // the patch kernels' warps fetch their patches from it
+    int sm_count;
     // two-depth forward (march_lists.cu, HZ variant): 0 = off, 1 = first phase (lists up to `horizon`), 2 = second
     int hz_phase;
     float horizon;
