@@ -26,7 +26,8 @@ constexpr int kMaxSlabs = 1 << 22;   // hard bound on slab iterations per ray
 struct WarpStage {      // staged hit records of one warp
     float4 recA[kStage];
     float4 recB[kStage];
-    float4 recC[kStage];
+    float4 recC[kStage / 2];     // the backward stages half as many
+    float4 recD[kStage / 2];
 };
 struct WarpShared : WarpStage {   // plus the search stack of the per-ray variant
     uint32_t stack[kStack];
@@ -428,21 +429,21 @@ __device__ __forceinline__ float reduce8(const float (&v)[8], int lane) {
 // Pass 2 over `count` (<= 32) staged Gaussians: each lane forms its sample's share of
 // the four per-Gaussian sums, the warp adds them up eight Gaussians at a time, and
 // lane j keeps the totals of staged Gaussian j.
-//   recA = (y_c.xyz, hk)  recB = (de.xyz, tbuffer - t_c)  recC = (chat_i, -, -, -)
-__device__ __forceinline__ void eval_backward(const WarpStage& ws, int count, float tau, float beta, float gamma,
+//   recA = (y_c.xyz, -)  recB = (de.xyz, tbuffer - t_c)  recC = (chat_i, -, -, -)  recD: the parabola, see eval_forward
+__device__ __forceinline__ void eval_backward(const WarpStage& ws, int count, float dt, float tau, float beta, float gamma,
                                               int lane, float& o_sb, float& o_n0, float& o_n1, float& o_n2) {
+    const float k2 = (float)(lane & ~1), h2 = (float)(lane & 1) + 0.5f;
     for (int j0 = 0; j0 < count; j0 += 8) {
         float vb[8], v0[8], v1[8], v2[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int j = j0 + e;
             if (j < count) {
-                float4 A = ws.recA[j], B = ws.recB[j], C = ws.recC[j];
-                float tc = __fadd_rn(tau, B.w);
-                float yx = fmaf(tc, B.x, A.x), yy = fmaf(tc, B.y, A.y), yz = fmaf(tc, B.z, A.z);
-                float q = fmaf(yx, yx, fmaf(yy, yy, __fmul_rn(yz, yz)));
-                float ex = q < 1.0f ? ex2_approx(__fmul_rn(-A.w, q)) : 0.0f;
-                float ga = __fmul_rn(ex, fmaf(C.x, beta, gamma));      // g * (alpha + beta*(chat_i - chat_s))
+                const float4 D = ws.recD[j];
+                const float d = fmaf(k2, dt, fmaf(h2, dt, -D.x)), d2 = __fmul_rn(d, d);      // the forward's own test of the sample
+                const float tc = __fadd_rn(tau, ws.recB[j].w);
+                const float ex = d2 < D.y ? ex2_approx(fmaf(D.z, d2, D.w)) : 0.0f;
+                float ga = __fmul_rn(ex, fmaf(ws.recC[j].x, beta, gamma));      // g * (alpha + beta*(chat_i - chat_s))
                 float g1 = __fmul_rn(ga, tc);
                 vb[e] = __fmul_rn(ex, beta); v0[e] = ga; v1[e] = g1; v2[e] = __fmul_rn(g1, tc);
             } else {
@@ -652,7 +653,7 @@ __device__ __forceinline__ void slab_gradients(const MarchLaunch& L, const rgx_m
     int nstage = 0, nhit = 0;
     auto drain = [&]() {
         float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
-        eval_backward(ws, nstage, tau, beta, gamma, lane, sb, n0, n1, n2);
+        eval_backward(ws, nstage, p.dt, tau, beta, gamma, lane, sb, n0, n1, n2);
         if (lane < nstage) {
             const int j = prim_of[lane];
             emit(j, expand_gradient(__ldg(&L.g.sdens[j]).w, ws.recA[lane], ws.recB[lane], sb, n0, n1, n2));
@@ -676,14 +677,13 @@ __device__ __forceinline__ void slab_gradients(const MarchLaunch& L, const rgx_m
             int slot = nstage + rank;
             float4 c = __ldg(&L.g.rgba[j]);
             // reference point: closest approach clamped to the slab, so that the moments stay small
-            float a = dot3(t.de, t.de);
-            float tca = __fdividef(-dot3(t.Oe, t.de), a);
-            tca = fminf(fmaxf(tca, tbuffer), __fadd_rn(tbuffer, p.slab));
+            const float tca = fminf(fmaxf(t.p.t0, tbuffer), __fadd_rn(tbuffer, p.slab));
             ws.recA[slot] = make_float4(fmaf(tca, t.de.x, t.Oe.x), fmaf(tca, t.de.y, t.Oe.y),
-                                        fmaf(tca, t.de.z, t.Oe.z), __ldg(&L.g.hk[j]));
+                                        fmaf(tca, t.de.z, t.Oe.z), 0.f);
             ws.recB[slot] = make_float4(t.de.x, t.de.y, t.de.z, __fadd_rn(tbuffer, -tca));
             float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
             ws.recC[slot] = make_float4(ci, 0.f, 0.f, 0.f);
+            ws.recD[slot] = parabola_record(t.p, tbuffer, __ldg(&L.g.hk[j]));
             prim_of[slot] = j;
         }
         nstage += n;
