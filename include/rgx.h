@@ -230,11 +230,16 @@ RGX_API int rgx_read_kernel_times(rgx_ctx* ctx, float* forward_ms, int* forward_
 /* Replaces: distCUDA2 of the reference's simple-knn submodule (submodules/simple-knn/simple_knn.cu,
  * SimpleKNN::knn; called from classes/point_cloud.py:252,592 to size the first Gaussians).
  * points [n,3] -> mean_dist2 [n]: the mean of the squared distances from each point to its three nearest
- * other points, exact (Morton sort, two levels of boxes of 32, one warp per 32 queries).  With fewer than
+ * other points, exact (Morton sort, three levels of boxes of 32, one warp per 32 queries).  With fewer than
  * four points the missing neighbours stay at FLT_MAX in the fp32 sum, as in the reference: one missing gives
  * about FLT_MAX / 3, two or three overflow to +inf.  Needs no context; allocates
  * and frees its scratch (about 70 bytes per point) inside the call and synchronises the stream. */
 RGX_API int rgx_knn_mean_dist2(int device, const float* points, int n, float* mean_dist2, rgx_stream stream);
+/* The same in scratch of the caller's (256-byte aligned, rgx_knn_scratch_bytes(n) bytes, from a framework's allocator
+ * say): enqueued on the stream without waiting for it, nothing allocated or freed. */
+RGX_API size_t rgx_knn_scratch_bytes(int n);
+RGX_API int rgx_knn_mean_dist2_scratch(int device, const float* points, int n, float* mean_dist2, void* scratch,
+                                       size_t scratch_bytes, rgx_stream stream);
 
 /* Test hook (no counterpart in the reference): the workspace allocation that follows `nth` more successful
  * ones fails as if the device were out of memory, without touching the device (nth < 0 switches the hook

@@ -76,6 +76,8 @@ SYMBOLS = {
     "rgx_read_near_lists": (C.c_int, [C.c_void_p, C.POINTER(C.c_longlong)]),
     "rgx_measure_peaks": (C.c_int, [C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
     "rgx_knn_mean_dist2": (C.c_int, [C.c_int, _fp, C.c_int, _fp, C.c_void_p]),
+    "rgx_knn_scratch_bytes": (C.c_size_t, [C.c_int]),
+    "rgx_knn_mean_dist2_scratch": (C.c_int, [C.c_int, _fp, C.c_int, _fp, _fp, C.c_size_t, C.c_void_p]),
     "rgx_reset_counters": (C.c_int, [C.c_void_p, C.c_void_p]),
     "rgx_read_counters": (C.c_int, [C.c_void_p, C.POINTER(Counters), C.c_void_p]),
     "rgx_workspace_bytes": (C.c_size_t, [C.c_void_p]),

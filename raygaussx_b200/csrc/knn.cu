@@ -3,117 +3,144 @@
 // simple-knn (classes/point_cloud.py:252,592 -> submodules/simple-knn/simple_knn.cu,
 // SimpleKNN::knn) to size the first Gaussians.
 //
-// Exact, like the reference: points are sorted along a Morton curve, every 32
-// consecutive points get a box and every 32 boxes a box of their own.  A warp owns 32
-// consecutive sorted points, one query per lane; it walks the upper boxes, opens the
-// ones that are nearer to some lane's query than that lane's third-best distance so
-// far, and inside them the boxes of 32 points by the same rule.  The 32 points of an
-// opened box are loaded with one coalesced read and handed round with shuffles.
-// Queries of a warp are neighbours in space, so after the seed (the warp's own box and
-// its two neighbours) nearly every box is rejected by all 32 lanes at once.
+// Exact, like the reference: points are sorted along a Hilbert curve, every 32
+// consecutive points get a box, every 32 boxes a box of their own, and 32 of those
+// again.  A warp owns 32 consecutive sorted points, one query per lane.  It descends
+// the three levels with lanes as nodes: 32 boxes at a time against the box of its 32
+// queries and the worst third-best distance among them.  A box of points that passes is
+// opened if it is nearer to some lane's query than that lane's third-best; its points
+// are then read by all lanes at once from shared memory.
+//   Queries of a warp are neighbours in space, so after the seed (the warp's own box and
+// its two neighbours) few boxes are opened and what bounds the kernel is the distance
+// arithmetic of those.  Testing every upper box by every warp, as an earlier version did, took 15.3 ms
+// for 3 M points (now 1.02 ms); the whole call, whose eleven allocations and frees cost more than
+// its kernels on small clouds, took 19.9 ms for 3 M (now 1.45) and 0.4 ms (in a process with a large
+// workspace several ms) for 100 k points (now 0.18, scratch from the caller).
 #include "rgx_internal.cuh"
+#include "device_math.cuh"
 #include <cub/device/device_radix_sort.cuh>
+#include <algorithm>
 
 namespace rgx {
 
 namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
+constexpr int kKnnWarps = 8;
 
-__device__ __forceinline__ int ordered(float f) {          // float -> int with the same order
-    int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
+// float -> unsigned with the same order, above zero for every number
+__device__ __forceinline__ unsigned ordered(float f) {
+    const unsigned u = __float_as_uint(f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
 }
-__device__ __forceinline__ float unordered(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+__device__ __forceinline__ float unordered(unsigned u) { return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u); }
 
-__global__ void knn_init_kernel(int* bounds) {
-    if (threadIdx.x < 3) bounds[threadIdx.x] = ordered(FLT_MAX);
-    else if (threadIdx.x < 6) bounds[threadIdx.x] = ordered(-FLT_MAX);
+// bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
+__global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, unsigned* bounds) {
+    __shared__ unsigned s_max[6];
+    if (threadIdx.x < 6) s_max[threadIdx.x] = 0u;
+    __syncthreads();
+    unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float v = pts[3 * (size_t)i + a];
+            m[a] = max(m[a], ordered(v));
+            m[3 + a] = max(m[3 + a], ordered(-v));
+        }
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+        const unsigned v = __reduce_max_sync(kAll, m[a]);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s_max[a], v);
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) atomicMax(&bounds[threadIdx.x], s_max[threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, int* bounds) {
+// Positions along a Hilbert curve.  A cell that holds many points leaves them in no order, their boxes of 32 all as large as
+// the cell: ten bits per axis do for small clouds, a large one whose extent is set by a few far points (an unbounded scene)
+// needs finer cells (3 M points, core and shell: query 14.4 ms with 10 bits per axis, 1.3 with 16).
+template <class Key>
+__global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ pts, int n, const unsigned* bounds,
+                                                       Key* keys, unsigned* vals) {
+    constexpr int kBits = sizeof(Key) == 8 ? 16 : 10;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    if (i < n)
-        for (int a = 0; a < 3; ++a) lo[a] = hi[a] = pts[3 * (size_t)i + a];
+    if (i >= n) return;
+    const float top = (float)((1 << kBits) - 1);
+    uint32_t q[3];
     for (int a = 0; a < 3; ++a) {
+        float lo = -unordered(bounds[3 + a]), hi = unordered(bounds[a]);
+        float ext = hi - lo;
+        float u = ext > 0.f ? (pts[3 * (size_t)i + a] - lo) / ext : 0.f;
+        q[a] = (uint32_t)fminf(fmaxf(u * top, 0.f), top);
+    }
+    hilbert_transpose(q, kBits);
+    keys[i] = (Key)((spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]));
+    vals[i] = (unsigned)i;
+}
+inline bool wide_keys(int n) { return n >= 65536; }
+
+// Boxes of one level: lo and hi per node.
+struct KnnLevel {
+    float4 *lo, *hi;
+    int count;
+};
+
+// The box of the warp's 32 boxes (an empty one is (+inf, -inf): at infinite distance), on lane 0.
+__device__ __forceinline__ void warp_box(float (&lo)[3], float (&hi)[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             lo[a] = fminf(lo[a], __shfl_xor_sync(kAll, lo[a], o));
             hi[a] = fmaxf(hi[a], __shfl_xor_sync(kAll, hi[a], o));
         }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&bounds[a], ordered(lo[a]));
-            atomicMax(&bounds[3 + a], ordered(hi[a]));
-        }
-    }
 }
 
-__device__ __forceinline__ unsigned spread10(unsigned v) {   // 10 bits -> every third bit
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
-__global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ pts, int n, const int* bounds,
-                                                       unsigned* keys, unsigned* vals) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    unsigned q[3];
-    for (int a = 0; a < 3; ++a) {
-        float lo = unordered(bounds[a]), hi = unordered(bounds[3 + a]);
-        float ext = hi - lo;
-        float u = ext > 0.f ? (pts[3 * (size_t)i + a] - lo) / ext : 0.f;
-        q[a] = (unsigned)fminf(fmaxf(u * 1023.0f, 0.f), 1023.f);
-    }
-    keys[i] = spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2);
-    vals[i] = (unsigned)i;
-}
-
-// Sorted copies of the points (w = 0), padded to a multiple of 1024 with points at infinity,
-// boxes of 32 points and of 32 such boxes.  One warp per box of 32 points.
-__global__ void __launch_bounds__(256) knn_gather_kernel(const float* __restrict__ pts, int n, int n_pad,
-                                                         const unsigned* __restrict__ order, float4* sorted,
-                                                         float4* box_lo, float4* box_hi) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int i = warp * 32 + lane;
-    if (i >= n_pad) return;
+// Sorted copies of the points, padded to a multiple of 32 with points at infinity, their boxes and, a block of 1,024 points
+// being one node of the level above, that node's.
+__global__ void __launch_bounds__(1024) knn_gather_kernel(const float* __restrict__ pts, int n, const unsigned* __restrict__ order,
+                                                          float4* sorted, KnnLevel leaf, KnnLevel mid) {
+    __shared__ float s_lo[32][3], s_hi[32][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * 1024 + threadIdx.x, b = blockIdx.x * 32 + warp;
     float4 p = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     if (i < n) {
         const size_t s = order[i];
         p = make_float4(pts[3 * s], pts[3 * s + 1], pts[3 * s + 2], 0.f);
     }
-    sorted[i] = p;
+    if (b < leaf.count) sorted[i] = p;
     float lo[3] = {p.x, p.y, p.z}, hi[3] = {i < n ? p.x : -INFINITY, i < n ? p.y : -INFINITY, i < n ? p.z : -INFINITY};
-    for (int a = 0; a < 3; ++a)
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(kAll, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(kAll, hi[a], o));
-        }
+    warp_box(lo, hi);
     if (lane == 0) {
-        box_lo[warp] = make_float4(lo[0], lo[1], lo[2], 0.f);      // an empty box is (+inf, -inf): at infinite distance
-        box_hi[warp] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        if (b < leaf.count) {
+            leaf.lo[b] = make_float4(lo[0], lo[1], lo[2], 0.f);
+            leaf.hi[b] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        }
+        for (int a = 0; a < 3; ++a) { s_lo[warp][a] = lo[a]; s_hi[warp][a] = hi[a]; }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        for (int a = 0; a < 3; ++a) { lo[a] = s_lo[lane][a]; hi[a] = s_hi[lane][a]; }
+        warp_box(lo, hi);
+        if (lane == 0) {
+            mid.lo[blockIdx.x] = make_float4(lo[0], lo[1], lo[2], 0.f);
+            mid.hi[blockIdx.x] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) knn_upper_kernel(const float4* box_lo, const float4* box_hi, int n_boxes,
-                                                        float4* up_lo, float4* up_hi) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int b = warp * 32 + lane;
-    if (warp * 32 >= n_boxes) return;
-    float4 l = b < n_boxes ? box_lo[b] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-    float4 h = b < n_boxes ? box_hi[b] : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+__global__ void __launch_bounds__(256) knn_upper_kernel(KnnLevel below, KnnLevel level) {
+    const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (node >= level.count) return;
+    const int b = node * 32 + lane;
+    const float4 l = b < below.count ? below.lo[b] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+    const float4 h = b < below.count ? below.hi[b] : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
     float lo[3] = {l.x, l.y, l.z}, hi[3] = {h.x, h.y, h.z};
-    for (int a = 0; a < 3; ++a)
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(kAll, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(kAll, hi[a], o));
-        }
+    warp_box(lo, hi);
     if (lane == 0) {
-        up_lo[warp] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        up_hi[warp] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        level.lo[node] = make_float4(lo[0], lo[1], lo[2], 0.f);
+        level.hi[node] = make_float4(hi[0], hi[1], hi[2], 0.f);
     }
 }
 
@@ -124,61 +151,144 @@ __device__ __forceinline__ float box_dist2(float4 lo, float4 hi, float4 p) {
     return dx * dx + dy * dy + dz * dz;
 }
 
-__device__ __forceinline__ void keep3(float d, float (&best)[3]) {     // the three smallest, ascending
-    if (d < best[2]) {
-        if (d < best[1]) {
-            best[2] = best[1];
-            if (d < best[0]) { best[1] = best[0]; best[0] = d; }
-            else best[1] = d;
-        } else best[2] = d;
-    }
-}
+struct KnnTree {
+    KnnLevel leaf, mid, top;
+};
 
-// All lanes: measure the 32 points of box `b` against this lane's query (skipping the query itself).
-__device__ __forceinline__ void open_box(const float4* __restrict__ sorted, int b, int self, float4 q, bool want,
-                                         float (&best)[3], int lane) {
-    const float4 mine = sorted[b * 32 + lane];
-    for (int k = 0; k < 32; ++k) {
-        const float x = __shfl_sync(kAll, mine.x, k), y = __shfl_sync(kAll, mine.y, k), z = __shfl_sync(kAll, mine.z, k);
-        const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
-        const float d = dx * dx + dy * dy + dz * dz;                 // +inf for the padding points
-        if (want && b * 32 + k != self) keep3(d, best);
-    }
-}
-
-__global__ void __launch_bounds__(256) knn_query_kernel(const float4* __restrict__ sorted, const unsigned* __restrict__ order,
-                                                        int n, int n_boxes, int n_upper, const float4* __restrict__ box_lo,
-                                                        const float4* __restrict__ box_hi, const float4* __restrict__ up_lo,
-                                                        const float4* __restrict__ up_hi, float* __restrict__ out) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n_boxes) return;
+__global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* __restrict__ sorted, const unsigned* __restrict__ order,
+                                                                   int n, KnnTree tree, float* __restrict__ out) {
+    __shared__ float s_pts[kKnnWarps][3][32];
+    const int warp = blockIdx.x * kKnnWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (warp >= tree.leaf.count) return;
+    float (*pts)[32] = s_pts[threadIdx.x >> 5];
     const int self = warp * 32 + lane;
     const bool live = self < n;
     const float4 q = sorted[self];
-    float best[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
-    // seed: the warp's own box and its neighbours along the curve
-    for (int b = max(warp - 1, 0); b <= min(warp + 1, n_boxes - 1); ++b) open_box(sorted, b, self, q, live, best, lane);
-    for (int u = 0; u < n_upper; ++u) {
-        const bool near_u = live && box_dist2(up_lo[u], up_hi[u], q) <= best[2];
-        if (!__any_sync(kAll, near_u)) continue;
-        const int b_end = min(u * 32 + 32, n_boxes);
-        // this lane looks at box u*32 + lane for every query of the warp ... by turns: each lane tests its own
-        // query against each of the 32 boxes, the warp opens a box if any lane wants it
-        for (int b = u * 32; b < b_end; ++b) {
-            if (b >= warp - 1 && b <= warp + 1) continue;            // seeded above
-            const bool near_b = near_u && box_dist2(box_lo[b], box_hi[b], q) <= best[2];
-            if (!__any_sync(kAll, near_b)) continue;
-            open_box(sorted, b, self, q, near_b, best, lane);
+    // the box of the queries
+    float qlo[3] = {live ? q.x : INFINITY, live ? q.y : INFINITY, live ? q.z : INFINITY};
+    float qhi[3] = {live ? q.x : -INFINITY, live ? q.y : -INFINITY, live ? q.z : -INFINITY};
+    warp_box(qlo, qhi);
+    float best0 = FLT_MAX, best1 = FLT_MAX, best2 = FLT_MAX;             // the three smallest, ascending
+    float worst = FLT_MAX;                                               // largest best2 of the warp
+    auto keep3 = [&](float d) {
+        const float t = fmaxf(best0, d), u = fmaxf(best1, t);
+        best0 = fminf(best0, d);
+        best1 = fminf(best1, t);
+        best2 = fminf(best2, u);
+    };
+    auto open_box = [&](int b, bool own) {
+        const float4 mine = sorted[b * 32 + lane];
+        __syncwarp();
+        pts[0][lane] = mine.x; pts[1][lane] = mine.y; pts[2][lane] = mine.z;
+        __syncwarp();
+#pragma unroll 4
+        for (int k = 0; k < 32; k += 2) {                                // two points at a time: packed fp32x2 arithmetic, same bits
+            const float2 dx = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[0][k]), make_float2(-q.x, -q.x)),
+                         dy = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[1][k]), make_float2(-q.y, -q.y)),
+                         dz = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[2][k]), make_float2(-q.z, -q.z));
+            float2 d = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));   // +inf for the padding points
+            if (own && k == lane) d.x = INFINITY;
+            if (own && k + 1 == lane) d.y = INFINITY;
+            keep3(d.x);
+            keep3(d.y);
         }
-    }
-    if (live) out[order[self]] = (best[0] + best[1] + best[2]) / 3.0f;   // simple_knn.cu: mean of the three
+    };
+    auto settle = [&]() { worst = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(live ? best2 : 0.f))); };
+    // nodes [base, base + 32) of a level that may hold something near enough for some query of the warp
+    auto near = [&](const KnnLevel& level, int base) -> unsigned {
+        const int b = base + lane;
+        bool ok = false;
+        if (b < level.count) {
+            const float4 lo = level.lo[b], hi = level.hi[b];
+            const float dx = fmaxf(fmaxf(lo.x - qhi[0], qlo[0] - hi.x), 0.f), dy = fmaxf(fmaxf(lo.y - qhi[1], qlo[1] - hi.y), 0.f),
+                        dz = fmaxf(fmaxf(lo.z - qhi[2], qlo[2] - hi.z), 0.f);
+            ok = dx * dx + dy * dy + dz * dz <= worst;
+        }
+        return __ballot_sync(kAll, ok);
+    };
+    // seed: the warp's own box and its neighbours along the curve
+    open_box(warp, true);
+    if (warp > 0) open_box(warp - 1, false);
+    if (warp + 1 < tree.leaf.count) open_box(warp + 1, false);
+    settle();
+    for (int t0 = 0; t0 < tree.top.count; t0 += 32)
+        for (unsigned mt = near(tree.top, t0); mt; mt &= mt - 1) {
+            const int t = t0 + __ffs(mt) - 1;
+            for (unsigned mm = near(tree.mid, t * 32); mm; mm &= mm - 1) {
+                const int m = t * 32 + __ffs(mm) - 1;
+                for (unsigned ml = near(tree.leaf, m * 32); ml; ml &= ml - 1) {
+                    const int b = m * 32 + __ffs(ml) - 1;
+                    if (b >= warp - 1 && b <= warp + 1) continue;        // seeded above
+                    if (!__any_sync(kAll, live && box_dist2(tree.leaf.lo[b], tree.leaf.hi[b], q) <= best2)) continue;
+                    open_box(b, false);
+                    settle();
+                }
+            }
+        }
+    if (live) out[order[self]] = (best0 + best1 + best2) / 3.0f;         // simple_knn.cu: mean of the three
 }
 
-template <class T>
-cudaError_t grab(T*& p, size_t count, cudaError_t prev) {
-    p = nullptr;
-    if (prev != cudaSuccess) return prev;
-    return cudaMalloc((void**)&p, (count > 0 ? count : 1) * sizeof(T));
+// The scratch of a call, carved out of one piece of memory.
+struct KnnScratch {
+    unsigned *bounds, *vals_in, *vals_out;
+    void *keys_in, *keys_out;          // 32 or 64 bits each, see wide_keys
+    float4* sorted;
+    KnnTree tree;
+    unsigned char* temp;
+    size_t temp_bytes, bytes;
+};
+
+template <class Key>
+cudaError_t sort_keys(KnnScratch& w, int n, int bits, cudaStream_t s) {
+    return cub::DeviceRadixSort::SortPairs(w.temp, w.temp_bytes, (const Key*)w.keys_in, (Key*)w.keys_out, w.vals_in, w.vals_out, n, 0,
+                                           bits, s);
+}
+cudaError_t sort_points(KnnScratch& w, int n, cudaStream_t s) {
+    return wide_keys(n) ? sort_keys<uint64_t>(w, n, 48, s) : sort_keys<uint32_t>(w, n, 30, s);
+}
+
+cudaError_t plan_scratch(int n, unsigned char* base, KnnScratch& w) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) -> unsigned char* {
+        unsigned char* p = base + at;
+        at += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    const size_t N = (size_t)n;
+    w.tree.leaf.count = (n + 31) / 32;
+    w.tree.mid.count = (w.tree.leaf.count + 31) / 32;
+    w.tree.top.count = (w.tree.mid.count + 31) / 32;
+    w.bounds = (unsigned*)take(6 * sizeof(unsigned));
+    const size_t key = wide_keys(n) ? 8 : 4;
+    w.keys_in = take(key * N); w.keys_out = take(key * N);
+    w.vals_in = (unsigned*)take(4 * N); w.vals_out = (unsigned*)take(4 * N);
+    w.sorted = (float4*)take(sizeof(float4) * 32 * (size_t)w.tree.leaf.count);
+    for (KnnLevel* l : {&w.tree.leaf, &w.tree.mid, &w.tree.top}) {
+        l->lo = (float4*)take(sizeof(float4) * (size_t)l->count);
+        l->hi = (float4*)take(sizeof(float4) * (size_t)l->count);
+    }
+    w.temp = nullptr;
+    w.temp_bytes = 0;
+    cudaError_t e = sort_points(w, n, (cudaStream_t)0);                   // size query
+    w.temp = take(w.temp_bytes);
+    w.bytes = at;
+    return e;
+}
+
+cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaStream_t s) {
+    const int tb = 256;
+    cudaError_t e = cudaMemsetAsync(w.bounds, 0, 6 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    note_launch(), knn_bounds_kernel<<<std::min((n + tb - 1) / tb, 592), tb, 0, s>>>(points, n, w.bounds);
+    if (wide_keys(n)) note_launch(), knn_keys_kernel<uint64_t><<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
+    else note_launch(), knn_keys_kernel<uint32_t><<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
+    e = sort_points(w, n, s);
+    if (e != cudaSuccess) return e;
+    note_launch(), knn_gather_kernel<<<w.tree.mid.count, 1024, 0, s>>>(points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
+    note_launch(), knn_upper_kernel<<<(w.tree.top.count + 7) / 8, 256, 0, s>>>(w.tree.mid, w.tree.top);
+    note_launch(), knn_query_kernel<<<(w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps, kKnnWarps * 32, 0, s>>>(w.sorted, w.vals_out, n,
+                                                                                                               w.tree, out);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -187,6 +297,26 @@ cudaError_t grab(T*& p, size_t count, cudaError_t prev) {
 
 using namespace rgx;
 
+extern "C" RGX_API size_t rgx_knn_scratch_bytes(int n) {
+    KnnScratch w;
+    return n > 0 && n <= (1 << 30) && plan_scratch(n, nullptr, w) == cudaSuccess ? w.bytes : 0;
+}
+
+extern "C" RGX_API int rgx_knn_mean_dist2_scratch(int device, const float* points, int n, float* mean_dist2, void* scratch,
+                                                  size_t scratch_bytes, rgx_stream stream) {
+    if (n < 0 || (n > 0 && (!points || !mean_dist2 || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 255u)))) return RGX_E_INVALID;
+    if (n > (1 << 30)) return RGX_E_TOO_LARGE;
+    if (n == 0) return RGX_OK;
+    DeviceGuard guard(device);
+    if (!guard.ok) { (void)cudaGetLastError(); return RGX_E_CUDA; }
+    KnnScratch w;
+    cudaError_t e = plan_scratch(n, (unsigned char*)scratch, w);
+    if (e == cudaSuccess && w.bytes > scratch_bytes) return RGX_E_INVALID;
+    if (e == cudaSuccess) e = run_knn(points, n, mean_dist2, w, (cudaStream_t)stream);
+    if (e != cudaSuccess) { (void)cudaGetLastError(); return RGX_E_CUDA; }
+    return RGX_OK;
+}
+
 extern "C" RGX_API int rgx_knn_mean_dist2(int device, const float* points, int n, float* mean_dist2, rgx_stream stream) {
     if (n < 0 || (n > 0 && (!points || !mean_dist2))) return RGX_E_INVALID;
     if (n > (1 << 30)) return RGX_E_TOO_LARGE;
@@ -194,35 +324,12 @@ extern "C" RGX_API int rgx_knn_mean_dist2(int device, const float* points, int n
     DeviceGuard guard(device);
     if (!guard.ok) { (void)cudaGetLastError(); return RGX_E_CUDA; }
     cudaStream_t s = (cudaStream_t)stream;
-    const int n_pad = ((n + 1023) / 1024) * 1024;
-    const int n_boxes = n_pad / 32, n_upper = n_boxes / 32;
-    int* bounds; unsigned *keys_in, *keys_out, *vals_in, *vals_out; float4 *sorted, *box_lo, *box_hi, *up_lo, *up_hi;
-    unsigned char* temp;
-    size_t temp_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, (const unsigned*)nullptr, (unsigned*)nullptr, (const unsigned*)nullptr,
-                                    (unsigned*)nullptr, n, 0, 30, s);
-    cudaError_t e = cudaSuccess;
-    e = grab(bounds, 6, e); e = grab(keys_in, n, e); e = grab(keys_out, n, e); e = grab(vals_in, n, e); e = grab(vals_out, n, e);
-    e = grab(sorted, n_pad, e); e = grab(box_lo, n_boxes, e); e = grab(box_hi, n_boxes, e); e = grab(up_lo, n_upper, e);
-    e = grab(up_hi, n_upper, e); e = grab(temp, temp_bytes, e);
-    if (e == cudaSuccess) {
-        const int tb = 256;
-        note_launch(), knn_init_kernel<<<1, 32, 0, s>>>(bounds);
-        note_launch(), knn_bounds_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, bounds);
-        note_launch(), knn_keys_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, bounds, keys_in, vals_in);
-        e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_in, keys_out, vals_in, vals_out, n, 0, 30, s);
-        if (e == cudaSuccess) {
-            note_launch(), knn_gather_kernel<<<(n_pad + tb - 1) / tb, tb, 0, s>>>(points, n, n_pad, vals_out, sorted, box_lo, box_hi);
-            note_launch(), knn_upper_kernel<<<(n_upper * 32 + tb - 1) / tb, tb, 0, s>>>(box_lo, box_hi, n_boxes, up_lo, up_hi);
-            note_launch(), knn_query_kernel<<<(n_boxes * 32 + tb - 1) / tb, tb, 0, s>>>(sorted, vals_out, n, n_boxes, n_upper, box_lo, box_hi,
-                                                                      up_lo, up_hi, mean_dist2);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);       // the scratch arrays are freed below
-    }
-    void* all[] = {bounds, keys_in, keys_out, vals_in, vals_out, sorted, box_lo, box_hi, up_lo, up_hi, temp};
-    for (void* p : all)
-        if (p) cudaFree(p);
+    void* scratch = nullptr;
+    const size_t bytes = rgx_knn_scratch_bytes(n);
+    cudaError_t e = bytes ? cudaMalloc(&scratch, bytes) : cudaErrorUnknown;
     if (e != cudaSuccess) { (void)cudaGetLastError(); return RGX_E_CUDA; }
-    return RGX_OK;
+    int rc = rgx_knn_mean_dist2_scratch(device, points, n, mean_dist2, scratch, bytes, stream);
+    if (rc == RGX_OK && cudaStreamSynchronize(s) != cudaSuccess) { (void)cudaGetLastError(); rc = RGX_E_CUDA; }   // the scratch is freed below
+    cudaFree(scratch);
+    return rc;
 }
