@@ -241,6 +241,56 @@ RGX_API size_t rgx_knn_scratch_bytes(int n);
 RGX_API int rgx_knn_mean_dist2_scratch(int device, const float* points, int n, float* mean_dist2, void* scratch,
                                        size_t scratch_bytes, rgx_stream stream);
 
+/* The parameterisation of the Gaussians (classes/point_cloud.py:509-559): scales = exp(log_scales), quaternions =
+ * raw / |raw|, color [n,3,sh_coeffs] = (rgb [n,3], sh [n,3,sh_coeffs-1]) side by side, sharpness = softplus(raw) (identity
+ * above 20), lobe_axis = raw / |raw|.  quaternions and, with 16 coefficients, color and its gradient are 16-byte
+ * aligned; quaternions and lobe_axis may be NULL: not wanted.
+ * Needs no context; one launch. */
+typedef struct rgx_activation {
+    int32_t n, sh_coeffs, num_lobes;
+    const float *log_scales, *raw_quaternions, *rgb, *sh, *raw_sharpness, *raw_axis;
+    float *scales, *quaternions, *color, *sharpness, *lobe_axis;
+} rgx_activation;
+/* Gradients of the activated values (in; NULL: none) and of the parameters (out; NULL: not wanted). */
+typedef struct rgx_activation_grads {
+    const float *scales, *quaternions, *color, *sharpness, *lobe_axis;
+    float *log_scales, *raw_quaternions, *rgb, *sh, *raw_sharpness, *raw_axis;
+} rgx_activation_grads;
+RGX_API int rgx_activate(int device, const rgx_activation* a, rgx_stream stream);
+/* Of `a` the sizes, the raw values and scales are read. */
+RGX_API int rgx_activate_backward(int device, const rgx_activation* a, const rgx_activation_grads* g, rgx_stream stream);
+
+/* Image loss of the training loop (scripts/train.py:128-137): rays [h*fy, w*fx, 3] averaged to pixels, then
+ * loss[0] = (1 - lambda) mean|image - target| + lambda (1 - SSIM), target [3,h,w]; SSIM as utils/loss_utils.py:37-62
+ * (11-tap Gaussian window of sigma 1.5, zero padding, constants 0.01^2 and 0.03^2).  maps: NULL, or 9*w*h floats that
+ * the backward reads when lambda is not 0; scratch: rgx_image_loss_scratch_floats(w, h) floats, 8-byte aligned.  The backward writes
+ * grad_loss[0] * dloss/drays to grad_rays [h*fy, w*fx, 3]; loss and grad_loss are device pointers.  Sums are fp32 per tile
+ * of 32x32 pixels and double over tiles, in a fixed order. */
+RGX_API size_t rgx_image_loss_scratch_floats(int w, int h);
+RGX_API int rgx_image_loss(int device, const float* rays, const float* target, int w, int h, int fx, int fy, float lambda_ssim,
+                           float* maps, float* scratch, float* loss, rgx_stream stream);
+RGX_API int rgx_image_loss_backward(int device, const float* rays, const float* target, int w, int h, int fx, int fy,
+                                    float lambda_ssim, const float* maps, const float* grad_loss, float* grad_rays,
+                                    rgx_stream stream);
+
+/* Densification statistics (classes/point_cloud.py:468-485): norm_sum[i] += |grad_i| max(|position_i - eye|, 1) and
+ * count[i] += 1 where |grad_i| > 0; norm_sum NULL: only the count.  eye [3] is a device pointer. */
+RGX_API int rgx_gradient_stats(int device, int n, const float* positions, const float* grad, const float* eye,
+                               float* norm_sum, float* count, rgx_stream stream);
+
+/* One Adam step of up to RGX_ADAM_MAX tensors in one launch: m += (1-beta1)(g-m), v = beta2 v + (1-beta2) g^2,
+ * param -= step_size m / (sqrt(v) inv_root + eps), with step_size = lr / (1 - beta1^t) and inv_root =
+ * 1 / sqrt(1 - beta2^t).  `tensors` is a host array. */
+enum { RGX_ADAM_MAX = 16 };
+typedef struct rgx_adam_tensor {
+    float *param, *exp_avg, *exp_avg_sq;
+    const float* grad;
+    int64_t n;
+    float step_size, inv_root;
+} rgx_adam_tensor;
+RGX_API int rgx_adam_step(int device, const rgx_adam_tensor* tensors, int count, double beta1, double beta2, double eps,
+                          rgx_stream stream);
+
 /* Test hook (no counterpart in the reference): the workspace allocation that follows `nth` more successful
  * ones fails as if the device were out of memory, without touching the device (nth < 0 switches the hook
  * off).  After any failed allocation the call in progress returns RGX_E_CUDA, and the next call on the context

@@ -41,6 +41,25 @@ class Grads(C.Structure):
                 ("color_features", _fp), ("sg_features", _fp), ("sharpness", _fp), ("lobe_axis", _fp)]
 
 
+class Activation(C.Structure):
+    _fields_ = [("n", C.c_int32), ("sh_coeffs", C.c_int32), ("num_lobes", C.c_int32)] + [
+        (k, _fp) for k in ("log_scales", "raw_quaternions", "rgb", "sh", "raw_sharpness", "raw_axis",
+                           "scales", "quaternions", "color", "sharpness", "lobe_axis")]
+
+
+class ActivationGrads(C.Structure):
+    _fields_ = [(k, _fp) for k in ("scales", "quaternions", "color", "sharpness", "lobe_axis",
+                                   "log_scales", "raw_quaternions", "rgb", "sh", "raw_sharpness", "raw_axis")]
+
+
+class AdamTensor(C.Structure):
+    _fields_ = [("param", _fp), ("exp_avg", _fp), ("exp_avg_sq", _fp), ("grad", _fp), ("n", C.c_int64),
+                ("step_size", C.c_float), ("inv_root", C.c_float)]
+
+
+ADAM_MAX = 16
+
+
 class Counters(C.Structure):
     _fields_ = [(k, C.c_uint64) for k in ("rays", "slabs", "slabs_hit", "closest_queries", "hits", "pairs_inside",
                                           "overflow_slabs", "node_tests", "prim_tests", "ellipsoid_tests",
@@ -76,6 +95,14 @@ SYMBOLS = {
     "rgx_read_near_lists": (C.c_int, [C.c_void_p, C.POINTER(C.c_longlong)]),
     "rgx_measure_peaks": (C.c_int, [C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
     "rgx_knn_mean_dist2": (C.c_int, [C.c_int, _fp, C.c_int, _fp, C.c_void_p]),
+    "rgx_activate": (C.c_int, [C.c_int, C.POINTER(Activation), C.c_void_p]),
+    "rgx_activate_backward": (C.c_int, [C.c_int, C.POINTER(Activation), C.POINTER(ActivationGrads), C.c_void_p]),
+    "rgx_image_loss_scratch_floats": (C.c_size_t, [C.c_int, C.c_int]),
+    "rgx_image_loss": (C.c_int, [C.c_int, _fp, _fp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, _fp, _fp, _fp, C.c_void_p]),
+    "rgx_image_loss_backward": (C.c_int, [C.c_int, _fp, _fp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, _fp, _fp, _fp,
+                                          C.c_void_p]),
+    "rgx_gradient_stats": (C.c_int, [C.c_int, C.c_int, _fp, _fp, _fp, _fp, _fp, C.c_void_p]),
+    "rgx_adam_step": (C.c_int, [C.c_int, C.POINTER(AdamTensor), C.c_int, C.c_double, C.c_double, C.c_double, C.c_void_p]),
     "rgx_knn_scratch_bytes": (C.c_size_t, [C.c_int]),
     "rgx_knn_mean_dist2_scratch": (C.c_int, [C.c_int, _fp, C.c_int, _fp, _fp, C.c_size_t, C.c_void_p]),
     "rgx_reset_counters": (C.c_int, [C.c_void_p, C.c_void_p]),

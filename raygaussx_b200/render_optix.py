@@ -89,15 +89,17 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None or t.numel() == 0 else t.data_ptr()
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t      # a row slice of a larger buffer: the kernels load 16 bytes at a time (rgx.h)
+
+
 def _as_input(t: torch.Tensor, name: str) -> torch.Tensor:
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if t.dtype != torch.float32:
         raise ValueError(f"{name} must be float32, got {t.dtype}")
-    t = t.detach().contiguous()
-    if t.data_ptr() % 16:            # a row slice of a larger buffer: the kernels load 16 bytes at a time (rgx.h)
-        t = t.clone()
-    return t
+    return _aligned(t.detach())
 
 
 def camera_struct(cam, supersampling=(1, 1)) -> _Camera:

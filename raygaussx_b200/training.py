@@ -20,6 +20,7 @@ and ``num_sph_gauss``.  ``SimplePointCloud`` is a small one for tests and benchm
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 import random
 from types import SimpleNamespace
@@ -28,6 +29,7 @@ from typing import Callable, List, Optional
 import torch
 import torch.nn.functional as F
 
+from . import _lib
 from . import render_optix as r_ox
 from .inference import reduce_supersampling
 
@@ -79,6 +81,99 @@ def isotropy_loss(scales: torch.Tensor) -> torch.Tensor:
     return (torch.clamp(r, min=10) - 10).mean()
 
 
+# ----------------------------------------------------------------------------- the same on the device, fused (csrc/train.cu)
+def _stream(t: torch.Tensor):
+    return torch.cuda.current_stream(t.device).cuda_stream
+
+
+def _check(rc: int, what: str):
+    if rc != 0:
+        raise _lib.RgxError(rc, what + " failed")
+
+
+def _fusable(*tensors) -> bool:
+    """fp32 CUDA tensors of one device, contiguous: what the fused kernels take."""
+    dev = tensors[0].device
+    return all(t.is_cuda and t.device == dev and t.dtype == torch.float32 and t.is_contiguous() for t in tensors)
+
+
+class _ImageLoss(torch.autograd.Function):
+    """``(1 - l) L1 + l (1 - SSIM)`` of the supersampled rays ``[R, 3]`` against ``[3, H, W]``: one kernel and a small sum
+    forward, one kernel backward, in place of some hundred operators on images."""
+
+    @staticmethod
+    def forward(ctx, rays, target, width, height, factor, lambda_ssim):
+        lib, dev = _lib.lib(), rays.device
+        maps = torch.empty(9 * width * height, device=dev) if lambda_ssim != 0 and ctx.needs_input_grad[0] else None
+        scratch = torch.empty(int(lib.rgx_image_loss_scratch_floats(width, height)), device=dev)
+        loss = torch.empty((), device=dev)
+        _check(lib.rgx_image_loss(dev.index or 0, rays.data_ptr(), target.data_ptr(), width, height, factor[0], factor[1],
+                                  lambda_ssim, maps.data_ptr() if maps is not None else None, scratch.data_ptr(),
+                                  loss.data_ptr(), _stream(rays)), "rgx_image_loss")
+        ctx.args = (width, height, factor, lambda_ssim)
+        ctx.save_for_backward(rays, target, maps)
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad_loss):
+        rays, target, maps = ctx.saved_tensors
+        width, height, factor, lambda_ssim = ctx.args
+        grad = torch.empty_like(rays)
+        _check(_lib.lib().rgx_image_loss_backward(rays.device.index or 0, rays.data_ptr(), target.data_ptr(), width, height, factor[0],
+                                                  factor[1], lambda_ssim, maps.data_ptr() if maps is not None else None,
+                                                  grad_loss.contiguous().data_ptr(), grad.data_ptr(), _stream(rays)),
+               "rgx_image_loss_backward")
+        return grad, None, None, None, None, None
+
+
+def image_loss(rays, target, width: int, height: int, supersampling=(1, 1), lambda_ssim: float = 0.2):
+    """``(1 - l) L1 + l (1 - SSIM)`` of the rays' image (``scripts/train.py:128-137``): fused where the tensors allow it,
+    else composed of :func:`l1_loss` and :func:`ssim`."""
+    if _fusable(rays, target) and target.dim() == 3:
+        return _ImageLoss.apply(rays, target, int(width), int(height), (int(supersampling[0]), int(supersampling[1])),
+                                float(lambda_ssim))
+    image = reduce_supersampling(width, height, rays, supersampling).permute(2, 0, 1)
+    loss = (1.0 - lambda_ssim) * l1_loss(image, target)
+    return loss + lambda_ssim * (1.0 - ssim(image, target)) if lambda_ssim != 0 else loss
+
+
+class _Activate(torch.autograd.Function):
+    """Parameters -> the operator's inputs that are not parameters themselves (``rgx_activate``), one kernel each way."""
+
+    @staticmethod
+    def forward(ctx, log_scales, quaternions, rgb, sh, sharpness, axis, normalize_q, normalize_axis):
+        n, g = log_scales.shape[0], sharpness.shape[1]
+        a = _lib.Activation()
+        a.n, a.sh_coeffs, a.num_lobes = n, 1 + sh.shape[2], g
+        scales, color = torch.empty_like(log_scales), torch.empty(n, 3, a.sh_coeffs, device=rgb.device)
+        sharp = torch.empty_like(sharpness)
+        quats = torch.empty_like(quaternions) if normalize_q else None
+        ax = torch.empty_like(axis) if normalize_axis else None
+        a.log_scales, a.raw_quaternions, a.rgb, a.sh = (r_ox._ptr(t) for t in (log_scales, quaternions, rgb, sh))
+        a.raw_sharpness, a.raw_axis = r_ox._ptr(sharpness), r_ox._ptr(axis)
+        a.scales, a.quaternions, a.color, a.sharpness, a.lobe_axis = (r_ox._ptr(t) for t in (scales, quats, color, sharp, ax))
+        _check(_lib.lib().rgx_activate(rgb.device.index or 0, C.byref(a), _stream(rgb)), "rgx_activate")
+        ctx.sizes = (a.n, a.sh_coeffs, a.num_lobes)
+        ctx.save_for_backward(scales, quaternions, sharpness, axis, rgb, sh)
+        ctx.set_materialize_grads(False)
+        return scales, quats, color, sharp, ax
+
+    @staticmethod
+    def backward(ctx, d_scales, d_quats, d_color, d_sharp, d_axis):
+        scales, quaternions, sharpness, axis, rgb, sh = ctx.saved_tensors
+        a, g = _lib.Activation(), _lib.ActivationGrads()
+        a.n, a.sh_coeffs, a.num_lobes = ctx.sizes
+        a.raw_quaternions, a.raw_sharpness, a.raw_axis, a.scales = (r_ox._ptr(t) for t in (quaternions, sharpness, axis, scales))
+        given = [r_ox._aligned(t) if t is not None else None for t in (d_scales, d_quats, d_color, d_sharp, d_axis)]
+        g.scales, g.quaternions, g.color, g.sharpness, g.lobe_axis = (r_ox._ptr(t) for t in given)
+        need = ctx.needs_input_grad
+        wanted = [torch.empty_like(like) if need[i] and given[src] is not None else None for i, src, like in (
+            (0, 0, scales), (1, 1, quaternions), (2, 2, rgb), (3, 2, sh), (4, 3, sharpness), (5, 4, axis))]
+        g.log_scales, g.raw_quaternions, g.rgb, g.sh, g.raw_sharpness, g.raw_axis = (r_ox._ptr(t) for t in wanted)
+        _check(_lib.lib().rgx_activate_backward(rgb.device.index or 0, C.byref(a), C.byref(g), _stream(rgb)), "rgx_activate_backward")
+        return (*wanted, None, None)
+
+
 # ----------------------------------------------------------------------------- the iteration
 class AccumulationSchedule:
     """Gradient accumulation of ``scripts/train.py:77-85,150-161``: from ``accum_start`` on, ``accum_steps``
@@ -124,12 +219,9 @@ def training_iteration(pointcloud, viewpoint_cam, config, iteration: int, schedu
                                       normalized_lobe_axis=not t.normalize_lobe_axis)
     image = r_ox.RenderOptixFunction.apply(positions, scales, quaternions, densities, color_features,
                                            sph_gauss_features, bandwidth_sharpness, lobe_axis, settings)
-    image_mean = reduce_supersampling(viewpoint_cam.image_width, viewpoint_cam.image_height, image, supersampling)
-    image_mean = image_mean.permute(2, 0, 1)
-    loss = (1.0 - t.lambda_ssim) * l1_loss(image_mean, gt_image)
-    if t.lambda_ssim != 0:
-        loss = loss + t.lambda_ssim * (1.0 - ssim(image_mean, gt_image))
-    loss = loss + t.lambda_iso * isotropy_loss(scales)
+    loss = image_loss(image, gt_image, viewpoint_cam.image_width, viewpoint_cam.image_height, supersampling, t.lambda_ssim)
+    if t.lambda_iso != 0:
+        loss = loss + t.lambda_iso * isotropy_loss(scales)
     if use_accum:
         loss = loss / float(schedule.accum_steps)
     loss.backward()
@@ -152,11 +244,48 @@ def training_iteration(pointcloud, viewpoint_cam, config, iteration: int, schedu
 
 
 # ----------------------------------------------------------------------------- a small point cloud
+class _Adam(torch.optim.Adam):
+    """``torch.optim.Adam`` whose step is one kernel over all tensors (``rgx_adam_step``) where the parameters are contiguous
+    fp32 CUDA tensors and nothing but the plain algorithm is asked for; state and results are those of the base class."""
+
+    _PLAIN = dict(weight_decay=0, amsgrad=False, maximize=False, capturable=False, differentiable=False, fused=None)
+
+    @torch.no_grad()
+    def step(self, closure=None):
+        work = [(p, grp) for grp in self.param_groups for p in grp["params"] if p.grad is not None]
+        if closure is not None or not work or not all(
+                all(grp[k] == v or (k == "fused" and not grp[k]) for k, v in self._PLAIN.items())
+                and not torch.is_tensor(grp["lr"]) for _, grp in work) or not all(
+                not p.grad.is_sparse and _fusable(p, p.grad) and p.device == work[0][0].device for p, _ in work):
+            return super().step(closure)
+        batches = {}
+        for p, grp in work:
+            st = self.state[p]
+            if len(st) == 0:
+                st["step"] = torch.tensor(0.0)
+                st["exp_avg"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+                st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.preserve_format)
+            st["step"] += 1
+            t = st["step"].item()                        # a host tensor
+            beta1, beta2 = grp["betas"]
+            batches.setdefault((beta1, beta2, grp["eps"]), []).append(
+                (p.data_ptr(), st["exp_avg"].data_ptr(), st["exp_avg_sq"].data_ptr(), p.grad.data_ptr(), p.numel(),
+                 grp["lr"] / (1 - beta1 ** t), 1.0 / math.sqrt(1 - beta2 ** t)))
+        dev = work[0][0].device
+        for (beta1, beta2, eps), rows in batches.items():
+            for lo in range(0, len(rows), _lib.ADAM_MAX):
+                part = rows[lo:lo + _lib.ADAM_MAX]
+                table = (_lib.AdamTensor * len(part))(*part)
+                _check(_lib.lib().rgx_adam_step(dev.index or 0, table, len(part), beta1, beta2, eps, _stream(work[0][0])),
+                       "rgx_adam_step")
+        torch.autograd.graph.increment_version([p for p, _ in work])       # written to behind torch's back
+
+
 class _Optimizers:
     """The part of the reference's optimizer manager the loop uses (``zero_grad``, ``step``, ``get_lrs``)."""
 
     def __init__(self, groups):
-        self.optimizer = torch.optim.Adam(groups, eps=1e-15)
+        self.optimizer = _Adam(groups, eps=1e-15)
 
     def zero_grad(self):
         self.optimizer.zero_grad(set_to_none=True)
@@ -220,6 +349,12 @@ class SimplePointCloud:
         return self.lobe_axis / torch.norm(self.lobe_axis, dim=2)[:, :, None]
 
     def get_data(self, normalized_quaternion=True, normalized_lobe_axis=True):
+        raw = (self.scales, self.quaternions, self.rgb, self.spherical_harmonics, self.bandwidth_sharpness, self.lobe_axis)
+        if _fusable(*raw):
+            with_axis = normalized_lobe_axis and self.lobe_axis.numel() > 0
+            scales, q, color, sharp, a = _Activate.apply(*raw, normalized_quaternion, with_axis)
+            return (self.positions, scales, q if normalized_quaternion else self.quaternions, self.get_density(), color,
+                    self.sph_gauss_features, sharp, a if with_axis else self.lobe_axis)
         q = self.get_normalized_quaternion() if normalized_quaternion else self.quaternions
         a = self.get_normalized_lobe_axis() if normalized_lobe_axis else self.lobe_axis
         return (self.positions, self.get_scale(), q, self.get_density(), self.get_color_features(),
@@ -235,6 +370,12 @@ class SimplePointCloud:
 
     @torch.no_grad()
     def accumulate_gradient(self, grad, camera):
+        eye = camera.camera_center
+        if _fusable(self.positions, grad, eye, self.xyz_gradient_accum_norm, self.num_accum):
+            _check(_lib.lib().rgx_gradient_stats(grad.device.index or 0, grad.shape[0], self.positions.data_ptr(), grad.data_ptr(),
+                                                 eye.data_ptr(), self.xyz_gradient_accum_norm.data_ptr(),
+                                                 self.num_accum.data_ptr(), _stream(grad)), "rgx_gradient_stats")
+            return
         dist = torch.clamp(torch.norm(self.positions - camera.camera_center[None, :], dim=1), min=1.0)
         norm = torch.norm(grad, dim=1)
         self.xyz_gradient_accum_norm += norm * dist
@@ -242,6 +383,10 @@ class SimplePointCloud:
 
     @torch.no_grad()
     def accumulate_gradient_gaussians_not_visible(self, grad):
+        if _fusable(grad, self.num_accum_gnv):
+            _check(_lib.lib().rgx_gradient_stats(grad.device.index or 0, grad.shape[0], None, grad.data_ptr(), None, None,
+                                                 self.num_accum_gnv.data_ptr(), _stream(grad)), "rgx_gradient_stats")
+            return
         self.num_accum_gnv += torch.where(torch.norm(grad, dim=1) > 0, 1.0, 0.0)
 
 
