@@ -306,7 +306,8 @@ RGX_API int rgx_debug_cap_recording(rgx_ctx* ctx, long long ints);
  * RGX_FLAG_SAVE_HITS, no counting) and whose view has at least `min_pairs_per_ray` (tile, Gaussian) pairs per
  * ray -- a dense scene whose rays end long before they have seen most of them -- sorts and marches only the pairs
  * that begin nearest to the eye first, about `budget_per_ray` per ray, and sorts the rest only for the tiles in
- * which some ray got further; the image is bit for bit that of the one-depth march.  Defaults 48 and 16;
+ * which some ray got further; the image is bit for bit that of the one-depth march.  Defaults 12 and 5
+ * (the budget doubles after a view in which more than an eighth of the rays went further);
  * min_pairs_per_ray < 0 switches the path off, 0 forces it; budget_per_ray = 0 keeps the current value.
  * rgx_read_two_depth returns and clears (pairs emitted, pairs sorted for the first depth, rays that went further,
  * pairs sorted for the second depth) of the latest such forward, zeros if there was none. */

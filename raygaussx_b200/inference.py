@@ -50,7 +50,10 @@ def reduce_supersampling(target_width, target_height, ray_colors, factor):
 
 
 def _tensors(pointcloud):
-    """The eight renderer inputs, as scripts/test.py:62-67 gathers them."""
+    """The eight renderer inputs, as scripts/test.py:62-67 gathers them (all at once where the cloud can do that)."""
+    at_once = getattr(pointcloud, "renderer_inputs", None)
+    if at_once is not None:
+        return list(at_once())
     return [pointcloud.positions, pointcloud.get_scale(), pointcloud.get_normalized_quaternion(),
             pointcloud.get_density(), pointcloud.get_color_features(), pointcloud.sph_gauss_features,
             pointcloud.get_bandwidth_sharpness(), pointcloud.get_normalized_lobe_axis()]
@@ -78,9 +81,45 @@ class _Settings:
         self.transmittance_eps = ro.TRANSMITTANCE_EPSILON
 
 
+class _HostCopies:
+    """Device tensors to numpy arrays of their own, by way of a few pinned buffers and a stream of their own: the copy and what the
+    host does with an image overlap the rendering of the next one."""
+
+    def __init__(self):
+        self._free = {}          # (shape, dtype) -> pinned buffers not in use
+        self._stream = None
+
+    def start(self, t: torch.Tensor):
+        """Begins the copy of ``t`` as it is at this point of the current stream."""
+        if not t.is_cuda:
+            return t.contiguous(), None, None
+        if self._stream is None:
+            self._stream = torch.cuda.Stream(t.device)
+        t = t.contiguous()
+        key = (tuple(t.shape), t.dtype)
+        buffers = self._free.setdefault(key, [])
+        buf = buffers.pop() if buffers else torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
+        self._stream.wait_stream(torch.cuda.current_stream(t.device))
+        with torch.cuda.stream(self._stream):
+            buf.copy_(t, non_blocking=True)
+            done = torch.cuda.Event()
+            done.record(self._stream)
+        t.record_stream(self._stream)
+        return buf, done, key
+
+    def finish(self, handle) -> np.ndarray:
+        buf, done, key = handle
+        if done is None:
+            return buf.numpy()
+        done.synchronize()
+        out = buf.numpy().copy()
+        self._free[key].append(buf)
+        return out
+
+
 def _render_list(tensors_of, cam_list, max_prim_slice, dt_step, supersampling, white_background, dynamic_sampling,
                  rebuild_each):
-    """Renders every camera; yields (camera, rays [R,3] on the device, milliseconds)."""
+    """Enqueues every camera; yields (camera, rays [R,3] on the device, start and end event of its rendering)."""
     renderer = None
     tensors = None
     for cam in cam_list:
@@ -95,8 +134,22 @@ def _render_list(tensors_of, cam_list, max_prim_slice, dt_step, supersampling, w
         start.record()
         rays, _, _ = renderer.forward(*tensors, cs, march)
         end.record()
-        torch.cuda.synchronize()
-        yield cam, rays, start.elapsed_time(end)
+        yield cam, rays, start, end
+
+
+def _one_behind(jobs):
+    """``job()`` of every job, each called once the next job has been made (and its work enqueued)."""
+    waiting = None
+    for job in jobs:
+        if waiting is not None:
+            waiting()
+        waiting = job
+    if waiting is not None:
+        waiting()
+
+
+def _clipped_image(cam, rays, supersampling):
+    return reduce_supersampling(cam.image_width, cam.image_height, rays, supersampling).clamp_(0, 1)
 
 
 def inference(hit_prim_idx, pointcloud, cam_list, max_prim_slice, dt_step, rnd_sample, supersampling,
@@ -107,15 +160,24 @@ def inference(hit_prim_idx, pointcloud, cam_list, max_prim_slice, dt_step, rnd_s
     with torch.no_grad():
         psnr_list, gt_list, img_list, times = [], [], [], []
         tensors_of = (lambda cam: _culled(pointcloud, cam)) if culling else (lambda cam: _tensors(pointcloud))
-        for cam, rays, ms in _render_list(tensors_of, cam_list, max_prim_slice, dt_step, supersampling,
-                                          white_background, dynamic_sampling, rebuild_each=culling):
-            times.append(ms)
-            image = reduce_supersampling(cam.image_width, cam.image_height, rays, supersampling)
-            image_np = image.detach().cpu().numpy().clip(0, 1)
-            gt_np = cam.original_image.permute(1, 2, 0).detach().cpu().numpy().clip(0, 1)
-            psnr_list.append(PSNR(image_np, gt_np))
-            gt_list.append(gt_np)
-            img_list.append(image_np)
+        copies = _HostCopies()
+
+        def jobs():
+            for cam, rays, start, end in _render_list(tensors_of, cam_list, max_prim_slice, dt_step, supersampling,
+                                                      white_background, dynamic_sampling, rebuild_each=culling):
+                image = _clipped_image(cam, rays, supersampling)
+                gt = cam.original_image.permute(1, 2, 0).detach().clamp(0, 1)
+                mse = (image - gt.to(image.device)).double().square().mean().reshape(1)
+                handles = [copies.start(t) for t in (image, gt, mse)]
+
+                def finish(handles=handles, start=start, end=end):
+                    image_np, gt_np, mse_np = (copies.finish(h) for h in handles)
+                    times.append(start.elapsed_time(end))
+                    psnr_list.append(100 if mse_np[0] == 0 else 20 * log10(1.0 / sqrt(mse_np[0])))
+                    gt_list.append(gt_np)
+                    img_list.append(image_np)
+                yield finish
+        _one_behind(jobs())
         return psnr_list, gt_list, img_list, float(np.mean(times)) if times else 0.0
 
 
@@ -125,11 +187,18 @@ def render(pointcloud, cam_list, max_prim_slice, dt_step, rnd_sample, supersampl
     ``[H, W, 3]`` numpy images clipped to [0, 1]."""
     with torch.no_grad():
         images, times = [], []
-        for cam, rays, ms in _render_list(lambda cam: _tensors(pointcloud), cam_list, max_prim_slice, dt_step,
-                                          supersampling, white_background, dynamic_sampling, rebuild_each=False):
-            times.append(ms)
-            image = reduce_supersampling(cam.image_width, cam.image_height, rays, supersampling)
-            images.append(image.detach().cpu().numpy().clip(0, 1))
+        copies = _HostCopies()
+
+        def jobs():
+            for cam, rays, start, end in _render_list(lambda cam: _tensors(pointcloud), cam_list, max_prim_slice, dt_step,
+                                                      supersampling, white_background, dynamic_sampling, rebuild_each=False):
+                handle = copies.start(_clipped_image(cam, rays, supersampling))
+
+                def finish(handle=handle, start=start, end=end):
+                    images.append(copies.finish(handle))
+                    times.append(start.elapsed_time(end))
+                yield finish
+        _one_behind(jobs())
         if times:
             print("Mean time", np.mean(times))
         return images

@@ -360,6 +360,10 @@ class SimplePointCloud:
         return (self.positions, self.get_scale(), q, self.get_density(), self.get_color_features(),
                 self.sph_gauss_features, self.get_bandwidth_sharpness(), a)
 
+    def renderer_inputs(self):
+        """The operator's eight inputs, activated (``inference.py``)."""
+        return self.get_data()
+
     # statistics of classes/point_cloud.py:468-485
     @torch.no_grad()
     def reset_gradient_accum(self):
