@@ -98,6 +98,7 @@ enum {
                                     sums (in the context's workspace, about 3 KB per ray) so that a backward for
                                     the same view replays them instead of searching and evaluating again; the
                                     backward falls back to searching where nothing was kept */
+    RGX_FLAG_GRADS_CLEAR = 64,   /* backward: the gradient tensors are already zero (a caller clears one buffer that holds them all) */
     RGX_FLAG_PER_RAY_SEARCH = 16 /* search the hierarchy once per ray and slab instead of sliding along the view's
                                     per-tile lists (same hits; the general path, kept for validation and used by
                                     rgx_forward_static) */

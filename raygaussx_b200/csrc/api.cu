@@ -36,6 +36,7 @@ struct rgx_ctx {
     float2 *bx = nullptr, *by = nullptr, *bz = nullptr;
     float4 *g0 = nullptr, *g1 = nullptr, *g2 = nullptr, *quat = nullptr, *sdens = nullptr, *rgba = nullptr;
     float4* grad_rows = nullptr;
+    bool build_scratch_clear = false; // bounds and refit_counters are zero (every build leaves them so)
     bool grad_rows_clear = false;     // every row is zero (the gradient kernel clears what it reads); false after a failed backward
     unsigned char* listed = nullptr; int listed_cap = 0;   // per sorted slot: on some list of the view whose colours rgba holds
     unsigned long long listed_serial = 0;                  // the colour evaluation `listed` belongs to (0: none)
@@ -59,9 +60,10 @@ struct rgx_ctx {
     size_t bin_pair_cap = 0, bin_ent_cap = 0, bin_cub_cap = 0;
     uint64_t *bin_keys_in = nullptr, *bin_keys_out = nullptr;
     uint32_t *bin_vals_in = nullptr, *bin_vals_out = nullptr;
-    int *tile_first = nullptr, *tile_last = nullptr, *tile_cnt = nullptr, *tile_pcnt = nullptr, *tile_pbegin = nullptr;
+    int *tile_cnt = nullptr, *tile_pbegin = nullptr;
+    // what an emission starts from zero, in one piece cleared by one memset (see ZeroedBins)
+    unsigned char* bin_zero = nullptr; size_t bin_zero_cap = 0;
     int *tile_iota = nullptr, *tile_cnt_sorted = nullptr, *tile_order = nullptr;
-    int* tile_unrecorded = nullptr;   // per tile: some ray of the latest recording forward could not be recorded
     int* ent_id = nullptr;
     float2 *ent_range = nullptr, *ent_blk = nullptr;
     float4* tile_dir = nullptr;
@@ -69,16 +71,17 @@ struct rgx_ctx {
     int* big_slot = nullptr;
     uint2* big_rect = nullptr;
     int big_cap = 0, sm_count = 0;
-    unsigned long long* bin_total_dev = nullptr;
-    unsigned long long* bin_total_host = nullptr;      // pinned
+    BinResult* bin_result_host = nullptr;              // pinned; the device's copy heads bin_zero
     // two-depth lists of forward-only views (binning.cu, march_lists.cu HZ variant)
-    int *tile_more = nullptr, *tile_resume = nullptr; int hz_tiles_cap = 0;
+    int *tile_more = nullptr;      // in bin_zero
+    int *tile_resume = nullptr; int hz_tiles_cap = 0;
     float4* hz_state = nullptr; long long hz_state_cap = 0;
     unsigned long long* hz_scalars = nullptr; unsigned long long* hz_scalars_host = nullptr;   // [0] selected pairs, [1] stopped rays (low 32 bits)
     // when to use them, how deep the first phase goes.  With the march by patches a view's time is largely that of its lists:
     // 7 M needles 34.8 ms (three frames) at 16 pairs per ray, 28.9 at 8, 26.7 at 5, 26.1 at 4; from 12 pairs per ray in the view on
     // it pays: 1 M Gaussians at 640x360 2.15 -> 1.63 ms, 3 M at 1256x828 8.2 -> 5.5 per frame.
     int hz_min_pairs_per_ray = 12, hz_budget_per_ray = 5;
+    int hz_budget_now = 5;         // doubled where rays go further than the first depth; back to the above with a set of another size
     long long hz_last[4] = {0, 0, 0, 0};                                          // pairs of the view (estimate), sorted in phase 1, rays stopped, sorted in phase 2
     // what the current lists were made for
     int last_pairs = 0;
@@ -100,11 +103,8 @@ struct rgx_ctx {
     long long beyond_kept = 0, beyond_lists_rays = 0; int beyond_budget = 0;   // of the lists that march used
     long long tape_beyond_rays = 0;              // rays of the current recording that went beyond (they are not recorded)
     long long near_min_pairs = 1ll << 21;     // views with fewer (estimated) pairs get complete lists
-    double near_ratio = 2.0;                  // estimated pairs (tile rectangles) per pair kept up to the horizon, from the latest such view
-    HorizonPick* near_pick = nullptr; HorizonPick* near_pick_host = nullptr;     // host copy pinned
-    unsigned long long* near_hist = nullptr;
+    double near_ratio = 2.0, hz_ratio = 2.0;  // estimated pairs (tile rectangles) per pair kept up to the horizon, from the latest such view (hz_: in the first depth)
     uint2* g_rect = nullptr; unsigned int* g_code = nullptr; int* kept_slot = nullptr; int g_rect_cap = 0;
-    int* tile_diff = nullptr; size_t tile_diff_cap = 0;
     unsigned long long lists_build_id = 0;
     rgx_camera lists_cam{};
     int lists_row_begin = 0, lists_row_end = 0;
@@ -112,7 +112,9 @@ struct rgx_ctx {
     // tape of forward hits for the backward (RGX_FLAG_SAVE_HITS)
     int* tape = nullptr;
     long long tape_cap = 0;
-    unsigned long long* tape_used = nullptr;
+    // [0] ints of the recording reserved, [4] rays that went beyond the horizon, [8 ...) per tile: some ray of the latest recording
+    // forward could not be recorded; cleared by one memset
+    unsigned long long* tape_used = nullptr; long long tape_used_cap = 0;
     unsigned long long* tape_used_host = nullptr;   // pinned; refreshed asynchronously after every recording forward
     long long* ray_head = nullptr;                  // first chunk of every patch, then a byte per ray: not recorded
     long long ray_head_cap = 0;
@@ -122,7 +124,8 @@ struct rgx_ctx {
     rgx_camera tape_cam{};
     rgx_march tape_march{};            // the parameters that shape the slabs of the recording
     int tape_row_begin = 0, tape_row_end = 0;
-    int* tape_tile_order = nullptr; int tape_order_cap = 0;   // order of the recording forward's CTAs, kept for the replay
+    int* tape_tile_order = nullptr; int tape_order_cap = 0;   // a second buffer for the order of the tiles: lists are made into the one ...
+    const int* tape_order = nullptr;                          // ... that the latest recording's replay does not need
     // lists of the view announced by rgx_hint_next_view, made on a stream of the context's own while the backward replays
     cudaStream_t side = nullptr;
     cudaEvent_t ev_main = nullptr, ev_lists = nullptr;
@@ -190,14 +193,12 @@ void release_workspace(rgx_ctx* ctx) {
                      (void**)&ctx->grad_rows, (void**)&ctx->hk, (void**)&ctx->refit_counters, (void**)&ctx->cub_temp,
                      (void**)&ctx->bounds, (void**)&ctx->box, (void**)&ctx->counters, (void**)&ctx->next_unit, (void**)&ctx->bin_keys_in,
                      (void**)&ctx->bin_keys_out, (void**)&ctx->bin_vals_in, (void**)&ctx->bin_vals_out,
-                     (void**)&ctx->tile_first, (void**)&ctx->tile_last, (void**)&ctx->tile_cnt, (void**)&ctx->tile_pcnt,
-                     (void**)&ctx->tile_pbegin, (void**)&ctx->ent_id, (void**)&ctx->ent_range, (void**)&ctx->ent_blk,
-                     (void**)&ctx->bin_cub, (void**)&ctx->bin_total_dev, (void**)&ctx->tape, (void**)&ctx->tape_used,
+                     (void**)&ctx->tile_cnt, (void**)&ctx->tile_pbegin, (void**)&ctx->ent_id, (void**)&ctx->ent_range, (void**)&ctx->ent_blk,
+                     (void**)&ctx->bin_cub, (void**)&ctx->bin_zero, (void**)&ctx->tape, (void**)&ctx->tape_used,
                      (void**)&ctx->ray_head, (void**)&ctx->tile_dir, (void**)&ctx->tile_iota,
                      (void**)&ctx->tile_cnt_sorted, (void**)&ctx->tile_order, (void**)&ctx->big_slot,
-                     (void**)&ctx->big_rect, (void**)&ctx->tile_unrecorded, (void**)&ctx->tile_more, (void**)&ctx->tile_resume,
-                     (void**)&ctx->hz_state, (void**)&ctx->hz_scalars, (void**)&ctx->tape_tile_order, (void**)&ctx->near_pick,
-                     (void**)&ctx->near_hist, (void**)&ctx->g_rect, (void**)&ctx->g_code, (void**)&ctx->kept_slot, (void**)&ctx->tile_diff,
+                     (void**)&ctx->big_rect, (void**)&ctx->tile_resume,
+                     (void**)&ctx->hz_state, (void**)&ctx->hz_scalars, (void**)&ctx->tape_tile_order, (void**)&ctx->g_rect, (void**)&ctx->g_code, (void**)&ctx->kept_slot,
                      (void**)&ctx->listed, (void**)&ctx->hz_rays};
     for (void** p : ptrs) {
         if (*p) cudaFree(*p);
@@ -216,7 +217,8 @@ void release_workspace(rgx_ctx* ctx) {
     ctx->lists_event_set = false;
     ctx->hint_set = false;
     ctx->hz_tiles_cap = 0; ctx->hz_state_cap = 0;
-    ctx->g_rect_cap = 0; ctx->tile_diff_cap = 0; ctx->listed_cap = 0; ctx->listed_serial = 0;
+    ctx->g_rect_cap = 0; ctx->bin_zero_cap = 0; ctx->tile_more = nullptr; ctx->tape_used_cap = 0; ctx->tape_order = nullptr;
+    ctx->build_scratch_clear = false; ctx->listed_cap = 0; ctx->listed_serial = 0;
     ctx->hz_rays_cap = 0; ctx->beyond_pending = false;
     ctx->grad_rows_clear = false;
     ctx->built = false;
@@ -258,6 +260,8 @@ int ensure_workspace(rgx_ctx* ctx, int n_pad, int boxes) {
         if ((e = regrow(ctx, ctx->box, 1)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
         if ((e = regrow(ctx, ctx->counters, 1)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
         if ((e = regrow(ctx, ctx->next_unit, 2)) != cudaSuccess) return cuda_fail(ctx, e, "workspace");
+        ctx->build_scratch_clear = false;
+        cudaMemset(ctx->next_unit, 0, 2 * sizeof(unsigned int));          // every march leaves it so
         cudaMemset(ctx->counters, 0, sizeof(DeviceCounters));
         cudaMemset(ctx->box, 0, sizeof(SceneBox));
     }
@@ -289,6 +293,7 @@ int ensure_workspace(rgx_ctx* ctx, int n_pad, int boxes) {
         if ((e = regrow(ctx, ctx->by, c)) != cudaSuccess) return cuda_fail(ctx, e, "workspace boxes");
         if ((e = regrow(ctx, ctx->bz, c)) != cudaSuccess) return cuda_fail(ctx, e, "workspace boxes");
         if ((e = regrow(ctx, ctx->refit_counters, c)) != cudaSuccess) return cuda_fail(ctx, e, "workspace boxes");
+        ctx->build_scratch_clear = false;
         ctx->cap_boxes = (int)c;
     }
     return RGX_OK;
@@ -346,7 +351,7 @@ int run_colors(rgx_ctx* ctx, const rgx_scene* sc, const float eye[3], cudaStream
     ColorLaunch c{};
     const bool listed = listed_only && ctx->lists_partial && ctx->g_code && ctx->listed && ctx->listed_cap >= ctx->n_pad;
     if (listed) {
-        c.listed_rect = ctx->g_rect; c.listed_code = ctx->g_code; c.listed_cut = ctx->near_pick_host->cut;
+        c.listed_rect = ctx->g_rect; c.listed_code = ctx->g_code; c.listed_cut = ctx->bin_result_host->pick.cut;
         c.listed_out = ctx->listed;
     }
     c.sc = *sc;
@@ -440,9 +445,8 @@ void rgx_destroy(rgx_ctx* ctx) {
     if (!ctx) return;
     DeviceGuard guard(ctx->device);
     release_workspace(ctx);
-    if (ctx->bin_total_host) cudaFreeHost(ctx->bin_total_host);
+    if (ctx->bin_result_host) cudaFreeHost(ctx->bin_result_host);
     if (ctx->tape_used_host) cudaFreeHost(ctx->tape_used_host);
-    if (ctx->near_pick_host) cudaFreeHost(ctx->near_pick_host);
     if (ctx->beyond_host) cudaFreeHost(ctx->beyond_host);
     if (ctx->ev_beyond) cudaEventDestroy(ctx->ev_beyond);
     if (ctx->hz_scalars_host) cudaFreeHost(ctx->hz_scalars_host);
@@ -476,6 +480,7 @@ int rgx_build(rgx_ctx* ctx, const rgx_scene* scene, float sigma_threshold, int m
     if ((rc = ensure_workspace(ctx, n_pad > 0 ? n_pad : kFan, lv.total))) return rc;
     ctx->built = false;
     ctx->build_id++;
+    if (n != ctx->n) ctx->hz_budget_now = ctx->hz_budget_per_ray;
     ctx->n = n;
     ctx->n_pad = n_pad;
     ctx->sigma_threshold = sigma_threshold;
@@ -503,8 +508,15 @@ int rgx_build(rgx_ctx* ctx, const rgx_scene* scene, float sigma_threshold, int m
     b.num_levels = lv.num_levels;
     for (int l = 0; l < kMaxLevels; ++l) { b.offset[l] = lv.offset[l]; b.count[l] = lv.count[l]; }
     b.cub_temp = ctx->cub_temp; b.cub_temp_bytes = ctx->cap_cub;
-    cudaError_t e = launch_build(b, s);
+    cudaError_t e = cudaSuccess;
+    if (!ctx->build_scratch_clear &&
+        ((e = cudaMemsetAsync(ctx->bounds, 0, 12 * sizeof(int), s)) != cudaSuccess ||
+         (e = cudaMemsetAsync(ctx->refit_counters, 0, sizeof(unsigned int) * (size_t)ctx->cap_boxes, s)) != cudaSuccess))
+        return cuda_fail(ctx, e, "build");
+    ctx->build_scratch_clear = false;
+    e = launch_build(b, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "build");
+    ctx->build_scratch_clear = true;
     ctx->built = true;
     return RGX_OK;
 }
@@ -550,6 +562,7 @@ struct Cull {
     int budget_per_ray;
     unsigned long long min_total;
     bool half;
+    double ratio;              // estimated pairs per pair kept
 };
 
 static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, BinLaunch& b, int& ntiles, const Cull* cull = nullptr) {
@@ -560,21 +573,24 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     const int ty_first = m->row_begin / tile, ty_last = (m->row_end - 1) / tile;
     const int tiles_y = ty_last - ty_first + 1;
     ntiles = tiles_x * tiles_y;
-    if (!ctx->bin_total_dev) {
-        RGB_(bin_total_dev, 4);
-        if (!ctx->bin_total_host && (e = cudaMallocHost((void**)&ctx->bin_total_host, 4 * sizeof(unsigned long long))) != cudaSuccess)
-            return cuda_fail(ctx, e, "pinned scalar");
-    }
+    if (!ctx->bin_result_host && (e = cudaMallocHost((void**)&ctx->bin_result_host, sizeof(BinResult))) != cudaSuccess)
+        return cuda_fail(ctx, e, "pinned scalars");
     if (ctx->n_pad > ctx->big_cap) {
         RGB_(big_slot, (size_t)ctx->n_pad); RGB_(big_rect, (size_t)ctx->n_pad);
         ctx->big_cap = ctx->n_pad;
     }
     if (ntiles + 1 > ctx->bin_tiles_cap) {
         size_t c = (size_t)ntiles + 1 + 64;
-        RGB_(tile_first, c); RGB_(tile_last, c); RGB_(tile_cnt, c); RGB_(tile_pcnt, c); RGB_(tile_pbegin, c);
-        RGB_(tile_dir, c); RGB_(tile_iota, c); RGB_(tile_cnt_sorted, c); RGB_(tile_order, c); RGB_(tile_unrecorded, c);
+        RGB_(tile_cnt, c); RGB_(tile_pbegin, c);
+        RGB_(tile_dir, c); RGB_(tile_iota, c); RGB_(tile_cnt_sorted, c); RGB_(tile_order, c);
         ctx->bin_tiles_cap = (int)c;
-        ctx->tape_valid = false;       // tile_unrecorded belongs to the recording and has just lost its contents
+        ctx->tape_valid = false;       // its order of the tiles may have been in the array that has just been replaced
+        ctx->tape_order = nullptr;
+    }
+    const ZeroedBins z = zeroed_bins(tiles_x, tiles_y);
+    if (z.bytes > ctx->bin_zero_cap) {
+        RGB_(bin_zero, z.bytes + z.bytes / 8);
+        ctx->bin_zero_cap = z.bytes + z.bytes / 8;
     }
     // first view of a context: room for eight tiles per Gaussian; a view that needs more runs the emission twice
     if (ctx->bin_pair_cap == 0 && (e = grow_pairs(ctx, (size_t)ctx->n_pad * 8)) != cudaSuccess)
@@ -588,17 +604,16 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     if (!camera_dual(*cam, b.dual)) return fail(ctx, RGX_E_INVALID, "camera axes are not linearly independent");
     b.row_begin = m->row_begin; b.row_end = m->row_end; b.tile = tile;
     b.tiles_x = tiles_x; b.tiles_y = tiles_y; b.ty_first = ty_first;
-    b.total_dev = ctx->bin_total_dev;
+    b.zero = ctx->bin_zero; b.zero_bytes = z.bytes;
+    b.total_dev = reinterpret_cast<BinResult*>(ctx->bin_zero)->total;
+    b.tile_first = reinterpret_cast<int*>(ctx->bin_zero + z.first); b.tile_last = reinterpret_cast<int*>(ctx->bin_zero + z.last);
+    b.tile_pcnt = reinterpret_cast<int*>(ctx->bin_zero + z.pcnt);
+    ctx->tile_more = reinterpret_cast<int*>(ctx->bin_zero + z.more);
     b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID;
     if (cull && cull->budget_per_ray > 0) {
         // only the pairs that begin before a horizon are emitted (binning.cu)
-        int rc = two_depth_workspace(ctx, ntiles);          // tile_more, and the counter of rays that reach the horizon
+        int rc = two_depth_workspace(ctx, ntiles);          // the counter of rays that reach the horizon
         if (rc) return rc;
-        if (!ctx->near_pick) {
-            RGB_(near_pick, 1); RGB_(near_hist, 2048);
-            if (!ctx->near_pick_host && (e = cudaMallocHost((void**)&ctx->near_pick_host, sizeof(HorizonPick))) != cudaSuccess)
-                return cuda_fail(ctx, e, "pinned horizon");
-        }
         if (ctx->n_pad > ctx->g_rect_cap) {
             RGB_(g_rect, (size_t)ctx->n_pad); RGB_(g_code, (size_t)ctx->n_pad); RGB_(kept_slot, (size_t)ctx->n_pad);
             ctx->g_rect_cap = ctx->n_pad;
@@ -608,15 +623,12 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
             ctx->listed_cap = ctx->n_pad;
             ctx->listed_serial = 0;
         }
-        const size_t diff = (size_t)(tiles_x + 1) * (size_t)(tiles_y + 1);
-        if (diff > ctx->tile_diff_cap) {
-            RGB_(tile_diff, diff + 64);
-            ctx->tile_diff_cap = diff + 64;
-        }
-        b.pick = ctx->near_pick; b.near_hist = ctx->near_hist; b.g_rect = ctx->g_rect; b.g_code = ctx->g_code; b.kept_slot = ctx->kept_slot;
-        b.tile_diff = ctx->tile_diff; b.tile_more = ctx->tile_more;
+        b.pick = &reinterpret_cast<BinResult*>(ctx->bin_zero)->pick;
+        b.near_hist = reinterpret_cast<unsigned long long*>(ctx->bin_zero + z.hist);
+        b.g_rect = ctx->g_rect; b.g_code = ctx->g_code; b.kept_slot = ctx->kept_slot;
+        b.tile_diff = reinterpret_cast<int*>(ctx->bin_zero + z.diff); b.tile_more = ctx->tile_more;
         const double rays = (double)cam->width * (double)(m->row_end - m->row_begin);
-        b.near_target = (unsigned long long)((double)cull->budget_per_ray * rays * ctx->near_ratio);
+        b.near_target = (unsigned long long)((double)cull->budget_per_ray * rays * cull->ratio);
         b.near_min_total = cull->min_total; b.near_half = cull->half ? 1 : 0;
     }
     return RGX_OK;
@@ -627,10 +639,9 @@ static int emit_launch(rgx_ctx* ctx, BinLaunch& b, cudaStream_t s) {
     cudaError_t e;
     b.keys_in = ctx->bin_keys_in; b.vals_in = ctx->bin_vals_in; b.pair_cap = ctx->bin_pair_cap;
     if ((e = launch_bin_emit(b, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list pairs");
-    if ((e = cudaMemcpyAsync(ctx->bin_total_host, ctx->bin_total_dev, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+    // the number of pairs and the horizon travel together
+    if ((e = cudaMemcpyAsync(ctx->bin_result_host, ctx->bin_zero, sizeof(BinResult), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "tile-list pair count read-back");
-    if (b.pick && (e = cudaMemcpyAsync(ctx->near_pick_host, b.pick, sizeof(HorizonPick), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        return cuda_fail(ctx, e, "horizon read-back");
     return RGX_OK;
 }
 
@@ -640,7 +651,7 @@ static int emit_finish(rgx_ctx* ctx, BinLaunch& b, cudaStream_t s, int& total) {
     cudaError_t e;
     for (int attempt = 0;; ++attempt) {
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list pair count read-back");
-        const unsigned long long total64 = ctx->bin_total_host[0];
+        const unsigned long long total64 = ctx->bin_result_host->total[0];
         if (total64 > (1ull << 30)) return fail(ctx, RGX_E_TOO_LARGE, "more than 2^30 (tile, Gaussian) pairs in this view");
         total = (int)total64;
         if (total64 <= ctx->bin_pair_cap) return RGX_OK;
@@ -676,14 +687,22 @@ static int fill_lists(rgx_ctx* ctx, BinLaunch& b, uint64_t* keys, uint32_t* vals
     b.keys_in = keys; b.vals_in = vals;
     b.keys_out = ctx->bin_keys_out; b.vals_out = ctx->bin_vals_out;
     b.pair_cap = ctx->bin_pair_cap;
-    b.tile_first = ctx->tile_first; b.tile_last = ctx->tile_last; b.tile_cnt = ctx->tile_cnt; b.tile_pcnt = ctx->tile_pcnt;
+    b.tile_cnt = ctx->tile_cnt;
     b.tile_pbegin = ctx->tile_pbegin;
-    b.tile_iota = ctx->tile_iota; b.tile_cnt_sorted = ctx->tile_cnt_sorted; b.tile_order = ctx->tile_order;
+    b.tile_iota = ctx->tile_iota; b.tile_cnt_sorted = ctx->tile_cnt_sorted;
+    b.tile_order = ctx->tile_order;
+    if (ctx->tape_valid && ctx->tape_order == ctx->tile_order) {          // the replay of the latest recording still needs that one
+        if (ntiles > ctx->tape_order_cap) {
+            RGB_(tape_tile_order, (size_t)ntiles + 64);
+            ctx->tape_order_cap = ntiles + 64;
+        }
+        b.tile_order = ctx->tape_tile_order;
+    }
     b.ent_id = ctx->ent_id; b.ent_range = ctx->ent_range; b.blk = ctx->ent_blk;
     b.cub_temp = ctx->bin_cub; b.cub_bytes = ctx->bin_cub_cap;
     if ((e = launch_bin_fill(b, count, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list fill");
     ctx->lists.ent_id = ctx->ent_id; ctx->lists.ent_range = ctx->ent_range; ctx->lists.blk = ctx->ent_blk;
-    ctx->lists.tile_pbegin = ctx->tile_pbegin; ctx->lists.tile_cnt = ctx->tile_cnt; ctx->lists.tile_order = ctx->tile_order;
+    ctx->lists.tile_pbegin = ctx->tile_pbegin; ctx->lists.tile_cnt = ctx->tile_cnt; ctx->lists.tile_order = b.tile_order;
     ctx->lists.tiles_x = b.tiles_x; ctx->lists.tiles_y = b.tiles_y; ctx->lists.ty_first = b.ty_first;
     ctx->lists.tile = b.tile;
     return RGX_OK;
@@ -706,7 +725,7 @@ static int two_depth_workspace(rgx_ctx* ctx, int ntiles) {
             return cuda_fail(ctx, e, "pinned scalars");
     }
     if (ntiles > ctx->hz_tiles_cap) {
-        RGB_(tile_more, (size_t)ntiles + 64); RGB_(tile_resume, (size_t)ntiles + 64);
+        RGB_(tile_resume, (size_t)ntiles + 64);
         ctx->hz_tiles_cap = ntiles + 64;
     }
     return RGX_OK;
@@ -714,11 +733,11 @@ static int two_depth_workspace(rgx_ctx* ctx, int ntiles) {
 
 // What a culled emission teaches about the next one: the estimate counts every tile of a Gaussian's rectangle, and
 // what that is worth in pairs is learnt from view to view.
-static void learn_ratio(rgx_ctx* ctx, int kept) {
-    if (kept > 0) ctx->near_ratio = std::min(8.0, std::max(1.0, (double)ctx->near_pick_host->est_kept / (double)kept));
+static void learn_ratio(const rgx_ctx* ctx, double& ratio, int kept) {
+    if (kept > 0) ratio = std::min(8.0, std::max(1.0, (double)ctx->bin_result_host->pick.est_kept / (double)kept));
 }
 
-static Cull near_cull(const rgx_ctx* ctx) { return Cull{ctx->near_budget_per_ray, (unsigned long long)ctx->near_min_pairs, true}; }
+static Cull near_cull(const rgx_ctx* ctx) { return Cull{ctx->near_budget_per_ray, (unsigned long long)ctx->near_min_pairs, true, ctx->near_ratio}; }
 
 // Turns the emitted pairs into ctx->lists.  The view of a recording forward -- a training view, whose rays end long
 // before they have seen most of their tile's list (on the 3 M-Gaussian scene every ray ends within the nearest eighth
@@ -731,13 +750,13 @@ static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, c
     int rc;
     if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
     lists_now_valid(ctx, cam, m, total);
-    if (b.pick && ctx->near_pick_host->cut != kAllBuckets) {
-        const HorizonPick& pk = *ctx->near_pick_host;
+    if (b.pick && ctx->bin_result_host->pick.cut != kAllBuckets) {
+        const HorizonPick& pk = ctx->bin_result_host->pick;
         ctx->lists_partial = true;
         ctx->lists_horizon = bin_hist_bucket_end(b, (int)pk.cut);
         ctx->lists_rays = (long long)cam->width * (m->row_end - m->row_begin);
         ctx->near_stats[0] += 1; ctx->near_stats[1] += (long long)pk.est_total; ctx->near_stats[2] += total;
-        learn_ratio(ctx, total);
+        learn_ratio(ctx, ctx->near_ratio, total);
     }
     return RGX_OK;
 }
@@ -777,7 +796,7 @@ static void lists_ahead_begin(rgx_ctx* ctx, cudaStream_t s, ListsAhead& a) {
     if (lists_cached(ctx, cam, m)) return;
     const int tile = bin_tile_size(*cam), tiles_x = (cam->width + tile - 1) / tile;
     const int ntiles = tiles_x * ((m->row_end - 1) / tile - m->row_begin / tile + 1);
-    if (!ctx->bin_total_dev || ctx->bin_pair_cap == 0 || ctx->n_pad > ctx->big_cap || ntiles + 1 > ctx->bin_tiles_cap) return;
+    if (!ctx->bin_zero || ctx->bin_pair_cap == 0 || ctx->n_pad > ctx->big_cap || ntiles + 1 > ctx->bin_tiles_cap) return;
     if (!ctx->side) {
         int lo = 0, hi = 0;
         cudaDeviceGetStreamPriorityRange(&lo, &hi);
@@ -833,21 +852,21 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_marc
         RGB_(hz_state, (size_t)(2 * all_rays));
         ctx->hz_state_cap = 2 * all_rays;
     }
-    // first depth: the pairs that begin nearest to the eye, about hz_budget_per_ray per ray -- or all of them, if the
+    // first depth: the pairs that begin nearest to the eye, about hz_budget_now per ray -- or all of them, if the
     // view has fewer than hz_min_pairs_per_ray per ray or the budget covers them
-    const Cull cull{ctx->hz_budget_per_ray > 0 ? ctx->hz_budget_per_ray : 1,
-                    (unsigned long long)((long long)ctx->hz_min_pairs_per_ray * rays), false};
+    const Cull cull{ctx->hz_budget_now,
+                    (unsigned long long)((long long)ctx->hz_min_pairs_per_ray * rays), false, ctx->hz_ratio};
     {
         ScopedTimer timer(ctx, s, 2);
         if ((rc = emit_pairs(ctx, cam, m, s, b, total, ntiles, &cull))) return rc;
         if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
     }
-    const HorizonPick pk = *ctx->near_pick_host;
+    const HorizonPick pk = ctx->bin_result_host->pick;
     if (pk.cut == kAllBuckets || total == 0) {                     // one depth is enough: these are the complete lists
         lists_now_valid(ctx, cam, m, total);
         return RGX_OK;
     }
-    learn_ratio(ctx, total);
+    learn_ratio(ctx, ctx->hz_ratio, total);
     if ((e = cudaMemsetAsync(ctx->tile_resume, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(ctx->hz_scalars, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess)
         return cuda_fail(ctx, e, "two-depth workspace");
@@ -882,7 +901,7 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_marc
         if (e != cudaSuccess) return cuda_fail(ctx, e, "forward march, second depth");
     }
     // a scene whose rays go further than the first depth pays for both: deeper next time
-    if (stopped * 8 > rays && ctx->hz_budget_per_ray < (1 << 18)) ctx->hz_budget_per_ray *= 2;
+    if (stopped * 8 > rays && ctx->hz_budget_now < (1 << 18)) ctx->hz_budget_now *= 2;
     ctx->hz_last[0] = (long long)pk.est_total; ctx->hz_last[1] = total; ctx->hz_last[2] = stopped; ctx->hz_last[3] = total2;
     ctx->last_pairs = total;
     handled = true;
@@ -950,11 +969,15 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         if (record) {
             const long long rays = (long long)cam->width * cam->height;
             const long long rows_rays = (long long)cam->width * (march->row_end - march->row_begin);
-            if (!ctx->tape_used) {
-                if ((e = regrow(ctx, ctx->tape_used, 4)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
-                if ((e = cudaMallocHost((void**)&ctx->tape_used_host, 4 * sizeof(unsigned long long))) != cudaSuccess)
+            const long long zero_words = 8 + ((long long)L.lists.tiles_x * L.lists.tiles_y + 1) / 2;
+            if (zero_words > ctx->tape_used_cap) {
+                if ((e = regrow(ctx, ctx->tape_used, (size_t)(zero_words + 64))) != cudaSuccess) return cuda_fail(ctx, e, "tape");
+                ctx->tape_used_cap = zero_words + 64;
+            }
+            if (!ctx->tape_used_host) {
+                if ((e = cudaMallocHost((void**)&ctx->tape_used_host, 8 * sizeof(unsigned long long))) != cudaSuccess)
                     return cuda_fail(ctx, e, "tape");
-                for (int i = 0; i < 4; ++i) ctx->tape_used_host[i] = 0;
+                for (int i = 0; i < 8; ++i) ctx->tape_used_host[i] = 0;
             }
             const int ntiles = L.lists.tiles_x * L.lists.tiles_y;
             const long long heads = (long long)ntiles * kMaxPatchesPerTile, head_words = heads + (rays + 7) / 8;
@@ -989,14 +1012,13 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
                     ctx->tape_cap = want;
                 }
             }
-            if ((e = cudaMemsetAsync(ctx->tape_used, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess ||
-                (e = cudaMemsetAsync(ctx->tile_unrecorded, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(ctx->tape_tile_order, L.lists.tile_order, sizeof(int) * (size_t)ntiles, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
+            if ((e = cudaMemsetAsync(ctx->tape_used, 0, (size_t)zero_words * sizeof(unsigned long long), s)) != cudaSuccess)
                 return cuda_fail(ctx, e, "tape");
+            ctx->tape_order = L.lists.tile_order;
             if (ctx->tape) {
                 L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
                 L.patch_head = ctx->ray_head; L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + heads);
-                L.tile_unrecorded = ctx->tile_unrecorded;
+                L.tile_unrecorded = reinterpret_cast<int*>(ctx->tape_used + 8);
                 if (ctx->tape_limit >= 0 && ctx->tape_limit < L.tape_cap) L.tape_cap = ctx->tape_limit;
             }
         }
@@ -1007,7 +1029,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         }
         if (e != cudaSuccess) return cuda_fail(ctx, e, "forward march");
         if (recorded) {
-            cudaMemcpyAsync(ctx->tape_used_host, ctx->tape_used, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(ctx->tape_used_host, ctx->tape_used, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
             ctx->tape_valid = true;
             ctx->tape_rgba_serial = ctx->rgba_serial;
             ctx->tape_build_id = ctx->build_id;
@@ -1114,8 +1136,8 @@ int rgx_backward(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* cam, co
         L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
         L.patch_head = ctx->ray_head;
         L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + (long long)L.lists.tiles_x * L.lists.tiles_y * kMaxPatchesPerTile);
-        L.tile_unrecorded = ctx->tile_unrecorded;
-        L.replay_order = ctx->tape_tile_order;
+        L.tile_unrecorded = reinterpret_cast<int*>(ctx->tape_used + 8);
+        L.replay_order = ctx->tape_order;
     }
     L.rgb_in = rgb; L.dl_drgb = dL_drgb; L.grad_rows = ctx->grad_rows; L.grad_copies = ctx->grad_copies;
     // rays without a recording first: theirs is the last launch that reads the view's lists, so the lists of an
@@ -1200,7 +1222,7 @@ int rgx_debug_fail_allocation(rgx_ctx* ctx, int nth) {
 int rgx_debug_two_depth(rgx_ctx* ctx, int min_pairs_per_ray, int budget_per_ray) {
     if (!ctx || budget_per_ray < 0) return RGX_E_INVALID;
     ctx->hz_min_pairs_per_ray = min_pairs_per_ray;
-    if (budget_per_ray > 0) ctx->hz_budget_per_ray = budget_per_ray;
+    if (budget_per_ray > 0) ctx->hz_budget_per_ray = ctx->hz_budget_now = budget_per_ray;
     return RGX_OK;
 }
 

@@ -652,19 +652,12 @@ cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s) {
     const int tb = 256;
     const int ntiles = b.tiles_x * b.tiles_y;
     cudaError_t e;
-    // total_dev: [0] pairs, [1] Gaussians listed by bin_list_kernel, [2] next listed Gaussian to take, [3] Gaussians
-    // listed by bin_compact_kernel
-    if ((e = cudaMemsetAsync(b.total_dev, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(b.zero, 0, b.zero_bytes, s)) != cudaSuccess) return e;
     const int blocks = (b.n_pad + kEmitThreads - 1) / kEmitThreads;
     if (b.pick) {
         // only the pairs that begin before a horizon, which is picked on the way (see bin_near_hist_kernel)
         const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
         if (kl.near_bits < kHistBits) return cudaErrorInvalidValue;
-        if ((e = cudaMemsetAsync(b.pick, 0, sizeof(HorizonPick), s)) != cudaSuccess ||
-            (e = cudaMemsetAsync(b.near_hist, 0, sizeof(unsigned long long) << kHistBits, s)) != cudaSuccess ||
-            (e = cudaMemsetAsync(b.tile_diff, 0, sizeof(int) * (size_t)(b.tiles_x + 1) * (size_t)(b.tiles_y + 1), s)) != cudaSuccess ||
-            (e = cudaMemsetAsync(b.tile_more, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess)
-            return e;
         note_launch(), bin_tile_dirs_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
         note_launch(), bin_near_hist_kernel<<<blocks, kEmitThreads, 0, s>>>(b);
         note_launch(), bin_pick_horizon_kernel<<<1, 1024, 0, s>>>(b);
@@ -686,9 +679,6 @@ cudaError_t launch_bin_fill(const BinLaunch& b, int total, cudaStream_t s) {
     // the layout is that of the whole image whatever the row range, so that a row range sees the same order
     const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
     cudaError_t e;
-    if ((e = cudaMemsetAsync(b.tile_first, 0, sizeof(int) * (ntiles + 1), s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(b.tile_last, 0, sizeof(int) * (ntiles + 1), s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(b.tile_pcnt, 0, sizeof(int) * (ntiles + 1), s)) != cudaSuccess) return e;
     size_t temp = b.cub_bytes;
     if (total > 0) {
         e = cub::DeviceRadixSort::SortPairs(b.cub_temp, temp, b.keys_in, b.keys_out, b.vals_in, b.vals_out, (int64_t)total, 0,

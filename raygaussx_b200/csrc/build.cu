@@ -13,14 +13,6 @@ namespace rgx {
 
 namespace {
 
-__device__ __forceinline__ int float_to_ordered(float f) {
-    int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float ordered_to_float(int i) {
-    return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff);
-}
-
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -30,14 +22,6 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
-}
-
-__global__ void init_bounds_kernel(int* bounds) {
-    int t = threadIdx.x;
-    if (t < 12) {
-        bool is_lo = (t % 6) < 3;
-        bounds[t] = float_to_ordered(is_lo ? INFINITY : -INFINITY);
-    }
 }
 
 // One thread per Gaussian: scene box over every Gaussian's box (degenerate ones
@@ -71,17 +55,20 @@ __global__ void __launch_bounds__(256) bounds_kernel(BuildLaunch b) {
         bool is_lo = (t % 6) < 3;
         float v = red[t][0];
         for (int w = 1; w < 8; ++w) v = is_lo ? fminf(v, red[t][w]) : fmaxf(v, red[t][w]);
-        if (is_lo) atomicMin(&b.bounds[t], float_to_ordered(v));
-        else atomicMax(&b.bounds[t], float_to_ordered(v));
+        atomicMax(reinterpret_cast<unsigned*>(&b.bounds[t]), ordered(is_lo ? -v : v));      // zero before: below every number
     }
 }
 
+__device__ __forceinline__ float bound_lo(const BuildLaunch& b, int t) { return -unordered((unsigned)b.bounds[t]); }
+__device__ __forceinline__ float bound_hi(const BuildLaunch& b, int t) { return unordered((unsigned)b.bounds[t]); }
+
+template <class Key>
 __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
         for (int a = 0; a < 3; ++a) {
-            b.box->lo[a] = ordered_to_float(b.bounds[a]);
-            b.box->hi[a] = ordered_to_float(b.bounds[3 + a]);
+            b.box->lo[a] = bound_lo(b, a);
+            b.box->hi[a] = bound_hi(b, 3 + a);
         }
     }
     if (i >= b.sc.n) return;
@@ -89,7 +76,7 @@ __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
     uint32_t q[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float lo = ordered_to_float(b.bounds[6 + a]), hi = ordered_to_float(b.bounds[9 + a]);
+        float lo = bound_lo(b, 6 + a), hi = bound_hi(b, 9 + a);
         float ext = hi - lo;
         float u = ext > 0.f ? (b.sc.positions[3 * i + a] - lo) / ext : 0.f;
         u = fminf(fmaxf(u * cells, 0.f), cells - 1.f);
@@ -103,7 +90,7 @@ __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
     } else {
         key = spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
     }
-    b.keys_in[i] = key;
+    reinterpret_cast<Key*>(b.keys_in)[i] = (Key)key;
     b.vals_in[i] = (uint32_t)i;
 }
 
@@ -111,7 +98,13 @@ __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
 // for the backward, and the level-0 box.
 __global__ void __launch_bounds__(256) gather_kernel(BuildLaunch b) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= b.n_pad) return;
+    if (j < 12) b.bounds[j] = 0;                       // for the next build
+    if (j >= b.n_pad) {                                // the upper levels start as boxes that are never hit
+        const int k = b.offset[1] + (j - b.n_pad);
+        const int end = b.offset[b.num_levels - 1] + ((b.count[b.num_levels - 1] + kFan - 1) / kFan) * kFan;
+        if (k < end) b.bx[k] = b.by[k] = b.bz[k] = make_float2(FLT_MAX, -FLT_MAX);
+        return;
+    }
     const float nanv = __int_as_float(0x7fc00000);
     float4 g0 = make_float4(0.f, 0.f, 0.f, nanv), g1 = make_float4(nanv, nanv, nanv, nanv), g2 = g1;
     float4 qq = make_float4(1.f, 0.f, 0.f, 0.f), sd = make_float4(1.f, 1.f, 1.f, 0.f);
@@ -158,11 +151,6 @@ __global__ void __launch_bounds__(256) gather_kernel(BuildLaunch b) {
     b.bz[j] = make_float2(lo.z, hi.z);
 }
 
-__global__ void fill_inverted_kernel(float2* bx, float2* by, float2* bz, int begin, int end) {
-    int j = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < end) bx[j] = by[j] = bz[j] = make_float2(FLT_MAX, -FLT_MAX);
-}
-
 // Bottom-up refit with arrival counters: one warp per level-1 node bounds its 32
 // Gaussians, then climbs; at every parent the last of the arriving children does
 // the work, the others leave.  No warp ever waits for another.
@@ -193,7 +181,9 @@ __global__ void __launch_bounds__(256) refit_kernel(BuildLaunch b) {
         unsigned int arrived = 0;
         if (lane == 0) {
             __threadfence();
-            arrived = atomicAdd(&b.refit_counters[b.offset[up + 1] + parent], 1u);
+            unsigned int* counter = &b.refit_counters[b.offset[up + 1] + parent];
+            arrived = atomicAdd(counter, 1u);
+            if ((int)arrived == siblings - 1) *counter = 0u;       // for the next build
         }
         arrived = __shfl_sync(0xffffffffu, arrived, 0);
         if ((int)arrived != siblings - 1) return;
@@ -205,29 +195,34 @@ __global__ void __launch_bounds__(256) refit_kernel(BuildLaunch b) {
 
 }  // namespace
 
+// Keys of up to 32 bits are sorted as such: half the bytes per pass.
+template <class Key>
+static cudaError_t sort_keys(const BuildLaunch& b, void* temp, size_t& bytes, int n, int bits, cudaStream_t s) {
+    return cub::DeviceRadixSort::SortPairs(temp, bytes, reinterpret_cast<const Key*>(b.keys_in), reinterpret_cast<Key*>(b.keys_out),
+                                           b.vals_in, b.vals_out, n, 0, bits, s);
+}
+
 size_t build_cub_temp_bytes(int n_pad) {
-    size_t bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr,
-                                    (const uint32_t*)nullptr, (uint32_t*)nullptr, n_pad, 0, 64, (cudaStream_t)0);
-    return bytes;
+    size_t narrow = 0, wide = 0;
+    sort_keys<uint32_t>(BuildLaunch{}, nullptr, narrow, n_pad, 30, (cudaStream_t)0);
+    sort_keys<uint64_t>(BuildLaunch{}, nullptr, wide, n_pad, 64, (cudaStream_t)0);
+    return narrow > wide ? narrow : wide;
 }
 
 cudaError_t launch_build(const BuildLaunch& b, cudaStream_t s) {
     const int n = b.sc.n;
-    const int tb = 256;
-    note_launch(), init_bounds_kernel<<<1, 32, 0, s>>>(b.bounds);
-    note_launch(), bounds_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(b);
-    note_launch(), morton_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(b);
+    const int tb = 256, blocks = (n + tb - 1) / tb;
+    const bool narrow = 3 * b.morton_bits <= 32;
+    note_launch(), bounds_kernel<<<blocks, tb, 0, s>>>(b);
+    if (narrow) note_launch(), morton_kernel<uint32_t><<<blocks, tb, 0, s>>>(b);
+    else note_launch(), morton_kernel<uint64_t><<<blocks, tb, 0, s>>>(b);
     size_t temp = b.cub_temp_bytes;
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(b.cub_temp, temp, b.keys_in, b.keys_out, b.vals_in, b.vals_out, n,
-                                                    0, 3 * b.morton_bits, s);
+    cudaError_t e = narrow ? sort_keys<uint32_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s)
+                           : sort_keys<uint64_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s);
     if (e != cudaSuccess) return e;
-    note_launch(), gather_kernel<<<(b.n_pad + tb - 1) / tb, tb, 0, s>>>(b);
-    int total = b.offset[b.num_levels - 1] + ((b.count[b.num_levels - 1] + kFan - 1) / kFan) * kFan;
-    int upper = total - b.offset[1];
-    note_launch(), fill_inverted_kernel<<<(upper + tb - 1) / tb, tb, 0, s>>>(b.bx, b.by, b.bz, b.offset[1], total);
-    e = cudaMemsetAsync(b.refit_counters, 0, sizeof(unsigned int) * (size_t)total, s);
-    if (e != cudaSuccess) return e;
+    const int total = b.offset[b.num_levels - 1] + ((b.count[b.num_levels - 1] + kFan - 1) / kFan) * kFan;
+    const int slots = b.n_pad + (total - b.offset[1]);
+    note_launch(), gather_kernel<<<(slots + tb - 1) / tb, tb, 0, s>>>(b);
     int warps = b.count[1];
     note_launch(), refit_kernel<<<(warps + 7) / 8, 256, 0, s>>>(b);
     return cudaGetLastError();

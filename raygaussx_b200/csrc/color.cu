@@ -290,7 +290,7 @@ cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s) {
 
 cudaError_t launch_finalize(const FinalizeLaunch& f, cudaStream_t s) {
     if (f.sc.n == 0) return cudaSuccess;
-    if (!(f.flags & RGX_FLAG_ACCUMULATE)) {       // the kernel writes the rows of the Gaussians some ray met, nothing else
+    if (!(f.flags & (RGX_FLAG_ACCUMULATE | RGX_FLAG_GRADS_CLEAR))) {       // the kernel writes the rows of the Gaussians some ray met, nothing else
         const size_t n = (size_t)f.sc.n, K = (size_t)f.sc.sh_coeffs, G = (size_t)f.sc.num_lobes;
         struct { float* p; size_t count; } clear[] = {
             {f.gr.positions, 3 * n}, {f.gr.scales, 3 * n}, {f.gr.quaternions, 4 * n}, {f.gr.densities, n},

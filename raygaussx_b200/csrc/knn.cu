@@ -28,13 +28,6 @@ namespace {
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kKnnWarps = 8;
 
-// float -> unsigned with the same order, above zero for every number
-__device__ __forceinline__ unsigned ordered(float f) {
-    const unsigned u = __float_as_uint(f);
-    return u & 0x80000000u ? ~u : u | 0x80000000u;
-}
-__device__ __forceinline__ float unordered(unsigned u) { return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u); }
-
 // bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
 __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, unsigned* bounds) {
     __shared__ unsigned s_max[6];

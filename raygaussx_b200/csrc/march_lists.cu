@@ -206,6 +206,14 @@ __device__ __forceinline__ void hz_note(const MarchLaunch& L, int ray_id) {
 
 // ---------------------------------------------------------------- what the sixteen rays of a patch share
 constexpr int kGroup = 8;          // entries that are tested before their hits are evaluated
+// The next patch.  Every warp of the grid fetches one number past the end; the one that fetches the last of those puts the counter
+// back to zero for the next launch.
+__device__ __forceinline__ unsigned fetch_unit(unsigned* next, unsigned units) {
+    const unsigned u = atomicAdd(next, 1u);
+    if (u == units + gridDim.x * kPatchWarps - 1u) *next = 0u;
+    return u;
+}
+
 constexpr int kStaged = 64;        // ring of list entries that passed the patch's filters
 
 struct PatchStage {                // per warp
@@ -497,7 +505,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, COUNT ? 1 : patch_ctas_per_s
 
     while (true) {
         unsigned unit = 0;
-        if (lane == 0) unit = atomicAdd(L.next_unit, 1u);
+        if (lane == 0) unit = fetch_unit(L.next_unit, units);
         unit = __shfl_sync(kFull, unit, 0);
         if (unit >= units) break;
         const int tile = __ldg(&L.lists.tile_order[unit / per_tile]), patch = (int)(unit % per_tile);   // longest lists first
@@ -863,7 +871,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, 4) march_backward_patches_ke
 
     while (true) {
         unsigned unit = 0;
-        if (lane == 0) unit = atomicAdd(L.next_unit, 1u);
+        if (lane == 0) unit = fetch_unit(L.next_unit + 1, units);
         unit = __shfl_sync(kFull, unit, 0);
         if (unit >= units) break;
         const int tile = __ldg(&L.replay_order[unit / per_tile]), patch = (int)(unit % per_tile);
@@ -1176,8 +1184,6 @@ static void launch_forward_lanes(const MarchLaunch& m, cudaStream_t s) {
 cudaError_t launch_march_forward(const MarchLaunch& m, cudaStream_t s) {
     if (!use_lists(m)) return launch_march_forward_per_ray(m, s);
     if (m.lists.tiles_x * m.lists.tiles_y <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(m.next_unit, 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess) return e;
     switch (patch_lanes(m)) {
         case 2: launch_forward_lanes<2>(m, s); break;
         case 4: launch_forward_lanes<4>(m, s); break;
@@ -1206,8 +1212,6 @@ static cudaError_t launch_replay(const MarchLaunch& m, cudaStream_t s) {
 cudaError_t launch_march_backward_replay(const MarchLaunch& m, cudaStream_t s) {
     if (!use_lists(m) || !m.tape) return cudaSuccess;
     if (m.lists.tiles_x * m.lists.tiles_y <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(m.next_unit, 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess) return e;
     switch (patch_lanes(m)) {
         case 2: return launch_replay<2>(m, s);
         case 4: return launch_replay<4>(m, s);

@@ -108,6 +108,30 @@ struct HorizonPick {
 };
 constexpr unsigned int kAllBuckets = 0xffffffffu;
 
+// What an emission leaves for the host, first in the piece of memory that it starts from zero.
+struct BinResult {
+    unsigned long long total[4];        // [0] pairs met (may exceed the capacity), [1] Gaussians listed by bin_list_kernel, [2] next listed
+                                        // Gaussian to take, [3] Gaussians listed by bin_compact_kernel
+    HorizonPick pick;
+};
+// That piece, as byte offsets: the result, the histogram of nearest distances, per tile first and last pair and padded count,
+// corners of culled rectangles, tiles that have more pairs.
+struct ZeroedBins {
+    size_t hist, first, last, pcnt, diff, more, bytes;
+};
+inline ZeroedBins zeroed_bins(int tiles_x, int tiles_y) {
+    const size_t tiles = (size_t)tiles_x * tiles_y, align = 255;
+    ZeroedBins z;
+    z.hist = (sizeof(BinResult) + align) & ~align;
+    z.first = z.hist + 2048 * sizeof(unsigned long long);
+    z.last = (z.first + sizeof(int) * (tiles + 1) + align) & ~align;
+    z.pcnt = (z.last + sizeof(int) * (tiles + 1) + align) & ~align;
+    z.diff = (z.pcnt + sizeof(int) * (tiles + 1) + align) & ~align;
+    z.more = (z.diff + sizeof(int) * (size_t)(tiles_x + 1) * (tiles_y + 1) + align) & ~align;
+    z.bytes = z.more + sizeof(int) * tiles;
+    return z;
+}
+
 struct BinLaunch {
     int n, n_pad;
     const float2 *bx, *by, *bz;            // level-0 boxes
@@ -124,7 +148,8 @@ struct BinLaunch {
     int* ent_id; float2* ent_range; float2* blk;
     float4* tile_dir;                      // [tiles] central ray direction, chord to the farthest corner ray
     void* cub_temp; size_t cub_bytes;
-    unsigned long long* total_dev;         // [4]; [0] = number of pairs met by the emission (may exceed pair_cap)
+    unsigned char* zero; size_t zero_bytes;// cleared before an emission; total_dev, pick ... tile_more point into it
+    unsigned long long* total_dev;         // [4], see BinResult
     int* big_slot; uint2* big_rect;        // [n_pad] complete emission: the Gaussians that touch a tile, and their tile rectangles
     int big_grid;                          // CTAs that work the list off (a few per SM)
     // culled emission (null / unused for a complete one): only the pairs that begin before a horizon are emitted
@@ -163,7 +188,7 @@ struct MarchLaunch {
     unsigned char* ray_unrecorded;   // [R] the ray could not be recorded: the backward searches it again
     int* tile_unrecorded;            // per tile (of the lists): set by the forward when a ray of the tile is unrecorded
     const int* replay_order;  // backward replay: tiles in the order of the recording forward (own copy: the lists may be remade meanwhile)
-    unsigned int* next_unit;  // the patch kernels' warps fetch their patches from it
+    unsigned int* next_unit;  // [2] the warps of the forward and of the replay fetch their patches from it; zero before and after
     int sm_count;
     // two-depth forward (march_lists.cu, HZ variant): 0 = off, 1 = first phase (lists up to `horizon`), 2 = second
     int hz_phase;
@@ -217,7 +242,8 @@ struct BuildLaunch {
     float2 *bx, *by, *bz;
     float4 *g0, *g1, *g2, *quat, *sdens;
     float* hk;
-    int* bounds;           // 12 ints: ordered-int encodings of scene box lo[3],hi[3], centre lo[3],hi[3]
+    int* bounds;           // 12 words: largest -lo[3], hi[3] of the scene box, then of the centres, ordered (device_math.cuh); zero
+                           // before and after a build, as are the refit counters
     SceneBox* box;
     unsigned int* refit_counters;
     int num_levels;

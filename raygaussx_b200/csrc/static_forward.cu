@@ -159,7 +159,10 @@ extern "C" RGX_API int rgx_forward_static(int device, const rgx_scene* scene, co
         b.n_pad = n_pad;
         b.num_levels = lv.num_levels;
         for (int l = 0; l < kMaxLevels; ++l) { b.offset[l] = lv.offset[l]; b.count[l] = lv.count[l]; }
-        if (launch_build(b, s) != cudaSuccess) return RGX_E_CUDA;
+        if (cudaMemsetAsync(b.bounds, 0, 12 * sizeof(int), s) != cudaSuccess ||
+            cudaMemsetAsync(b.refit_counters, 0, sizeof(unsigned int) * (size_t)lv.total, s) != cudaSuccess ||
+            launch_build(b, s) != cudaSuccess)
+            return RGX_E_CUDA;
         ColorLaunch c{};
         c.sc = *scene;
         c.eye[0] = cam->eye[0]; c.eye[1] = cam->eye[1]; c.eye[2] = cam->eye[2];

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) activate_kernel(rgx_activation a) {
         for (int c = 0; c < 3; ++c) a.scales[3 * i + c] = expf(a.log_scales[3 * i + c]);
         if (a.quaternions) {
             const float q0 = a.raw_quaternions[4 * i], q1 = a.raw_quaternions[4 * i + 1], q2 = a.raw_quaternions[4 * i + 2], q3 = a.raw_quaternions[4 * i + 3];
-            const float len = sqrtf(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3);
+            const float len = sqrtf((q0 * q0 + q2 * q2) + (q1 * q1 + q3 * q3));      // the order of torch.norm: same bits
             reinterpret_cast<float4*>(a.quaternions)[i] = make_float4(q0 / len, q1 / len, q2 / len, q3 / len);
         }
     }

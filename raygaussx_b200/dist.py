@@ -120,7 +120,9 @@ class GradBuffer:
         self.layout = gradient_layout(n, sh_coeffs)
         name, off, shape = self.layout[-1]
         total = off + (shape[0] * shape[1] * shape[2])
-        self.flat = torch.zeros(total, dtype=torch.float32, device=device)
+        # the colour rows are moved 16 bytes at a time: the buffer begins where its last tensor falls on such a boundary
+        pad = -off % 4
+        self.flat = torch.zeros(total + pad, dtype=torch.float32, device=device)[pad:]
         self.views = {}
         for name, off, shape in self.layout:
             size = 1

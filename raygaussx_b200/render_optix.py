@@ -156,7 +156,7 @@ class Renderer:
 
     # -- helpers
     def _stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _lib.raw_stream(self.device)
 
     @staticmethod
     def _scene(positions, scales, quaternions, densities, color_features=None, sg_features=None, sharpness=None,
@@ -391,7 +391,10 @@ class RenderOptixFunction(torch.autograd.Function):
             flags |= _lib.FLAG_ACCUMULATE
             march = _settings_march(settings, cam, flags=flags, rows=getattr(settings, "rows", None))
         else:
-            grads = [torch.empty_like(t) for t in tensors]
+            # one buffer for all of them, cleared at once; every tensor starts on a 16-byte boundary
+            sizes = [(t.numel() + 3) & ~3 for t in tensors]
+            grads = [g[:t.numel()].view(t.shape) for g, t in zip(torch.zeros(sum(sizes), device=rgb.device).split(sizes), tensors)]
+            march.flags |= _lib.FLAG_GRADS_CLEAR
         if r._build_serial != ctx.build_serial:
             # another build came between this view's forward and its backward (a second model, an evaluation copy,
             # a finite-difference probe): the backward reads the geometry of the latest build, so build again from

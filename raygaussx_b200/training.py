@@ -83,7 +83,7 @@ def isotropy_loss(scales: torch.Tensor) -> torch.Tensor:
 
 # ----------------------------------------------------------------------------- the same on the device, fused (csrc/train.cu)
 def _stream(t: torch.Tensor):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.raw_stream(t.device)
 
 
 def _check(rc: int, what: str):
@@ -93,8 +93,11 @@ def _check(rc: int, what: str):
 
 def _fusable(*tensors) -> bool:
     """fp32 CUDA tensors of one device, contiguous: what the fused kernels take."""
-    dev = tensors[0].device
-    return all(t.is_cuda and t.device == dev and t.dtype == torch.float32 and t.is_contiguous() for t in tensors)
+    index = tensors[0].get_device()                      # -1: not on a GPU
+    for t in tensors:
+        if t.layout != torch.strided or t.get_device() != index or t.dtype != torch.float32 or not t.is_contiguous():
+            return False
+    return index >= 0
 
 
 class _ImageLoss(torch.autograd.Function):
@@ -248,18 +251,19 @@ class _Adam(torch.optim.Adam):
     """``torch.optim.Adam`` whose step is one kernel over all tensors (``rgx_adam_step``) where the parameters are contiguous
     fp32 CUDA tensors and nothing but the plain algorithm is asked for; state and results are those of the base class."""
 
-    _PLAIN = dict(weight_decay=0, amsgrad=False, maximize=False, capturable=False, differentiable=False, fused=None)
+    @staticmethod
+    def _plain(grp) -> bool:
+        return not (grp["weight_decay"] or grp["amsgrad"] or grp["maximize"] or grp["capturable"] or grp["differentiable"]
+                    or grp["fused"] or torch.is_tensor(grp["lr"]))
 
     @torch.no_grad()
     def step(self, closure=None):
-        work = [(p, grp) for grp in self.param_groups for p in grp["params"] if p.grad is not None]
-        if closure is not None or not work or not all(
-                all(grp[k] == v or (k == "fused" and not grp[k]) for k, v in self._PLAIN.items())
-                and not torch.is_tensor(grp["lr"]) for _, grp in work) or not all(
-                not p.grad.is_sparse and _fusable(p, p.grad) and p.device == work[0][0].device for p, _ in work):
+        work = [(p, p.grad, grp) for grp in self.param_groups for p in grp["params"] if p.grad is not None]
+        if closure is not None or not work or not all(self._plain(grp) for grp in self.param_groups) or not _fusable(
+                *[p for p, _, _ in work], *[g for _, g, _ in work]):
             return super().step(closure)
         batches = {}
-        for p, grp in work:
+        for p, grad, grp in work:
             st = self.state[p]
             if len(st) == 0:
                 st["step"] = torch.tensor(0.0)
@@ -269,7 +273,7 @@ class _Adam(torch.optim.Adam):
             t = st["step"].item()                        # a host tensor
             beta1, beta2 = grp["betas"]
             batches.setdefault((beta1, beta2, grp["eps"]), []).append(
-                (p.data_ptr(), st["exp_avg"].data_ptr(), st["exp_avg_sq"].data_ptr(), p.grad.data_ptr(), p.numel(),
+                (p.data_ptr(), st["exp_avg"].data_ptr(), st["exp_avg_sq"].data_ptr(), grad.data_ptr(), p.numel(),
                  grp["lr"] / (1 - beta1 ** t), 1.0 / math.sqrt(1 - beta2 ** t)))
         dev = work[0][0].device
         for (beta1, beta2, eps), rows in batches.items():
@@ -278,7 +282,7 @@ class _Adam(torch.optim.Adam):
                 table = (_lib.AdamTensor * len(part))(*part)
                 _check(_lib.lib().rgx_adam_step(dev.index or 0, table, len(part), beta1, beta2, eps, _stream(work[0][0])),
                        "rgx_adam_step")
-        torch.autograd.graph.increment_version([p for p, _ in work])       # written to behind torch's back
+        torch.autograd.graph.increment_version([p for p, _, _ in work])       # written to behind torch's back
 
 
 class _Optimizers:

@@ -18,7 +18,7 @@ def distCUDA2(points: torch.Tensor) -> torch.Tensor:
     need = int(lib.rgx_knn_scratch_bytes(n))
     scratch = torch.empty(need, device=dev, dtype=torch.uint8)
     rc = lib.rgx_knn_mean_dist2_scratch(dev.index or 0, pts.data_ptr(), n, out.data_ptr(), scratch.data_ptr(), need,
-                                        torch.cuda.current_stream(dev).cuda_stream)
+                                        _lib.raw_stream(dev))
     if rc != 0:
         raise _lib.RgxError(rc, "rgx_knn_mean_dist2 failed")
     return out
