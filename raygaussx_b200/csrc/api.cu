@@ -20,6 +20,7 @@ using namespace rgx;
 #define RGX_NEAR_BUDGET 5
 #endif
 
+constexpr double kFirstRatio = 2.0;      // (estimated pairs per pair before a view of the scene has been seen)
 struct rgx_ctx {
     int device = 0;
     std::string error;
@@ -103,7 +104,7 @@ struct rgx_ctx {
     long long beyond_kept = 0, beyond_lists_rays = 0; int beyond_budget = 0;   // of the lists that march used
     long long tape_beyond_rays = 0;              // rays of the current recording that went beyond (they are not recorded)
     long long near_min_pairs = 1ll << 21;     // views with fewer (estimated) pairs get complete lists
-    double near_ratio = 2.0, hz_ratio = 2.0;  // estimated pairs (tile rectangles) per pair kept up to the horizon, from the latest such view (hz_: in the first depth)
+    double near_ratio = kFirstRatio, hz_ratio = kFirstRatio;  // estimated pairs (tile rectangles) per pair kept up to the horizon, from the latest such view (hz_: in the first depth)
     uint2* g_rect = nullptr; unsigned int* g_code = nullptr; int* kept_slot = nullptr; int g_rect_cap = 0;
     unsigned long long lists_build_id = 0;
     rgx_camera lists_cam{};
@@ -480,7 +481,7 @@ int rgx_build(rgx_ctx* ctx, const rgx_scene* scene, float sigma_threshold, int m
     if ((rc = ensure_workspace(ctx, n_pad > 0 ? n_pad : kFan, lv.total))) return rc;
     ctx->built = false;
     ctx->build_id++;
-    if (n != ctx->n) ctx->hz_budget_now = ctx->hz_budget_per_ray;
+    if (n != ctx->n) { ctx->hz_budget_now = ctx->hz_budget_per_ray; ctx->hz_ratio = ctx->near_ratio = kFirstRatio; }
     ctx->n = n;
     ctx->n_pad = n_pad;
     ctx->sigma_threshold = sigma_threshold;
@@ -732,7 +733,8 @@ static int two_depth_workspace(rgx_ctx* ctx, int ntiles) {
 }
 
 // What a culled emission teaches about the next one: the estimate counts every tile of a Gaussian's rectangle, and
-// what that is worth in pairs is learnt from view to view.
+// what that is worth in pairs is learnt from view to view, from those that keep every pair as well: else a ratio too large for the
+// scene, under which everything is kept, would stay.
 static void learn_ratio(const rgx_ctx* ctx, double& ratio, int kept) {
     if (kept > 0) ratio = std::min(8.0, std::max(1.0, (double)ctx->bin_result_host->pick.est_kept / (double)kept));
 }
@@ -750,13 +752,13 @@ static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, c
     int rc;
     if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
     lists_now_valid(ctx, cam, m, total);
+    if (b.pick) learn_ratio(ctx, ctx->near_ratio, total);
     if (b.pick && ctx->bin_result_host->pick.cut != kAllBuckets) {
         const HorizonPick& pk = ctx->bin_result_host->pick;
         ctx->lists_partial = true;
         ctx->lists_horizon = bin_hist_bucket_end(b, (int)pk.cut);
         ctx->lists_rays = (long long)cam->width * (m->row_end - m->row_begin);
         ctx->near_stats[0] += 1; ctx->near_stats[1] += (long long)pk.est_total; ctx->near_stats[2] += total;
-        learn_ratio(ctx, ctx->near_ratio, total);
     }
     return RGX_OK;
 }
@@ -862,11 +864,11 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_marc
         if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
     }
     const HorizonPick pk = ctx->bin_result_host->pick;
+    learn_ratio(ctx, ctx->hz_ratio, total);
     if (pk.cut == kAllBuckets || total == 0) {                     // one depth is enough: these are the complete lists
         lists_now_valid(ctx, cam, m, total);
         return RGX_OK;
     }
-    learn_ratio(ctx, ctx->hz_ratio, total);
     if ((e = cudaMemsetAsync(ctx->tile_resume, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(ctx->hz_scalars, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess)
         return cuda_fail(ctx, e, "two-depth workspace");

@@ -127,7 +127,7 @@ __device__ __forceinline__ bool ellipsoid_stretch(float3 Oe, float3 de, RayParab
     p.inv_a = __fdividef(1.0f, p.a);
     const float t = __fmul_rn(b, p.inv_a);
     p.t0 = fmaf(fmaf(-t, p.a, b), p.inv_a, t);
-    float3 P = make_float3(fmaf(p.t0, de.x, Oe.x), fmaf(p.t0, de.y, Oe.y), fmaf(p.t0, de.z, Oe.z));
+    float3 P = make_float3(fmaf(t, de.x, Oe.x), fmaf(t, de.y, Oe.y), fmaf(t, de.z, Oe.z));   // from the quotient as it is: q is flat there
     p.q = dot3(P, P);
     p.disc = 1.0f - p.q;
     p.w2 = __fmul_rn(p.disc, p.inv_a);
