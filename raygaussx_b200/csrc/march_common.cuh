@@ -116,6 +116,7 @@ __device__ __forceinline__ void whiten_ray(const Ray& r, float4 g0, float4 g1, f
 // quotient is exact in an FMA), good to an ulp: the response is evaluated as a parabola about it.
 struct RayParabola {
     float a, inv_a, t0, q, disc, w2, hw;      // disc = 1 - q; w2 = disc / a, hw its root: the ray is inside for |t - t0| < hw
+    float root, far;                          // root of disc * a; the larger root (b + root) / a
 };
 
 // The stretch of the ray Oe + t de inside the truncation ellipsoid (the unit sphere of the whitened frame), t0 - hw .. t0 + hw
@@ -131,20 +132,22 @@ __device__ __forceinline__ bool ellipsoid_stretch(float3 Oe, float3 de, RayParab
     p.q = dot3(P, P);
     p.disc = 1.0f - p.q;
     p.w2 = __fmul_rn(p.disc, p.inv_a);
-    p.hw = sqrt_approx(p.w2);
-    return p.disc > 1e-7f && p.t0 >= 0.f;
+    p.root = sqrt_approx(__fmul_rn(p.disc, p.a));
+    p.hw = __fmul_rn(p.root, p.inv_a);
+    p.far = __fmul_rn(__fadd_rn(b, p.root), p.inv_a);
+    return p.disc > 1e-7f && b >= 0.f;
 }
 // Where the ray enters: the smaller root, from the form that does not cancel (c / q).  c = |Oe|^2 - 1.
 __device__ __forceinline__ float whitened_c(float3 Oe) {
     return fmaf(Oe.x, Oe.x, fmaf(Oe.y, Oe.y, fmaf(Oe.z, Oe.z, -1.0f)));
 }
 __device__ __forceinline__ float entry_root(float3 Oe, float3 de, float c, const RayParabola& p) {
-    const float b = -dot3(Oe, de);
-    return __fdividef(c, b + copysignf(sqrt_approx(__fmul_rn(p.disc, p.a)), b));
+    return __fdividef(c, __fadd_rn(-dot3(Oe, de), p.root));
 }
-// Whether the stretch meets [tmin, tmax].
+// Whether the stretch meets [tmin, tmax].  Its far end is the quadratic formula's root and nothing that rounds otherwise: where a
+// Gaussian ends as a slab begins, the one decides whether the slab is empty, and so where the ray's next slab lies.
 __device__ __forceinline__ bool stretch_meets(const RayParabola& p, float tmin, float tmax) {
-    return __fadd_rn(p.t0, -p.hw) <= tmax && __fadd_rn(p.t0, p.hw) >= tmin;
+    return __fadd_rn(p.t0, -p.hw) <= tmax && p.far >= tmin;
 }
 
 struct LeafTest {
