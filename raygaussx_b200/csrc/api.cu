@@ -60,7 +60,7 @@ struct rgx_ctx {
     int bin_tiles_cap = 0;
     size_t bin_pair_cap = 0, bin_ent_cap = 0, bin_cub_cap = 0;
     uint64_t *bin_keys_in = nullptr, *bin_keys_out = nullptr;
-    uint32_t *bin_vals_in = nullptr, *bin_vals_out = nullptr;
+    uint32_t *bin_vals_in = nullptr, *bin_vals_out = nullptr, *bin_ranks = nullptr;
     int *tile_cnt = nullptr, *tile_pbegin = nullptr;
     // what an emission starts from zero, in one piece cleared by one memset (see ZeroedBins)
     unsigned char* bin_zero = nullptr; size_t bin_zero_cap = 0;
@@ -193,7 +193,7 @@ void release_workspace(rgx_ctx* ctx) {
                      (void**)&ctx->g2, (void**)&ctx->quat, (void**)&ctx->sdens, (void**)&ctx->rgba,
                      (void**)&ctx->grad_rows, (void**)&ctx->hk, (void**)&ctx->refit_counters, (void**)&ctx->cub_temp,
                      (void**)&ctx->bounds, (void**)&ctx->box, (void**)&ctx->counters, (void**)&ctx->next_unit, (void**)&ctx->bin_keys_in,
-                     (void**)&ctx->bin_keys_out, (void**)&ctx->bin_vals_in, (void**)&ctx->bin_vals_out,
+                     (void**)&ctx->bin_keys_out, (void**)&ctx->bin_vals_in, (void**)&ctx->bin_vals_out, (void**)&ctx->bin_ranks,
                      (void**)&ctx->tile_cnt, (void**)&ctx->tile_pbegin, (void**)&ctx->ent_id, (void**)&ctx->ent_range, (void**)&ctx->ent_blk,
                      (void**)&ctx->bin_cub, (void**)&ctx->bin_zero, (void**)&ctx->tape, (void**)&ctx->tape_used,
                      (void**)&ctx->ray_head, (void**)&ctx->tile_dir, (void**)&ctx->tile_iota,
@@ -547,7 +547,8 @@ static cudaError_t grow_pairs(rgx_ctx* ctx, size_t pairs) {
     size_t c = pairs + pairs / 4 + 1024;
     cudaError_t err;
     if ((err = regrow(ctx, ctx->bin_keys_in, c)) != cudaSuccess || (err = regrow(ctx, ctx->bin_keys_out, c)) != cudaSuccess ||
-        (err = regrow(ctx, ctx->bin_vals_in, c)) != cudaSuccess || (err = regrow(ctx, ctx->bin_vals_out, c)) != cudaSuccess)
+        (err = regrow(ctx, ctx->bin_vals_in, c)) != cudaSuccess || (err = regrow(ctx, ctx->bin_vals_out, c)) != cudaSuccess ||
+        (err = regrow(ctx, ctx->bin_ranks, c)) != cudaSuccess)
         return err;
     ctx->bin_pair_cap = c;
     return cudaSuccess;
@@ -606,8 +607,20 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     b.row_begin = m->row_begin; b.row_end = m->row_end; b.tile = tile;
     b.tiles_x = tiles_x; b.tiles_y = tiles_y; b.ty_first = ty_first;
     b.zero = ctx->bin_zero; b.zero_bytes = z.bytes;
+    b.result = reinterpret_cast<BinResult*>(ctx->bin_zero);
+    b.tile_cnt = ctx->tile_cnt;
+    b.tile_pbegin = ctx->tile_pbegin;
+    b.tile_iota = ctx->tile_iota; b.tile_cnt_sorted = ctx->tile_cnt_sorted;
+    b.tile_order = ctx->tile_order;
+    if (ctx->tape_valid && ctx->tape_order == ctx->tile_order) {          // the replay of the latest recording still needs that one
+        if (ntiles > ctx->tape_order_cap) {
+            RGB_(tape_tile_order, (size_t)ntiles + 64);
+            ctx->tape_order_cap = ntiles + 64;
+        }
+        b.tile_order = ctx->tape_tile_order;
+    }
     b.total_dev = reinterpret_cast<BinResult*>(ctx->bin_zero)->total;
-    b.tile_first = reinterpret_cast<int*>(ctx->bin_zero + z.first); b.tile_last = reinterpret_cast<int*>(ctx->bin_zero + z.last);
+    b.tile_first = reinterpret_cast<int*>(ctx->bin_zero + z.first);
     b.tile_pcnt = reinterpret_cast<int*>(ctx->bin_zero + z.pcnt);
     ctx->tile_more = reinterpret_cast<int*>(ctx->bin_zero + z.more);
     b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID;
@@ -638,7 +651,7 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
 // ... the kernels and the copy of the pair count to the host, enqueued ...
 static int emit_launch(rgx_ctx* ctx, BinLaunch& b, cudaStream_t s) {
     cudaError_t e;
-    b.keys_in = ctx->bin_keys_in; b.vals_in = ctx->bin_vals_in; b.pair_cap = ctx->bin_pair_cap;
+    b.keys_in = ctx->bin_keys_in; b.vals_in = ctx->bin_vals_in; b.ranks = ctx->bin_ranks; b.pair_cap = ctx->bin_pair_cap;
     if ((e = launch_bin_emit(b, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list pairs");
     // the number of pairs and the horizon travel together
     if ((e = cudaMemcpyAsync(ctx->bin_result_host, ctx->bin_zero, sizeof(BinResult), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
@@ -688,20 +701,9 @@ static int fill_lists(rgx_ctx* ctx, BinLaunch& b, uint64_t* keys, uint32_t* vals
     b.keys_in = keys; b.vals_in = vals;
     b.keys_out = ctx->bin_keys_out; b.vals_out = ctx->bin_vals_out;
     b.pair_cap = ctx->bin_pair_cap;
-    b.tile_cnt = ctx->tile_cnt;
-    b.tile_pbegin = ctx->tile_pbegin;
-    b.tile_iota = ctx->tile_iota; b.tile_cnt_sorted = ctx->tile_cnt_sorted;
-    b.tile_order = ctx->tile_order;
-    if (ctx->tape_valid && ctx->tape_order == ctx->tile_order) {          // the replay of the latest recording still needs that one
-        if (ntiles > ctx->tape_order_cap) {
-            RGB_(tape_tile_order, (size_t)ntiles + 64);
-            ctx->tape_order_cap = ntiles + 64;
-        }
-        b.tile_order = ctx->tape_tile_order;
-    }
     b.ent_id = ctx->ent_id; b.ent_range = ctx->ent_range; b.blk = ctx->ent_blk;
     b.cub_temp = ctx->bin_cub; b.cub_bytes = ctx->bin_cub_cap;
-    if ((e = launch_bin_fill(b, count, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list fill");
+    if ((e = launch_bin_fill(b, count, *ctx->bin_result_host, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list fill");
     ctx->lists.ent_id = ctx->ent_id; ctx->lists.ent_range = ctx->ent_range; ctx->lists.blk = ctx->ent_blk;
     ctx->lists.tile_pbegin = ctx->tile_pbegin; ctx->lists.tile_cnt = ctx->tile_cnt; ctx->lists.tile_order = b.tile_order;
     ctx->lists.tiles_x = b.tiles_x; ctx->lists.tiles_y = b.tiles_y; ctx->lists.ty_first = b.ty_first;

@@ -2,9 +2,9 @@
 //
 // All rays of a view leave from one point, so which Gaussians a ray can meet is
 // decided by where the Gaussian projects on the image.  Once per view every
-// Gaussian is projected to a rectangle of 16x16-pixel tiles and paired with each
-// tile it touches; the pairs are sorted by (tile, nearest distance from the eye)
-// with one radix sort, and every tile ends up with a front-to-back list of
+// Gaussian is projected to a rectangle of tiles (bin_tile_size) and paired with each
+// tile it touches; the pairs are dealt to their tiles and sorted there by the nearest
+// distance from the eye, and every tile ends up with a front-to-back list of
 // candidate Gaussians with, per entry, the range of distances its box spans.  A ray
 // then never searches the hierarchy: it slides along its tile's list.
 //
@@ -14,7 +14,6 @@
 #include "rgx_internal.cuh"
 #include "device_math.cuh"
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 #include <cub/block/block_scan.cuh>
 #include <cstring>
 
@@ -543,7 +542,8 @@ __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunc
         __syncwarp();
         for (int i = lane; i < nbuf; i += 32) {
             const unsigned long long k = base + (unsigned long long)i;
-            if (k < b.pair_cap) { b.keys_in[k] = keys[i]; b.vals_in[k] = __float_as_uint(fars[i]); }
+            const unsigned rank = atomicAdd(&b.tile_pcnt[(int)(keys[i] >> (kl.near_bits + kl.id_bits))], 1);
+            if (k < b.pair_cap) { b.keys_in[k] = keys[i]; b.vals_in[k] = __float_as_uint(fars[i]); b.ranks[k] = rank; }
         }
         nbuf = 0;
         __syncwarp();
@@ -581,21 +581,181 @@ __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunc
     flush();
 }
 
-__global__ void __launch_bounds__(256) bin_ranges_kernel(BinLaunch b, int total, int tile_shift) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= total) return;
-    int t = (int)(b.keys_out[k] >> tile_shift);
-    if (k == 0 || (int)(b.keys_out[k - 1] >> tile_shift) != t) b.tile_first[t] = k;
-    if (k == total - 1 || (int)(b.keys_out[k + 1] >> tile_shift) != t) b.tile_last[t] = k + 1;
+// ---------------------------------------------------------------- lists that fit shared memory
+//
+// The emission has counted every tile's pairs and numbered each pair among them.  From that, one block lays the lists out
+// (bin_layout_kernel: begin of each tile's pairs and of its padded list, the order of the tiles), the pairs are put in their tile's
+// place (bin_place_kernel), and a block per tile sorts them and writes the list (bin_sort_tiles_kernel).  Three launches and two
+// passes over the pairs in place of a radix sort of all of them by 48 bits (six passes and a histogram), the ranges, counts,
+// scan, sort of the tiles, padding, scatter and summaries that follow it: some twenty launches.  Lists per view: 3 M-Gaussian
+// window 0.63 -> 0.35 ms, 1 M at 640x360 0.51 -> 0.39, 30 k at 400x400 0.24 -> 0.17, 4 k at 64x64 0.18 -> 0.09 (launches and the
+// host's wait bound the last two).  Lists of more than kSortLong pairs do not fit a block (12 bytes a pair in 227 KB); a view that
+// has one takes the radix sort.
+
+// (begin of tile t's pairs in tile_first, of its padded list in tile_pbegin, tiles by falling number of pairs in tile_order)
+constexpr int kLayoutThreads = 1024;
+__global__ void __launch_bounds__(kLayoutThreads) bin_layout_kernel(BinLaunch b, int ntiles) {
+    using Scan = cub::BlockScan<int2, kLayoutThreads>;
+    __shared__ typename Scan::TempStorage tmp;
+    __shared__ int s_bucket[256];
+    __shared__ int s_longest, s_many;
+    const int t = threadIdx.x;
+    if (t == 0) { s_longest = 0; s_many = 0; }
+    if (t < 256) s_bucket[t] = 0;
+    __syncthreads();
+    int2 carry = make_int2(0, 0);
+    int longest = 0, many = 0;
+    for (int base = 0; base <= ntiles; base += kLayoutThreads) {
+        const int i = base + t, n = i < ntiles ? b.tile_pcnt[i] : 0;
+        int2 at, sum;
+        Scan(tmp).ExclusiveScan(make_int2(n, (n + 31) & ~31), at, make_int2(0, 0), [](int2 x, int2 y) { return make_int2(x.x + y.x, x.y + y.y); }, sum);
+        if (i <= ntiles) { b.tile_first[i] = carry.x + at.x; b.tile_pbegin[i] = carry.y + at.y; }
+        if (i < ntiles) b.tile_cnt[i] = n;
+        carry = make_int2(carry.x + sum.x, carry.y + sum.y);
+        longest = max(longest, n);
+        many += n > kSortShort ? 1 : 0;
+        __syncthreads();
+    }
+    longest = __reduce_max_sync(kFullMask, longest);
+    many = __reduce_add_sync(kFullMask, many);
+    if ((t & 31) == 0) { atomicMax(&s_longest, longest); if (many) atomicAdd(&s_many, many); }
+    __syncthreads();
+    longest = s_longest;
+    if (t == 0) { b.result->longest = (unsigned)longest; b.result->long_tiles = (unsigned)s_many; }
+    // Buckets by length, the longest first; bucket boundaries put every list of more than kSortShort pairs before all others.
+    auto bucket = [&](int n) {
+        if (n > kSortShort) return 127 - (int)((long long)(n - kSortShort) * 127 / max(longest - kSortShort, 1));
+        return 255 - n * 127 / kSortShort;
+    };
+    for (int i = t; i < ntiles; i += kLayoutThreads) atomicAdd(&s_bucket[bucket(b.tile_pcnt[i])], 1);
+    __syncthreads();
+    if (t < 32) {                                                        // exclusive scan of 256 counts by one warp
+        int run = 0;
+        for (int k = 0; k < 256; k += 32) {
+            int v = s_bucket[k + t], incl = v;
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(kFullMask, incl, o); if (t >= o) incl += u; }
+            s_bucket[k + t] = run + incl - v;
+            run += __shfl_sync(kFullMask, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < ntiles; i += kLayoutThreads) b.tile_order[atomicAdd(&s_bucket[bucket(b.tile_pcnt[i])], 1)] = i;
 }
 
-__global__ void bin_tile_counts_kernel(BinLaunch b, int ntiles) {
+__global__ void __launch_bounds__(256) bin_place_kernel(BinLaunch b, int total, int tile_shift) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= total) return;
+    const uint64_t key = b.keys_in[k];
+    const int dest = b.tile_first[(int)(key >> tile_shift)] + (int)b.ranks[k];
+    b.keys_out[dest] = key;
+    b.vals_out[dest] = b.vals_in[k];
+}
+
+// A block sorts the pairs of one tile by (near, slot) -- distinct keys, so the order does not depend on that of emission -- and writes
+// its list, padded to blocks of 32 with empty ranges, and the block summaries.  The pairs are dealt into kSortBuckets buckets by
+// near distance, about one pair each, and ranked inside their bucket by comparison; where many share a distance (an eye inside
+// many Gaussians) a bucket would be too long for that, and the block sorts with a bitonic network.  1024 threads for the lists of
+// more than kSortShort pairs, of which an SM holds few blocks; 256 for the others, eight blocks an SM.
+constexpr int kSortCrowd = 96;
+__host__ __device__ constexpr size_t sort_smem(int cap) { return (size_t)cap * (8 + 4) + (size_t)(cap / 32) * 4; }
+template <int kSortThreads, int kSortBuckets>
+__global__ void __launch_bounds__(kSortThreads) bin_sort_tiles_kernel(BinLaunch b, KeyLayout kl, int first_unit, int cap) {
+    extern __shared__ __align__(16) unsigned char sort_mem[];
+    uint64_t* key = reinterpret_cast<uint64_t*>(sort_mem);               // [cap] near | slot
+    unsigned* at = reinterpret_cast<unsigned*>(key + cap);               // [cap] pair numbers by bucket, or in order
+    unsigned* far_max = at + cap;                                        // [cap / 32]
+    __shared__ unsigned s_start[kSortBuckets];
+    __shared__ unsigned s_lo, s_hi, s_most, s_warp[kSortThreads / 32];
+    const int t = threadIdx.x, lane = t & 31;
+    const int tile = b.tile_order[first_unit + blockIdx.x];
+    const int n = b.tile_cnt[tile];
+    if (n == 0) return;
+    const int seg = b.tile_first[tile], out = b.tile_pbegin[tile];
+    const uint64_t mask = (1ull << (kl.near_bits + kl.id_bits)) - 1ull;
+    for (int i = t; i < kSortBuckets; i += kSortThreads) s_start[i] = 0u;
+    for (int i = t; i < (n + 31) / 32; i += kSortThreads) far_max[i] = 0u;
+    if (t == 0) { s_lo = ~0u; s_hi = 0u; s_most = 0u; }
+    __syncthreads();
+    unsigned lo = ~0u, hi = 0u;
+    for (int i = t; i < n; i += kSortThreads) {
+        const uint64_t k = b.keys_out[seg + i] & mask;
+        key[i] = k;
+        const unsigned q = (unsigned)(k >> kl.id_bits);
+        lo = min(lo, q); hi = max(hi, q);
+    }
+    lo = __reduce_min_sync(kFullMask, lo); hi = __reduce_max_sync(kFullMask, hi);
+    if (lane == 0) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
+    __syncthreads();
+    lo = s_lo;
+    const float scale = (float)kSortBuckets / (float)(s_hi - lo + 1u);
+    auto bucket = [&](uint64_t k) { return min((int)((float)((unsigned)(k >> kl.id_bits) - lo) * scale), kSortBuckets - 1); };   // monotone in the distance
+    for (int i = t; i < n; i += kSortThreads) atomicAdd(&s_start[bucket(key[i])], 1u);
+    __syncthreads();
+    // exclusive scan of the buckets, eight per thread
+    constexpr int kPer = kSortBuckets / kSortThreads;
+    unsigned c[kPer], sum = 0u, most = 0u;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) { c[k] = s_start[t * kPer + k]; sum += c[k]; most = max(most, c[k]); }
+    unsigned incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned u = __shfl_up_sync(kFullMask, incl, o); if (lane >= o) incl += u; }
+    if (lane == 31) s_warp[t >> 5] = incl;
+    most = __reduce_max_sync(kFullMask, most);
+    if (lane == 0) atomicMax(&s_most, most);
+    __syncthreads();
+    unsigned run = incl - sum;
+    for (int w = 0; w < (t >> 5); ++w) run += s_warp[w];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) { s_start[t * kPer + k] = run; run += c[k]; }
+    __syncthreads();
+    const bool crowded = s_most > (unsigned)kSortCrowd;
+    if (crowded) {
+        int size = 1;
+        while (size < n) size <<= 1;
+        for (int i = t; i < size; i += kSortThreads) at[i] = (unsigned)i;                  // numbers past the end compare as largest
+        __syncthreads();
+        auto value = [&](unsigned i) { return i < (unsigned)n ? key[i] : ~0ull; };
+        for (int k = 2; k <= size; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int p = t; p < size / 2; p += kSortThreads) {
+                    const int x = ((p & ~(j - 1)) << 1) | (p & (j - 1)), y = x | j;
+                    const unsigned ax = at[x], ay = at[y];
+                    if ((value(ax) > value(ay)) == ((x & k) == 0)) { at[x] = ay; at[y] = ax; }
+                }
+                __syncthreads();
+            }
+    } else {
+        for (int i = t; i < n; i += kSortThreads) at[atomicAdd(&s_start[bucket(key[i])], 1u)] = (unsigned)i;    // s_start: now the ends
+        __syncthreads();
+    }
+    for (int p = t; p < n; p += kSortThreads) {
+        const unsigned i = at[p];
+        const uint64_t k = key[i];
+        int rank = p;
+        if (!crowded) {
+            const int w = bucket(k), begin = w ? (int)s_start[w - 1] : 0, end = (int)s_start[w];
+            rank = begin;
+            for (int q = begin; q < end; ++q) rank += key[at[q]] < k ? 1 : 0;
+        }
+        const float near = near_stored((unsigned)(k >> kl.id_bits), kl);
+        const unsigned far = b.vals_out[seg + i];
+        b.ent_id[out + rank] = (int)(k & ((1ull << kl.id_bits) - 1ull));
+        b.ent_range[out + rank] = make_float2(near, __uint_as_float(far));
+        atomicMax(&far_max[rank >> 5], far);                                               // distances: positive, ordered like their bits
+        if ((rank & 31) == 0) b.blk[(out + rank) >> 5].x = near;
+    }
+    for (int i = n + t; i < ((n + 31) & ~31); i += kSortThreads) {
+        b.ent_id[out + i] = 0;
+        b.ent_range[out + i] = make_float2(INFINITY, -INFINITY);
+    }
+    __syncthreads();
+    for (int i = t; i < (n + 31) / 32; i += kSortThreads) b.blk[(out >> 5) + i].y = __uint_as_float(far_max[i]);
+}
+
+// ---------------------------------------------------------------- lists of any length: after the radix sort
+__global__ void bin_tile_iota_kernel(BinLaunch b, int ntiles) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntiles) return;
-    int cnt = b.tile_last[t] - b.tile_first[t];
-    b.tile_cnt[t] = cnt;
-    b.tile_pcnt[t] = ((cnt + 31) / 32) * 32;
-    b.tile_iota[t] = t;
+    if (t < ntiles) b.tile_iota[t] = t;
 }
 
 __global__ void __launch_bounds__(256) bin_fill_kernel(BinLaunch b, size_t n_entries) {
@@ -634,15 +794,13 @@ __global__ void __launch_bounds__(256) bin_blocks_kernel(BinLaunch b, size_t n_b
 }  // namespace
 
 size_t binning_cub_temp_bytes(size_t pair_cap, int ntiles) {
-    size_t a = 0, d = 0;
+    size_t a = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, a, (const uint64_t*)nullptr, (uint64_t*)nullptr, (const uint32_t*)nullptr,
                                     (uint32_t*)nullptr, (int64_t)pair_cap, 0, 64, (cudaStream_t)0);
-    cub::DeviceScan::ExclusiveSum(nullptr, d, (const int*)nullptr, (int*)nullptr, ntiles + 1, (cudaStream_t)0);
     size_t o = 0;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, o, (const int*)nullptr, (int*)nullptr, (const int*)nullptr,
                                               (int*)nullptr, ntiles, 0, 32, (cudaStream_t)0);
-    if (o > a) a = o;
-    return a > d ? a : d;
+    return o > a ? o : a;
 }
 
 // Phase 1: all (tile, Gaussian) pairs -- with b.pick those that begin before the horizon picked on the way --,
@@ -664,38 +822,49 @@ cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s) {
         note_launch(), bin_compact_kernel<<<(b.n_pad + 255) / 256, 256, 0, s>>>(b);
         note_launch(), bin_emit_pairs_kernel<true><<<b.big_grid, kBigWarps * 32, 0, s>>>(b);
         note_launch(), bin_tile_more_kernel<<<1, 1024, 0, s>>>(b);
+        note_launch(), bin_layout_kernel<<<1, kLayoutThreads, 0, s>>>(b, ntiles);
         return cudaGetLastError();
     }
     note_launch(), bin_tile_dirs_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
     note_launch(), bin_list_kernel<<<blocks, kEmitThreads, 0, s>>>(b);
     note_launch(), bin_emit_pairs_kernel<false><<<b.big_grid, kBigWarps * 32, 0, s>>>(b);
+    note_launch(), bin_layout_kernel<<<1, kLayoutThreads, 0, s>>>(b, ntiles);
     return cudaGetLastError();
 }
 
-// Phase 2: sort, per-tile ranges, padded layout, block summaries.
-cudaError_t launch_bin_fill(const BinLaunch& b, int total, cudaStream_t s) {
+// Phase 2: the pairs of every tile in order, padded layout, block summaries.  r: what the emission left for the host.
+cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, cudaStream_t s) {
     const int tb = 256;
     const int ntiles = b.tiles_x * b.tiles_y;
+    if (total == 0) return cudaSuccess;                    // every list is empty: the counts say so
     // the layout is that of the whole image whatever the row range, so that a row range sees the same order
     const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
+    if (r.longest <= (unsigned)kSortLong) {
+        note_launch(), bin_place_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl.near_bits + kl.id_bits);
+        int cap = kSortShort;
+        while (cap < (int)r.longest) cap <<= 1;
+        if (r.long_tiles) {                                // tile_order has these first
+            cudaError_t e = cudaFuncSetAttribute(bin_sort_tiles_kernel<1024, 4096>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortLong));
+            if (e != cudaSuccess) return e;
+            note_launch(), bin_sort_tiles_kernel<1024, 4096><<<r.long_tiles, 1024, sort_smem(cap), s>>>(b, kl, 0, cap);
+        }
+        if ((int)r.long_tiles < ntiles)
+            note_launch(), bin_sort_tiles_kernel<256, 2048><<<ntiles - (int)r.long_tiles, 256, sort_smem(kSortShort), s>>>(b, kl, (int)r.long_tiles, kSortShort);
+        return cudaGetLastError();
+    }
     cudaError_t e;
     size_t temp = b.cub_bytes;
-    if (total > 0) {
-        e = cub::DeviceRadixSort::SortPairs(b.cub_temp, temp, b.keys_in, b.keys_out, b.vals_in, b.vals_out, (int64_t)total, 0,
-                                            kl.tile_bits + kl.near_bits + kl.id_bits, s);
-        if (e != cudaSuccess) return e;
-        note_launch(), bin_ranges_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl.near_bits + kl.id_bits);
-    }
-    note_launch(), bin_tile_counts_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
-    temp = b.cub_bytes;
-    if ((e = cub::DeviceScan::ExclusiveSum(b.cub_temp, temp, b.tile_pcnt, b.tile_pbegin, ntiles + 1, s)) != cudaSuccess) return e;
+    e = cub::DeviceRadixSort::SortPairs(b.cub_temp, temp, b.keys_in, b.keys_out, b.vals_in, b.vals_out, (int64_t)total, 0,
+                                        kl.tile_bits + kl.near_bits + kl.id_bits, s);
+    if (e != cudaSuccess) return e;
     // CTAs take the tiles with the longest lists first: the march ends with short tiles, not with one long one
+    note_launch(), bin_tile_iota_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
     temp = b.cub_bytes;
     if ((e = cub::DeviceRadixSort::SortPairsDescending(b.cub_temp, temp, b.tile_cnt, b.tile_cnt_sorted, b.tile_iota, b.tile_order,
                                                        ntiles, 0, 32, s)) != cudaSuccess) return e;
     const size_t n_entries = (((size_t)total + 32u * (size_t)ntiles + 31) / 32) * 32;   // upper bound of the padded layout
     note_launch(), bin_fill_kernel<<<(unsigned)((n_entries + tb - 1) / tb), tb, 0, s>>>(b, n_entries);
-    if (total > 0) note_launch(), bin_scatter_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl);
+    note_launch(), bin_scatter_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl);
     const size_t n_blocks = (n_entries + 31) / 32;
     note_launch(), bin_blocks_kernel<<<(unsigned)((n_blocks + 7) / 8), 256, 0, s>>>(b, n_blocks);
     return cudaGetLastError();

@@ -113,19 +113,20 @@ struct BinResult {
     unsigned long long total[4];        // [0] pairs met (may exceed the capacity), [1] Gaussians listed by bin_list_kernel, [2] next listed
                                         // Gaussian to take, [3] Gaussians listed by bin_compact_kernel
     HorizonPick pick;
+    unsigned int longest, long_tiles;   // pairs of the longest list; lists of more than kSortShort pairs (bin_layout_kernel)
 };
+constexpr int kSortShort = 2048, kSortLong = 16384;   // lists that a block sorts in shared memory (binning.cu)
 // That piece, as byte offsets: the result, the histogram of nearest distances, per tile first and last pair and padded count,
 // corners of culled rectangles, tiles that have more pairs.
 struct ZeroedBins {
-    size_t hist, first, last, pcnt, diff, more, bytes;
+    size_t hist, first, pcnt, diff, more, bytes;     // pcnt: pairs per tile, counted by the emission
 };
 inline ZeroedBins zeroed_bins(int tiles_x, int tiles_y) {
     const size_t tiles = (size_t)tiles_x * tiles_y, align = 255;
     ZeroedBins z;
     z.hist = (sizeof(BinResult) + align) & ~align;
     z.first = z.hist + 2048 * sizeof(unsigned long long);
-    z.last = (z.first + sizeof(int) * (tiles + 1) + align) & ~align;
-    z.pcnt = (z.last + sizeof(int) * (tiles + 1) + align) & ~align;
+    z.pcnt = (z.first + sizeof(int) * (tiles + 1) + align) & ~align;
     z.diff = (z.pcnt + sizeof(int) * (tiles + 1) + align) & ~align;
     z.more = (z.diff + sizeof(int) * (size_t)(tiles_x + 1) * (tiles_y + 1) + align) & ~align;
     z.bytes = z.more + sizeof(int) * tiles;
@@ -142,8 +143,10 @@ struct BinLaunch {
     int row_begin, row_end, tile, tiles_x, tiles_y, ty_first;
     uint64_t *keys_in, *keys_out;          // [pair capacity] (tile, near distance, sorted slot)
     uint32_t *vals_in, *vals_out;          // [pair capacity] far distance (float bits)
+    uint32_t* ranks;                       // [pair capacity] the pair's number among its tile's, in no particular order
+    BinResult* result;
     unsigned long long pair_cap;
-    int *tile_first, *tile_last, *tile_cnt, *tile_pcnt, *tile_pbegin;   // [tiles + 1]
+    int *tile_first, *tile_cnt, *tile_pcnt, *tile_pbegin;   // [tiles + 1]
     int *tile_iota, *tile_cnt_sorted, *tile_order;                      // [tiles]
     int* ent_id; float2* ent_range; float2* blk;
     float4* tile_dir;                      // [tiles] central ray direction, chord to the farthest corner ray
@@ -262,7 +265,7 @@ cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeLaunch& f, cudaStream_t s);
 size_t binning_cub_temp_bytes(size_t pair_cap, int ntiles);
 cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s);
-cudaError_t launch_bin_fill(const BinLaunch& b, int total, cudaStream_t s);
+cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, cudaStream_t s);
 float bin_hist_bucket_end(const BinLaunch& b, int bucket);
 cudaError_t launch_march_forward(const MarchLaunch& m, cudaStream_t s);
 // The rays listed in m.hz_rays by a march over lists that stop at a horizon, again by per-ray search (march.cu).
