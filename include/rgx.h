@@ -265,7 +265,7 @@ RGX_API int rgx_activate_backward(int device, const rgx_activation* a, const rgx
  * loss[0] = (1 - lambda) mean|image - target| + lambda (1 - SSIM), target [3,h,w]; SSIM as utils/loss_utils.py:37-62
  * (11-tap Gaussian window of sigma 1.5, zero padding, constants 0.01^2 and 0.03^2).  maps: NULL, or 9*w*h floats that
  * the backward reads when lambda is not 0; scratch: rgx_image_loss_scratch_floats(w, h) floats, 8-byte aligned.  The backward writes
- * grad_loss[0] * dloss/drays to grad_rays [h*fy, w*fx, 3]; loss and grad_loss are device pointers.  Sums are fp32 per tile
+ * grad_loss[0] * dloss/drays to grad_rays [h*fy, w*fx, 3]; loss and grad_loss are device pointers (grad_loss null: 1).  Sums are fp32 per tile
  * of 32x32 pixels and double over tiles, in a fixed order. */
 RGX_API size_t rgx_image_loss_scratch_floats(int w, int h);
 RGX_API int rgx_image_loss(int device, const float* rays, const float* target, int w, int h, int fx, int fy, float lambda_ssim,

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_backward_kernel(Loss
         }
         __syncthreads();
     }
-    const float per_value = *grad_loss / (float)(3 * plane) / (float)(a.fx * a.fy);
+    const float per_value = (grad_loss ? *grad_loss : 1.0f) / (float)(3 * plane) / (float)(a.fx * a.fy);
     for (int j = ty; j < kTile; j += kRows) {
         const int x = x0 + tx, y = y0 + j;
         if (x >= a.w || y >= a.h) continue;
@@ -433,7 +433,7 @@ extern "C" RGX_API int rgx_image_loss(int device, const float* rays, const float
 
 extern "C" RGX_API int rgx_image_loss_backward(int device, const float* rays, const float* target, int w, int h, int fx, int fy,
                                                float lambda_ssim, const float* maps, const float* grad_loss, float* grad_rays, rgx_stream stream) {
-    if (bad_image(rays, target, w, h, fx, fy) || !grad_loss || !grad_rays || (lambda_ssim != 0.f && !maps)) return RGX_E_INVALID;
+    if (bad_image(rays, target, w, h, fx, fy) || !grad_rays || (lambda_ssim != 0.f && !maps)) return RGX_E_INVALID;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
     cudaStream_t s = (cudaStream_t)stream;

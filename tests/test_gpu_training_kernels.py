@@ -104,3 +104,32 @@ def test_densification_statistics(tr, n):
     a, b = clouds
     assert torch.allclose(a.xyz_gradient_accum_norm.cpu(), b.xyz_gradient_accum_norm, rtol=1e-5)
     assert torch.equal(a.num_accum.cpu(), b.num_accum) and torch.equal(a.num_accum_gnv.cpu(), b.num_accum_gnv)
+
+
+@pytest.mark.parametrize("coeffs,lobes,normalize,factor", [(1, 0, False, 1), (16, 0, True, 1), (4, 2, False, 2), (4, 3, True, 1)])
+def test_iteration_without_a_graph_is_the_one_with(tr, coeffs, lobes, normalize, factor):
+    """training_iteration calls its Functions itself where nothing asks for a graph; a hook asks for one."""
+    from raygaussx_b200 import scenes
+    sc = scenes.tiny_scene(n=700, width=33, height=21, log_scale_mean=-2.5, sh_degree=int(coeffs ** 0.5) - 1, lobes=lobes, seed=coeffs)
+    cam = sc.cameras[0].to("cuda")
+    cam.original_image = torch.rand(3, 21, 33, generator=torch.Generator().manual_seed(1))
+    cfg = tr.default_config(dt=0.01)
+    cfg.training.normalize_quaternion = cfg.training.normalize_lobe_axis = normalize
+    cfg.training.supersampling_x = factor
+    got = []
+    for hooked in (False, True):
+        pc = tr.SimplePointCloud(*[t.cuda() for t in sc.tensors()])
+        if hooked:
+            pc.positions.register_hook(lambda g: None)
+        grads = {}
+        step = pc.optim_managers.step
+        names = [g["name"] for g in pc.optim_managers.optimizer.param_groups]
+        pc.optim_managers.step = lambda: (grads.update({k: getattr(pc, k).grad.clone() for k in names}), step())
+        loss, stepped = tr.training_iteration(pc, cam, cfg, 0, tr.AccumulationSchedule())
+        assert stepped and not loss.requires_grad and all(getattr(pc, k).grad is None for k in names)
+        got.append((loss, grads, pc))
+    assert torch.equal(got[0][0], got[1][0])
+    for k, a in got[0][1].items():
+        b = got[1][1][k]
+        assert a.shape == b.shape and (a - b).abs().max() <= 2e-5 * b.abs().max().clamp_min(1e-30), k
+    assert torch.equal(got[0][2].num_accum, got[1][2].num_accum)
