@@ -91,6 +91,7 @@ struct rgx_ctx {
     bool lists_valid = false;
     // lists of a recording forward's view may hold only the pairs that begin before a horizon (lists_from_pairs)
     bool lists_partial = false;
+    bool lists_noted = false;          // g_rect, g_code and the pick on the host are those of the current lists
     float lists_horizon = 0.f;
     long long lists_rays = 0;          // rays of the view the partial lists were made for
     int near_budget_per_ray = RGX_NEAR_BUDGET;   // pairs per ray such lists keep; doubled whenever a ray reached the horizon
@@ -346,11 +347,12 @@ void fill_sorted(const rgx_ctx* ctx, SortedGaussians& g) {
     g.n = ctx->n; g.n_pad = ctx->n_pad;
 }
 
-// listed_only: the current lists stop at a horizon; only the Gaussians that were emitted for them get their colours
-// (the march, the replay of its recording and a search over the same lists meet no others).
+// listed_only: only the Gaussians that were emitted for the current lists get their colours, if the emission left a note of
+// them -- those whose rectangle lies in the image and which begin before the horizon, should the lists stop at one (the march, the
+// replay of its recording and a search over the same lists meet no others).
 int run_colors(rgx_ctx* ctx, const rgx_scene* sc, const float eye[3], cudaStream_t s, bool listed_only = false) {
     ColorLaunch c{};
-    const bool listed = listed_only && ctx->lists_partial && ctx->g_code && ctx->listed && ctx->listed_cap >= ctx->n_pad;
+    const bool listed = listed_only && ctx->lists_noted && ctx->g_code && ctx->listed && ctx->listed_cap >= ctx->n_pad;
     if (listed) {
         c.listed_rect = ctx->g_rect; c.listed_code = ctx->g_code; c.listed_cut = ctx->bin_result_host->pick.cut;
         c.listed_out = ctx->listed;
@@ -623,7 +625,7 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     b.tile_first = reinterpret_cast<int*>(ctx->bin_zero + z.first);
     b.tile_pcnt = reinterpret_cast<int*>(ctx->bin_zero + z.pcnt);
     ctx->tile_more = reinterpret_cast<int*>(ctx->bin_zero + z.more);
-    b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID;
+    b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID; b.sm_count = ctx->sm_count;
     if (cull && cull->budget_per_ray > 0) {
         // only the pairs that begin before a horizon are emitted (binning.cu)
         int rc = two_depth_workspace(ctx, ntiles);          // the counter of rays that reach the horizon
@@ -711,12 +713,13 @@ static int fill_lists(rgx_ctx* ctx, BinLaunch& b, uint64_t* keys, uint32_t* vals
     return RGX_OK;
 }
 
-static void lists_now_valid(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, int total) {
+static void lists_now_valid(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, int total, bool noted) {
     ctx->lists_cam = *cam;
     ctx->lists_row_begin = m->row_begin; ctx->lists_row_end = m->row_end;
     ctx->lists_build_id = ctx->build_id;
     ctx->lists_valid = true;
     ctx->lists_partial = false;
+    ctx->lists_noted = noted;
     ctx->last_pairs = total;
 }
 
@@ -753,7 +756,7 @@ static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, c
                             cudaStream_t s) {
     int rc;
     if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
-    lists_now_valid(ctx, cam, m, total);
+    lists_now_valid(ctx, cam, m, total, b.pick != nullptr);
     if (b.pick) learn_ratio(ctx, ctx->near_ratio, total);
     if (b.pick && ctx->bin_result_host->pick.cut != kAllBuckets) {
         const HorizonPick& pk = ctx->bin_result_host->pick;
@@ -770,7 +773,7 @@ static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, c
 static int ensure_lists(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, cudaStream_t s, bool near_only = false,
                         bool near_cached_ok = false) {
     if (lists_cached(ctx, cam, m) && (!ctx->lists_partial || near_only || near_cached_ok)) return RGX_OK;
-    ctx->lists_valid = false;
+    ctx->lists_valid = ctx->lists_noted = false;
     if (m->row_end <= m->row_begin || ctx->n == 0) return RGX_OK;   // nothing to march
     ScopedTimer timer(ctx, s, 2);
     BinLaunch b;
@@ -816,7 +819,7 @@ static void lists_ahead_begin(rgx_ctx* ctx, cudaStream_t s, ListsAhead& a) {
         }
     }
     if (cudaEventRecord(ctx->ev_main, s) != cudaSuccess || cudaStreamWaitEvent(ctx->side, ctx->ev_main, 0) != cudaSuccess) return;
-    ctx->lists_valid = false;                      // from here on the list arrays belong to the announced view
+    ctx->lists_valid = ctx->lists_noted = false;   // from here on the list arrays belong to the announced view
     const bool near_only = (m->flags & RGX_FLAG_SAVE_HITS) && !(m->flags & RGX_FLAG_COUNT_WORK);
     const Cull cull = near_cull(ctx);
     if (emit_setup(ctx, cam, m, a.b, a.ntiles, near_only ? &cull : nullptr) || emit_launch(ctx, a.b, ctx->side)) {
@@ -843,7 +846,7 @@ static void lists_ahead_end(rgx_ctx* ctx, ListsAhead& a) {
 // Forward-only march of a view with many more (tile, Gaussian) pairs than its rays will look at: the lists
 // are made in two depths (binning.cu) and the march runs in two phases (march_lists.cu, HZ variant).
 // handled = false: the view does not qualify; its complete lists have been made instead.
-static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, MarchLaunch& L, cudaStream_t s,
+static int forward_two_depth(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* cam, const rgx_march* m, MarchLaunch& L, cudaStream_t s,
                              bool& handled) {
     handled = false;
     cudaError_t e = cudaSuccess;
@@ -868,12 +871,14 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_marc
     const HorizonPick pk = ctx->bin_result_host->pick;
     learn_ratio(ctx, ctx->hz_ratio, total);
     if (pk.cut == kAllBuckets || total == 0) {                     // one depth is enough: these are the complete lists
-        lists_now_valid(ctx, cam, m, total);
+        lists_now_valid(ctx, cam, m, total, true);
         return RGX_OK;
     }
     if ((e = cudaMemsetAsync(ctx->tile_resume, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(ctx->hz_scalars, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess)
         return cuda_fail(ctx, e, "two-depth workspace");
+    ctx->lists_noted = true;
+    if ((rc = run_colors(ctx, scene, cam->eye, s, true))) return rc;
     L.lists = ctx->lists;
     L.hz_phase = 1; L.horizon = bin_hist_bucket_end(b, (int)pk.cut); L.hz_state = ctx->hz_state; L.tile_more = ctx->tile_more;
     L.tile_resume = ctx->tile_resume; L.hz_count = reinterpret_cast<unsigned int*>(ctx->hz_scalars + 1);
@@ -889,6 +894,7 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_camera* cam, const rgx_marc
     int total2 = 0;
     if (stopped > 0) {
         // second depth: all pairs of the tiles in which a ray stopped
+        if ((rc = run_colors(ctx, scene, cam->eye, s))) return rc;
         {
             ScopedTimer timer(ctx, s, 2);
             b.pick = nullptr;
@@ -944,7 +950,6 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
     join_side(ctx, s);
     L.rgb = rgb; L.alpha = alpha; L.depth = depth; L.frame = frame;
     const bool counting = (march->flags & RGX_FLAG_COUNT_WORK) != 0;
-    bool have_colors = false;
     if (!(march->flags & (RGX_FLAG_BRUTE_FORCE | RGX_FLAG_PER_RAY_SEARCH))) {
         // a forward that nothing follows (no recording, no counting) and whose lists are yet to be made may take
         // the two-depth path, if the view turns out to have far more pairs than rays
@@ -952,9 +957,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
                                   march->row_end > march->row_begin && ctx->hz_min_pairs_per_ray >= 0;
         if (forward_only && !lists_cached(ctx, cam, march)) {
             bool handled = false;
-            if ((rc = run_colors(ctx, scene, cam->eye, s))) return rc;
-            have_colors = true;
-            if ((rc = forward_two_depth(ctx, cam, march, L, s, handled))) return rc;
+            if ((rc = forward_two_depth(ctx, scene, cam, march, L, s, handled))) return rc;
             if (handled) return RGX_OK;
         } else {
             const bool counts = (march->flags & RGX_FLAG_COUNT_WORK) != 0;
@@ -963,7 +966,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         }
         L.lists = ctx->lists;
     }
-    if (!have_colors && (rc = run_colors(ctx, scene, cam->eye, s, L.lists.ent_id != nullptr && ctx->lists_partial && !counting)))
+    if ((rc = run_colors(ctx, scene, cam->eye, s, L.lists.ent_id != nullptr && !counting)))
         return rc;
     // one march of the view over the lists in L.lists (a lambda: a view whose lists stop at a horizon may need a second one)
     auto march_once = [&]() -> int {

@@ -154,7 +154,7 @@ struct BinLaunch {
     unsigned char* zero; size_t zero_bytes;// cleared before an emission; total_dev, pick ... tile_more point into it
     unsigned long long* total_dev;         // [4], see BinResult
     int* big_slot; uint2* big_rect;        // [n_pad] complete emission: the Gaussians that touch a tile, and their tile rectangles
-    int big_grid;                          // CTAs that work the list off (a few per SM)
+    int big_grid, sm_count;                // CTAs that work the list off (a few per SM)
     // culled emission (null / unused for a complete one): only the pairs that begin before a horizon are emitted
     HorizonPick* pick;
     unsigned long long* near_hist;         // [2048] estimated pairs by nearest distance of the Gaussian
