@@ -608,6 +608,7 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     if (!camera_dual(*cam, b.dual)) return fail(ctx, RGX_E_INVALID, "camera axes are not linearly independent");
     b.row_begin = m->row_begin; b.row_end = m->row_end; b.tile = tile;
     b.tiles_x = tiles_x; b.tiles_y = tiles_y; b.ty_first = ty_first;
+    b.proj = make_projector(b);
     b.zero = ctx->bin_zero; b.zero_bytes = z.bytes;
     b.result = reinterpret_cast<BinResult*>(ctx->bin_zero);
     b.tile_cnt = ctx->tile_cnt;

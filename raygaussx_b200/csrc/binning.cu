@@ -16,6 +16,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/block/block_scan.cuh>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace rgx {
@@ -23,34 +24,6 @@ namespace rgx {
 namespace {
 
 constexpr unsigned kFullMask = 0xffffffffu;
-
-struct Projector {     // pixel coordinates of a world point: px = (a / (2 tan) + pp) * size - 0.5
-    float eye[3], du[3], dv[3], dw[3];   // dual basis of (u, v, w)
-    float sx, sy, ox, oy;                // px = a * sx + ox, py = b * sy + oy
-    float plane[4][4];                   // the view's four side planes through the eye: inward normal, and its length
-};
-
-__device__ __forceinline__ Projector make_projector(const BinLaunch& b) {
-    Projector p;
-    for (int k = 0; k < 3; ++k) { p.eye[k] = b.cam.eye[k]; p.du[k] = b.dual[0][k]; p.dv[k] = b.dual[1][k]; p.dw[k] = b.dual[2][k]; }
-    p.sx = (float)b.cam.width / (2.0f * b.cam.tan_half_fov[0]);
-    p.sy = (float)b.cam.height / (2.0f * b.cam.tan_half_fov[1]);
-    p.ox = b.cam.pp[0] * (float)b.cam.width - 0.5f;
-    p.oy = b.cam.pp[1] * (float)b.cam.height - 0.5f;
-    // a point eye + t (a u + b v + w), t > 0, of a ray of the rows at hand has a within [a0, a1] and b within [b0, b1]
-    // (one pixel of margin), that is x_c - a0 z_c >= 0, a1 z_c - x_c >= 0 and the same for rows
-    const float a0 = (-1.0f - p.ox) / p.sx, a1 = ((float)b.cam.width - p.ox) / p.sx;
-    const float b0 = ((float)b.row_begin - 1.0f - p.oy) / p.sy, b1 = ((float)b.row_end - p.oy) / p.sy;
-    for (int k = 0; k < 3; ++k) {
-        p.plane[0][k] = p.du[k] - a0 * p.dw[k];
-        p.plane[1][k] = a1 * p.dw[k] - p.du[k];
-        p.plane[2][k] = p.dv[k] - b0 * p.dw[k];
-        p.plane[3][k] = b1 * p.dw[k] - p.dv[k];
-    }
-    for (int q = 0; q < 4; ++q)
-        p.plane[q][3] = sqrtf(p.plane[q][0] * p.plane[q][0] + p.plane[q][1] * p.plane[q][1] + p.plane[q][2] * p.plane[q][2]);
-    return p;
-}
 
 // Camera coordinates (x right, y down, z forward, in units of the ray parametrisation a = x/z, b = y/z).
 __device__ __forceinline__ void to_camera(const Projector& p, float x, float y, float z, float& xc, float& yc, float& zc) {
@@ -74,7 +47,8 @@ __device__ __forceinline__ int project_corners(const Projector& p, const float* 
         all_front = all_front && front;
         all_behind = all_behind && !(zc[c] > 0.f);
         if (front) {
-            float px = xc[c] / zc[c] * p.sx + p.ox, py = yc[c] / zc[c] * p.sy + p.oy;
+            const float inv = __fdividef(1.0f, zc[c]);               // the margins about the rectangle cover its rounding
+            float px = xc[c] * inv * p.sx + p.ox, py = yc[c] * inv * p.sy + p.oy;
             lox = fminf(lox, px); hix = fmaxf(hix, px);
             loy = fminf(loy, py); hiy = fmaxf(hiy, py);
         }
@@ -171,6 +145,18 @@ struct PairGeom {
 // the box and the ellipsoid grown by that much.
 __device__ __forceinline__ bool pair_range(const float* eye, float4 td, const PairGeom& g, float& tn, float& tf) {
     const float infl = g.far_box * td.w * 1.0001f + 1e-6f;
+    // ellipsoid |M (x - p)| <= 1 grown to radius rho in the whitened frame; first, since it turns away the more: a needle's
+    // rectangle is full of tiles beside it
+    const float rho = 1.0f + infl * g.rho_scale;
+    const float3 O = make_float3(eye[0] - g.g0.x, eye[1] - g.g0.y, eye[2] - g.g0.z);
+    const float3 Oe = make_float3(g.g0.w * O.x + g.g1.x * O.y + g.g1.y * O.z, g.g1.z * O.x + g.g1.w * O.y + g.g2.x * O.z,
+                                  g.g2.y * O.x + g.g2.z * O.y + g.g2.w * O.z);
+    const float3 de = make_float3(g.g0.w * td.x + g.g1.x * td.y + g.g1.y * td.z, g.g1.z * td.x + g.g1.w * td.y + g.g2.x * td.z,
+                                  g.g2.y * td.x + g.g2.z * td.y + g.g2.w * td.z);
+    const float qa = dot3(de, de), qb = -dot3(Oe, de), qc = dot3(Oe, Oe) - rho * rho;
+    const float disc = qb * qb - qa * qc;
+    const float mag = qb * qb + fabsf(qa * qc);
+    if (disc < -1e-5f * mag) return false;
     tn = 0.f; tf = INFINITY;
     const float o[3] = {eye[0], eye[1], eye[2]}, d[3] = {td.x, td.y, td.z};
     const float lo[3] = {g.bx.x - infl, g.by.x - infl, g.bz.x - infl}, hi[3] = {g.bx.y + infl, g.by.y + infl, g.bz.y + infl};
@@ -186,17 +172,6 @@ __device__ __forceinline__ bool pair_range(const float* eye, float4 td, const Pa
         }
     }
     if (tn > tf * (1.0f + 1e-5f) + 1e-6f) return false;
-    // ellipsoid |M (x - p)| <= 1 grown to radius rho in the whitened frame
-    const float rho = 1.0f + infl * g.rho_scale;
-    float3 O = make_float3(o[0] - g.g0.x, o[1] - g.g0.y, o[2] - g.g0.z);
-    float3 Oe = make_float3(g.g0.w * O.x + g.g1.x * O.y + g.g1.y * O.z, g.g1.z * O.x + g.g1.w * O.y + g.g2.x * O.z,
-                            g.g2.y * O.x + g.g2.z * O.y + g.g2.w * O.z);
-    float3 de = make_float3(g.g0.w * d[0] + g.g1.x * d[1] + g.g1.y * d[2], g.g1.z * d[0] + g.g1.w * d[1] + g.g2.x * d[2],
-                            g.g2.y * d[0] + g.g2.z * d[1] + g.g2.w * d[2]);
-    const float qa = dot3(de, de), qb = -dot3(Oe, de), qc = dot3(Oe, Oe) - rho * rho;
-    const float disc = qb * qb - qa * qc;
-    const float mag = qb * qb + fabsf(qa * qc);
-    if (disc < -1e-5f * mag) return false;
     if (qa > 1e-30f) {
         const float sq = sqrtf(fmaxf(disc, 0.f) + 1e-5f * mag);
         const float inv_qa = __fdividef(1.0f, qa);
@@ -348,6 +323,8 @@ __device__ __forceinline__ int gaussian_rect(const BinLaunch& b, const Projector
     return (int)((tx1 - tx0 + 1) * (ty1 - ty0 + 1));
 }
 
+constexpr unsigned kWideTiles = 128;     // rectangles of more tiles are listed apart
+__device__ __forceinline__ unsigned rect_tiles(uint2 r) { return ((r.x >> 16) - (r.x & 0xffffu) + 1u) * ((r.y >> 16) - (r.y & 0xffffu) + 1u); }
 constexpr int kHistBits = 11;      // leading bits of the quantised near distance: its exponent bits and 3 to 6 of the mantissa
 constexpr unsigned kNoRect = 0xffffffffu;
 
@@ -378,7 +355,7 @@ __global__ void __launch_bounds__(kEmitThreads) bin_near_hist_kernel(BinLaunch b
     if (j < b.n) {
         const float2 bx = b.bx[j], by = b.by[j], bz = b.bz[j];
         if (bx.x <= bx.y) {
-            const Projector p = make_projector(b);
+            const Projector& p = b.proj;
             const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
             uint2 r;
             const int count = gaussian_rect(b, p, j, bx, by, bz, r);
@@ -440,7 +417,7 @@ constexpr int kDiffShared = 11900;
 constexpr int kCompactThreads = 1024;
 __global__ void __launch_bounds__(kCompactThreads) bin_compact_kernel(BinLaunch b) {
     __shared__ int s_diff[kDiffShared];
-    __shared__ unsigned s_count[kCompactThreads / 32 + 1];
+    __shared__ unsigned s_count[2][kCompactThreads / 32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const unsigned cut = b.pick->cut;
     const int Wd = b.tiles_x + 1, cells = Wd * (b.tiles_y + 1);
@@ -450,7 +427,7 @@ __global__ void __launch_bounds__(kCompactThreads) bin_compact_kernel(BinLaunch 
     __syncthreads();
     for (int base = blockIdx.x * kCompactThreads; base < b.n; base += gridDim.x * kCompactThreads) {
         const int j = base + t;
-        bool keep = false;
+        bool keep = false, wide = false;
         if (j < b.n) {
             const uint2 rect = b.g_rect[j];
             if (rect.x != kNoRect) {
@@ -461,24 +438,26 @@ __global__ void __launch_bounds__(kCompactThreads) bin_compact_kernel(BinLaunch 
                     atomicAdd(&diff[(ty1 + 1) * Wd + tx0], -1);
                     atomicAdd(&diff[(ty1 + 1) * Wd + tx1 + 1], 1);
                 } else {
-                    keep = true;
+                    wide = rect_tiles(rect) > kWideTiles;
+                    keep = !wide;
                 }
             }
         }
-        const unsigned m = __ballot_sync(kFullMask, keep);
-        if (lane == 0) s_count[warp] = (unsigned)__popc(m);
+        const unsigned m = __ballot_sync(kFullMask, keep), mw = __ballot_sync(kFullMask, wide);
+        if (lane == 0) { s_count[0][warp] = (unsigned)__popc(m); s_count[1][warp] = (unsigned)__popc(mw); }
         __syncthreads();
-        if (warp == 0) {
-            const unsigned c = s_count[lane];
+        if (warp < 2) {
+            const unsigned c = s_count[warp][lane];
             unsigned incl = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const unsigned u = __shfl_up_sync(kFullMask, incl, o); if (lane >= o) incl += u; }
             unsigned at = 0;
-            if (lane == 31 && incl) at = (unsigned)atomicAdd(b.total_dev + 3, (unsigned long long)incl);
-            s_count[lane] = __shfl_sync(kFullMask, at, 31) + incl - c;
+            if (lane == 31 && incl) at = (unsigned)atomicAdd(b.total_dev + (warp == 0 ? 1 : 3), (unsigned long long)incl);
+            s_count[warp][lane] = __shfl_sync(kFullMask, at, 31) + incl - c;
         }
         __syncthreads();
-        if (keep) b.kept_slot[s_count[warp] + __popc(m & ((1u << lane) - 1u))] = j;
+        if (keep) b.kept_slot[s_count[0][warp] + __popc(m & ((1u << lane) - 1u))] = j;
+        if (wide) b.kept_slot[b.n_pad - 1 - (int)(s_count[1][warp] + __popc(mw & ((1u << lane) - 1u)))] = j;
         __syncthreads();
     }
     for (int i = t; local && i < cells; i += kCompactThreads)
@@ -511,7 +490,7 @@ __global__ void __launch_bounds__(1024) bin_tile_more_kernel(BinLaunch b) {
 }
 
 // Complete emission, first step: every Gaussian's rectangle of tiles; those that have one are listed (big_slot,
-// big_rect, their number in total_dev[1]) for bin_emit_pairs_kernel.  (A culled emission has the rectangles from
+// big_rect, those of many tiles from the back) for bin_emit_pairs_kernel.  (A culled emission has the rectangles from
 // bin_near_hist_kernel and the list from bin_compact_kernel.)
 __global__ void __launch_bounds__(kEmitThreads) bin_list_kernel(BinLaunch b) {
     const int j = blockIdx.x * kEmitThreads + threadIdx.x, lane = threadIdx.x & 31;
@@ -520,20 +499,29 @@ __global__ void __launch_bounds__(kEmitThreads) bin_list_kernel(BinLaunch b) {
     if (j < b.n) {
         const float2 bx = b.bx[j], by = b.by[j], bz = b.bz[j];
         if (bx.x <= bx.y) {
-            const Projector p = make_projector(b);
+            const Projector& p = b.proj;
             keep = gaussian_rect(b, p, j, bx, by, bz, rect) > 0;
         }
     }
-    const unsigned m = __ballot_sync(kFullMask, keep);
-    if (m) {
+    const bool wide = keep && rect_tiles(rect) > kWideTiles;
+    auto append = [&](bool mine, int counter) {
+        const unsigned m = __ballot_sync(kFullMask, mine);
+        if (!m) return;
         unsigned long long at = 0;
-        if (lane == __ffs(m) - 1) at = atomicAdd(b.total_dev + 1, (unsigned long long)__popc(m));
+        if (lane == __ffs(m) - 1) at = atomicAdd(b.total_dev + counter, (unsigned long long)__popc(m));
         at = __shfl_sync(kFullMask, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
-        if (keep) { b.big_slot[at] = j; b.big_rect[at] = rect; }
-    }
+        if (mine) {
+            const size_t slot = counter == 3 ? (size_t)b.n_pad - 1 - (size_t)at : (size_t)at;
+            b.big_slot[slot] = j;
+            b.big_rect[slot] = rect;
+        }
+    };
+    append(keep && !wide, 1);
+    append(wide, 3);
 }
 
-// The pairs of the listed Gaussians.  Warps take the Gaussians one at a time, 32 tiles of the rectangle per step:
+// The pairs of the listed Gaussians.  Warps take the Gaussians a few at a time (one, where there are few for each), 32 tiles
+// of a rectangle per step:
 // the tile's central ray against the box and the ellipsoid, both grown by the tile's angular radius (pair_range),
 // keeps the pairs in which some ray of the tile can meet the Gaussian.  Every warp gathers its pairs in a buffer
 // of its own in shared memory and appends them with one atomic per 256; pairs past the capacity are counted but
@@ -545,16 +533,21 @@ __global__ void __launch_bounds__(kEmitThreads) bin_list_kernel(BinLaunch b) {
 // CULL: the list is bin_compact_kernel's; single pairs that begin beyond the cut are dropped and their tile marked.
 constexpr int kBigWarps = 8;
 constexpr int kBigBuf = 256;
+constexpr int kBigBatch = 8;
 
 template <bool CULL>
 __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunch b) {
     const unsigned cut = CULL ? b.pick->cut : kAllBuckets;
     __shared__ unsigned long long s_keys[kBigWarps][kBigBuf];
     __shared__ float s_fars[kBigWarps][kBigBuf];
+    __shared__ PairGeom s_geom[kBigWarps][kBigBatch];
+    __shared__ uint2 s_rect[kBigWarps][kBigBatch];
+    __shared__ int s_slot[kBigWarps][kBigBatch];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned long long* keys = s_keys[warp];
     float* fars = s_fars[warp];
-    const unsigned long long nlisted = CULL ? b.total_dev[3] : b.total_dev[1];
+    const unsigned long long nlisted = b.total_dev[1], nwide = b.total_dev[3];
+    bool wide = true;                        // those of many tiles first, one at a time
     const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
     int nbuf = 0;
     auto flush = [&]() {
@@ -570,25 +563,52 @@ __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunc
         nbuf = 0;
         __syncwarp();
     };
+    const unsigned long long warps = (unsigned long long)gridDim.x * kBigWarps;
+    const int batch = (int)min(max(nlisted / (8ull * warps), 1ull), (unsigned long long)kBigBatch);
+    int have = 0, next = 0;
+    unsigned long long idx = 0;
     while (true) {
-        unsigned long long idx = 0;
-        if (lane == 0) idx = atomicAdd(b.total_dev + 2, 1ull);
-        idx = __shfl_sync(kFullMask, idx, 0);
-        if (idx >= nlisted) break;
-        const int j = CULL ? b.kept_slot[idx] : b.big_slot[idx];
-        const uint2 rect = CULL ? b.g_rect[j] : b.big_rect[idx];
-        const float4 sd = b.sdens[j];
-        const float kk = sqrtf(2.0f * 0.6931471805599453f * b.hk[j]);
-        const PairGeom g = make_pair_geom(b.cam.eye, b.bx[j], b.by[j], b.bz[j], b.g0[j], b.g1[j], b.g2[j], sd, b.quat[j], kk);
+        if (next == have) {
+            // the next few Gaussians, a lane for each: one atomic for them, and their loads in flight together
+            if (wide) {
+                if (lane == 0) idx = atomicAdd(b.total_dev + 4, 1ull);
+                idx = __shfl_sync(kFullMask, idx, 0);
+                wide = idx < nwide;
+                idx = (unsigned long long)b.n_pad - 1ull - idx;
+                have = 1;
+            }
+            if (!wide) {
+                if (lane == 0) idx = atomicAdd(b.total_dev + 2, (unsigned long long)batch);
+                idx = __shfl_sync(kFullMask, idx, 0);
+                if (idx >= nlisted) break;
+                have = (int)min((unsigned long long)batch, nlisted - idx);
+            }
+            next = 0;
+            __syncwarp();
+            if (lane < have) {
+                const int j = CULL ? b.kept_slot[idx + lane] : b.big_slot[idx + lane];
+                s_slot[warp][lane] = j;
+                s_rect[warp][lane] = CULL ? b.g_rect[j] : b.big_rect[idx + lane];
+                const float kk = sqrtf(2.0f * 0.6931471805599453f * b.hk[j]);
+                s_geom[warp][lane] = make_pair_geom(b.cam.eye, b.bx[j], b.by[j], b.bz[j], b.g0[j], b.g1[j], b.g2[j], b.sdens[j], b.quat[j], kk);
+            }
+            __syncwarp();
+        }
+        const int j = s_slot[warp][next];
+        const uint2 rect = s_rect[warp][next];
+        const PairGeom g = s_geom[warp][next];
+        ++next;
         const unsigned tx0 = rect.x & 0xffffu, tx1 = rect.x >> 16, ty0 = rect.y & 0xffffu, ty1 = rect.y >> 16;
         const unsigned w = tx1 - tx0 + 1, count = w * (ty1 - ty0 + 1);
+        const float inv_w = 1.0f / (float)w;
         for (unsigned it0 = 0; it0 < count; it0 += 32) {
             const unsigned item = it0 + lane;
             bool keep = false;
             unsigned long long key = 0;
             float tf = 0.f;
             if (item < count) {
-                const unsigned t = (ty0 + item / w) * (unsigned)b.tiles_x + tx0 + item % w;
+                const unsigned row = count < (1u << 22) ? __float2uint_rz(((float)item + 0.5f) * inv_w) : item / w;    // item / w either way
+                const unsigned t = (ty0 + row) * (unsigned)b.tiles_x + tx0 + item - row * w;
                 float tn = 0.f;
                 keep = (!b.tile_flag || b.tile_flag[t] != 0) && pair_range(b.cam.eye, b.tile_dir[t], g, tn, tf);
                 if (CULL && keep && hist_bucket(tn, kl) > cut) { keep = false; b.tile_more[t] = 1; }
@@ -823,6 +843,29 @@ size_t binning_cub_temp_bytes(size_t pair_cap, int ntiles) {
     cub::DeviceRadixSort::SortPairsDescending(nullptr, o, (const int*)nullptr, (int*)nullptr, (const int*)nullptr,
                                               (int*)nullptr, ntiles, 0, 32, (cudaStream_t)0);
     return o > a ? o : a;
+}
+
+// The view's projection, the same for every Gaussian: made once on the host.
+Projector make_projector(const BinLaunch& b) {
+    Projector p;
+    for (int k = 0; k < 3; ++k) { p.eye[k] = b.cam.eye[k]; p.du[k] = b.dual[0][k]; p.dv[k] = b.dual[1][k]; p.dw[k] = b.dual[2][k]; }
+    p.sx = (float)b.cam.width / (2.0f * b.cam.tan_half_fov[0]);
+    p.sy = (float)b.cam.height / (2.0f * b.cam.tan_half_fov[1]);
+    p.ox = b.cam.pp[0] * (float)b.cam.width - 0.5f;
+    p.oy = b.cam.pp[1] * (float)b.cam.height - 0.5f;
+    // a point eye + t (a u + b v + w), t > 0, of a ray of the rows at hand has a within [a0, a1] and b within [b0, b1]
+    // (one pixel of margin), that is x_c - a0 z_c >= 0, a1 z_c - x_c >= 0 and the same for rows
+    const float a0 = (-1.0f - p.ox) / p.sx, a1 = ((float)b.cam.width - p.ox) / p.sx;
+    const float b0 = ((float)b.row_begin - 1.0f - p.oy) / p.sy, b1 = ((float)b.row_end - p.oy) / p.sy;
+    for (int k = 0; k < 3; ++k) {
+        p.plane[0][k] = p.du[k] - a0 * p.dw[k];
+        p.plane[1][k] = a1 * p.dw[k] - p.du[k];
+        p.plane[2][k] = p.dv[k] - b0 * p.dw[k];
+        p.plane[3][k] = b1 * p.dw[k] - p.dv[k];
+    }
+    for (int q = 0; q < 4; ++q)
+        p.plane[q][3] = std::sqrt(p.plane[q][0] * p.plane[q][0] + p.plane[q][1] * p.plane[q][1] + p.plane[q][2] * p.plane[q][2]);
+    return p;
 }
 
 // Phase 1: all (tile, Gaussian) pairs -- with b.pick those that begin before the horizon picked on the way --,

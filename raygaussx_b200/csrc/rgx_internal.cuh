@@ -110,8 +110,8 @@ constexpr unsigned int kAllBuckets = 0xffffffffu;
 
 // What an emission leaves for the host, first in the piece of memory that it starts from zero.
 struct BinResult {
-    unsigned long long total[4];        // [0] pairs met (may exceed the capacity), [1] Gaussians listed by bin_list_kernel, [2] next listed
-                                        // Gaussian to take, [3] Gaussians listed by bin_compact_kernel
+    unsigned long long total[6];        // [0] pairs met (may exceed the capacity); Gaussians listed for the emission: [1] of few tiles, [3] of
+                                        // many; [2], [4] the next of each
     HorizonPick pick;
     unsigned int longest, long_tiles;   // pairs of the longest list; lists of more than kSortShort pairs (bin_layout_kernel)
 };
@@ -133,7 +133,14 @@ inline ZeroedBins zeroed_bins(int tiles_x, int tiles_y) {
     return z;
 }
 
+struct Projector {     // pixel coordinates of a world point: px = (a / (2 tan) + pp) * size - 0.5
+    float eye[3], du[3], dv[3], dw[3];   // dual basis of (u, v, w)
+    float sx, sy, ox, oy;                // px = a * sx + ox, py = b * sy + oy
+    float plane[4][4];                   // the view's four side planes through the eye: inward normal, and its length
+};
+
 struct BinLaunch {
+    Projector proj;                        // of cam, for the rows at hand
     int n, n_pad;
     const float2 *bx, *by, *bz;            // level-0 boxes
     const float4 *g0, *g1, *g2, *quat, *sdens;
@@ -152,14 +159,14 @@ struct BinLaunch {
     float4* tile_dir;                      // [tiles] central ray direction, chord to the farthest corner ray
     void* cub_temp; size_t cub_bytes;
     unsigned char* zero; size_t zero_bytes;// cleared before an emission; total_dev, pick ... tile_more point into it
-    unsigned long long* total_dev;         // [4], see BinResult
+    unsigned long long* total_dev;         // [6], see BinResult
     int* big_slot; uint2* big_rect;        // [n_pad] complete emission: the Gaussians that touch a tile, and their tile rectangles
     int big_grid, sm_count;                // CTAs that work the list off (a few per SM)
     // culled emission (null / unused for a complete one): only the pairs that begin before a horizon are emitted
     HorizonPick* pick;
     unsigned long long* near_hist;         // [2048] estimated pairs by nearest distance of the Gaussian
     uint2* g_rect; unsigned int* g_code;   // [n_pad] tile rectangle (x = ~0: none) and histogram bucket of every Gaussian
-    int* kept_slot;                        // [n_pad] the Gaussians before the cut, in no particular order; their number in total_dev[3]
+    int* kept_slot;                        // [n_pad] the Gaussians before the cut, in no particular order: from the front, of many tiles from the back
     int* tile_diff;                        // [(tiles_x + 1) * (tiles_y + 1)] corners of the rectangles of culled Gaussians
     int* tile_more;                        // [tiles] the tile has pairs that were not emitted
     unsigned long long near_target;        // estimated pairs to keep
@@ -264,6 +271,7 @@ size_t build_cub_temp_bytes(int n_pad);
 cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeLaunch& f, cudaStream_t s);
 size_t binning_cub_temp_bytes(size_t pair_cap, int ntiles);
+Projector make_projector(const BinLaunch& b);
 cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s);
 cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, cudaStream_t s);
 float bin_hist_bucket_end(const BinLaunch& b, int bucket);
