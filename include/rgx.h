@@ -95,7 +95,7 @@ enum {
     RGX_FLAG_EXACT_SH_GRAD = 4,  /* backward: exact d(basis 9)/dy instead of the reference's term (utils/sh_utils.cu:367) */
     RGX_FLAG_ACCUMULATE = 8,     /* backward: add into the gradient tensors instead of overwriting them */
     RGX_FLAG_SAVE_HITS = 32,     /* forward: keep, per ray and slab, the Gaussians that were hit and the per-sample
-                                    sums (in the context's workspace, about 3 KB per ray) so that a backward for
+                                    sums (in the context's workspace, about 2.5 KB per ray) so that a backward for
                                     the same view replays them instead of searching and evaluating again; the
                                     backward falls back to searching where nothing was kept */
     RGX_FLAG_GRADS_CLEAR = 64,   /* backward: the gradient tensors are already zero (a caller clears one buffer that holds them all) */
@@ -131,16 +131,16 @@ typedef struct rgx_counters {
     uint64_t ellipsoid_tests;/* exact ray/ellipsoid tests */
     uint64_t stack_overflows;/* traversal-stack overflows (results invalid if non-zero) */
     uint64_t hits_hash;     /* order-independent hash of every (ray, slab, Gaussian) hit triple */
-    uint64_t candidates;    /* tile-list march: list entries looked at (32 per opened block of a tile's list) */
-    /* tile-list forward march, counting variant: warp-cycles spent per phase (clock64 differences summed over
-     * warps).  cycles_search contains cycles_wait, which contains cycles_window and most of cycles_eval. */
+    uint64_t candidates;    /* tile-list march: list entries looked at (32 per opened block of a tile's list), once per patch of rays */
+    /* counting forward march: warp-cycles spent per phase (clock64 differences summed over warps).  The march by patches fills
+     * cycles_seek, cycles_search, cycles_composite and cycles_total, per patch; the others are the per-ray search's. */
     uint64_t cycles_window;   /* staging of hits for the evaluation */
     uint64_t cycles_seek;     /* closest-hit queries over the tile's list */
     uint64_t cycles_search;   /* slab queries: list scan, exact tests, staging, evaluation */
     uint64_t cycles_eval;     /* per-sample evaluation of staged Gaussians */
     uint64_t cycles_composite;/* compositing of a slab */
     uint64_t cycles_wait;     /* exact tests of 32 candidates and what follows from their hits */
-    uint64_t cycles_total;    /* whole ray */
+    uint64_t cycles_total;    /* whole ray or patch */
 } rgx_counters;
 
 /* Replaces: ox.DeviceContext / module / pipeline creation (optix_utils.py:154-210). */
@@ -231,7 +231,7 @@ RGX_API int rgx_read_kernel_times(rgx_ctx* ctx, float* forward_ms, int* forward_
 /* Replaces: distCUDA2 of the reference's simple-knn submodule (submodules/simple-knn/simple_knn.cu,
  * SimpleKNN::knn; called from classes/point_cloud.py:252,592 to size the first Gaussians).
  * points [n,3] -> mean_dist2 [n]: the mean of the squared distances from each point to its three nearest
- * other points, exact (Morton sort, three levels of boxes of 32, one warp per 32 queries).  With fewer than
+ * other points, exact (Hilbert sort, three levels of boxes, one warp per 32 queries).  With fewer than
  * four points the missing neighbours stay at FLT_MAX in the fp32 sum, as in the reference: one missing gives
  * about FLT_MAX / 3, two or three overflow to +inf.  Needs no context; allocates
  * and frees its scratch (about 70 bytes per point) inside the call and synchronises the stream. */
