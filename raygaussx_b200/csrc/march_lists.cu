@@ -38,7 +38,6 @@ struct Patch {
     // recording, in ints: header, tbuffer and sample spacing per ray, sums, list
     static constexpr int kTapeDt = 8 + kRays, kTapeSums = 8 + 2 * kRays, kTapeList = kTapeSums + 4 * kSamples * 32;
 };
-constexpr int kPatchWarps = 4;                              // warps per CTA of the patch kernels; they share nothing
 
 constexpr int kHitList = 256;      // hits of a slab remembered between the two passes of the backward search
 
@@ -210,7 +209,7 @@ constexpr int kGroup = 8;          // entries that are tested before their hits 
 // back to zero for the next launch.
 __device__ __forceinline__ unsigned fetch_unit(unsigned* next, unsigned units) {
     const unsigned u = atomicAdd(next, 1u);
-    if (u == units + gridDim.x * kPatchWarps - 1u) *next = 0u;
+    if (u == units + gridDim.x - 1u) *next = 0u;
     return u;
 }
 
@@ -439,8 +438,8 @@ __device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq,
 // evaluation of both halves in one body missed the instruction cache) and the evaluation runs over entries that were hit only.
 //   Slabs of the rays are taken in steps: the ray that is furthest behind leads, and every ray whose slab begins before the
 // leader's ends marches with it.  The list is walked once per step over the union of the windows.
-//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.1 -> 4.3, 300 k object 9.25 -> 3.75 (7.8 -> 2.95
-// without recording), 7 M needles 11.6 -> 4.6 (two depths), 1 M at 640x360 1.67 -> 0.79.
+//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.1 -> 3.5, 300 k object 9.25 -> 3.4 (7.8 -> 2.9
+// without recording), 7 M needles 11.6 -> 4.55 (two depths), 1 M at 640x360 1.67 -> 0.76.
 //
 // HZ: the two-depth variant for forward-only views whose rays end early (binning.cu).  In its first phase
 // (L.hz_phase == 1) the tile lists hold only the pairs that begin before L.horizon; a ray that would need more
@@ -480,17 +479,22 @@ struct SampleTree {
         else part[level] = v;
     }
 };
-// CTAs per SM that a forward kernel is compiled for.  With the recording 168 registers and twelve warps are faster than 128 and
-// sixteen: what spills at 128 is read back in the inner loops (300 k object 3.75 against 4.28 ms, 3 M-Gaussian view 4.30 against 4.60).
-template <int P, bool SAVE>
-__host__ __device__ constexpr int patch_ctas_per_sm() { return SAVE ? 3 : 4; }
+// CTAs of one warp per SM that a forward kernel is compiled for, and so its registers: 128 with 16, 136 with 15.  The warps of a
+// patch kernel share nothing, and in CTAs of one warp their number per SM, and with it the registers of each, can be chosen one by
+// one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward takes 3.52
+// instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  14 or 15 warps are slower there (3.78 / 3.83), 17 to 20
+// (96 registers) as fast on the 3 M view and slower on the object (3.74).  Without recording the object, whose slabs hold few
+// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles 4.72 with 15 and 4.55 with 16.
+template <bool COUNT, bool SAVE, int HZ>
+__host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ != 0 ? 16 : 15; }
+// The replay, of 109 registers: 2.55 and 3.00 ms with 18 to 20 warps per SM, 2.66 and 3.11 with 16 (four CTAs of four).
+constexpr int kReplayCtas = 18;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
-__global__ void __launch_bounds__(kPatchWarps * 32, COUNT ? 1 : patch_ctas_per_sm<P, SAVE>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+__global__ void __launch_bounds__(32, forward_ctas<COUNT, SAVE, HZ>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
     using Pt = Patch<P>;
-    __shared__ PatchShared<P> shared[kPatchWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
-    PatchShared<P>& sh = shared[warp];
+    __shared__ PatchShared<P> sh;
+    const int lane = threadIdx.x, sub = lane / Pt::kRays, r = lane % Pt::kRays;
     PatchStage& st = sh.st;
     TapeState& tq = sh.tq;
     const float eps = L.m.transmittance_eps;
@@ -850,20 +854,19 @@ __global__ void __launch_bounds__(kPatchWarps * 32, COUNT ? 1 : patch_ctas_per_s
 // patch's rays; a lane walks the samples that lie inside that Gaussian on its ray (a handful of the 32) and keeps the four
 // moment sums in registers.  The thirteen sums of the Gaussian's gradient row are then added up over the rays in shared memory and
 // leave the SM as one coalesced reduction of 52 bytes, where a reduction per ray and hit kept the L2 and the L1 data pipe busy.
-// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 3.2 ms, 300 k object 4.7 -> 2.6 ms.
+// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 3.0 ms, 300 k object 4.7 -> 2.55 ms.
 template <int P>
-struct ReplayShared {              // per warp
+struct ReplayShared {
     PatchStage st;
     float2 bg[kSlab][Patch<P>::kRays];  // beta, gamma of every sample
     float red[13][36];             // one row per component, 32 lanes (+4: rows start in other banks)
 };
 
 template <int P>
-__global__ void __launch_bounds__(kPatchWarps * 32, 4) march_backward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+__global__ void __launch_bounds__(32, kReplayCtas) march_backward_patches_kernel(const __grid_constant__ MarchLaunch L) {
     using Pt = Patch<P>;
-    extern __shared__ __align__(16) unsigned char replay_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
-    ReplayShared<P>& sh = reinterpret_cast<ReplayShared<P>*>(replay_smem)[warp];
+    __shared__ ReplayShared<P> sh;
+    const int lane = threadIdx.x, sub = lane / Pt::kRays, r = lane % Pt::kRays;
     PatchStage& st = sh.st;
     const float eps = L.m.transmittance_eps;
     const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
@@ -1155,17 +1158,17 @@ static int patch_lanes(const MarchLaunch& m) {
     return rays <= 128 * 128 ? 8 : rays <= 200 * 200 ? 4 : 2;
 }
 
-// CTAs of a patch kernel: as many as fit the device at once (their warps fetch patches until there are none left).
+// CTAs of a patch kernel: as many as fit the device at once (they fetch patches until there are none left).
 template <int P>
 static int patch_ctas(const MarchLaunch& m, int ctas_per_sm) {
-    const long long warps = (long long)m.lists.tiles_x * m.lists.tiles_y * (m.lists.tile * m.lists.tile / Patch<P>::kRays);
-    const long long want = (warps + kPatchWarps - 1) / kPatchWarps, fit = (long long)m.sm_count * ctas_per_sm;
+    const long long want = (long long)m.lists.tiles_x * m.lists.tiles_y * (m.lists.tile * m.lists.tile / Patch<P>::kRays),
+                    fit = (long long)m.sm_count * ctas_per_sm;
     return (int)(want < fit ? want : fit);
 }
 
 template <int P, bool COUNT, bool SAVE, int HZ>
 static void launch_patches(const MarchLaunch& m, cudaStream_t s) {
-    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, COUNT ? 1 : patch_ctas_per_sm<P, SAVE>()), kPatchWarps * 32, 0, s>>>(m);
+    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, forward_ctas<COUNT, SAVE, HZ>()), 32, 0, s>>>(m);
 }
 
 template <int P>
@@ -1202,10 +1205,7 @@ cudaError_t launch_march_backward_search(const MarchLaunch& m, cudaStream_t s) {
 
 template <int P>
 static cudaError_t launch_replay(const MarchLaunch& m, cudaStream_t s) {
-    const int bytes = (int)sizeof(ReplayShared<P>) * kPatchWarps;
-    cudaError_t e = cudaFuncSetAttribute(march_backward_patches_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    note_launch(), march_backward_patches_kernel<P><<<patch_ctas<P>(m, 4), kPatchWarps * 32, bytes, s>>>(m);
+    note_launch(), march_backward_patches_kernel<P><<<patch_ctas<P>(m, kReplayCtas), 32, 0, s>>>(m);
     return cudaGetLastError();
 }
 
