@@ -204,12 +204,13 @@ __device__ __forceinline__ void hz_note(const MarchLaunch& L, int ray_id) {
 }
 
 // ---------------------------------------------------------------- what the sixteen rays of a patch share
+constexpr int kPatchWarps = 1;     // warps per CTA of the patch kernels, see forward_ctas
 constexpr int kGroup = 8;          // entries that are tested before their hits are evaluated
 // The next patch.  Every warp of the grid fetches one number past the end; the one that fetches the last of those puts the counter
 // back to zero for the next launch.
 __device__ __forceinline__ unsigned fetch_unit(unsigned* next, unsigned units) {
     const unsigned u = atomicAdd(next, 1u);
-    if (u == units + gridDim.x - 1u) *next = 0u;
+    if (u == units + gridDim.x * (blockDim.x >> 5) - 1u) *next = 0u;
     return u;
 }
 
@@ -491,10 +492,11 @@ __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ
 constexpr int kReplayCtas = 18;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
-__global__ void __launch_bounds__(32, forward_ctas<COUNT, SAVE, HZ>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+__global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
     using Pt = Patch<P>;
-    __shared__ PatchShared<P> sh;
-    const int lane = threadIdx.x, sub = lane / Pt::kRays, r = lane % Pt::kRays;
+    __shared__ PatchShared<P> shared[kPatchWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
+    PatchShared<P>& sh = shared[warp];
     PatchStage& st = sh.st;
     TapeState& tq = sh.tq;
     const float eps = L.m.transmittance_eps;
@@ -863,7 +865,7 @@ struct ReplayShared {
 };
 
 template <int P>
-__global__ void __launch_bounds__(32, kReplayCtas) march_backward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+__global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_patches_kernel(const __grid_constant__ MarchLaunch L) {
     using Pt = Patch<P>;
     __shared__ ReplayShared<P> sh;
     const int lane = threadIdx.x, sub = lane / Pt::kRays, r = lane % Pt::kRays;
@@ -1168,7 +1170,7 @@ static int patch_ctas(const MarchLaunch& m, int ctas_per_sm) {
 
 template <int P, bool COUNT, bool SAVE, int HZ>
 static void launch_patches(const MarchLaunch& m, cudaStream_t s) {
-    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, forward_ctas<COUNT, SAVE, HZ>()), 32, 0, s>>>(m);
+    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, forward_ctas<COUNT, SAVE, HZ>()), kPatchWarps * 32, 0, s>>>(m);
 }
 
 template <int P>
@@ -1205,7 +1207,7 @@ cudaError_t launch_march_backward_search(const MarchLaunch& m, cudaStream_t s) {
 
 template <int P>
 static cudaError_t launch_replay(const MarchLaunch& m, cudaStream_t s) {
-    note_launch(), march_backward_patches_kernel<P><<<patch_ctas<P>(m, kReplayCtas), 32, 0, s>>>(m);
+    note_launch(), march_backward_patches_kernel<P><<<patch_ctas<P>(m, kReplayCtas), kPatchWarps * 32, 0, s>>>(m);
     return cudaGetLastError();
 }
 
