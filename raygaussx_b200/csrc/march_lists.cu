@@ -957,7 +957,6 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
             __syncwarp();
             // ---- second pass: the Gaussians of the step
             const float inv_dt = __fdividef(1.0f, dt);
-            const float tend = __fadd_rn(tbuffer, __fmul_rn(dt, (float)kSlab));
             const float2* bg = &sh.bg[0][r];
             const int2* list = reinterpret_cast<const int2*>(chunk + Pt::kTapeList);
             int n = h0.x;
@@ -994,29 +993,26 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const int s_lo = max(__float2int_ru(fmaf(rel - hw, inv_dt, -0.55f)), 0);
                         const int s_hi = min(__float2int_rd(fmaf(rel + hw, inv_dt, -0.45f)), kSlab - 1);
                         const int len = hit ? s_hi - s_lo + 1 : 0;
-                        // moments about the closest approach clamped to the slab, so that they stay small
-                        const float tcr = fminf(fmaxf(tca, tbuffer), tend);
+                        // moments about the closest approach: there the whitened ray is at right angles to its direction, so the
+                        // terms do not cancel, and inside the ellipsoid none is larger than one
                         const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
-                        const float off_d = __fadd_rn(tbuffer, -tca), off_c = __fadd_rn(tbuffer, -tcr);
+                        const float off_d = __fadd_rn(tbuffer, -tca);
                         float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
                         float x = (float)s_lo + 0.5f;
-                        const float2* at = bg + s_lo * Pt::kRays;
-                        for (int i = 0; i < len; ++i) {
+                        const float2 *at = bg + s_lo * Pt::kRays, *const end = at + max(len, 0) * Pt::kRays;
+                        for (; at != end; at += Pt::kRays) {
                             const float d = fmaf(x, dt, off_d);
                             const float d2 = __fmul_rn(d, d);
                             const float2 w = *at;
                             const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
-                            const float tc = fmaf(x, dt, off_c);
                             const float ga = __fmul_rn(g, fmaf(ci, w.x, w.y));        // g * (alpha + beta*(chat_i - chat_s))
-                            const float g1 = __fmul_rn(ga, tc);
                             sb = fmaf(g, w.x, sb);
                             n0 = __fadd_rn(n0, ga);
-                            n1 = __fadd_rn(n1, g1);
-                            n2 = fmaf(g1, tc, n2);
+                            n1 = fmaf(ga, d, n1);
+                            n2 = fmaf(ga, d2, n2);
                             x += 1.0f;
-                            at += Pt::kRays;
                         }
-                        const float4 A = make_float4(fmaf(tcr, de.x, Oe.x), fmaf(tcr, de.y, Oe.y), fmaf(tcr, de.z, Oe.z), 0.f);
+                        const float4 A = make_float4(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z), 0.f);
                         GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sb, n0, n1, n2);
                         if (!hit) gg = GaussGrad{};
                         sh.red[0][lane] = gg.mu.x; sh.red[1][lane] = gg.mu.y; sh.red[2][lane] = gg.mu.z;
