@@ -488,7 +488,7 @@ struct SampleTree {
 // Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles 4.72 with 15 and 4.55 with 16.
 template <bool COUNT, bool SAVE, int HZ>
 __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ != 0 ? 16 : 15; }
-// The replay, of 109 registers: 2.55 and 3.00 ms with 18 to 20 warps per SM, 2.66 and 3.11 with 16 (four CTAs of four).
+// The replay, of 95 registers: 18 to 20 warps per SM are 4 % faster than 16 (four CTAs of four).
 constexpr int kReplayCtas = 18;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
 // patch's rays; a lane walks the samples that lie inside that Gaussian on its ray (a handful of the 32) and keeps the four
 // moment sums in registers.  The thirteen sums of the Gaussian's gradient row are then added up over the rays in shared memory and
 // leave the SM as one coalesced reduction of 52 bytes, where a reduction per ray and hit kept the L2 and the L1 data pipe busy.
-// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 3.0 ms, 300 k object 4.7 -> 2.55 ms.
+// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 2.6 ms, 300 k object 4.7 -> 2.2 ms.
 template <int P>
 struct ReplayShared {
     PatchStage st;
@@ -997,23 +997,22 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         // terms do not cancel, and inside the ellipsoid none is larger than one
                         const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
                         const float off_d = __fadd_rn(tbuffer, -tca);
-                        float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
+                        float2 sn = make_float2(0.f, 0.f), n12 = make_float2(0.f, 0.f);          // sums of beta g and of w; of w d and w d^2
                         float x = (float)s_lo + 0.5f;
                         const float2 *at = bg + s_lo * Pt::kRays, *const end = at + max(len, 0) * Pt::kRays;
+#pragma unroll 2
                         for (; at != end; at += Pt::kRays) {
                             const float d = fmaf(x, dt, off_d);
                             const float d2 = __fmul_rn(d, d);
                             const float2 w = *at;
                             const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
-                            const float ga = __fmul_rn(g, fmaf(ci, w.x, w.y));        // g * (alpha + beta*(chat_i - chat_s))
-                            sb = fmaf(g, w.x, sb);
-                            n0 = __fadd_rn(n0, ga);
-                            n1 = fmaf(ga, d, n1);
-                            n2 = fmaf(ga, d2, n2);
+                            const float u = fmaf(ci, w.x, w.y), ga = __fmul_rn(g, u);  // w = g * (alpha + beta*(chat_i - chat_s))
+                            sn = __ffma2_rn(make_float2(g, g), make_float2(w.x, u), sn);
+                            n12 = __ffma2_rn(make_float2(ga, ga), make_float2(d, d2), n12);
                             x += 1.0f;
                         }
                         const float4 A = make_float4(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z), 0.f);
-                        GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sb, n0, n1, n2);
+                        GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sn.x, sn.y, n12.x, n12.y);
                         if (!hit) gg = GaussGrad{};
                         sh.red[0][lane] = gg.mu.x; sh.red[1][lane] = gg.mu.y; sh.red[2][lane] = gg.mu.z;
                         sh.red[3][lane] = gg.y00; sh.red[4][lane] = gg.y11; sh.red[5][lane] = gg.y22;
