@@ -99,7 +99,7 @@ def _as_input(t: torch.Tensor, name: str) -> torch.Tensor:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if t.dtype != torch.float32:
         raise ValueError(f"{name} must be float32, got {t.dtype}")
-    return _aligned(t.detach())
+    return _aligned(t.detach() if t.requires_grad else t)
 
 
 def camera_struct(cam, supersampling=(1, 1)) -> _Camera:
@@ -392,8 +392,12 @@ class RenderOptixFunction(torch.autograd.Function):
             march = _settings_march(settings, cam, flags=flags, rows=getattr(settings, "rows", None))
         else:
             # one buffer for all of them, cleared at once; every tensor starts on a 16-byte boundary
-            sizes = [(t.numel() + 3) & ~3 for t in tensors]
-            grads = [g[:t.numel()].view(t.shape) for g, t in zip(torch.zeros(sum(sizes), device=rgb.device).split(sizes), tensors)]
+            at, total = [], 0
+            for t in tensors:
+                at.append(total)
+                total += (t.numel() + 3) & ~3
+            flat = torch.zeros(total, device=rgb.device)
+            grads = [flat.as_strided(t.shape, t.stride(), a) for t, a in zip(tensors, at)]
             march.flags |= _lib.FLAG_GRADS_CLEAR
         if r._build_serial != ctx.build_serial:
             # another build came between this view's forward and its backward (a second model, an evaluation copy,
