@@ -288,17 +288,7 @@ __device__ __forceinline__ int gaussian_rect(const BinLaunch& b, const Projector
         straddle_tiles(xc, zc, p.sx, p.ox, tiles_x_all, b.tile, W, lox, hix);
         straddle_tiles(yc, zc, p.sy, p.oy, tiles_y_all, b.tile, H, loy, hiy);
     }
-    // rays sit at integer pixel coordinates; keep a small safety margin for rounding
-    const float m = 0.02f;
-    float fx0, fx1, fy0, fy1;
-    auto pixels = [&]() {
-        fx0 = fmaxf(ceilf(lox - m - 1e-5f * fabsf(lox)), 0.f); fx1 = fminf(floorf(hix + m + 1e-5f * fabsf(hix)), (float)W - 1.f);
-        fy0 = fmaxf(ceilf(loy - m - 1e-5f * fabsf(loy)), (float)b.row_begin); fy1 = fminf(floorf(hiy + m + 1e-5f * fabsf(hiy)), (float)b.row_end - 1.f);
-        return fx0 <= fx1 && fy0 <= fy1;
-    };
-    if (!pixels()) return 0;
-    // a box within one tile has one pair at most, which the emission tests exactly: no second box, none of its loads
-    if ((unsigned)fx0 / b.tile != (unsigned)fx1 / b.tile || (unsigned)fy0 / b.tile != (unsigned)fy1 / b.tile) {
+    {
         // oriented box of the ellipsoid {x : |S^-1 R^T (x - p)| <= k}: centre +- k s_a col_a
         const float4 sd = b.sdens[j], q = b.quat[j], g0 = b.g0[j];
         const float k = sqrtf(2.0f * 0.6931471805599453f * b.hk[j]) * 1.0001f;
@@ -319,8 +309,14 @@ __device__ __forceinline__ int gaussian_rect(const BinLaunch& b, const Projector
             straddle_tiles(yc, zc, p.sy, p.oy, tiles_y_all, b.tile, H, oly, ohy);
         }
         lox = fmaxf(lox, olx); hix = fminf(hix, ohx); loy = fmaxf(loy, oly); hiy = fminf(hiy, ohy);
-        if (!pixels()) return 0;
     }
+    // rays sit at integer pixel coordinates; keep a small safety margin for rounding
+    const float m = 0.02f;
+    float fx0 = ceilf(lox - m - 1e-5f * fabsf(lox)), fx1 = floorf(hix + m + 1e-5f * fabsf(hix));
+    float fy0 = ceilf(loy - m - 1e-5f * fabsf(loy)), fy1 = floorf(hiy + m + 1e-5f * fabsf(hiy));
+    fx0 = fmaxf(fx0, 0.f); fx1 = fminf(fx1, (float)W - 1.f);
+    fy0 = fmaxf(fy0, (float)b.row_begin); fy1 = fminf(fy1, (float)b.row_end - 1.f);
+    if (!(fx0 <= fx1 && fy0 <= fy1)) return 0;
     const unsigned tx0 = (unsigned)fx0 / b.tile, tx1 = (unsigned)fx1 / b.tile;
     const unsigned ty0 = (unsigned)fy0 / b.tile - b.ty_first, ty1 = (unsigned)fy1 / b.tile - b.ty_first;
     rect = make_uint2(tx0 | (tx1 << 16), ty0 | (ty1 << 16));
