@@ -275,9 +275,9 @@ RGX_API int rgx_image_loss_backward(int device, const float* rays, const float* 
                                     rgx_stream stream);
 
 /* Densification statistics (classes/point_cloud.py:468-485): norm_sum[i] += |grad_i| max(|position_i - eye|, 1) and
- * count[i] += 1 where |grad_i| > 0; norm_sum NULL: only the count.  eye [3] is a device pointer. */
+ * count[i] += 1 (and also[i] += 1, unless NULL) where |grad_i| > 0; norm_sum NULL: only the count.  eye [3] is a device pointer. */
 RGX_API int rgx_gradient_stats(int device, int n, const float* positions, const float* grad, const float* eye,
-                               float* norm_sum, float* count, rgx_stream stream);
+                               float* norm_sum, float* count, float* also, rgx_stream stream);
 
 /* One Adam step of up to RGX_ADAM_MAX tensors in one launch: m += (1-beta1)(g-m), v = beta2 v + (1-beta2) g^2,
  * param -= step_size m / (sqrt(v) inv_root + eps), with step_size = lr / (1 - beta1^t) and inv_root =

@@ -102,7 +102,7 @@ SYMBOLS = {
     "rgx_image_loss": (C.c_int, [C.c_int, _fp, _fp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, _fp, _fp, _fp, C.c_void_p]),
     "rgx_image_loss_backward": (C.c_int, [C.c_int, _fp, _fp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, _fp, _fp, _fp,
                                           C.c_void_p]),
-    "rgx_gradient_stats": (C.c_int, [C.c_int, C.c_int, _fp, _fp, _fp, _fp, _fp, C.c_void_p]),
+    "rgx_gradient_stats": (C.c_int, [C.c_int, C.c_int, _fp, _fp, _fp, _fp, _fp, _fp, C.c_void_p]),
     "rgx_adam_step": (C.c_int, [C.c_int, C.POINTER(AdamTensor), C.c_int, C.c_double, C.c_double, C.c_double, C.c_void_p]),
     "rgx_knn_scratch_bytes": (C.c_size_t, [C.c_int]),
     "rgx_knn_mean_dist2_scratch": (C.c_int, [C.c_int, _fp, C.c_int, _fp, _fp, C.c_size_t, C.c_void_p]),

@@ -627,7 +627,8 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     b.tile_pcnt = reinterpret_cast<int*>(ctx->bin_zero + z.pcnt);
     ctx->tile_more = reinterpret_cast<int*>(ctx->bin_zero + z.more);
     b.big_slot = ctx->big_slot; b.big_rect = ctx->big_rect; b.big_grid = ctx->sm_count * RGX_BIG_GRID; b.sm_count = ctx->sm_count;
-    if (cull && cull->budget_per_ray > 0) {
+    // (fewer Gaussians times tiles than that threshold: nothing could be cut, and three kernels are saved)
+    if (cull && cull->budget_per_ray > 0 && (unsigned long long)ctx->n * (unsigned long long)ntiles >= cull->min_total) {
         // only the pairs that begin before a horizon are emitted (binning.cu)
         int rc = two_depth_workspace(ctx, ntiles);          // the counter of rays that reach the horizon
         if (rc) return rc;
@@ -870,9 +871,9 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_scene* scene, const rgx_cam
         if ((rc = fill_lists(ctx, b, ctx->bin_keys_in, ctx->bin_vals_in, total, ntiles, s))) return rc;
     }
     const HorizonPick pk = ctx->bin_result_host->pick;
-    learn_ratio(ctx, ctx->hz_ratio, total);
-    if (pk.cut == kAllBuckets || total == 0) {                     // one depth is enough: these are the complete lists
-        lists_now_valid(ctx, cam, m, total, true);
+    if (b.pick) learn_ratio(ctx, ctx->hz_ratio, total);
+    if (!b.pick || pk.cut == kAllBuckets || total == 0) {          // one depth is enough: these are the complete lists
+        lists_now_valid(ctx, cam, m, total, b.pick != nullptr);
         return RGX_OK;
     }
     if ((e = cudaMemsetAsync(ctx->tile_resume, 0, sizeof(int) * (size_t)ntiles, s)) != cudaSuccess ||

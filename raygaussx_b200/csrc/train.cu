@@ -294,7 +294,8 @@ dim3 loss_grid(int w, int h) { return dim3((w + kTile - 1) / kTile, (h + kTile -
 
 // ---------------------------------------------------------------- statistics, Adam
 // classes/point_cloud.py:468-485; a null norm_sum counts only (gradients of Gaussians not visible).
-__global__ void __launch_bounds__(256) gradient_stats_kernel(int n, const float* pos, const float* grad, const float* eye, float* norm_sum, float* count) {
+__global__ void __launch_bounds__(256) gradient_stats_kernel(int n, const float* pos, const float* grad, const float* eye, float* norm_sum, float* count,
+                                                             float* also) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gx = grad[3 * (size_t)i], gy = grad[3 * (size_t)i + 1], gz = grad[3 * (size_t)i + 2];
@@ -303,7 +304,10 @@ __global__ void __launch_bounds__(256) gradient_stats_kernel(int n, const float*
         const float dx = pos[3 * (size_t)i] - eye[0], dy = pos[3 * (size_t)i + 1] - eye[1], dz = pos[3 * (size_t)i + 2] - eye[2];
         norm_sum[i] += norm * fmaxf(sqrtf(dx * dx + dy * dy + dz * dz), 1.0f);
     }
-    if (norm > 0.f) count[i] += 1.0f;
+    if (norm > 0.f) {
+        count[i] += 1.0f;
+        if (also) also[i] += 1.0f;
+    }
 }
 
 constexpr int kAdamChunk = 4096;     // values per block: sixteen per thread
@@ -445,12 +449,12 @@ extern "C" RGX_API int rgx_image_loss_backward(int device, const float* rays, co
 }
 
 extern "C" RGX_API int rgx_gradient_stats(int device, int n, const float* positions, const float* grad, const float* eye, float* norm_sum,
-                                          float* count, rgx_stream stream) {
+                                          float* count, float* also, rgx_stream stream) {
     if (n < 0 || (n > 0 && (!grad || !count || (norm_sum && (!positions || !eye))))) return RGX_E_INVALID;
     if (n == 0) return RGX_OK;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
-    note_launch(), gradient_stats_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, positions, grad, eye, norm_sum, count);
+    note_launch(), gradient_stats_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, positions, grad, eye, norm_sum, count, also);
     return done(cudaGetLastError());
 }
 

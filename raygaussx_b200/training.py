@@ -278,8 +278,13 @@ def training_iteration(pointcloud, viewpoint_cam, config, iteration: int, schedu
             loss = loss / float(schedule.accum_steps)
         loss.backward()
     if pointcloud.positions.grad is not None:
-        pointcloud.accumulate_gradient(pointcloud.positions.grad, viewpoint_cam)
-        pointcloud.accumulate_gradient_gaussians_not_visible(pointcloud.positions.grad)
+        grad = pointcloud.positions.grad
+        if type(pointcloud) is SimplePointCloud and _fusable(grad, pointcloud.num_accum_gnv):     # both statistics in one pass
+            if not pointcloud.accumulate_gradient(grad, viewpoint_cam, pointcloud.num_accum_gnv.data_ptr()):
+                pointcloud.accumulate_gradient_gaussians_not_visible(grad)
+        else:
+            pointcloud.accumulate_gradient(grad, viewpoint_cam)
+            pointcloud.accumulate_gradient_gaussians_not_visible(grad)
     stepped = False
     if use_accum:
         schedule.counter += 1
@@ -427,23 +432,24 @@ class SimplePointCloud:
         self.num_accum_gnv = torch.zeros(n, device=dev)
 
     @torch.no_grad()
-    def accumulate_gradient(self, grad, camera):
+    def accumulate_gradient(self, grad, camera, _also=None):
         eye = camera.camera_center
         if _fusable(self.positions, grad, eye, self.xyz_gradient_accum_norm, self.num_accum):
             _check(_lib.lib().rgx_gradient_stats(grad.device.index or 0, grad.shape[0], self.positions.data_ptr(), grad.data_ptr(),
                                                  eye.data_ptr(), self.xyz_gradient_accum_norm.data_ptr(),
-                                                 self.num_accum.data_ptr(), _stream(grad)), "rgx_gradient_stats")
-            return
+                                                 self.num_accum.data_ptr(), _also, _stream(grad)), "rgx_gradient_stats")
+            return True
         dist = torch.clamp(torch.norm(self.positions - camera.camera_center[None, :], dim=1), min=1.0)
         norm = torch.norm(grad, dim=1)
         self.xyz_gradient_accum_norm += norm * dist
         self.num_accum += torch.where(norm > 0, 1.0, 0.0)
+        return False
 
     @torch.no_grad()
     def accumulate_gradient_gaussians_not_visible(self, grad):
         if _fusable(grad, self.num_accum_gnv):
             _check(_lib.lib().rgx_gradient_stats(grad.device.index or 0, grad.shape[0], None, grad.data_ptr(), None, None,
-                                                 self.num_accum_gnv.data_ptr(), _stream(grad)), "rgx_gradient_stats")
+                                                 self.num_accum_gnv.data_ptr(), None, _stream(grad)), "rgx_gradient_stats")
             return
         self.num_accum_gnv += torch.where(torch.norm(grad, dim=1) > 0, 1.0, 0.0)
 
