@@ -454,6 +454,15 @@ __device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq,
 // HZ = 1: the two phases (L.hz_phase 1 or 2); HZ = 2: counting only (L.hz_phase 3), nothing is put aside.
 enum RayMode { kSeekFirst, kSeekNext, kInSlab, kDone };
 
+// Packed a b + c, evaluated where it stands: left to itself the compiler lifts the sample positions of a slab, sixteen registers,
+// out of the loop over its hits and spills others for them (recording forward of the 300 k object 3.66 ms, 3.34 this way).
+__device__ __forceinline__ float2 fma2_in_place(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm volatile("{ .reg .b64 a, b, c, r; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7};"
+                 " fma.rn.f32x2 r, a, b, c; mov.b64 {%0, %1}, r; }" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
 // Sum of one value over the P lanes of a ray (P consecutive samples), as a balanced tree; `before`: over the lanes before this one.
 template <int P>
 __device__ __forceinline__ float across_ray(float x, int sub, float& before) {
@@ -503,7 +512,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
     // recording 3 M view 3.52 -> 3.46.  On the object, whose slabs hold few Gaussians, it costs 7 to 10 %.
     constexpr int kTestUnroll = HZ != 0 ? 2 : 1;
     const float eps = L.m.transmittance_eps;
-    const float sub_even = (float)(sub & ~1), sub_off = (float)(sub & 1) + 0.5f;       // see eval_forward
+    const float sub_half = (float)sub + 0.5f;
     const int cap = L.m.max_prim_slice;
     const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
     const unsigned units = (unsigned)(L.lists.tiles_x * L.lists.tiles_y) * per_tile;
@@ -640,7 +649,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
             if (!__any_sync(kFull, act)) continue;
             const long long c_q = COUNT ? clock64() : 0;
             const float tmin = act ? p.tmin : INFINITY, tmax = act ? p.tmax : -INFINITY;
-            const float dt = p.dt, inv_part = __fdividef((float)Pt::kParts / (float)kSlab, p.dt);
+            const float dt = p.dt, sub_dt = sub ? dt : 0.f, inv_part = __fdividef((float)Pt::kParts / (float)kSlab, p.dt);
             float2 S[Pt::kPairs], R[Pt::kPairs], G[Pt::kPairs], B[Pt::kPairs];
 #pragma unroll
             for (int i = 0; i < Pt::kPairs; ++i) S[i] = R[i] = G[i] = B[i] = make_float2(0.f, 0.f);
@@ -721,15 +730,15 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
                         reach &= ~(kPartBits << (Pt::kParts * e));
                         const float4 A = sh.rec[e][r];
                         const float4 c = st.rgba[(f + e) & (kStaged - 1)];
-                        const float off = fmaf(sub_off, dt, -A.x);
 #pragma unroll
                         for (int g = 0; g < Pt::kParts; ++g) {
                             if (!((here >> g) & 1u)) continue;
 #pragma unroll
                             for (int i = Pt::kPairsPerPart * g; i < Pt::kPairsPerPart * (g + 1); ++i) {
-                                const float2 s2 = P == 2 ? make_float2((float)(4 * i), (float)(4 * i + 2))
-                                                         : make_float2((float)(2 * P * i) + sub_even, (float)(2 * P * i + P) + sub_even);
-                                const float2 d = __ffma2_rn(s2, make_float2(dt, dt), make_float2(off, off));
+                                // (s + 1/2) dt rounded once, as in eval_forward: with two lanes per ray sub dt is exact
+                                const float2 tau = P == 2 ? fma2_in_place(make_float2((float)(4 * i) + 0.5f, (float)(4 * i + 2) + 0.5f), make_float2(dt, dt), make_float2(sub_dt, sub_dt))
+                                                          : __fmul2_rn(make_float2((float)(2 * P * i) + sub_half, (float)(2 * P * i + P) + sub_half), make_float2(dt, dt));
+                                const float2 d = __fadd2_rn(tau, make_float2(-A.x, -A.x));
                                 const float2 d2 = __fmul2_rn(d, d);
                                 const float2 arg = __ffma2_rn(make_float2(A.z, A.z), d2, make_float2(A.w, A.w));
                                 const float2 ee = make_float2(d2.x < A.y ? ex2_approx(arg.x) : 0.0f, d2.y < A.y ? ex2_approx(arg.y) : 0.0f);
@@ -863,7 +872,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
 template <int P>
 struct ReplayShared {
     PatchStage st;
-    float2 bg[kSlab][Patch<P>::kRays];  // beta, gamma of every sample
+    float2 bg[kSlab + kRun - 1][Patch<P>::kRays];  // beta, gamma of every sample; zero past the last, where a run may end
     float red[13][36];             // one row per component, 32 lanes (+4: rows start in other banks)
 };
 
@@ -876,6 +885,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
     const float eps = L.m.transmittance_eps;
     const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
     const unsigned units = (unsigned)(L.lists.tiles_x * L.lists.tiles_y) * per_tile;
+    for (int i = lane; i < (kRun - 1) * Pt::kRays; i += 32) (&sh.bg[kSlab][0])[i] = make_float2(0.f, 0.f);
 
     while (true) {
         unsigned unit = 0;
@@ -983,35 +993,38 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
                         const float a = dot3(de, de), inv_a = __fdividef(1.0f, a), b = -dot3(Oe, de);
                         const float t0 = __fmul_rn(b, inv_a), tca = fmaf(fmaf(-t0, a, b), inv_a, t0);    // as in ellipsoid_stretch
-                        const float3 P = make_float3(fmaf(t0, de.x, Oe.x), fmaf(t0, de.y, Oe.y), fmaf(t0, de.z, Oe.z));
-                        const float disc = 1.0f - dot3(P, P);
-                        const float ay = __fmul_rn(disc, inv_a), az = __fmul_rn(-ex.x, a), aw = fmaf(ex.x, disc, -ex.x);
-                        // samples (s + 1/2) dt inside the ellipsoid, and those within a twentieth of a sample of it against rounding;
-                        // d^2 < ay decides.  (A whole sample more on each side cost two of a dozen turns of the loop below.)
+                        const float3 yc = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
+                        const float qmin = dot3(yc, yc);
+                        const float ay = __fmul_rn(1.0f - qmin, inv_a), az = __fmul_rn(-ex.x, a), aw = __fmul_rn(-ex.x, qmin);
+                        // runs of samples that may lie inside (first_run), up to the last one within a twentieth of a sample of the
+                        // ellipsoid (positions are good to a few 2^-24 t, so up to t = 10^5 dt); d^2 < ay decides
                         const float hw = sqrt_approx(fmaxf(ay, 0.f));
-                        const float rel = __fadd_rn(tca, -tbuffer);
-                        const int s_lo = max(__float2int_ru(fmaf(rel - hw, inv_dt, -0.55f)), 0);
-                        const int s_hi = min(__float2int_rd(fmaf(rel + hw, inv_dt, -0.45f)), kSlab - 1);
-                        const int len = hit ? s_hi - s_lo + 1 : 0;
+                        const int s_lo = first_run(tca, hw, tbuffer, inv_dt);
+                        const int s_hi = min(__float2int_rd(slab_sample(__fadd_rn(tca, hw), tbuffer, inv_dt) + 0.05f), kSlab - 1);
+                        const int runs = hit && s_hi >= s_lo ? (s_hi - s_lo) / kRun + 1 : 0;
                         // moments about the closest approach: there the whitened ray is at right angles to its direction, so the
                         // terms do not cancel, and inside the ellipsoid none is larger than one
                         const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
                         const float off_d = __fadd_rn(tbuffer, -tca);
                         float2 sn = make_float2(0.f, 0.f), n12 = make_float2(0.f, 0.f);          // sums of beta g and of w; of w d and w d^2
                         float x = (float)s_lo + 0.5f;
-                        const float2 *at = bg + s_lo * Pt::kRays, *const end = at + max(len, 0) * Pt::kRays;
-#pragma unroll 2
-                        for (; at != end; at += Pt::kRays) {
-                            const float d = fmaf(x, dt, off_d);
-                            const float d2 = __fmul_rn(d, d);
-                            const float2 w = *at;
-                            const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
-                            const float u = fmaf(ci, w.x, w.y), ga = __fmul_rn(g, u);  // w = g * (alpha + beta*(chat_i - chat_s))
-                            sn = __ffma2_rn(make_float2(g, g), make_float2(w.x, u), sn);
-                            n12 = __ffma2_rn(make_float2(ga, ga), make_float2(d, d2), n12);
-                            x += 1.0f;
+                        const float2 *at = bg + s_lo * Pt::kRays, *const end = at + runs * (kRun * Pt::kRays);
+#pragma unroll 1
+                        for (; at != end; at += kRun * Pt::kRays) {
+                            float d = __fadd_rn(__fmul_rn(x, dt), off_d);
+#pragma unroll
+                            for (int i = 0; i < kRun; ++i) {
+                                const float d2 = __fmul_rn(d, d);
+                                const float2 w = at[i * Pt::kRays];
+                                const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
+                                const float u = fmaf(ci, w.x, w.y), ga = __fmul_rn(g, u);  // w = g * (alpha + beta*(chat_i - chat_s))
+                                sn = __ffma2_rn(make_float2(g, g), make_float2(w.x, u), sn);
+                                n12 = __ffma2_rn(make_float2(ga, ga), make_float2(d, d2), n12);
+                                d = __fadd_rn(d, dt);
+                            }
+                            x += (float)kRun;
                         }
-                        const float4 A = make_float4(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z), 0.f);
+                        const float4 A = make_float4(yc.x, yc.y, yc.z, 0.f);
                         GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sn.x, sn.y, n12.x, n12.y);
                         if (!hit) gg = GaussGrad{};
                         sh.red[0][lane] = gg.mu.x; sh.red[1][lane] = gg.mu.y; sh.red[2][lane] = gg.mu.z;
