@@ -325,7 +325,8 @@ RGX_API int rgx_read_two_depth(rgx_ctx* ctx, long long out[4]);
  * that of complete lists to summation rounding (1e-5); it is not recorded, and the backward searches it again over
  * complete lists, which it then makes.  Every other ray is bit for bit what complete lists give.  No host
  * synchronisation is added: the number of such rays reaches the host behind the forward and is looked at by the next
- * call on the context; a view that had any doubles the budget for the views to come.
+ * call on the context; a view that had any doubles the budget for the views to come, 64 views in a row without any
+ * halve it again, down to what was asked for; a build of a set of another size begins there.
  * budget_per_ray = 0 switches the feature off, < 0 leaves it as it is; min_pairs >= 0 replaces the 2^21 (tests use 0
  * to take small views through it).  rgx_read_near_lists returns and clears (views whose lists stopped at a horizon,
  * the estimated number of all pairs of those views, pairs kept, views in which some ray went beyond the horizon); it

@@ -20,6 +20,7 @@ using namespace rgx;
 #define RGX_NEAR_BUDGET 5
 #endif
 
+constexpr int kNearWait = 64;
 constexpr double kFirstRatio = 2.0;      // (estimated pairs per pair before a view of the scene has been seen)
 struct rgx_ctx {
     int device = 0;
@@ -94,7 +95,10 @@ struct rgx_ctx {
     bool lists_noted = false;          // g_rect, g_code and the pick on the host are those of the current lists
     float lists_horizon = 0.f;
     long long lists_rays = 0;          // rays of the view the partial lists were made for
-    int near_budget_per_ray = RGX_NEAR_BUDGET;   // pairs per ray such lists keep; doubled whenever a ray reached the horizon
+    int near_budget_per_ray = RGX_NEAR_BUDGET;   // pairs per ray such lists keep to begin with
+    int near_budget_now = RGX_NEAR_BUDGET;       // ... and now: see near_deeper, near_went_well; back to the above with a set of another size
+    int near_clean = 0, near_wait = kNearWait;   // views in a row in which no ray went beyond, of the number after which the lists get shallower
+    bool near_lowered = false;                   // they have since the last time they got deeper
     long long near_stats[4] = {0, 0, 0, 0};   // views with such lists, pairs of those views (estimate), pairs kept, views marched again
     // rays that went beyond the horizon in the latest march over such lists: counted on the device, finished there by a
     // per-ray search, and known to the host only later (settle_beyond)
@@ -384,9 +388,33 @@ int run_colors_if_beyond(rgx_ctx* ctx, const rgx_scene* sc, const float eye[3], 
     return e == cudaSuccess ? RGX_OK : cuda_fail(ctx, e, "colour kernel");
 }
 
+// How deep the lists of recording forwards are.  Twice as deep after a view in which any ray went beyond them: a few rays cost
+// milliseconds (1,164 of 260,000 rays searched one by one: 4.9 ms a view instead of 1.7), lists of 10 pairs per ray instead of 5 cost
+// 0.1 to 0.3 (1 M Gaussians at 628x414, 3 M at 1256x828).  But complete lists cost 3 ms on the latter, and a few awkward views of a
+// long run would lead there, so after kNearWait views without such rays half as deep again; twice as long a wait where that was
+// one time too many.
+void near_deeper(rgx_ctx* ctx) {
+    if (ctx->near_budget_now < (1 << 18)) ctx->near_budget_now *= 2;
+    if (ctx->near_lowered) ctx->near_wait = std::min(2 * ctx->near_wait, 64 * kNearWait);
+    ctx->near_clean = 0;
+    ctx->near_lowered = false;
+}
+void near_went_well(rgx_ctx* ctx) {
+    if (ctx->near_budget_now <= ctx->near_budget_per_ray || ++ctx->near_clean < ctx->near_wait) return;
+    ctx->near_budget_now = std::max(ctx->near_budget_now / 2, ctx->near_budget_per_ray);
+    ctx->near_clean = 0;
+    ctx->near_lowered = true;
+}
+void near_begin(rgx_ctx* ctx, int budget_per_ray) {
+    ctx->near_budget_per_ray = ctx->near_budget_now = budget_per_ray;
+    ctx->near_clean = 0;
+    ctx->near_wait = kNearWait;
+    ctx->near_lowered = false;
+}
+
 // The number of rays that went beyond the horizon in the latest march over lists that stop at one was copied to the
 // host behind that march; whoever needs it waits for the copy here (by then long done).  A view in which it is not
-// zero makes the lists of the views to come twice as deep -- unless its own lists had fallen short of the budget:
+// zero makes the lists of the views to come deeper -- unless its own lists had fallen short of the budget:
 // then the estimate was off, and has been corrected already.
 void settle_beyond(rgx_ctx* ctx) {
     if (!ctx->beyond_pending) return;
@@ -394,11 +422,11 @@ void settle_beyond(rgx_ctx* ctx) {
     if (cudaEventSynchronize(ctx->ev_beyond) != cudaSuccess) { (void)cudaGetLastError(); return; }
     const long long n = (long long)(*ctx->beyond_host & 0xffffffffull);
     if (ctx->beyond_recorded) ctx->tape_beyond_rays = n;
-    if (n == 0) return;
+    if (n == 0) { near_went_well(ctx); return; }
     ctx->near_stats[3] += 1;
     if ((double)ctx->beyond_kept >= 0.75 * (double)ctx->beyond_budget * (double)ctx->beyond_lists_rays &&
-        ctx->near_budget_per_ray == ctx->beyond_budget && ctx->near_budget_per_ray < (1 << 18))
-        ctx->near_budget_per_ray *= 2;
+        ctx->near_budget_now == ctx->beyond_budget)
+        near_deeper(ctx);
 }
 
 struct ScopedTimer {   // brackets one kernel launch with events when profiling is on
@@ -483,7 +511,7 @@ int rgx_build(rgx_ctx* ctx, const rgx_scene* scene, float sigma_threshold, int m
     if ((rc = ensure_workspace(ctx, n_pad > 0 ? n_pad : kFan, lv.total))) return rc;
     ctx->built = false;
     ctx->build_id++;
-    if (n != ctx->n) { ctx->hz_budget_now = ctx->hz_budget_per_ray; ctx->hz_ratio = ctx->near_ratio = kFirstRatio; }
+    if (n != ctx->n) { ctx->hz_budget_now = ctx->hz_budget_per_ray; ctx->hz_ratio = ctx->near_ratio = kFirstRatio; near_begin(ctx, ctx->near_budget_per_ray); }
     ctx->n = n;
     ctx->n_pad = n_pad;
     ctx->sigma_threshold = sigma_threshold;
@@ -746,7 +774,7 @@ static void learn_ratio(const rgx_ctx* ctx, double& ratio, int kept) {
     if (kept > 0) ratio = std::min(8.0, std::max(1.0, (double)ctx->bin_result_host->pick.est_kept / (double)kept));
 }
 
-static Cull near_cull(const rgx_ctx* ctx) { return Cull{ctx->near_budget_per_ray, (unsigned long long)ctx->near_min_pairs, true, ctx->near_ratio}; }
+static Cull near_cull(const rgx_ctx* ctx) { return Cull{ctx->near_budget_now, (unsigned long long)ctx->near_min_pairs, true, ctx->near_ratio}; }
 
 // Turns the emitted pairs into ctx->lists.  The view of a recording forward -- a training view, whose rays end long
 // before they have seen most of their tile's list (on the 3 M-Gaussian scene every ray ends within the nearest eighth
@@ -766,6 +794,8 @@ static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, c
         ctx->lists_horizon = bin_hist_bucket_end(b, (int)pk.cut);
         ctx->lists_rays = (long long)cam->width * (m->row_end - m->row_begin);
         ctx->near_stats[0] += 1; ctx->near_stats[1] += (long long)pk.est_total; ctx->near_stats[2] += total;
+    } else if (b.pick && ctx->bin_result_host->pick.est_total >= (unsigned long long)ctx->near_min_pairs) {
+        near_went_well(ctx);           // complete because the budget covers the view
     }
     return RGX_OK;
 }
@@ -1080,7 +1110,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         return cuda_fail(ctx, e, "rays beyond the horizon");
     ctx->beyond_pending = true;
     ctx->beyond_recorded = L.tape != nullptr;
-    ctx->beyond_kept = ctx->last_pairs; ctx->beyond_lists_rays = ctx->lists_rays; ctx->beyond_budget = ctx->near_budget_per_ray;
+    ctx->beyond_kept = ctx->last_pairs; ctx->beyond_lists_rays = ctx->lists_rays; ctx->beyond_budget = ctx->near_budget_now;
     return RGX_OK;
 }
 
@@ -1239,7 +1269,7 @@ int rgx_debug_near_lists(rgx_ctx* ctx, int budget_per_ray, long long min_pairs) 
     if (!ctx) return RGX_E_INVALID;
     DeviceGuard guard(ctx->device);
     settle_beyond(ctx);
-    if (budget_per_ray >= 0) ctx->near_budget_per_ray = budget_per_ray;
+    if (budget_per_ray >= 0) near_begin(ctx, budget_per_ray);
     if (min_pairs >= 0) ctx->near_min_pairs = min_pairs;
     ctx->lists_valid = false;          // lists made under the old setting are not reused
     return RGX_OK;
