@@ -279,6 +279,26 @@ __global__ void __launch_bounds__(128) finalize_kernel(FinalizeLaunch f) {
     for (int a = 0; a < 3; ++a) put(f.gr.positions + 3 * (size_t)i + a, dpos[a], acc);
 }
 
+// Zeroes up to eight tensors in one launch, a block per kClearFloats floats of one of them; 16 bytes at a time where the tensor
+// begins on such a boundary.  (One memset per tensor was five to eight launches, as much as a small scene's gradients themselves.)
+constexpr int kClearFloats = 8192;
+struct ClearTable {
+    struct Piece { float* p; size_t count; } piece[8];
+    unsigned blocks_upto[8];           // inclusive prefix
+    int n;
+};
+__global__ void __launch_bounds__(128) clear_kernel(const __grid_constant__ ClearTable t) {
+    int k = 0;
+    while (blockIdx.x >= t.blocks_upto[k]) ++k;                // the grid has blocks_upto[n - 1] blocks
+    const size_t begin = (size_t)(blockIdx.x - (k > 0 ? t.blocks_upto[k - 1] : 0u)) * kClearFloats;
+    const size_t left = t.piece[k].count - begin;
+    float* p = t.piece[k].p + begin;
+    const int count = left < (size_t)kClearFloats ? (int)left : kClearFloats;
+    const int wide = (reinterpret_cast<unsigned long long>(p) & 15ull) == 0 ? count / 4 : 0;
+    for (int i = threadIdx.x; i < wide; i += 128) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 4 * wide + threadIdx.x; i < count; i += 128) p[i] = 0.f;
+}
+
 }  // namespace
 
 cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s) {
@@ -292,15 +312,19 @@ cudaError_t launch_finalize(const FinalizeLaunch& f, cudaStream_t s) {
     if (f.sc.n == 0) return cudaSuccess;
     if (!(f.flags & (RGX_FLAG_ACCUMULATE | RGX_FLAG_GRADS_CLEAR))) {       // the kernel writes the rows of the Gaussians some ray met, nothing else
         const size_t n = (size_t)f.sc.n, K = (size_t)f.sc.sh_coeffs, G = (size_t)f.sc.num_lobes;
-        struct { float* p; size_t count; } clear[] = {
+        const ClearTable::Piece all[8] = {
             {f.gr.positions, 3 * n}, {f.gr.scales, 3 * n}, {f.gr.quaternions, 4 * n}, {f.gr.densities, n},
             {f.gr.color_features, 3 * K * n}, {f.gr.sg_features, 3 * G * n}, {f.gr.sharpness, G * n},
             {f.gr.lobe_axis, 3 * G * n}};
-        for (auto& c : clear) {
+        ClearTable t{};
+        size_t blocks = 0;
+        for (const auto& c : all) {
             if (!c.p || c.count == 0) continue;
-            cudaError_t e = cudaMemsetAsync(c.p, 0, c.count * sizeof(float), s);
-            if (e != cudaSuccess) return e;
+            blocks += (c.count + kClearFloats - 1) / kClearFloats;
+            t.piece[t.n] = c;
+            t.blocks_upto[t.n++] = (unsigned)blocks;
         }
+        if (blocks) note_launch(), clear_kernel<<<(unsigned)blocks, 128, 0, s>>>(t);
     }
     note_launch(), finalize_kernel<<<(f.sc.n + 127) / 128, 128, 0, s>>>(f);
     return cudaGetLastError();

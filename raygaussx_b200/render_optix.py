@@ -391,14 +391,8 @@ class RenderOptixFunction(torch.autograd.Function):
             flags |= _lib.FLAG_ACCUMULATE
             march = _settings_march(settings, cam, flags=flags, rows=getattr(settings, "rows", None))
         else:
-            # one buffer for all of them, cleared at once; every tensor starts on a 16-byte boundary
-            at, total = [], 0
-            for t in tensors:
-                at.append(total)
-                total += (t.numel() + 3) & ~3
-            flat = torch.zeros(total, device=rgb.device)
-            grads = [flat.as_strided(t.shape, t.stride(), a) for t, a in zip(tensors, at)]
-            march.flags |= _lib.FLAG_GRADS_CLEAR
+            # a tensor of its own for each, so that keeping one keeps no other; rgx_backward clears them in one launch
+            grads = [torch.empty_like(t) for t in tensors]
         if r._build_serial != ctx.build_serial:
             # another build came between this view's forward and its backward (a second model, an evaluation copy,
             # a finite-difference probe): the backward reads the geometry of the latest build, so build again from
