@@ -192,13 +192,36 @@ class _Node:
         pass
 
 
+class _Edges(torch.autograd.Function):
+    """A graph node that leads to the accumulators of the parameters given."""
+
+    @staticmethod
+    def forward(ctx, *params):
+        return params[0].new_empty(0)
+
+
+def _accumulators_held(params) -> bool:
+    """Whether something else holds a parameter's gradient accumulator -- a hook on it, a graph that is still in use.  Autograd
+    makes an accumulator when one is asked for and drops it with its last holder, so one that something is written on is
+    found again only if it has another."""
+    for again in (False, True):
+        end = _Edges.apply(*params)
+        nodes = [node for node, _ in end.grad_fn.next_functions]
+        if again:
+            return any([node.metadata.pop("rgx_seen", False) for node in nodes])
+        for node in nodes:
+            node.metadata["rgx_seen"] = True
+        del end, nodes, node
+
+
 def _gradients_directly(pc, settings, target, cam, supersampling, t):
     """Loss, and the gradients left in the parameters' empty ``.grad``: the iteration's three Functions called one after the
     other.  Built and run by autograd they cost a small scene's iteration more host time than its kernels take (4 k Gaussians
-    at 64x64: 0.70 ms of host time around 0.35 ms of kernels, 0.41 this way).  None: something here is for autograd to look after -- another
-    class of point cloud, frozen parameters, hooks, gradients to add to, another loss."""
+    at 64x64: 0.70 ms of host time around 0.35 ms of kernels, 0.41 this way).  None: something here is for autograd to look after -- a
+    point cloud with accessors of its own, frozen parameters, hooks on them, gradients to add to, another loss.  Where something holds
+    an accumulator, autograd hands the gradients over, and with them to the hooks there."""
     params = (pc.positions, pc.scales, pc.quaternions, pc.densities, pc.rgb, pc.spherical_harmonics, pc.sph_gauss_features,
-              pc.bandwidth_sharpness, pc.lobe_axis) if type(pc) is SimplePointCloud else ()
+              pc.bandwidth_sharpness, pc.lobe_axis) if _as_defined(pc, _ACCESSORS) else ()
     if (not params or t.lambda_iso != 0 or target.dim() != 3 or target.requires_grad or not _fusable(*params, target)
             or not torch.is_grad_enabled()):
         return None
@@ -218,9 +241,13 @@ def _gradients_directly(pc, settings, target, cam, supersampling, t):
         d_image = _ImageLoss.backward(compare, None)[0]
         g_pos, g_scales, g_q, g_dens, g_color, g_sg, g_sharp, g_axis, _ = r_ox.RenderOptixFunction.backward(render, d_image)
         d = _Activate.backward(activate, g_scales, g_q if with_q else None, g_color, g_sharp, g_axis if with_axis else None)
-    positions.grad, densities.grad, sg.grad = g_pos, g_dens, g_sg
-    scales.grad, quaternions.grad, rgb.grad, sh.grad, sharpness.grad = d[0], d[1] if with_q else g_q, d[2], d[3], d[4]
-    axis.grad = d[5] if with_axis else g_axis
+    grads = (g_pos, d[0], d[1] if with_q else g_q, g_dens, d[2], d[3], g_sg, d[4], d[5] if with_axis else g_axis)
+    if _accumulators_held([p for p in params if p.numel() > 0]):
+        there = [(p, g) for p, g in zip(params, grads) if g is not None]
+        torch.autograd.backward([p for p, _ in there], [g for _, g in there])
+    else:
+        for p, g in zip(params, grads):
+            p.grad = g
     return loss
 
 
@@ -279,7 +306,7 @@ def training_iteration(pointcloud, viewpoint_cam, config, iteration: int, schedu
         loss.backward()
     if pointcloud.positions.grad is not None:
         grad = pointcloud.positions.grad
-        if type(pointcloud) is SimplePointCloud and _fusable(grad, pointcloud.num_accum_gnv):     # both statistics in one pass
+        if _as_defined(pointcloud, _STATISTICS) and _fusable(grad, pointcloud.num_accum_gnv):     # both statistics in one pass
             if not pointcloud.accumulate_gradient(grad, viewpoint_cam, pointcloud.num_accum_gnv.data_ptr()):
                 pointcloud.accumulate_gradient_gaussians_not_visible(grad)
         else:
@@ -452,6 +479,19 @@ class SimplePointCloud:
                                                  self.num_accum_gnv.data_ptr(), None, _stream(grad)), "rgx_gradient_stats")
             return
         self.num_accum_gnv += torch.where(torch.norm(grad, dim=1) > 0, 1.0, 0.0)
+
+
+#: What the fused paths above take the place of, as it is defined here.
+_ACCESSORS = {k: vars(SimplePointCloud)[k] for k in (
+    "get_data", "get_color_features", "get_scale", "get_normalized_quaternion", "get_density", "get_bandwidth_sharpness",
+    "get_normalized_lobe_axis")}
+_STATISTICS = {k: vars(SimplePointCloud)[k] for k in ("accumulate_gradient", "accumulate_gradient_gaussians_not_visible")}
+
+
+def _as_defined(pc, methods) -> bool:
+    """A SimplePointCloud, or a class derived from it, that has replaced none of ``methods``, neither in its class nor on the object."""
+    own = getattr(pc, "__dict__", {})
+    return isinstance(pc, SimplePointCloud) and all(getattr(type(pc), k) is f and k not in own for k, f in methods.items())
 
 
 def default_config(dt=0.01, dynamic_sampling=False, white_background=False, max_prim_slice=512, lambda_ssim=0.2,
