@@ -36,9 +36,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 N_VIEWS = 20
-# DRAM bytes of one recording forward launch per byte it records, from ncu captures (profiles/): the recording is
-# written once, the Gaussian records and the lists stream through once
-TRAFFIC_PER_RECORDED_BYTE = 1.018
+# DRAM bytes of one recording forward launch per byte it records, from ncu captures of smaller cases (0.927 and 0.930,
+# profiles/march_forward_dram_traffic_unbounded-2M_and_1M_628x414.md): the recording is written once, what of it is still in the
+# L2 at the end of the launch is not counted, and little is read
+TRAFFIC_PER_RECORDED_BYTE = 0.93
 WORKLOAD = "unbounded-3M"
 METRIC = "fwd+bwd Mrays/s (3M Gaussians, 1256x828)"
 

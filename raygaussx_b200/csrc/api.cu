@@ -99,7 +99,7 @@ struct rgx_ctx {
     int near_budget_now = RGX_NEAR_BUDGET;       // ... and now: see near_deeper, near_went_well; back to the above with a set of another size
     int near_clean = 0, near_wait = kNearWait;   // views in a row in which no ray went beyond, of the number after which the lists get shallower
     bool near_lowered = false;                   // they have since the last time they got deeper
-    long long near_stats[4] = {0, 0, 0, 0};   // views with such lists, pairs of those views (estimate), pairs kept, views marched again
+    long long near_stats[4] = {0, 0, 0, 0};   // views with such lists, pairs of those views (estimate), pairs kept, views with rays beyond
     // rays that went beyond the horizon in the latest march over such lists: counted on the device, finished there by a
     // per-ray search, and known to the host only later (settle_beyond)
     int* hz_rays = nullptr; long long hz_rays_cap = 0;
@@ -122,8 +122,8 @@ struct rgx_ctx {
     // forward could not be recorded; cleared by one memset
     unsigned long long* tape_used = nullptr; long long tape_used_cap = 0;
     unsigned long long* tape_used_host = nullptr;   // pinned; refreshed asynchronously after every recording forward
-    long long* ray_head = nullptr;                  // first chunk of every patch, then a byte per ray: not recorded
-    long long ray_head_cap = 0;
+    long long* patch_heads = nullptr;               // first chunk of every patch, then a byte per ray: not recorded
+    long long patch_head_cap = 0;
     bool tape_valid = false;
     unsigned long long rgba_serial = 0, tape_rgba_serial = 0;   // which evaluation of the per-view colours is in rgba / was recorded with
     unsigned long long tape_build_id = 0;
@@ -201,7 +201,7 @@ void release_workspace(rgx_ctx* ctx) {
                      (void**)&ctx->bin_keys_out, (void**)&ctx->bin_vals_in, (void**)&ctx->bin_vals_out, (void**)&ctx->bin_ranks,
                      (void**)&ctx->tile_cnt, (void**)&ctx->tile_pbegin, (void**)&ctx->ent_id, (void**)&ctx->ent_range, (void**)&ctx->ent_blk,
                      (void**)&ctx->bin_cub, (void**)&ctx->bin_zero, (void**)&ctx->tape, (void**)&ctx->tape_used,
-                     (void**)&ctx->ray_head, (void**)&ctx->tile_dir, (void**)&ctx->tile_iota,
+                     (void**)&ctx->patch_heads, (void**)&ctx->tile_dir, (void**)&ctx->tile_iota,
                      (void**)&ctx->tile_cnt_sorted, (void**)&ctx->tile_order, (void**)&ctx->big_slot,
                      (void**)&ctx->big_rect, (void**)&ctx->tile_resume,
                      (void**)&ctx->hz_state, (void**)&ctx->hz_scalars, (void**)&ctx->tape_tile_order, (void**)&ctx->g_rect, (void**)&ctx->g_code, (void**)&ctx->kept_slot,
@@ -218,7 +218,7 @@ void release_workspace(rgx_ctx* ctx) {
     ctx->bin_pair_cap = ctx->bin_ent_cap = ctx->bin_cub_cap = 0;
     ctx->big_cap = 0;
     ctx->tape_cap = 0;
-    ctx->ray_head_cap = 0;
+    ctx->patch_head_cap = 0;
     ctx->tape_order_cap = 0;
     ctx->lists_event_set = false;
     ctx->hint_set = false;
@@ -779,9 +779,9 @@ static Cull near_cull(const rgx_ctx* ctx) { return Cull{ctx->near_budget_now, (u
 // Turns the emitted pairs into ctx->lists.  The view of a recording forward -- a training view, whose rays end long
 // before they have seen most of their tile's list (on the 3 M-Gaussian scene every ray ends within the nearest eighth
 // of the pairs) -- was emitted only up to a horizon (emit_setup with near_only; binning.cu picks the horizon so that
-// about near_budget_per_ray pairs per ray begin before it): such lists are marked partial, the march counts the rays
-// that would have needed more (march_lists.cu, hz_phase 3), and forward_impl, should there be any, makes the complete
-// lists and marches the view again.  Emission and sorting are nearly all of a view's list construction.
+// about near_budget_now pairs per ray begin before it): such lists are marked partial, the march counts and lists the rays
+// that would have needed more (march_lists.cu, hz_phase 3), and march_forward_listed_rays_kernel finishes them by a search of
+// the hierarchy.  Emission and sorting are nearly all of a view's list construction.
 static int lists_from_pairs(rgx_ctx* ctx, BinLaunch& b, int total, int ntiles, const rgx_camera* cam, const rgx_march* m,
                             cudaStream_t s) {
     int rc;
@@ -1000,7 +1000,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
     }
     if ((rc = run_colors(ctx, scene, cam->eye, s, L.lists.ent_id != nullptr && !counting)))
         return rc;
-    // one march of the view over the lists in L.lists (a lambda: a view whose lists stop at a horizon may need a second one)
+    // the march of the view over the lists in L.lists
     auto march_once = [&]() -> int {
         cudaError_t e;
         const bool record = (march->flags & RGX_FLAG_SAVE_HITS) && L.lists.ent_id != nullptr && ctx->n > 0;
@@ -1020,9 +1020,9 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
             }
             const int ntiles = L.lists.tiles_x * L.lists.tiles_y;
             const long long heads = (long long)ntiles * kMaxPatchesPerTile, head_words = heads + (rays + 7) / 8;
-            if (head_words > ctx->ray_head_cap) {
-                if ((e = regrow(ctx, ctx->ray_head, (size_t)head_words)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
-                ctx->ray_head_cap = head_words;
+            if (head_words > ctx->patch_head_cap) {
+                if ((e = regrow(ctx, ctx->patch_heads, (size_t)head_words)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
+                ctx->patch_head_cap = head_words;
             }
             if (ntiles > ctx->tape_order_cap) {
                 if ((e = regrow(ctx, ctx->tape_tile_order, (size_t)ntiles + 64)) != cudaSuccess) return cuda_fail(ctx, e, "tape");
@@ -1056,7 +1056,7 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
             ctx->tape_order = L.lists.tile_order;
             if (ctx->tape) {
                 L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
-                L.patch_head = ctx->ray_head; L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + heads);
+                L.patch_head = ctx->patch_heads; L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->patch_heads + heads);
                 L.tile_unrecorded = reinterpret_cast<int*>(ctx->tape_used + 8);
                 if (ctx->tape_limit >= 0 && ctx->tape_limit < L.tape_cap) L.tape_cap = ctx->tape_limit;
             }
@@ -1173,8 +1173,8 @@ int rgx_backward(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* cam, co
     }
     if (L.lists.ent_id && tape_matches) {
         L.tape = ctx->tape; L.tape_used = ctx->tape_used; L.tape_cap = ctx->tape_cap;
-        L.patch_head = ctx->ray_head;
-        L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->ray_head + (long long)L.lists.tiles_x * L.lists.tiles_y * kMaxPatchesPerTile);
+        L.patch_head = ctx->patch_heads;
+        L.ray_unrecorded = reinterpret_cast<unsigned char*>(ctx->patch_heads + (long long)L.lists.tiles_x * L.lists.tiles_y * kMaxPatchesPerTile);
         L.tile_unrecorded = reinterpret_cast<int*>(ctx->tape_used + 8);
         L.replay_order = ctx->tape_order;
     }

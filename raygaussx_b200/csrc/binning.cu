@@ -336,9 +336,10 @@ __device__ __forceinline__ unsigned hist_bucket(float tn, const KeyLayout& kl) {
 //
 // Rays that end early -- those of a training view, of a dense scene -- look at the beginning of their tile's list
 // only.  Such a view's lists need only hold the pairs that begin before a horizon (about near_target of them), and
-// the pairs beyond need not even be emitted.  A recording forward counts the rays that reach the horizon after all
-// and, if there are any, starts over with complete lists; a forward that records nothing puts those rays aside and
-// takes them up again with the complete lists of their tiles (b.tile_flag) -- lists in two depths (march_lists.cu).  The horizon is picked before the emission, on the device, from what is cheap to know of a Gaussian:
+// the pairs beyond need not even be emitted.  A recording forward lists the rays that reach the horizon after all,
+// and march_forward_listed_rays_kernel finishes them by a search of the hierarchy; a forward that records nothing puts
+// those rays aside and takes them up again with the complete lists of their tiles (b.tile_flag) -- lists in two depths
+// (march_lists.cu).  The horizon is picked before the emission, on the device, from what is cheap to know of a Gaussian:
 // the rectangle of tiles it can touch (an upper bound of its pairs) and a lower bound of the distance at which any
 // of its pairs begins.  bin_near_hist_kernel: those two per Gaussian, and their histogram; bin_pick_horizon_kernel:
 // the bucket at which the running sum reaches the target; the emission kernels then skip Gaussians and pairs that

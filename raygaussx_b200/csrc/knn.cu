@@ -51,8 +51,11 @@ __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict
 }
 
 // Positions along a Hilbert curve.  A cell that holds many points leaves them in no order, their boxes of 32 all as large as
-// the cell: ten bits per axis do for small clouds, a large one whose extent is set by a few far points (an unbounded scene)
-// needs finer cells (3 M points, core and shell: query 14.4 ms with 10 bits per axis, 1.3 with 16).
+// the cell, so a cloud whose extent is set by a few far points needs fine cells: sixteen points at 1,000 times the size of a cloud of
+// 1 M on surfaces take the whole call from 6.1 ms to 38.2 with 10 bits per axis instead of 16, 300 k from 2.0 to 5.3, 100 k from 0.70 to
+// 1.19, 65 k from 0.48 to 0.67, 30 k from 0.31 to 0.35, and 3 M points of a core and a shell from 1.43 to 1.78.  Where there are none,
+// sorting 64-bit keys costs 0.02 to 0.07 ms (100 k on surfaces 0.153 -> 0.177, 1 M 0.446 -> 0.509).  The extent cannot be told without
+// waiting for the device, so the line is the count from which the loss outweighs that price.
 template <class Key>
 __global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ pts, int n, const unsigned* bounds,
                                                        Key* keys, unsigned* vals) {

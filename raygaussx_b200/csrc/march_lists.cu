@@ -432,15 +432,15 @@ __device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq,
 // entries are tested, lane group h tests entry e + h for all the rays; while hits are evaluated, lane h of a ray holds the samples
 // P i + h of its slab, 32 / P samples times four sums in registers.  Hits are evaluated only in the parts of the slab that some ray's
 // stretch inside the Gaussian reaches.
-//   What bounds it: instruction issue (66 % of the slots on the 300 k object, 2,376 M warp instructions; a warp per ray took
-// 7,800 M) and, recording, the 512 bytes of sums per ray and slab.  With P = 1 the sums of a slab would be 128 registers and eight
+//   What bounds it: instruction issue (67 % of the slots on 2 M Gaussians at 628x414, 63 % on the 300 k object at 400x400; the rest
+// waits on dependent chains at sixteen warps per SM) and, recording, the 512 bytes of sums per ray and slab.  With P = 1 the sums of a slab would be 128 registers and eight
 // warps would fill an SM; P = 2 halves them at the price of one exchange per sample in the compositing.
 //   Tests of a group of entries come before their evaluation, through shared memory: the loops are short (a unit of tests and the
 // evaluation of both halves in one body missed the instruction cache) and the evaluation runs over entries that were hit only.
 //   Slabs of the rays are taken in steps: the ray that is furthest behind leads, and every ray whose slab begins before the
 // leader's ends marches with it.  The list is walked once per step over the union of the windows.
-//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.1 -> 3.5, 300 k object 9.25 -> 3.4 (7.8 -> 2.9
-// without recording), 7 M needles 11.6 -> 4.55 (two depths), 1 M at 640x360 1.67 -> 0.76.
+//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.3 -> 3.6, 300 k object 9.3 -> 3.3 (7.8 -> 2.9
+// without recording), 7 M needles 14.6 -> 5.65 (two depths), 1 M at 640x360 1.83 -> 0.81.
 //
 // HZ: the two-depth variant for forward-only views whose rays end early (binning.cu).  In its first phase
 // (L.hz_phase == 1) the tile lists hold only the pairs that begin before L.horizon; a ray that would need more
@@ -489,12 +489,12 @@ struct SampleTree {
         else part[level] = v;
     }
 };
-// CTAs of one warp per SM that a forward kernel is compiled for, and so its registers: 128 with 16, 136 with 15.  The warps of a
-// patch kernel share nothing, and in CTAs of one warp their number per SM, and with it the registers of each, can be chosen one by
-// one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward takes 3.52
+// CTAs of one warp per SM that a forward kernel is compiled for and launched with: 128 registers with 15 or 16.  The warps of a
+// patch kernel share nothing, and in CTAs of one warp their number per SM can be chosen one by
+// one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward took 3.52
 // instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  14 or 15 warps are slower there (3.78 / 3.83), 17 to 20
 // (96 registers) as fast on the 3 M view and slower on the object (3.74).  Without recording the object, whose slabs hold few
-// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles 4.72 with 15 and 4.55 with 16.
+// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles 4.72 with 15 and 4.55 with 16 (its first depth).
 template <bool COUNT, bool SAVE, int HZ>
 __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ != 0 ? 16 : 15; }
 // The replay, of 95 registers: 18 to 20 warps per SM are 4 % faster than 16 (four CTAs of four).
@@ -508,9 +508,10 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
     PatchShared<P>& sh = shared[warp];
     PatchStage& st = sh.st;
     TapeState& tq = sh.tq;
-    // Two test steps at once where lists are culled, that is in dense scenes: 7 M needles 4.55 -> 4.38 ms, 1 M at 640x360 0.76 -> 0.74,
-    // recording 3 M view 3.52 -> 3.46.  On the object, whose slabs hold few Gaussians, it costs 7 to 10 %.
-    constexpr int kTestUnroll = HZ != 0 ? 2 : 1;
+    // Two test steps at once in recording forwards whose lists stop at a horizon, that is in dense scenes: window of four 3 M views
+    // 15.11 -> 14.53 ms, 1 M with lobes 0.98 -> 0.94.  No difference in two depths (three frames of 7 M needles 16.93, 1 M at 640x360
+    // 0.81 either way); on the object, whose slabs hold few Gaussians, it costs 7 to 10 %.
+    constexpr int kTestUnroll = HZ == 2 ? 2 : 1;
     const float eps = L.m.transmittance_eps;
     const float sub_half = (float)sub + 0.5f;
     const int cap = L.m.max_prim_slice;
@@ -868,7 +869,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
 // patch's rays; a lane walks the samples that lie inside that Gaussian on its ray (a handful of the 32) and keeps the four
 // moment sums in registers.  The thirteen sums of the Gaussian's gradient row are then added up over the rays in shared memory and
 // leave the SM as one coalesced reduction of 52 bytes, where a reduction per ray and hit kept the L2 and the L1 data pipe busy.
-// Bound by instruction issue (77 % of the slots).  3 M-Gaussian view 7.7 -> 2.6 ms, 300 k object 4.7 -> 2.2 ms.
+// Bound by instruction issue (78 % of the slots).  Against a warp per ray: 3 M-Gaussian view 7.7 -> 2.7 ms, 300 k object 4.7 -> 2.15 ms.
 template <int P>
 struct ReplayShared {
     PatchStage st;

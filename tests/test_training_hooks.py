@@ -76,14 +76,9 @@ def test_hooks_on_accumulators_run(iteration):
 @pytest.mark.gpu
 def test_accessors_of_the_callers_own_run(iteration):
     called = []
-
-    class Other(tr.SimplePointCloud):
-        def accumulate_gradient(self, grad, camera):
-            called.append("statistics")
-            return super().accumulate_gradient(grad, camera)
-
-    pc = cloud(Other, "cuda")
-    data = pc.get_data
+    pc = cloud(device="cuda")
+    data, stats = pc.get_data, pc.accumulate_gradient
     pc.get_data = lambda *a, **k: called.append("data") or data(*a, **k)
+    pc.accumulate_gradient = lambda grad, camera: called.append("statistics") or stats(grad, camera)
     iteration(pc)
     assert called == ["data", "statistics"] and float(pc.num_accum.sum()) > 0 and float(pc.num_accum_gnv.sum()) > 0
