@@ -494,7 +494,7 @@ struct SampleTree {
 // one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward took 3.52
 // instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  14 or 15 warps are slower there (3.78 / 3.83), 17 to 20
 // (96 registers) as fast on the 3 M view and slower on the object (3.74).  Without recording the object, whose slabs hold few
-// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles 4.72 with 15 and 4.55 with 16 (its first depth).
+// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles (three frames) 17.65 with 15 and 16.93 with 16.
 template <bool COUNT, bool SAVE, int HZ>
 __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ != 0 ? 16 : 15; }
 // The replay, of 95 registers: 18 to 20 warps per SM are 4 % faster than 16 (four CTAs of four).
