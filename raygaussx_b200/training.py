@@ -214,16 +214,22 @@ def _accumulators_held(params) -> bool:
         del end, nodes, node
 
 
+def _autograd_watched() -> bool:
+    """Whether somebody looks on: hooks on saved tensors (``torch.autograd.graph.saved_tensors_hooks``), anomaly detection, a mode."""
+    return (torch._C._autograd._top_saved_tensors_default_hooks(True) is not None or torch.is_anomaly_enabled()
+            or torch._C._is_torch_function_mode_enabled() or torch._C._len_torch_dispatch_stack() > 0)
+
+
 def _gradients_directly(pc, settings, target, cam, supersampling, t):
     """Loss, and the gradients left in the parameters' empty ``.grad``: the iteration's three Functions called one after the
     other.  Built and run by autograd they cost a small scene's iteration more host time than its kernels take (4 k Gaussians
     at 64x64: 0.70 ms of host time around 0.35 ms of kernels, 0.41 this way).  None: something here is for autograd to look after -- a
-    point cloud with accessors of its own, frozen parameters, hooks on them, gradients to add to, another loss.  Where something holds
+    point cloud with accessors of its own, frozen parameters, hooks on them or on saved tensors, gradients to add to, another loss.  Where something holds
     an accumulator, autograd hands the gradients over, and with them to the hooks there."""
     params = (pc.positions, pc.scales, pc.quaternions, pc.densities, pc.rgb, pc.spherical_harmonics, pc.sph_gauss_features,
               pc.bandwidth_sharpness, pc.lobe_axis) if _as_defined(pc, _ACCESSORS) else ()
     if (not params or t.lambda_iso != 0 or target.dim() != 3 or target.requires_grad or not _fusable(*params, target)
-            or not torch.is_grad_enabled()):
+            or not torch.is_grad_enabled() or _autograd_watched()):
         return None
     for p in params:
         if not p.requires_grad or not p.is_leaf or p.grad is not None or p._backward_hooks or p._post_accumulate_grad_hooks:

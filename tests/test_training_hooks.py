@@ -44,6 +44,18 @@ def test_replaced_methods_are_noticed():
     assert not tr._as_defined(pc, tr._STATISTICS) and not tr._as_defined(object(), tr._ACCESSORS)
 
 
+def test_onlookers_are_noticed():
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    assert not tr._autograd_watched()
+    same = lambda t: t
+    for onlooker in (torch.autograd.graph.saved_tensors_hooks(same, same), torch.autograd.detect_anomaly(check_nan=False),
+                     TorchFunctionMode(), TorchDispatchMode()):
+        with onlooker:
+            assert tr._autograd_watched(), onlooker
+    assert not tr._autograd_watched()
+
+
 @pytest.fixture
 def iteration():
     if not torch.cuda.is_available():
@@ -82,3 +94,11 @@ def test_accessors_of_the_callers_own_run(iteration):
     pc.accumulate_gradient = lambda grad, camera: called.append("statistics") or stats(grad, camera)
     iteration(pc)
     assert called == ["data", "statistics"] and float(pc.num_accum.sum()) > 0 and float(pc.num_accum_gnv.sum()) > 0
+
+
+@pytest.mark.gpu
+def test_hooks_on_saved_tensors_run(iteration):
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+        iteration(cloud(device="cuda"))
+    assert packed
