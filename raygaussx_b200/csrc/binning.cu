@@ -137,12 +137,18 @@ struct PairGeom {
     float4 g0, g1, g2;
     float far_box;      // largest distance from the eye to the box
     float rho_scale;    // operator norm of the whitening map: 1 / (k s_min), with slack for non-unit quaternions
+    float away, slack;  // see pair_range
 };
 
 // Range of ray parameters at which some ray of the tile can be inside the Gaussian's box and
 // inside its truncation ellipsoid; false if no ray of the tile can.  Every ray of the tile is, at
 // parameter t, within t * chord of the central ray's point, so the central ray is tested against
 // the box and the ellipsoid grown by that much.
+// A ray whose closest approach lies behind the eye misses, even from inside (ellipsoid_stretch in march_common.cuh): for M the whitening
+// map and Oe = M (eye - centre), if -Oe . M d < 0.  `away` = |M^T Oe|, so for a ray of the tile that is at most the central ray's plus
+// chord * away; `slack` is ten times what rounding can make of it.  Such pairs are those of Gaussians that hold the eye and lie
+// behind it: a third of the entries that the march of 30 k large Gaussians about the camera tested, a seventh of 1 M
+// (forward of the former at 399x301 0.278 -> 0.229 ms, of the latter at 628x414 0.907 -> 0.851, four views of 3 M 14.47 -> 14.02).
 __device__ __forceinline__ bool pair_range(const float* eye, float4 td, const PairGeom& g, float& tn, float& tf) {
     const float infl = g.far_box * td.w * 1.0001f + 1e-6f;
     // ellipsoid |M (x - p)| <= 1 grown to radius rho in the whitened frame; first, since it turns away the more: a needle's
@@ -154,6 +160,7 @@ __device__ __forceinline__ bool pair_range(const float* eye, float4 td, const Pa
     const float3 de = make_float3(g.g0.w * td.x + g.g1.x * td.y + g.g1.y * td.z, g.g1.z * td.x + g.g1.w * td.y + g.g2.x * td.z,
                                   g.g2.y * td.x + g.g2.z * td.y + g.g2.w * td.z);
     const float qa = dot3(de, de), qb = -dot3(Oe, de), qc = dot3(Oe, Oe) - rho * rho;
+    if (fmaf(td.w, g.away, qb) < -g.slack) return false;       // behind the eye for every ray of the tile
     const float disc = qb * qb - qa * qc;
     const float mag = qb * qb + fabsf(qa * qc);
     if (disc < -1e-5f * mag) return false;
@@ -252,6 +259,11 @@ __device__ __forceinline__ PairGeom make_pair_geom(const float* eye, float2 bx, 
     float smin = fminf(sd.x, fminf(sd.y, sd.z));
     float qn = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
     g.rho_scale = 1.02f * fmaxf(1.0f, qn) / (kk * smin);
+    const float3 O = make_float3(eye[0] - g0.x, eye[1] - g0.y, eye[2] - g0.z);
+    const float3 r0 = make_float3(g0.w, g1.x, g1.y), r1 = make_float3(g1.z, g1.w, g2.x), r2 = make_float3(g2.y, g2.z, g2.w);
+    const float3 Oe = make_float3(dot3(r0, O), dot3(r1, O), dot3(r2, O)), v = r0 * Oe.x + r1 * Oe.y + r2 * Oe.z;
+    g.away = sqrtf(dot3(v, v));
+    g.slack = 1e-5f * sqrtf(dot3(Oe, Oe) * (dot3(r0, r0) + dot3(r1, r1) + dot3(r2, r2)));
     return g;
 }
 
