@@ -129,7 +129,7 @@ struct RayParabola {
 __device__ __forceinline__ bool ellipsoid_stretch(float3 Oe, float3 de, RayParabola& p) {
     p.a = dot3(de, de);
     const float b = -dot3(Oe, de);
-    p.inv_a = __fdividef(1.0f, p.a);
+    p.inv_a = rcp_approx(p.a);
     const float t = __fmul_rn(b, p.inv_a);
     p.t0 = fmaf(fmaf(-t, p.a, b), p.inv_a, t);
     // both points and both squared distances (dot3's order) in packed instructions: the bits of two scalar ones each
@@ -150,7 +150,7 @@ __device__ __forceinline__ float whitened_c(float3 Oe) {
     return fmaf(Oe.x, Oe.x, fmaf(Oe.y, Oe.y, fmaf(Oe.z, Oe.z, -1.0f)));
 }
 __device__ __forceinline__ float entry_root(float3 Oe, float3 de, float c, const RayParabola& p) {
-    return __fdividef(c, __fadd_rn(-dot3(Oe, de), p.root));
+    return quotient(c, __fadd_rn(-dot3(Oe, de), p.root));
 }
 // Whether the stretch meets [tmin, tmax].  Its far end is the quadratic formula's root and nothing that rounds otherwise: where a
 // Gaussian ends as a slab begins, the one decides whether the slab is empty, and so where the ray's next slab lies.
@@ -585,7 +585,7 @@ __device__ __forceinline__ void composite_forward(const SlabPlan& p, float tbuff
                                                   RayColor& st) {
     SlabTrans tr = slab_transmittance(s, p.dt, st.T, eps, lane);
     float one_m_w = 1.0f - tr.w;
-    float f = tr.live ? __fmul_rn(tr.Ts, __fmul_rn(p.dt, __fdividef(one_m_w, fmaxf(tr.x, 1e-6f)))) : 0.f;
+    float f = tr.live ? __fmul_rn(tr.Ts, __fmul_rn(p.dt, quotient(one_m_w, fmaxf(tr.x, 1e-6f)))) : 0.f;
     st.Cr = __fadd_rn(st.Cr, warp_sum(__fmul_rn(f, cr)));
     st.Cg = __fadd_rn(st.Cg, warp_sum(__fmul_rn(f, cg)));
     st.Cb = __fadd_rn(st.Cb, warp_sum(__fmul_rn(f, cb)));
@@ -621,7 +621,7 @@ __device__ __forceinline__ SlabBackTerms slab_back_terms(float s, float dc, floa
                                                          int lane) {
     SlabBackTerms o;
     o.tr = slab_transmittance(s, dt, T, eps, lane);
-    float inv_s = s > 0.f ? __fdividef(1.0f, s) : 0.f;
+    float inv_s = s > 0.f ? rcp_approx(s) : 0.f;
     float chat = __fmul_rn(dc, inv_s);
     float one_m_w = 1.0f - o.tr.w;
     float step = __fmul_rn(__fmul_rn(o.tr.Ts, one_m_w), chat);                 // T_s (1-w_s) chat_s
@@ -678,7 +678,7 @@ __device__ __forceinline__ void slab_gradients(const MarchLaunch& L, const rgx_m
                                                float gamma, WarpStage& ws, int* prim_of, int lane,
                                                Enum&& enumerate, Emit&& emit) {
     int nstage = 0, nhit = 0;
-    const float inv_dt = __fdividef(1.0f, p.dt);
+    const float inv_dt = rcp_approx(p.dt);
     auto drain = [&]() {
         float sb = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
         eval_backward(ws, nstage, p.dt, tau, beta, gamma, lane, sb, n0, n1, n2);
@@ -709,7 +709,7 @@ __device__ __forceinline__ void slab_gradients(const MarchLaunch& L, const rgx_m
             ws.recA[slot] = make_float4(fmaf(tca, t.de.x, t.Oe.x), fmaf(tca, t.de.y, t.Oe.y),
                                         fmaf(tca, t.de.z, t.Oe.z), 0.f);
             ws.recB[slot] = make_float4(t.de.x, t.de.y, t.de.z, __fadd_rn(tbuffer, -tca));
-            float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
+            float ci = quotient(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
             const int run = first_run(t.p.t0, sqrt_approx(fmaxf(t.p.w2, 0.f)), tbuffer, inv_dt);
             ws.recC[slot] = make_float4(ci, __int_as_float(run), 0.f, 0.f);
             ws.recD[slot] = parabola_record(t.p, tbuffer, __ldg(&L.g.hk[j]));

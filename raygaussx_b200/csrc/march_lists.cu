@@ -265,7 +265,7 @@ __device__ __forceinline__ bool patch_misses(const float4* cone, float4 g0, floa
     const float4 c = cone[0], p = cone[1], q = cone[2];
     const float3 de = whiten_dir(m0, m1, m2, make_float3(c.x, c.y, c.z));
     const float3 dp = whiten_dir(m0, m1, m2, make_float3(p.x, p.y, p.z)), dq = whiten_dir(m0, m1, m2, make_float3(q.x, q.y, q.z));
-    const float inv_a = __fdividef(1.0f, dot3(de, de)), t = -dot3(Oe, de) * inv_a;
+    const float inv_a = rcp_approx(dot3(de, de)), t = -dot3(Oe, de) * inv_a;
     const float3 P = make_float3(fmaf(t, de.x, Oe.x), fmaf(t, de.y, Oe.y), fmaf(t, de.z, Oe.z));
     const float rho = fmaf(__fmul_rn(far, c.w), sqrt_approx(fmaxf(dot3(dp, dp), dot3(dq, dq))), 1.0f);
     const float room = fmaf(__fmul_rn(rho, rho), 1.0005f, 1e-5f) - dot3(P, P);
@@ -516,10 +516,6 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
     PatchShared<P>& sh = shared[warp];
     PatchStage& st = sh.st;
     TapeState& tq = sh.tq;
-    // Two test steps at once in recording forwards whose lists stop at a horizon, that is in dense scenes: window of four 3 M views
-    // 15.11 -> 14.53 ms, 1 M with lobes 0.98 -> 0.94.  No difference in two depths (three frames of 7 M needles 16.93, 1 M at 640x360
-    // 0.81 either way); on the object, whose slabs hold few Gaussians, it costs 7 to 10 %.
-    constexpr int kTestUnroll = HZ == 2 ? 2 : 1;
     const float eps = L.m.transmittance_eps;
     const float sub_half = (float)sub + 0.5f;
     const int cap = L.m.max_prim_slice;
@@ -658,7 +654,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
             if (!__any_sync(kFull, act)) continue;
             const long long c_q = COUNT ? clock64() : 0;
             const float tmin = act ? p.tmin : INFINITY, tmax = act ? p.tmax : -INFINITY;
-            const float dt = p.dt, sub_dt = sub ? dt : 0.f, inv_part = __fdividef((float)Pt::kParts / (float)kSlab, p.dt);
+            const float dt = p.dt, sub_dt = sub ? dt : 0.f, inv_part = quotient((float)Pt::kParts / (float)kSlab, p.dt);
             float2 S[Pt::kPairs], R[Pt::kPairs], G[Pt::kPairs], B[Pt::kPairs];
 #pragma unroll
             for (int i = 0; i < Pt::kPairs; ++i) S[i] = R[i] = G[i] = B[i] = make_float2(0.f, 0.f);
@@ -685,9 +681,9 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
 #pragma unroll 1
                 for (int base = 0; base < count; base += kGroup) {
                     const int f = first + base, n = min(count - base, kGroup), nhit0 = nhit;
-                    // test: lane group h of the warp takes entry e + h; no branches, so that the tests of two steps overlap
+                    // test: lane group h of the warp takes entry e + h
                     unsigned reach = 0u;               // kParts bits per entry: parts of the slab that some ray's stretch inside reaches
-#pragma unroll kTestUnroll
+#pragma unroll 1
                     for (int e = 0; e < n; e += P) {
                         const int q = (f + e + sub) & (kStaged - 1);
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
@@ -815,7 +811,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ
                     run = __fadd_rn(run, all);
                     const float one_m_w = 1.0f - exp_neg(x);
                     const float Ts = live ? __fmul_rn(T, exp_neg(excl)) : 0.f;
-                    const float f = __fmul_rn(Ts, __fmul_rn(dt, __fdividef(one_m_w, fmaxf(x, 1e-6f))));
+                    const float f = __fmul_rn(Ts, __fmul_rn(dt, quotient(one_m_w, fmaxf(x, 1e-6f))));
                     cr = fmaf(f, i & 1 ? R[i / 2].y : R[i / 2].x, cr);
                     cg = fmaf(f, i & 1 ? G[i / 2].y : G[i / 2].x, cg);
                     cb = fmaf(f, i & 1 ? B[i / 2].y : B[i / 2].x, cb);
@@ -956,7 +952,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                     run = __fadd_rn(run, all);
                     const float one_m_w = 1.0f - exp_neg(x);
                     const float Ts = __fmul_rn(T, exp_neg(excl));
-                    const float inv_s = c.x > 0.f ? __fdividef(1.0f, c.x) : 0.f;
+                    const float inv_s = c.x > 0.f ? rcp_approx(c.x) : 0.f;
                     const float chat = __fmul_rn(fmaf(dl.x, c.y, fmaf(dl.y, c.z, __fmul_rn(dl.z, c.w))), inv_s);
                     const float tw = __fmul_rn(Ts, one_m_w);
                     const float step = __fmul_rn(tw, chat);                       // T_s (1 - w_s) chat_s
@@ -975,7 +971,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
             }
             __syncwarp();
             // ---- second pass: the Gaussians of the step
-            const float inv_dt = __fdividef(1.0f, dt);
+            const float inv_dt = rcp_approx(dt);
             const float2* bg = &sh.bg[0][r];
             const int2* list = reinterpret_cast<const int2*>(chunk + Pt::kTapeList);
             int n = h0.x;
@@ -1000,7 +996,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const float2 ex = make_float2(st.ex[q].x, st.ex[q].z);
                         const float4 c = st.rgba[q];
                         const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
-                        const float a = dot3(de, de), inv_a = __fdividef(1.0f, a), b = -dot3(Oe, de);
+                        const float a = dot3(de, de), inv_a = rcp_approx(a), b = -dot3(Oe, de);
                         const float t0 = __fmul_rn(b, inv_a), tca = fmaf(fmaf(-t0, a, b), inv_a, t0);    // as in ellipsoid_stretch
                         const float3 yc = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
                         const float qmin = dot3(yc, yc);
@@ -1013,7 +1009,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const int runs = hit && s_hi >= s_lo ? (s_hi - s_lo) / kRun + 1 : 0;
                         // moments about the closest approach: there the whitened ray is at right angles to its direction, so the
                         // terms do not cancel, and inside the ellipsoid none is larger than one
-                        const float ci = __fdividef(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
+                        const float ci = quotient(fmaf(dl.x, c.x, fmaf(dl.y, c.y, __fmul_rn(dl.z, c.z))), c.w);
                         const float off_d = __fadd_rn(tbuffer, -tca);
                         float2 sn = make_float2(0.f, 0.f), n12 = make_float2(0.f, 0.f);          // sums of beta g and of w; of w d and w d^2
                         float x = (float)s_lo + 0.5f;
