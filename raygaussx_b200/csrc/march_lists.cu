@@ -502,19 +502,18 @@ struct SampleTree {
         else part[level] = v;
     }
 };
-// CTAs of one warp per SM that a forward kernel is compiled for and launched with: 128 registers with 15 or 16.  The warps of a
+// CTAs of one warp per SM that a forward kernel is compiled for and launched with: 128 registers with 16.  The warps of a
 // patch kernel share nothing, and in CTAs of one warp their number per SM can be chosen one by
 // one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward took 3.52
-// instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  14 or 15 warps are slower there (3.78 / 3.83), 17 to 20
-// (96 registers) as fast on the 3 M view and slower on the object (3.74).  Without recording the object, whose slabs hold few
-// Gaussians, takes 2.88 ms with 15 and 3.04 with 16, the two-depth forward of 7 M needles (three frames) 17.65 with 15 and 16.93 with 16.
-template <bool COUNT, bool SAVE, int HZ>
-__host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : SAVE || HZ != 0 ? 16 : 15; }
+// instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  15 warps are slower (four 3 M views 13.98 against
+// 13.46 ms, the object 3.09 against 3.05), 18 of 112 registers much slower (15.25, 3.89): the sums of a slab alone are 64.
+template <bool COUNT>
+__host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : 16; }
 // The replay, of 95 registers: 18 to 20 warps per SM are 4 % faster than 16 (four CTAs of four).
 constexpr int kReplayCtas = 18;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
-__global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT, SAVE, HZ>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
+__global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
     using Pt = Patch<P>;
     __shared__ PatchShared<P> shared[kPatchWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / Pt::kRays, r = lane % Pt::kRays;
@@ -1191,7 +1190,7 @@ static int patch_ctas(const MarchLaunch& m, int ctas_per_sm) {
 
 template <int P, bool COUNT, bool SAVE, int HZ>
 static void launch_patches(const MarchLaunch& m, cudaStream_t s) {
-    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, forward_ctas<COUNT, SAVE, HZ>()), kPatchWarps * 32, 0, s>>>(m);
+    note_launch(), march_forward_patches_kernel<P, COUNT, SAVE, HZ><<<patch_ctas<P>(m, forward_ctas<COUNT>()), kPatchWarps * 32, 0, s>>>(m);
 }
 
 template <int P>
