@@ -31,7 +31,6 @@ struct Patch {
     static constexpr int kLanes = P, kRays = 32 / P;
     static constexpr int kW = P == 8 ? 2 : 4, kH = kRays / kW;
     static constexpr unsigned kRayBits = (1u << kRays) - 1u;          // the lanes of one list entry in a ballot
-    static constexpr unsigned kSameRay = P == 2 ? 0x10001u : P == 4 ? 0x01010101u : 0x11111111u;   // the lanes of ray 0
     static constexpr int kSamples = kSlab / P;                        // samples of a lane
     static constexpr int kParts = P == 8 ? 2 : 4;                     // a slab is evaluated in this many parts
     static constexpr int kPairs = kSamples / 2, kPairsPerPart = kPairs / kParts;
@@ -220,10 +219,11 @@ struct PatchStage {                // per warp
     float4 m0[kStaged];            // rows of M = S^-1 R^T / k, and the eye in the whitened frame:
     float4 m1[kStaged];            // (m00, m01, m02, Oe.x), (m10, ...), (m20, ...)
     float4 m2[kStaged];
-    float4 ex[kStaged];            // hk, |Oe|^2 - 1, sorted slot (bits), -
+    float4 ex[kStaged];            // hk, |Oe|^2 - 1, sorted slot (bits), rays that hit it (bits, set once tested)
     float4 rgba[kStaged];          // (r sigma, g sigma, b sigma, sigma)
-    unsigned mask[kStaged];        // rays that hit it
 };
+
+__device__ __forceinline__ unsigned& hit_by(PatchStage& st, int q) { return reinterpret_cast<unsigned*>(&st.ex[q])[3]; }
 
 // smallest / largest of non-negative floats over the warp (they order like their bits)
 __device__ __forceinline__ float warp_min_pos(float v) { return __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(v))); }
@@ -401,11 +401,11 @@ __device__ __forceinline__ void put_offset(int* at, long long off) {
 __device__ __forceinline__ long long get_offset(int lo, int hi) { return ((long long)hi << 32) | (unsigned int)lo; }
 
 // Appends the staged entries [first, first + count) that some ray hit to the list of the current step.
-__device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq, const PatchStage& st, int first, int count, int lane) {
+__device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq, PatchStage& st, int first, int count, int lane) {
     if (tq.chunk < 0) return;
     for (int base = 0; base < count; base += 32) {
         const int q = (first + base + lane) & (kStaged - 1);
-        const unsigned mask = base + lane < count ? st.mask[q] : 0u;
+        const unsigned mask = base + lane < count ? hit_by(st, q) : 0u;
         const unsigned m = __ballot_sync(kFull, mask != 0u);
         const int n = __popc(m);
         if (n == 0) continue;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
             float2 S[Pt::kPairs], R[Pt::kPairs], G[Pt::kPairs], B[Pt::kPairs];
 #pragma unroll
             for (int i = 0; i < Pt::kPairs; ++i) S[i] = R[i] = G[i] = B[i] = make_float2(0.f, 0.f);
-            int nhit = 0, most = 0;                     // hits of this ray; bound on the hits of any ray of the patch
+            int nhit = 0, most = 0;                     // hits of this ray that this lane found; bound on the hits of any ray of the patch
             bool overflow = false;
             if (SAVE) {
                 if (lane == 0 && tq.ok) {
@@ -696,8 +696,9 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         hit = hit && e + sub < n && stretch_meets(pb, tmin, tmax);
                         if (COUNT && act && e + sub < n) { tl.v[C_PRIM_TESTS] += 1; tl.v[C_ELL_TESTS] += 1; }
                         const unsigned m = __ballot_sync(kFull, hit);
-                        nhit += __popc(m & (Pt::kSameRay << r));
-                        if (r == 0) st.mask[q] = (m >> (Pt::kRays * sub)) & Pt::kRayBits;
+                        nhit += hit ? 1 : 0;
+                        // by all lanes alike: a branch around the store, as any in this loop, costs 4 % of the kernel
+                        if (SAVE || COUNT) hit_by(st, q) = (m >> (Pt::kRays * sub)) & Pt::kRayBits;
                         float4 A = parabola_record(pb, t, st.ex[q].x);
                         // parts of the slab that the ray's stretch inside reaches, with a fiftieth of one on either side against
                         // rounding (the test of each sample decides)
@@ -712,21 +713,23 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                     most += n;
                     if (most > cap) {                   // cuda_train/forward/gaussians_aabb.cu:352-356: hits past the cap are dropped
                         int seen = nhit0;
+                        for (int o = Pt::kRays; o < 32; o <<= 1) seen += __shfl_xor_sync(kFull, seen, o);
                         for (int e = 0; e < n; ++e) {
                             const int q = (f + e) & (kStaged - 1);
-                            bool hit = (st.mask[q] >> r) & 1u;
+                            bool hit = sh.rec[e][r].y != -1.0f;
+                            __syncwarp();
                             if (hit && seen >= cap) { hit = false; overflow = true; if (sub == 0) sh.rec[e][r].y = -1.0f; }
                             seen += hit ? 1 : 0;
                             const unsigned m = __ballot_sync(kFull, hit) & Pt::kRayBits;
-                            if (lane == 0) st.mask[q] = m;
+                            if (lane == 0) hit_by(st, q) = m;
                             __syncwarp();
                         }
-                        nhit = seen;
+                        nhit = sub == 0 ? seen : 0;
                     }
                     if (COUNT)
                         for (int e = 0; e < n; ++e) {
                             const int q = (f + e) & (kStaged - 1);
-                            if (sub == 0 && ((st.mask[q] >> r) & 1u))
+                            if (sub == 0 && ((hit_by(st, q) >> r) & 1u))
                                 tl.v[C_HASH] += mix64(((unsigned long long)ray_id << 40) ^ ((unsigned long long)sh.slabs[r] << 24) ^
                                                       (unsigned long long)__ldg(&L.g.perm[__float_as_int(st.ex[q].z)]));
                         }
@@ -763,6 +766,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                 }
                 if (SAVE) tape_append(L, tq, st, first, count, lane);
             });
+            for (int o = Pt::kRays; o < 32; o <<= 1) nhit += __shfl_xor_sync(kFull, nhit, o);
             const bool hits = act && nhit > 0;
             if (COUNT) {
                 if (lane == 0) tl.v[C_CYC_SEARCH] += clock64() - c_q;
@@ -988,14 +992,14 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const int j = en.x;
                         const float4 g0 = __ldg(&L.g.g0[j]), g1 = __ldg(&L.g.g1[j]), g2 = __ldg(&L.g.g2[j]);
                         stage_record(st, lane, j, g0, g1, g2, whiten_eye(L, g0, g1, g2), __ldg(&L.g.hk[j]), __ldg(&L.g.rgba[j]));
-                        st.mask[lane] = (unsigned)en.y & rays;
+                        hit_by(st, lane) = (unsigned)en.y & rays;
                     } else {
-                        st.mask[lane] = 0u;
+                        hit_by(st, lane) = 0u;
                     }
                     __syncwarp();
                     for (int e = 0; e < cnt; e += P) {
                         const int q = e + sub;
-                        const bool hit = (st.mask[q] >> r) & 1u;
+                        const bool hit = (hit_by(st, q) >> r) & 1u;
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         const float2 ex = make_float2(st.ex[q].x, st.ex[q].z);
                         const float4 c = st.rgba[q];
