@@ -216,8 +216,8 @@ __device__ __forceinline__ unsigned fetch_unit(unsigned* next, unsigned units) {
 constexpr int kStaged = 64;        // ring of list entries that passed the patch's filters
 
 struct PatchStage {                // per warp
-    float4 m0[kStaged];            // rows of M = S^-1 R^T / k, and the eye in the whitened frame:
-    float4 m1[kStaged];            // (m00, m01, m02, Oe.x), (m10, ...), (m20, ...)
+    float4 m0[kStaged];            // M = S^-1 R^T / k, and the eye in the whitened frame, the first two rows side by side for
+    float4 m1[kStaged];            // packed instructions: (m00, m10, m01, m11), (m02, m12, Oe.x, Oe.y), (m20, m21, m22, Oe.z)
     float4 m2[kStaged];
     float4 ex[kStaged];            // hk, |Oe|^2 - 1, sorted slot (bits), rays that hit it (bits, set once tested)
     float4 rgba[kStaged];          // (r sigma, g sigma, b sigma, sigma)
@@ -231,8 +231,8 @@ __device__ __forceinline__ float warp_max_pos(float v) { return __uint_as_float(
 
 // One Gaussian's record, as the sorted arrays hold it, into slot `q` (by one lane).
 __device__ __forceinline__ void stage_record(PatchStage& st, int q, int j, float4 g0, float4 g1, float4 g2, float3 Oe, float hk, float4 rgba) {
-    st.m0[q] = make_float4(g0.w, g1.x, g1.y, Oe.x);
-    st.m1[q] = make_float4(g1.z, g1.w, g2.x, Oe.y);
+    st.m0[q] = make_float4(g0.w, g1.z, g1.x, g1.w);
+    st.m1[q] = make_float4(g1.y, g2.x, Oe.x, Oe.y);
     st.m2[q] = make_float4(g2.y, g2.z, g2.w, Oe.z);
     st.ex[q] = make_float4(hk, whitened_c(Oe), __int_as_float(j), 0.f);
     st.rgba[q] = rgba;
@@ -250,6 +250,15 @@ __device__ __forceinline__ float3 whiten_dir(float4 m0, float4 m1, float4 m2, fl
                        fmaf(m1.x, d.x, fmaf(m1.y, d.y, __fmul_rn(m1.z, d.z))),
                        fmaf(m2.x, d.x, fmaf(m2.y, d.y, __fmul_rn(m2.z, d.z))));
 }
+
+// whiten_dir for a staged record: the same bits, six instructions instead of nine (recording forward of four 3 M views 12.38 -> 12.29 ms, of
+// the 300 k object 2.91 -> 2.87).
+__device__ __forceinline__ float3 staged_dir(float4 m0, float4 m1, float4 m2, float3 d) {
+    const float2 xy = __ffma2_rn(make_float2(m0.x, m0.y), make_float2(d.x, d.x), __ffma2_rn(make_float2(m0.z, m0.w), make_float2(d.y, d.y),
+                                 __fmul2_rn(make_float2(m1.x, m1.y), make_float2(d.z, d.z))));
+    return make_float3(xy.x, xy.y, fmaf(m2.x, d.x, fmaf(m2.y, d.y, __fmul_rn(m2.z, d.z))));
+}
+__device__ __forceinline__ float3 staged_eye(float4 m1, float4 m2) { return make_float3(m1.z, m1.w, m2.w); }
 
 // No ray of the patch can meet the Gaussian at a parameter in [wlo, whi].  The rays' directions lie in the parallelogram
 // mid +- e1 +- e2 (cone[0..2], the directions scaled to the middle one's projection; what the normalisation of each ray takes off only
@@ -615,7 +624,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         const int q = (first + e + sub) & (kStaged - 1);
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         RayParabola pb;
-                        const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
+                        const float3 Oe = staged_eye(m1, m2), de = staged_dir(m0, m1, m2, dir);
                         if (ellipsoid_stretch(Oe, de, pb) && e + sub < count && from <= best && stretch_meets(pb, from, best)) {
                             const float at = fmaxf(from, entry_root(Oe, de, st.ex[q].y, pb));
                             if (at <= best) { best = at; found = true; }
@@ -692,7 +701,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         const int q = (f + e + sub) & (kStaged - 1);
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         RayParabola pb;
-                        bool hit = ellipsoid_stretch(make_float3(m0.w, m1.w, m2.w), whiten_dir(m0, m1, m2, dir), pb);
+                        bool hit = ellipsoid_stretch(staged_eye(m1, m2), staged_dir(m0, m1, m2, dir), pb);
                         hit = hit && e + sub < n && stretch_meets(pb, tmin, tmax);
                         if (COUNT && act && e + sub < n) { tl.v[C_PRIM_TESTS] += 1; tl.v[C_ELL_TESTS] += 1; }
                         const unsigned m = __ballot_sync(kFull, hit);
@@ -1003,7 +1012,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         const float2 ex = make_float2(st.ex[q].x, st.ex[q].z);
                         const float4 c = st.rgba[q];
-                        const float3 Oe = make_float3(m0.w, m1.w, m2.w), de = whiten_dir(m0, m1, m2, dir);
+                        const float3 Oe = staged_eye(m1, m2), de = staged_dir(m0, m1, m2, dir);
                         const float a = dot3(de, de), inv_a = rcp_approx(a), b = -dot3(Oe, de);
                         const float t0 = __fmul_rn(b, inv_a), tca = fmaf(fmaf(-t0, a, b), inv_a, t0);    // as in ellipsoid_stretch
                         const float3 yc = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
