@@ -815,25 +815,36 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                 bool live = true;
                 SampleTree<P> tree;
 #pragma unroll
-                for (int i = 0; i < Pt::kSamples; ++i) {
-                    const float x = __fmul_rn(i & 1 ? S[i / 2].y : S[i / 2].x, dt);
-                    float before;
-                    const float all = across_ray<P>(x, sub, before);
-                    if (i == Pt::kSamples / 2) {
+                for (int i = 0; i < Pt::kPairs; ++i) {                   // two samples of the lane at a time, in packed instructions
+                    const float2 dt2 = make_float2(dt, dt), log2e = make_float2(-1.4426950408889634f, -1.4426950408889634f);
+                    const float2 x = __fmul2_rn(S[i], dt2), wx = __fmul2_rn(x, log2e);
+                    if (i == Pt::kPairs / 2) {
                         x16 = tree.half;
                         T16 = __fmul_rn(T, exp_neg(x16));
                         live = T16 > eps;                                // :190-201: the second chunk only counts while T is above the threshold
                     }
-                    const float excl = __fadd_rn(run, before);
-                    run = __fadd_rn(run, all);
-                    const float one_m_w = 1.0f - exp_neg(x);
-                    const float Ts = live ? __fmul_rn(T, exp_neg(excl)) : 0.f;
-                    const float f = __fmul_rn(Ts, __fmul_rn(dt, quotient(one_m_w, fmaxf(x, 1e-6f))));
-                    cr = fmaf(f, i & 1 ? R[i / 2].y : R[i / 2].x, cr);
-                    cg = fmaf(f, i & 1 ? G[i / 2].y : G[i / 2].x, cg);
-                    cb = fmaf(f, i & 1 ? B[i / 2].y : B[i / 2].x, cb);
-                    if (L.depth) cd = fmaf(__fmul_rn(Ts, one_m_w), __fadd_rn(t, __fmul_rn((float)(P * i) + (float)sub + 0.5f, dt)), cd);
-                    tree.add(i, all);
+                    float2 before, excl;
+                    const float all0 = across_ray<P>(x.x, sub, before.x), all1 = across_ray<P>(x.y, sub, before.y);
+                    excl.x = __fadd_rn(run, before.x);
+                    run = __fadd_rn(run, all0);
+                    excl.y = __fadd_rn(run, before.y);
+                    run = __fadd_rn(run, all1);
+                    tree.add(2 * i, all0);
+                    tree.add(2 * i + 1, all1);
+                    const float2 one_m_w = __fadd2_rn(make_float2(1.0f, 1.0f), make_float2(-ex2_approx(wx.x), -ex2_approx(wx.y)));
+                    const float2 tx = __fmul2_rn(excl, log2e);
+                    const float T_live = live ? T : 0.f;
+                    const float2 Ts = __fmul2_rn(make_float2(T_live, T_live), make_float2(ex2_approx(tx.x), ex2_approx(tx.y)));
+                    const float2 per_x = __fmul2_rn(one_m_w, make_float2(rcp_approx(fmaxf(x.x, 1e-6f)), rcp_approx(fmaxf(x.y, 1e-6f))));
+                    const float2 f = __fmul2_rn(Ts, __fmul2_rn(dt2, per_x));
+                    cr = fmaf(f.y, R[i].y, fmaf(f.x, R[i].x, cr));
+                    cg = fmaf(f.y, G[i].y, fmaf(f.x, G[i].x, cg));
+                    cb = fmaf(f.y, B[i].y, fmaf(f.x, B[i].x, cb));
+                    if (L.depth) {
+                        const float2 lost = __fmul2_rn(Ts, one_m_w);
+                        cd = fmaf(lost.x, __fadd_rn(t, __fmul_rn((float)(2 * P * i) + sub_half, dt)), cd);
+                        cd = fmaf(lost.y, __fadd_rn(t, __fmul_rn((float)(2 * P * i + P) + sub_half, dt)), cd);
+                    }
                 }
                 for (int o = Pt::kRays; o < 32; o <<= 1) {
                     cr = __fadd_rn(cr, __shfl_xor_sync(kFull, cr, o));
