@@ -745,18 +745,16 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                                 tl.v[C_HASH] += mix64(((unsigned long long)ray_id << 40) ^ ((unsigned long long)sh.slabs[r] << 24) ^
                                                       (unsigned long long)__ldg(&L.g.perm[__float_as_int(st.ex[q].z)]));
                         }
-                    // evaluate
+                    // Evaluate, entry after entry: to pick those that reach something out of the bits costs more than to pass by the
+                    // others (four 3 M views 12.17 -> 11.72 ms, three frames of 7 M needles 12.83 -> 12.30, the object 2.81 -> 2.79).
+                    // The records of the next entry fetched ahead: 12.57 and 13.09, registers.
+                    const float4 *rec = &sh.rec[0][r], *payload = &st.rgba[f & (kStaged - 1)];     // a group does not wrap around the ring
 #pragma unroll 1
-                    while (reach) {
-                        const int e = (__ffs(reach) - 1) / Pt::kParts;
-                        constexpr unsigned kPartBits = (1u << Pt::kParts) - 1u;
-                        const unsigned here = (reach >> (Pt::kParts * e)) & kPartBits;
-                        reach &= ~(kPartBits << (Pt::kParts * e));
-                        const float4 A = sh.rec[e][r];
-                        const float4 c = st.rgba[(f + e) & (kStaged - 1)];
+                    for (; reach; reach >>= Pt::kParts, rec += Pt::kRays, ++payload) {
+                        const float4 A = *rec, c = *payload;
 #pragma unroll
                         for (int g = 0; g < Pt::kParts; ++g) {
-                            if (!((here >> g) & 1u)) continue;
+                            if (!((reach >> g) & 1u)) continue;
 #pragma unroll
                             for (int i = Pt::kPairsPerPart * g; i < Pt::kPairsPerPart * (g + 1); ++i) {
                                 // (s + 1/2) dt rounded once, as in eval_forward: with two lanes per ray sub dt is exact
