@@ -696,12 +696,12 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
             walk_list<COUNT>(L, tv, sh.cone, wall, warp_min_pos(tmin), whi, cursor, st, 3 * kGroup, lane, tl, [&](int first, int count) {
 #pragma unroll 1
                 for (int base = 0; base < count; base += kGroup) {
-                    const int f = first + base, n = min(count - base, kGroup), nhit0 = nhit;
+                    const int f = (first + base) & (kStaged - 1), n = min(count - base, kGroup), nhit0 = nhit;   // a group does not wrap around the ring
                     // test: lane group h of the warp takes entry e + h
                     unsigned reach = 0u;               // kParts bits per entry: parts of the slab that some ray's stretch inside reaches
 #pragma unroll 1
                     for (int e = 0; e < n; e += P) {
-                        const int q = (f + e + sub) & (kStaged - 1);
+                        const int q = f + e + sub;
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         RayParabola pb;
                         bool hit = ellipsoid_stretch(staged_eye(m1, m2), staged_dir(m0, m1, m2, dir), pb);
@@ -727,7 +727,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         int seen = nhit0;
                         for (int o = Pt::kRays; o < 32; o <<= 1) seen += __shfl_xor_sync(kFull, seen, o);
                         for (int e = 0; e < n; ++e) {
-                            const int q = (f + e) & (kStaged - 1);
+                            const int q = f + e;
                             bool hit = sh.rec[e][r].y != -1.0f;
                             __syncwarp();
                             if (hit && seen >= cap) { hit = false; overflow = true; if (sub == 0) sh.rec[e][r].y = -1.0f; }
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                     }
                     if (COUNT)
                         for (int e = 0; e < n; ++e) {
-                            const int q = (f + e) & (kStaged - 1);
+                            const int q = f + e;
                             if (sub == 0 && ((hit_by(st, q) >> r) & 1u))
                                 tl.v[C_HASH] += mix64(((unsigned long long)ray_id << 40) ^ ((unsigned long long)sh.slabs[r] << 24) ^
                                                       (unsigned long long)__ldg(&L.g.perm[__float_as_int(st.ex[q].z)]));
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                     // Evaluate, entry after entry: to pick those that reach something out of the bits costs more than to pass by the
                     // others (four 3 M views 12.17 -> 11.72 ms, three frames of 7 M needles 12.83 -> 12.30, the object 2.81 -> 2.79).
                     // The records of the next entry fetched ahead: 12.57 and 13.09, registers.
-                    const float4 *rec = &sh.rec[0][r], *payload = &st.rgba[f & (kStaged - 1)];     // a group does not wrap around the ring
+                    const float4 *rec = &sh.rec[0][r], *payload = &st.rgba[f];
 #pragma unroll 1
                     for (; reach; reach >>= Pt::kParts, rec += Pt::kRays, ++payload) {
                         const float4 A = *rec, c = *payload;
