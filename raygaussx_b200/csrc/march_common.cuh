@@ -652,19 +652,19 @@ struct GaussGrad {
 __device__ __forceinline__ GaussGrad expand_gradient(float sigma, float4 A, float4 B, float sb, float n0, float n1,
                                                      float n2) {
     const float m0 = __fmul_rn(sigma, n0), m1 = __fmul_rn(sigma, n1), m2 = __fmul_rn(sigma, n2);
-    const float3 yc = make_float3(A.x, A.y, A.z), de = make_float3(B.x, B.y, B.z);
-    const float3 U = make_float3(fmaf(m0, yc.x, __fmul_rn(m1, de.x)), fmaf(m0, yc.y, __fmul_rn(m1, de.y)),
-                                 fmaf(m0, yc.z, __fmul_rn(m1, de.z)));
-    const float3 V = make_float3(fmaf(m1, yc.x, __fmul_rn(m2, de.x)), fmaf(m1, yc.y, __fmul_rn(m2, de.y)),
-                                 fmaf(m1, yc.z, __fmul_rn(m2, de.z)));
+    // x and y in packed instructions
+    const float2 y = make_float2(A.x, A.y), d = make_float2(B.x, B.y), M0 = make_float2(m0, m0), M1 = make_float2(m1, m1), M2 = make_float2(m2, m2);
+    const float2 U = __ffma2_rn(M0, y, __fmul2_rn(M1, d)), V = __ffma2_rn(M1, y, __fmul2_rn(M2, d));
+    const float Uz = fmaf(m0, A.z, __fmul_rn(m1, B.z)), Vz = fmaf(m1, A.z, __fmul_rn(m2, B.z));
+    const float2 diag = __ffma2_rn(y, U, __fmul2_rn(d, V)), last = __ffma2_rn(y, make_float2(Uz, Uz), __fmul2_rn(d, make_float2(Vz, Vz)));
     GaussGrad g;
-    g.mu = U;
-    g.y00 = fmaf(yc.x, U.x, __fmul_rn(de.x, V.x));
-    g.y11 = fmaf(yc.y, U.y, __fmul_rn(de.y, V.y));
-    g.y22 = fmaf(yc.z, U.z, __fmul_rn(de.z, V.z));
-    g.y01 = fmaf(yc.x, U.y, __fmul_rn(de.x, V.y));
-    g.y02 = fmaf(yc.x, U.z, __fmul_rn(de.x, V.z));
-    g.y12 = fmaf(yc.y, U.z, __fmul_rn(de.y, V.z));
+    g.mu = make_float3(U.x, U.y, Uz);
+    g.y00 = diag.x;
+    g.y11 = diag.y;
+    g.y22 = fmaf(A.z, Uz, __fmul_rn(B.z, Vz));
+    g.y01 = fmaf(A.x, U.y, __fmul_rn(B.x, V.y));
+    g.y02 = last.x;
+    g.y12 = last.y;
     g.dsigma = n0;
     g.drgb_scale = __fmul_rn(sigma, sb);
     return g;

@@ -1040,7 +1040,9 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         const float4 c = st.rgba[q];
                         const float3 Oe = staged_eye(m1, m2), de = staged_dir(m0, m1, m2, dir);
                         const float a = dot3(de, de), inv_a = rcp_approx(a), b = -dot3(Oe, de);
-                        const float t0 = __fmul_rn(b, inv_a), tca = fmaf(fmaf(-t0, a, b), inv_a, t0);    // as in ellipsoid_stretch
+                        // the closest approach as in ellipsoid_stretch; a lane without a hit adds up nothing, and whatever its ray is to the
+                        // Gaussian, zero times a point near it is zero
+                        const float t0 = __fmul_rn(b, inv_a), tca = hit ? fmaf(fmaf(-t0, a, b), inv_a, t0) : 0.f;
                         const float3 yc = make_float3(fmaf(tca, de.x, Oe.x), fmaf(tca, de.y, Oe.y), fmaf(tca, de.z, Oe.z));
                         const float qmin = dot3(yc, yc);
                         const float ay = __fmul_rn(1.0f - qmin, inv_a), az = __fmul_rn(-ex.x, a), aw = __fmul_rn(-ex.x, qmin);
@@ -1073,8 +1075,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                             x += (float)kRun;
                         }
                         const float4 A = make_float4(yc.x, yc.y, yc.z, 0.f);
-                        GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sn.x, sn.y, n12.x, n12.y);
-                        if (!hit) gg = GaussGrad{};
+                        const GaussGrad gg = expand_gradient(c.w, A, make_float4(de.x, de.y, de.z, 0.f), sn.x, sn.y, n12.x, n12.y);
                         sh.red[0][lane] = gg.mu.x; sh.red[1][lane] = gg.mu.y; sh.red[2][lane] = gg.mu.z;
                         sh.red[3][lane] = gg.y00; sh.red[4][lane] = gg.y11; sh.red[5][lane] = gg.y22;
                         sh.red[6][lane] = gg.y01; sh.red[7][lane] = gg.y02; sh.red[8][lane] = gg.y12;
@@ -1083,21 +1084,18 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                         sh.red[11][lane] = __fmul_rn(dl.y, gg.drgb_scale);
                         sh.red[12][lane] = __fmul_rn(dl.z, gg.drgb_scale);
                         __syncwarp();
-                        // the lanes of entry e + h add its components over the rays (row layout: emit_global)
-                        if (q < cnt) {
-                            float* row = reinterpret_cast<float*>(L.grad_rows) +
-                                         16 * ((size_t)((unsigned)tile & (unsigned)(L.grad_copies - 1)) * (size_t)L.g.n_pad + (size_t)__float_as_int(ex.y));
+                        // the lanes of entry e + h add its components over the rays (row layout: emit_global); lanes past the thirteenth add up
+                        // the last one too and keep it to themselves
+                        float* row = reinterpret_cast<float*>(L.grad_rows) +
+                                     16 * ((size_t)((unsigned)tile & (unsigned)(L.grad_copies - 1)) * (size_t)L.g.n_pad + (size_t)__float_as_int(ex.y));
 #pragma unroll
-                            for (int k0 = 0; k0 < 13; k0 += Pt::kRays) {
-                                const int k = k0 + r;
-                                if (k < 13) {
-                                    const float4* v = reinterpret_cast<const float4*>(&sh.red[k][Pt::kRays * sub]);
-                                    float sum = 0.f;
+                        for (int k0 = 0; k0 < 13; k0 += Pt::kRays) {
+                            const int k = min(k0 + r, 12);
+                            const float4* v = reinterpret_cast<const float4*>(&sh.red[k][Pt::kRays * sub]);
+                            float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-                                    for (int i = 0; i < Pt::kRays / 4; ++i) { const float4 a4 = v[i]; sum += (a4.x + a4.y) + (a4.z + a4.w); }
-                                    atomicAdd(row + k, sum);
-                                }
-                            }
+                            for (int i = 0; i < Pt::kRays / 4; ++i) { const float4 a4 = v[i]; sum = __fadd2_rn(sum, __fadd2_rn(make_float2(a4.x, a4.y), make_float2(a4.z, a4.w))); }
+                            if (q < cnt && k0 + r < 13) atomicAdd(row + k, __fadd_rn(sum.x, sum.y));
                         }
                         __syncwarp();
                     }
