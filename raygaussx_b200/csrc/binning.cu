@@ -115,6 +115,7 @@ __device__ __forceinline__ float3 pixel_dir(const rgx_camera& c, float px, float
 // Per tile: direction of the ray through the tile centre and the largest chord |d - d_c| to a
 // ray of the tile (the rays of a tile lie inside the pyramid of its four corner rays).
 __global__ void bin_tile_dirs_kernel(BinLaunch b, int ntiles) {
+    after_previous();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntiles) return;
     int tx = t % b.tiles_x, ty = t / b.tiles_x + b.ty_first;
@@ -359,6 +360,7 @@ __device__ __forceinline__ unsigned hist_bucket(float tn, const KeyLayout& kl) {
 // of its rectangle, added up from rectangle corners by bin_tile_more_kernel).
 
 __global__ void __launch_bounds__(kEmitThreads) bin_near_hist_kernel(BinLaunch b) {
+    after_previous();
     __shared__ unsigned int local[1 << kHistBits];
     for (int i = threadIdx.x; i < (1 << kHistBits); i += kEmitThreads) local[i] = 0u;
     __syncthreads();
@@ -397,6 +399,7 @@ __global__ void __launch_bounds__(kEmitThreads) bin_near_hist_kernel(BinLaunch b
 // one if none does).  Everything is kept (cut = kAllBuckets) when the view has fewer than near_min_total estimated
 // pairs or the cut would keep all of them (half of them or more, with near_half).
 __global__ void __launch_bounds__(1024) bin_pick_horizon_kernel(BinLaunch b) {
+    after_previous();
     using Scan = cub::BlockScan<unsigned long long, 1024>;
     __shared__ typename Scan::TempStorage scan_tmp;
     __shared__ int s_cut, s_first;
@@ -429,6 +432,7 @@ __global__ void __launch_bounds__(1024) bin_pick_horizon_kernel(BinLaunch b) {
 constexpr int kDiffShared = 11900;
 constexpr int kCompactThreads = 1024;
 __global__ void __launch_bounds__(kCompactThreads) bin_compact_kernel(BinLaunch b) {
+    after_previous();
     __shared__ int s_diff[kDiffShared];
     __shared__ unsigned s_count[2][kCompactThreads / 32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -480,6 +484,7 @@ __global__ void __launch_bounds__(kCompactThreads) bin_compact_kernel(BinLaunch 
 // tile_diff holds +1 / -1 at the corners of the rectangles of the skipped Gaussians; its two-dimensional running
 // sum is the number of skipped rectangles over each tile.
 __global__ void __launch_bounds__(1024) bin_tile_more_kernel(BinLaunch b) {
+    after_previous();
     __shared__ int s_diff[kDiffShared];
     const int W = b.tiles_x + 1, H = b.tiles_y + 1;
     int* d = b.tile_diff;
@@ -506,6 +511,7 @@ __global__ void __launch_bounds__(1024) bin_tile_more_kernel(BinLaunch b) {
 // big_rect, those of many tiles from the back) for bin_emit_pairs_kernel.  (A culled emission has the rectangles from
 // bin_near_hist_kernel and the list from bin_compact_kernel.)
 __global__ void __launch_bounds__(kEmitThreads) bin_list_kernel(BinLaunch b) {
+    after_previous();
     const int j = blockIdx.x * kEmitThreads + threadIdx.x, lane = threadIdx.x & 31;
     uint2 rect = make_uint2(kNoRect, 0u);
     bool keep = false;
@@ -550,6 +556,7 @@ constexpr int kBigBatch = 8;
 
 template <bool CULL>
 __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunch b) {
+    after_previous();
     const unsigned cut = CULL ? b.pick->cut : kAllBuckets;
     __shared__ unsigned long long s_keys[kBigWarps][kBigBuf];
     __shared__ float s_fars[kBigWarps][kBigBuf];
@@ -650,6 +657,7 @@ __global__ void __launch_bounds__(kBigWarps * 32) bin_emit_pairs_kernel(BinLaunc
 // (begin of tile t's pairs in tile_first, of its padded list in tile_pbegin, tiles by falling number of pairs in tile_order)
 constexpr int kLayoutThreads = 1024;
 __global__ void __launch_bounds__(kLayoutThreads) bin_layout_kernel(BinLaunch b, int ntiles) {
+    after_previous();
     using Scan = cub::BlockScan<int2, kLayoutThreads>;
     __shared__ typename Scan::TempStorage tmp;
     __shared__ int s_bucket[256];
@@ -698,6 +706,7 @@ __global__ void __launch_bounds__(kLayoutThreads) bin_layout_kernel(BinLaunch b,
 }
 
 __global__ void __launch_bounds__(256) bin_place_kernel(BinLaunch b, int total, int tile_shift) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= total) return;
     const uint64_t key = b.keys_in[k];
@@ -715,6 +724,7 @@ constexpr int kSortCrowd = 96;
 __host__ __device__ constexpr size_t sort_smem(int cap) { return (size_t)cap * (8 + 4) + (size_t)(cap / 32) * 4; }
 template <int kSortThreads, int kSortBuckets>
 __global__ void __launch_bounds__(kSortThreads) bin_sort_tiles_kernel(BinLaunch b, KeyLayout kl, int first_unit, int cap) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char sort_mem[];
     uint64_t* key = reinterpret_cast<uint64_t*>(sort_mem);               // [cap] near | slot
     unsigned* at = reinterpret_cast<unsigned*>(key + cap);               // [cap] pair numbers by bucket, or in order
@@ -809,11 +819,13 @@ __global__ void __launch_bounds__(kSortThreads) bin_sort_tiles_kernel(BinLaunch 
 
 // ---------------------------------------------------------------- lists of any length: after the radix sort
 __global__ void bin_tile_iota_kernel(BinLaunch b, int ntiles) {
+    after_previous();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < ntiles) b.tile_iota[t] = t;
 }
 
 __global__ void __launch_bounds__(256) bin_fill_kernel(BinLaunch b, size_t n_entries) {
+    after_previous();
     size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_entries) return;
     b.ent_id[k] = 0;
@@ -821,6 +833,7 @@ __global__ void __launch_bounds__(256) bin_fill_kernel(BinLaunch b, size_t n_ent
 }
 
 __global__ void __launch_bounds__(256) bin_scatter_kernel(BinLaunch b, int total, KeyLayout kl) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= total) return;
     const uint64_t key = b.keys_out[k];
@@ -833,6 +846,7 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(BinLaunch b, int total
 
 // One warp per block of 32 entries: nearest near distance and farthest far distance.
 __global__ void __launch_bounds__(256) bin_blocks_kernel(BinLaunch b, size_t n_blocks) {
+    after_previous();
     size_t blk = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (blk >= n_blocks) return;
@@ -894,19 +908,19 @@ cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s) {
         // only the pairs that begin before a horizon, which is picked on the way (see bin_near_hist_kernel)
         const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
         if (kl.near_bits < kHistBits) return cudaErrorInvalidValue;
-        note_launch(), bin_tile_dirs_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
-        note_launch(), bin_near_hist_kernel<<<blocks, kEmitThreads, 0, s>>>(b);
-        note_launch(), bin_pick_horizon_kernel<<<1, 1024, 0, s>>>(b);
-        note_launch(), bin_compact_kernel<<<std::min((b.n + kCompactThreads - 1) / kCompactThreads, 2 * b.sm_count), kCompactThreads, 0, s>>>(b);
-        note_launch(), bin_emit_pairs_kernel<true><<<b.big_grid, kBigWarps * 32, 0, s>>>(b);
-        note_launch(), bin_tile_more_kernel<<<1, 1024, 0, s>>>(b);
-        note_launch(), bin_layout_kernel<<<1, kLayoutThreads, 0, s>>>(b, ntiles);
+        launch_after(bin_tile_dirs_kernel, (ntiles + tb - 1) / tb, tb, 0, s, b, ntiles);
+        launch_after(bin_near_hist_kernel, blocks, kEmitThreads, 0, s, b);
+        launch_after(bin_pick_horizon_kernel, 1, 1024, 0, s, b);
+        launch_after(bin_compact_kernel, std::min((b.n + kCompactThreads - 1) / kCompactThreads, 2 * b.sm_count), kCompactThreads, 0, s, b);
+        launch_after(bin_emit_pairs_kernel<true>, b.big_grid, kBigWarps * 32, 0, s, b);
+        launch_after(bin_tile_more_kernel, 1, 1024, 0, s, b);
+        launch_after(bin_layout_kernel, 1, kLayoutThreads, 0, s, b, ntiles);
         return cudaGetLastError();
     }
-    note_launch(), bin_tile_dirs_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
-    note_launch(), bin_list_kernel<<<blocks, kEmitThreads, 0, s>>>(b);
-    note_launch(), bin_emit_pairs_kernel<false><<<b.big_grid, kBigWarps * 32, 0, s>>>(b);
-    note_launch(), bin_layout_kernel<<<1, kLayoutThreads, 0, s>>>(b, ntiles);
+    launch_after(bin_tile_dirs_kernel, (ntiles + tb - 1) / tb, tb, 0, s, b, ntiles);
+    launch_after(bin_list_kernel, blocks, kEmitThreads, 0, s, b);
+    launch_after(bin_emit_pairs_kernel<false>, b.big_grid, kBigWarps * 32, 0, s, b);
+    launch_after(bin_layout_kernel, 1, kLayoutThreads, 0, s, b, ntiles);
     return cudaGetLastError();
 }
 
@@ -918,16 +932,16 @@ cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, c
     // the layout is that of the whole image whatever the row range, so that a row range sees the same order
     const KeyLayout kl = key_layout(b.tiles_x * ((b.cam.height + b.tile - 1) / b.tile), b.n_pad);
     if (r.longest <= (unsigned)kSortLong) {
-        note_launch(), bin_place_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl.near_bits + kl.id_bits);
+        launch_after(bin_place_kernel, (total + tb - 1) / tb, tb, 0, s, b, total, kl.near_bits + kl.id_bits);
         int cap = kSortShort;
         while (cap < (int)r.longest) cap <<= 1;
         if (r.long_tiles) {                                // tile_order has these first
             cudaError_t e = cudaFuncSetAttribute(bin_sort_tiles_kernel<1024, 4096>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem(kSortLong));
             if (e != cudaSuccess) return e;
-            note_launch(), bin_sort_tiles_kernel<1024, 4096><<<r.long_tiles, 1024, sort_smem(cap), s>>>(b, kl, 0, cap);
+            launch_after((bin_sort_tiles_kernel<1024, 4096>), r.long_tiles, 1024, sort_smem(cap), s, b, kl, 0, cap);
         }
         if ((int)r.long_tiles < ntiles)
-            note_launch(), bin_sort_tiles_kernel<256, 2048><<<ntiles - (int)r.long_tiles, 256, sort_smem(kSortShort), s>>>(b, kl, (int)r.long_tiles, kSortShort);
+            launch_after((bin_sort_tiles_kernel<256, 2048>), ntiles - (int)r.long_tiles, 256, sort_smem(kSortShort), s, b, kl, (int)r.long_tiles, kSortShort);
         return cudaGetLastError();
     }
     cudaError_t e;
@@ -936,15 +950,15 @@ cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, c
                                         kl.tile_bits + kl.near_bits + kl.id_bits, s);
     if (e != cudaSuccess) return e;
     // CTAs take the tiles with the longest lists first: the march ends with short tiles, not with one long one
-    note_launch(), bin_tile_iota_kernel<<<(ntiles + tb - 1) / tb, tb, 0, s>>>(b, ntiles);
+    launch_after(bin_tile_iota_kernel, (ntiles + tb - 1) / tb, tb, 0, s, b, ntiles);
     temp = b.cub_bytes;
     if ((e = cub::DeviceRadixSort::SortPairsDescending(b.cub_temp, temp, b.tile_cnt, b.tile_cnt_sorted, b.tile_iota, b.tile_order,
                                                        ntiles, 0, 32, s)) != cudaSuccess) return e;
     const size_t n_entries = (((size_t)total + 32u * (size_t)ntiles + 31) / 32) * 32;   // upper bound of the padded layout
-    note_launch(), bin_fill_kernel<<<(unsigned)((n_entries + tb - 1) / tb), tb, 0, s>>>(b, n_entries);
-    note_launch(), bin_scatter_kernel<<<(total + tb - 1) / tb, tb, 0, s>>>(b, total, kl);
+    launch_after(bin_fill_kernel, (unsigned)((n_entries + tb - 1) / tb), tb, 0, s, b, n_entries);
+    launch_after(bin_scatter_kernel, (total + tb - 1) / tb, tb, 0, s, b, total, kl);
     const size_t n_blocks = (n_entries + 31) / 32;
-    note_launch(), bin_blocks_kernel<<<(unsigned)((n_blocks + 7) / 8), 256, 0, s>>>(b, n_blocks);
+    launch_after(bin_blocks_kernel, (unsigned)((n_blocks + 7) / 8), 256, 0, s, b, n_blocks);
     return cudaGetLastError();
 }
 

@@ -27,6 +27,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // One thread per Gaussian: scene box over every Gaussian's box (degenerate ones
 // included, as the reference's min/max reductions do) and the box of the centres.
 __global__ void __launch_bounds__(256) bounds_kernel(BuildLaunch b) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -64,6 +65,7 @@ __device__ __forceinline__ float bound_hi(const BuildLaunch& b, int t) { return 
 
 template <class Key>
 __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
         for (int a = 0; a < 3; ++a) {
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(256) morton_kernel(BuildLaunch b) {
 // One thread per sorted slot: whitening matrix, truncation constant, raw copies
 // for the backward, and the level-0 box.
 __global__ void __launch_bounds__(256) gather_kernel(BuildLaunch b) {
+    after_previous();
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j < 12) b.bounds[j] = 0;                       // for the next build
     if (j >= b.n_pad) {                                // the upper levels start as boxes that are never hit
@@ -155,6 +158,7 @@ __global__ void __launch_bounds__(256) gather_kernel(BuildLaunch b) {
 // Gaussians, then climbs; at every parent the last of the arriving children does
 // the work, the others leave.  No warp ever waits for another.
 __global__ void __launch_bounds__(256) refit_kernel(BuildLaunch b) {
+    after_previous();
     int node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (node >= b.count[1]) return;
@@ -213,18 +217,18 @@ cudaError_t launch_build(const BuildLaunch& b, cudaStream_t s) {
     const int n = b.sc.n;
     const int tb = 256, blocks = (n + tb - 1) / tb;
     const bool narrow = 3 * b.morton_bits <= 32;
-    note_launch(), bounds_kernel<<<blocks, tb, 0, s>>>(b);
-    if (narrow) note_launch(), morton_kernel<uint32_t><<<blocks, tb, 0, s>>>(b);
-    else note_launch(), morton_kernel<uint64_t><<<blocks, tb, 0, s>>>(b);
+    launch_after(bounds_kernel, blocks, tb, 0, s, b);
+    if (narrow) launch_after(morton_kernel<uint32_t>, blocks, tb, 0, s, b);
+    else launch_after(morton_kernel<uint64_t>, blocks, tb, 0, s, b);
     size_t temp = b.cub_temp_bytes;
     cudaError_t e = narrow ? sort_keys<uint32_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s)
                            : sort_keys<uint64_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s);
     if (e != cudaSuccess) return e;
     const int total = b.offset[b.num_levels - 1] + ((b.count[b.num_levels - 1] + kFan - 1) / kFan) * kFan;
     const int slots = b.n_pad + (total - b.offset[1]);
-    note_launch(), gather_kernel<<<(slots + tb - 1) / tb, tb, 0, s>>>(b);
+    launch_after(gather_kernel, (slots + tb - 1) / tb, tb, 0, s, b);
     int warps = b.count[1];
-    note_launch(), refit_kernel<<<(warps + 7) / 8, 256, 0, s>>>(b);
+    launch_after(refit_kernel, (warps + 7) / 8, 256, 0, s, b);
     return cudaGetLastError();
 }
 

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(128) colors_kernel(ColorLaunch c) {
 __device__ __forceinline__ void put(float* p, float v, bool acc) { *p = acc ? *p + v : v; }
 
 __global__ void __launch_bounds__(128) finalize_kernel(FinalizeLaunch f) {
+    after_previous();
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = f.sc.n;
     if (j >= n) return;
@@ -288,6 +289,7 @@ struct ClearTable {
     int n;
 };
 __global__ void __launch_bounds__(128) clear_kernel(const __grid_constant__ ClearTable t) {
+    after_previous();
     int k = 0;
     while (blockIdx.x >= t.blocks_upto[k]) ++k;                // the grid has blocks_upto[n - 1] blocks
     const size_t begin = (size_t)(blockIdx.x - (k > 0 ? t.blocks_upto[k - 1] : 0u)) * kClearFloats;
@@ -324,9 +326,9 @@ cudaError_t launch_finalize(const FinalizeLaunch& f, cudaStream_t s) {
             t.piece[t.n] = c;
             t.blocks_upto[t.n++] = (unsigned)blocks;
         }
-        if (blocks) note_launch(), clear_kernel<<<(unsigned)blocks, 128, 0, s>>>(t);
+        if (blocks) launch_after(clear_kernel, (unsigned)blocks, 128, 0, s, t);
     }
-    note_launch(), finalize_kernel<<<(f.sc.n + 127) / 128, 128, 0, s>>>(f);
+    launch_after(finalize_kernel, (f.sc.n + 127) / 128, 128, 0, s, f);
     return cudaGetLastError();
 }
 

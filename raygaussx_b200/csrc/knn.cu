@@ -30,6 +30,7 @@ constexpr int kKnnWarps = 8;
 
 // bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
 __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, unsigned* bounds) {
+    after_previous();
     __shared__ unsigned s_max[6];
     if (threadIdx.x < 6) s_max[threadIdx.x] = 0u;
     __syncthreads();
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict
 template <class Key>
 __global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ pts, int n, const unsigned* bounds,
                                                        Key* keys, unsigned* vals) {
+    after_previous();
     constexpr int kBits = sizeof(Key) == 8 ? 16 : 10;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -97,6 +99,7 @@ __device__ __forceinline__ void warp_box(float (&lo)[3], float (&hi)[3]) {
 // being one node of the level above, that node's.
 __global__ void __launch_bounds__(1024) knn_gather_kernel(const float* __restrict__ pts, int n, const unsigned* __restrict__ order,
                                                           float4* sorted, KnnLevel leaf, KnnLevel mid) {
+    after_previous();
     __shared__ float s_lo[32][3], s_hi[32][3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * 1024 + threadIdx.x, b = blockIdx.x * 32 + warp;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(1024) knn_gather_kernel(const float* __restric
 }
 
 __global__ void __launch_bounds__(256) knn_upper_kernel(KnnLevel below, KnnLevel level) {
+    after_previous();
     const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (node >= level.count) return;
     const int b = node * 32 + lane;
@@ -151,8 +155,9 @@ struct KnnTree {
     KnnLevel leaf, mid, top;
 };
 
-__global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* __restrict__ sorted, const unsigned* __restrict__ order,
+__global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* sorted, const unsigned* __restrict__ order,
                                                                    int n, KnnTree tree, float* __restrict__ out) {
+    after_previous();
     __shared__ float s_pts[kKnnWarps][3][32];
     const int warp = blockIdx.x * kKnnWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (warp >= tree.leaf.count) return;
@@ -275,14 +280,14 @@ cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaS
     const int tb = 256;
     cudaError_t e = cudaMemsetAsync(w.bounds, 0, 6 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
-    note_launch(), knn_bounds_kernel<<<std::min((n + tb - 1) / tb, 592), tb, 0, s>>>(points, n, w.bounds);
-    if (wide_keys(n)) note_launch(), knn_keys_kernel<uint64_t><<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
-    else note_launch(), knn_keys_kernel<uint32_t><<<(n + tb - 1) / tb, tb, 0, s>>>(points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
+    launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 592), tb, 0, s, points, n, w.bounds);
+    if (wide_keys(n)) launch_after(knn_keys_kernel<uint64_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
+    else launch_after(knn_keys_kernel<uint32_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
     e = sort_points(w, n, s);
     if (e != cudaSuccess) return e;
-    note_launch(), knn_gather_kernel<<<w.tree.mid.count, 1024, 0, s>>>(points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
-    note_launch(), knn_upper_kernel<<<(w.tree.top.count + 7) / 8, 256, 0, s>>>(w.tree.mid, w.tree.top);
-    note_launch(), knn_query_kernel<<<(w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps, kKnnWarps * 32, 0, s>>>(w.sorted, w.vals_out, n,
+    launch_after(knn_gather_kernel, w.tree.mid.count, 1024, 0, s, points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
+    launch_after(knn_upper_kernel, (w.tree.top.count + 7) / 8, 256, 0, s, w.tree.mid, w.tree.top);
+    launch_after(knn_query_kernel, (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n,
                                                                                                                w.tree, out);
     return cudaGetLastError();
 }

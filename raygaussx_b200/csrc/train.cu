@@ -21,6 +21,7 @@ __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1p
 // Bound by memory: reads and writes every value once (3 M Gaussians, degree 3: 1.4 GB each way in 0.23 ms, 6 TB/s; one value per thread 0.52).
 template <int K>                     // coefficients per channel; 0: any number
 __global__ void __launch_bounds__(256) activate_kernel(rgx_activation a) {
+    after_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int k_all = K ? K : a.sh_coeffs;
     if (K == 16) {                       // four values per thread, written 16 bytes at a time
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(256) activate_kernel(rgx_activation a) {
 // the parameters are written to g_*.
 template <int K>
 __global__ void __launch_bounds__(256) activate_backward_kernel(rgx_activation a, rgx_activation_grads g) {
+    after_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int k_all = K ? K : a.sh_coeffs;
     if (K == 16) {
@@ -159,6 +161,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // About 190 arithmetic instructions per pixel and channel; 1256x828: 66 us and 51 us for the backward, where framework operators took 1.9 ms for both.
 template <bool SSIM>
 __global__ void __launch_bounds__(kTile * kRows) image_loss_kernel(LossArgs a, float* maps, float2* partial) {
+    after_previous();
     __shared__ float s_x[SSIM ? kSpan : 1][kSpan + 1], s_y[SSIM ? kSpan : 1][kSpan + 1];
     __shared__ float s_h[5][SSIM ? kSpan : 1][kTile];
     __shared__ float red[kRows];
@@ -219,6 +222,7 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_kernel(LossArgs a, f
 
 // The partial sums in a fixed order, in double: (1 - l) L1 + l (1 - SSIM).
 __global__ void __launch_bounds__(256) image_loss_sum_kernel(const float2* partial, int count, double values, float lambda, float* loss) {
+    after_previous();
     __shared__ double s_a[256], s_b[256];
     double l1 = 0., ss = 0.;
     for (int i = threadIdx.x; i < count; i += 256) { l1 += partial[i].x; ss += partial[i].y; }
@@ -238,6 +242,7 @@ __global__ void __launch_bounds__(256) image_loss_sum_kernel(const float2* parti
 // Gradient of the loss with respect to the rays: the three maps blurred, and the sign of the difference.
 template <bool SSIM>
 __global__ void __launch_bounds__(kTile * kRows) image_loss_backward_kernel(LossArgs a, const float* maps, const float* grad_loss, float* out) {
+    after_previous();
     __shared__ float s_m[3][SSIM ? kSpan : 1][kSpan + 1];
     __shared__ float s_h[3][SSIM ? kSpan : 1][kTile];
     const int c = blockIdx.z, x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, tx = threadIdx.x, ty = threadIdx.y;
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_backward_kernel(Loss
                 const int x = x0 + i - kRad, y = y0 + j - kRad;
                 const bool in = x >= 0 && y >= 0 && x < a.w && y < a.h;
 #pragma unroll
-                for (int q = 0; q < 3; ++q) s_m[q][j][i] = in ? __ldg(&maps[(size_t)(3 * q + c) * plane + (size_t)y * a.w + x]) : 0.f;
+                for (int q = 0; q < 3; ++q) s_m[q][j][i] = in ? maps[(size_t)(3 * q + c) * plane + (size_t)y * a.w + x] : 0.f;
             }
         __syncthreads();
         for (int j = ty; j < kSpan; j += kRows) {
@@ -296,6 +301,7 @@ dim3 loss_grid(int w, int h) { return dim3((w + kTile - 1) / kTile, (h + kTile -
 // classes/point_cloud.py:468-485; a null norm_sum counts only (gradients of Gaussians not visible).
 __global__ void __launch_bounds__(256) gradient_stats_kernel(int n, const float* pos, const float* grad, const float* eye, float* norm_sum, float* count,
                                                              float* also) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gx = grad[3 * (size_t)i], gy = grad[3 * (size_t)i + 1], gz = grad[3 * (size_t)i + 2];
@@ -329,6 +335,7 @@ __device__ __forceinline__ void adam_value(float& p, float g, float& m, float& v
 // All tensors of a step in one launch.  Bound by memory: 16 bytes read and 12 written per value; 177 M values: 0.76 ms, 6.5 TB/s (foreach
 // operators, a launch and a round trip per term of the formula: 3.0 ms).
 __global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamTable a) {
+    after_previous();
     int k = 0;
     while (k + 1 < a.count && blockIdx.x >= a.first[k + 1]) ++k;
     const rgx_adam_tensor& t = a.t[k];
@@ -379,14 +386,13 @@ extern "C" RGX_API int rgx_activate(int device, const rgx_activation* a, rgx_str
         return RGX_E_INVALID;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
-    note_launch();
     const unsigned blocks = (unsigned)((activation_threads(a) + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     switch (a->sh_coeffs) {
-        case 4: activate_kernel<4><<<blocks, 256, 0, s>>>(*a); break;
-        case 9: activate_kernel<9><<<blocks, 256, 0, s>>>(*a); break;
-        case 16: activate_kernel<16><<<blocks, 256, 0, s>>>(*a); break;
-        default: activate_kernel<0><<<blocks, 256, 0, s>>>(*a);
+        case 4: launch_after(activate_kernel<4>, blocks, 256, 0, s, *a); break;
+        case 9: launch_after(activate_kernel<9>, blocks, 256, 0, s, *a); break;
+        case 16: launch_after(activate_kernel<16>, blocks, 256, 0, s, *a); break;
+        default: launch_after(activate_kernel<0>, blocks, 256, 0, s, *a);
     }
     return done(cudaGetLastError());
 }
@@ -399,14 +405,13 @@ extern "C" RGX_API int rgx_activate_backward(int device, const rgx_activation* a
         return RGX_E_INVALID;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
-    note_launch();
     const unsigned blocks = (unsigned)((activation_threads(a) + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     switch (a->sh_coeffs) {
-        case 4: activate_backward_kernel<4><<<blocks, 256, 0, s>>>(*a, *g); break;
-        case 9: activate_backward_kernel<9><<<blocks, 256, 0, s>>>(*a, *g); break;
-        case 16: activate_backward_kernel<16><<<blocks, 256, 0, s>>>(*a, *g); break;
-        default: activate_backward_kernel<0><<<blocks, 256, 0, s>>>(*a, *g);
+        case 4: launch_after(activate_backward_kernel<4>, blocks, 256, 0, s, *a, *g); break;
+        case 9: launch_after(activate_backward_kernel<9>, blocks, 256, 0, s, *a, *g); break;
+        case 16: launch_after(activate_backward_kernel<16>, blocks, 256, 0, s, *a, *g); break;
+        default: launch_after(activate_backward_kernel<0>, blocks, 256, 0, s, *a, *g);
     }
     return done(cudaGetLastError());
 }
@@ -429,9 +434,9 @@ extern "C" RGX_API int rgx_image_loss(int device, const float* rays, const float
     const LossArgs a = loss_args(rays, target, w, h, fx, fy, lambda_ssim);
     const dim3 grid = loss_grid(w, h), block(kTile, kRows);
     float2* partial = reinterpret_cast<float2*>(scratch);
-    if (lambda_ssim != 0.f) note_launch(), image_loss_kernel<true><<<grid, block, 0, s>>>(a, maps, partial);
-    else note_launch(), image_loss_kernel<false><<<grid, block, 0, s>>>(a, nullptr, partial);
-    note_launch(), image_loss_sum_kernel<<<1, 256, 0, s>>>(partial, (int)(grid.x * grid.y * grid.z), 3.0 * (double)w * (double)h, lambda_ssim, loss);
+    if (lambda_ssim != 0.f) launch_after(image_loss_kernel<true>, grid, block, 0, s, a, maps, partial);
+    else launch_after(image_loss_kernel<false>, grid, block, 0, s, a, nullptr, partial);
+    launch_after(image_loss_sum_kernel, 1, 256, 0, s, partial, (int)(grid.x * grid.y * grid.z), 3.0 * (double)w * (double)h, lambda_ssim, loss);
     return done(cudaGetLastError());
 }
 
@@ -443,8 +448,8 @@ extern "C" RGX_API int rgx_image_loss_backward(int device, const float* rays, co
     cudaStream_t s = (cudaStream_t)stream;
     const LossArgs a = loss_args(rays, target, w, h, fx, fy, lambda_ssim);
     const dim3 grid = loss_grid(w, h), block(kTile, kRows);
-    if (lambda_ssim != 0.f) note_launch(), image_loss_backward_kernel<true><<<grid, block, 0, s>>>(a, maps, grad_loss, grad_rays);
-    else note_launch(), image_loss_backward_kernel<false><<<grid, block, 0, s>>>(a, nullptr, grad_loss, grad_rays);
+    if (lambda_ssim != 0.f) launch_after(image_loss_backward_kernel<true>, grid, block, 0, s, a, maps, grad_loss, grad_rays);
+    else launch_after(image_loss_backward_kernel<false>, grid, block, 0, s, a, nullptr, grad_loss, grad_rays);
     return done(cudaGetLastError());
 }
 
@@ -454,7 +459,7 @@ extern "C" RGX_API int rgx_gradient_stats(int device, int n, const float* positi
     if (n == 0) return RGX_OK;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
-    note_launch(), gradient_stats_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, positions, grad, eye, norm_sum, count, also);
+    launch_after(gradient_stats_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, n, positions, grad, eye, norm_sum, count, also);
     return done(cudaGetLastError());
 }
 
@@ -475,6 +480,6 @@ extern "C" RGX_API int rgx_adam_step(int device, const rgx_adam_tensor* tensors,
     if (a.count == 0) return RGX_OK;
     DeviceGuard guard(device);
     if (!guard.ok) return done(cudaErrorInvalidDevice);
-    note_launch(), adam_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(a);
+    launch_after(adam_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, a);
     return done(cudaGetLastError());
 }
