@@ -13,9 +13,9 @@
 //   Queries of a warp are neighbours in space, so after the seed (the warp's own box and
 // its two neighbours) few boxes are opened and what bounds the kernel is the distance
 // arithmetic of those.  Testing every upper box by every warp, as an earlier version did, took 15.3 ms
-// for 3 M points (now 1.02 ms); the whole call, whose eleven allocations and frees cost more than
-// its kernels on small clouds, took 19.9 ms for 3 M (now 1.45) and 0.4 ms (in a process with a large
-// workspace several ms) for 100 k points (now 0.18, scratch from the caller).
+// for 3 M points (now 0.85 ms); the whole call, whose eleven allocations and frees cost more than
+// its kernels on small clouds, took 19.9 ms for 3 M (now 1.27) and 0.4 ms (in a process with a large
+// workspace several ms) for 100 k points (now 0.17, scratch from the caller).
 #include "rgx_internal.cuh"
 #include "device_math.cuh"
 #include <cub/device/device_radix_sort.cuh>
@@ -27,6 +27,7 @@ namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kKnnWarps = 8;
+constexpr int kFilterWarps = 148 * 64;     // as many warps as the device holds at once (303 k points), see knn_query_kernel
 
 // bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
 __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, unsigned* bounds) {
@@ -155,6 +156,11 @@ struct KnnTree {
     KnnLevel leaf, mid, top;
 };
 
+// FILTER: eight points at a time are passed by where none of them is nearer to its query than what a lane has.  Of the points opened
+// few are, so that saves most of the bookkeeping where the kernel is bound by arithmetic (whole call, 3 M points of a core and a shell
+// 1,424 -> 1,271 us, 1 M of an object 539 -> 489, 1 M on surfaces 493 -> 483); with fewer warps than the device holds the vote is one more
+// thing to wait for (30 k points 225 -> 235 us, 100 k 176 -> 178).
+template <bool FILTER>
 __global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* sorted, const unsigned* __restrict__ order,
                                                                    int n, KnnTree tree, float* __restrict__ out) {
     after_previous();
@@ -171,27 +177,40 @@ __global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4*
     warp_box(qlo, qhi);
     float best0 = FLT_MAX, best1 = FLT_MAX, best2 = FLT_MAX;             // the three smallest, ascending
     float worst = FLT_MAX;                                               // largest best2 of the warp
-    auto keep3 = [&](float d) {
-        const float t = fmaxf(best0, d), u = fmaxf(best1, t);
-        best0 = fminf(best0, d);
-        best1 = fminf(best1, t);
-        best2 = fminf(best2, u);
+    auto keep = [&](float2 d) {                                          // the three smallest of those and two more
+        const float lo = fminf(d.x, d.y), hi = fmaxf(d.x, d.y);
+        const float second = fminf(fminf(fmaxf(best0, lo), best1), hi), third = fminf(fminf(best2, fmaxf(best1, lo)), fmaxf(best0, hi));
+        best0 = fminf(best0, lo);
+        best1 = second;
+        best2 = third;
+    };
+    auto dist2 = [&](int k, bool own, const float (*pts)[32]) {          // to points k and k + 1 in packed fp32x2 arithmetic, same bits
+        const float2 dx = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[0][k]), make_float2(-q.x, -q.x)),
+                     dy = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[1][k]), make_float2(-q.y, -q.y)),
+                     dz = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[2][k]), make_float2(-q.z, -q.z));
+        float2 d = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));   // +inf for the padding points
+        if (own && k == lane) d.x = INFINITY;
+        if (own && k + 1 == lane) d.y = INFINITY;
+        return d;
     };
     auto open_box = [&](int b, bool own) {
         const float4 mine = sorted[b * 32 + lane];
         __syncwarp();
         pts[0][lane] = mine.x; pts[1][lane] = mine.y; pts[2][lane] = mine.z;
         __syncwarp();
-#pragma unroll 4
-        for (int k = 0; k < 32; k += 2) {                                // two points at a time: packed fp32x2 arithmetic, same bits
-            const float2 dx = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[0][k]), make_float2(-q.x, -q.x)),
-                         dy = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[1][k]), make_float2(-q.y, -q.y)),
-                         dz = __fadd2_rn(*reinterpret_cast<const float2*>(&pts[2][k]), make_float2(-q.z, -q.z));
-            float2 d = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));   // +inf for the padding points
-            if (own && k == lane) d.x = INFINITY;
-            if (own && k + 1 == lane) d.y = INFINITY;
-            keep3(d.x);
-            keep3(d.y);
+        constexpr int kPairs = FILTER ? 4 : 1;
+#pragma unroll(FILTER ? 1 : 4)
+        for (int k = 0; k < 32; k += 2 * kPairs) {
+            float2 d[kPairs];
+            float least = INFINITY;
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) {
+                d[i] = dist2(k + 2 * i, own, pts);
+                least = fminf(fminf(d[i].x, d[i].y), least);
+            }
+            if (FILTER && !__any_sync(kAll, least < best2)) continue;
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) keep(d[i]);
         }
     };
     auto settle = [&]() { worst = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(live ? best2 : 0.f))); };
@@ -287,8 +306,9 @@ cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaS
     if (e != cudaSuccess) return e;
     launch_after(knn_gather_kernel, w.tree.mid.count, 1024, 0, s, points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
     launch_after(knn_upper_kernel, (w.tree.top.count + 7) / 8, 256, 0, s, w.tree.mid, w.tree.top);
-    launch_after(knn_query_kernel, (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n,
-                                                                                                               w.tree, out);
+    const int blocks = (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps;
+    if (w.tree.leaf.count > kFilterWarps) launch_after(knn_query_kernel<true>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
+    else launch_after(knn_query_kernel<false>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
     return cudaGetLastError();
 }
 
