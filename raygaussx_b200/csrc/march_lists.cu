@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         const float4 m0 = st.m0[q], m1 = st.m1[q], m2 = st.m2[q];
                         RayParabola pb;
                         bool hit = ellipsoid_stretch(staged_eye(m1, m2), staged_dir(m0, m1, m2, dir), pb);
-                        hit = hit && e + sub < n && stretch_meets(pb, tmin, tmax);
+                        hit = hit & (e + sub < n) & stretch_meets(pb, tmin, tmax);
                         if (COUNT && act && e + sub < n) { tl.v[C_PRIM_TESTS] += 1; tl.v[C_ELL_TESTS] += 1; }
                         const unsigned m = __ballot_sync(kFull, hit);
                         nhit += hit ? 1 : 0;
@@ -726,9 +726,13 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                         float4 A = parabola_record(pb, t, st.ex[q].x);
                         // parts of the slab that the ray's stretch inside reaches, with a fiftieth of one on either side against
                         // rounding (the test of each sample decides)
-                        const int lo = max(__float2int_rd(fmaf(A.x - pb.hw, inv_part, -0.5f * Pt::kParts / kSlab - 0.02f)), 0);
-                        const int hi = min(__float2int_rd(fmaf(A.x + pb.hw, inv_part, -0.5f * Pt::kParts / kSlab + 0.02f)), Pt::kParts - 1);
-                        const unsigned groups = hit && lo <= hi ? (2u << hi) - (1u << lo) : 0u;
+                        const float begin = fmaxf(fmaf(A.x - pb.hw, inv_part, -0.5f * Pt::kParts / kSlab - 0.02f), 0.f);
+                        const float end = fminf(fmaf(A.x + pb.hw, inv_part, -0.5f * Pt::kParts / kSlab + 0.02f), (float)Pt::kParts - 1e-6f);
+                        // their whole numbers are the last bits of the sums with 2^23, rounded down (a shift takes the last five): with conversions
+                        // and short-circuit logic in place of this and of `hit` above the object took 2.67 ms instead of 2.58, four 3 M views 11.32
+                        // instead of 11.19
+                        const unsigned lo = __float_as_uint(__fadd_rd(begin, 8388608.0f)), hi = __float_as_uint(__fadd_rd(end, 8388608.0f));
+                        const unsigned groups = hit && begin <= end ? (2u << (hi & 31u)) - (1u << (lo & 31u)) : 0u;
                         if (!hit) A.y = -1.0f;
                         sh.rec[e + sub][r] = A;
                         reach |= __reduce_or_sync(kFull, groups << (Pt::kParts * sub)) << (Pt::kParts * e);
