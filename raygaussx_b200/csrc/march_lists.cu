@@ -218,22 +218,26 @@ __device__ __forceinline__ unsigned fetch_unit(unsigned* next, unsigned units) {
 
 constexpr int kStaged = 64;        // ring of list entries that passed the patch's filters
 
-struct PatchStage {                // per warp
-    float4 m0[kStaged];            // M = S^-1 R^T / k, and the eye in the whitened frame, the first two rows side by side for
-    float4 m1[kStaged];            // packed instructions: (m00, m10, m01, m11), (m02, m12, Oe.x, Oe.y), (m20, m21, m22, Oe.z)
-    float4 m2[kStaged];
-    float4 ex[kStaged];            // hk, |Oe|^2 - 1, sorted slot (bits), rays that hit it (bits, set once tested)
-    float4 rgba[kStaged];          // (r sigma, g sigma, b sigma, sigma)
+template <int N>
+struct Staged {                    // per warp
+    float4 m0[N];                  // M = S^-1 R^T / k, and the eye in the whitened frame, the first two rows side by side for
+    float4 m1[N];                  // packed instructions: (m00, m10, m01, m11), (m02, m12, Oe.x, Oe.y), (m20, m21, m22, Oe.z)
+    float4 m2[N];
+    float4 ex[N];                  // hk, |Oe|^2 - 1, sorted slot (bits), rays that hit it (bits, set once tested)
+    float4 rgba[N];                // (r sigma, g sigma, b sigma, sigma)
 };
+using PatchStage = Staged<kStaged>;
 
-__device__ __forceinline__ unsigned& hit_by(PatchStage& st, int q) { return reinterpret_cast<unsigned*>(&st.ex[q])[3]; }
+template <int N>
+__device__ __forceinline__ unsigned& hit_by(Staged<N>& st, int q) { return reinterpret_cast<unsigned*>(&st.ex[q])[3]; }
 
 // smallest / largest of non-negative floats over the warp (they order like their bits)
 __device__ __forceinline__ float warp_min_pos(float v) { return __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(v))); }
 __device__ __forceinline__ float warp_max_pos(float v) { return __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(v))); }
 
 // One Gaussian's record, as the sorted arrays hold it, into slot `q` (by one lane): what is computed from the geometry, then the rest.
-__device__ __forceinline__ void stage_geometry(PatchStage& st, int q, int j, float4 g0, float4 g1, float4 g2, float3 Oe) {
+template <int N>
+__device__ __forceinline__ void stage_geometry(Staged<N>& st, int q, int j, float4 g0, float4 g1, float4 g2, float3 Oe) {
     st.m0[q] = make_float4(g0.w, g1.z, g1.x, g1.w);
     st.m1[q] = make_float4(g1.y, g2.x, Oe.x, Oe.y);
     st.m2[q] = make_float4(g2.y, g2.z, g2.w, Oe.z);
@@ -533,8 +537,9 @@ struct SampleTree {
 // 13.46 ms, the object 3.09 against 3.05), 18 of 112 registers much slower (15.25, 3.89): the sums of a slab alone are 64.
 template <bool COUNT>
 __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : 16; }
-// The replay, of 95 registers: 18 to 20 warps per SM are 4 % faster than 16 (four CTAs of four).
-constexpr int kReplayCtas = 18;
+// The replay, of 96 registers and 8.9 KB: 20 warps per SM.  18 are 1.5 to 3 % slower (four 3 M views 10.57 against 10.40 ms, the 300 k
+// object 1.95 against 1.89), 17 another 4 % on the 3 M views, 21 (80 registers) as slow as 18.
+constexpr int kReplayCtas = 20;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
 __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march_forward_patches_kernel(const __grid_constant__ MarchLaunch L) {
@@ -921,7 +926,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
 // Bound by instruction issue (78 % of the slots).  Against a warp per ray: 3 M-Gaussian view 7.7 -> 2.7 ms, 300 k object 4.7 -> 2.15 ms.
 template <int P>
 struct ReplayShared {
-    PatchStage st;
+    Staged<kFan> st;
     float2 bg[kSlab + kRun - 1][Patch<P>::kRays];  // beta, gamma of every sample; zero past the last, where a run may end
     float red[13][36];             // one row per component, 32 lanes (+4: rows start in other banks)
 };
@@ -931,7 +936,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
     using Pt = Patch<P>;
     __shared__ ReplayShared<P> sh;
     const int lane = threadIdx.x, sub = lane / Pt::kRays, r = lane % Pt::kRays;
-    PatchStage& st = sh.st;
+    Staged<kFan>& st = sh.st;
     const float eps = L.m.transmittance_eps;
     const unsigned per_row = (unsigned)(L.lists.tile / Pt::kW), per_tile = per_row * (unsigned)(L.lists.tile / Pt::kH);
     const unsigned units = (unsigned)(L.lists.tiles_x * L.lists.tiles_y) * per_tile;
@@ -1076,7 +1081,8 @@ __global__ void __launch_bounds__(kPatchWarps * 32, kReplayCtas) march_backward_
                             for (int i = 0; i < kRun; ++i) {
                                 const float d2 = __fmul_rn(d, d);
                                 const float2 w = at[i * Pt::kRays];
-                                const float g = d2 < ay ? ex2_approx(fmaf(az, d2, aw)) : 0.f;
+                                // 2^-inf is the zero outside: what is chosen is the exponent, before the slow unit (1.5 % of the kernel)
+                                const float g = ex2_approx(d2 < ay ? fmaf(az, d2, aw) : -INFINITY);
                                 const float u = fmaf(ci, w.x, w.y), ga = __fmul_rn(g, u);  // w = g * (alpha + beta*(chat_i - chat_s))
                                 sn = __ffma2_rn(make_float2(g, g), make_float2(w.x, u), sn);
                                 n12 = __ffma2_rn(make_float2(ga, ga), make_float2(d, d2), n12);
