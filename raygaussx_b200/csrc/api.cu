@@ -639,6 +639,7 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     b.proj = make_projector(b);
     b.zero = ctx->bin_zero; b.zero_bytes = z.bytes;
     b.result = reinterpret_cast<BinResult*>(ctx->bin_zero);
+    b.result_host = ctx->bin_result_host;
     b.tile_cnt = ctx->tile_cnt;
     b.tile_pbegin = ctx->tile_pbegin;
     b.tile_iota = ctx->tile_iota; b.tile_cnt_sorted = ctx->tile_cnt_sorted;
@@ -680,15 +681,12 @@ static int emit_setup(rgx_ctx* ctx, const rgx_camera* cam, const rgx_march* m, B
     return RGX_OK;
 }
 
-// ... the kernels and the copy of the pair count to the host, enqueued ...
+// ... the kernels, enqueued ...
 static int emit_launch(rgx_ctx* ctx, BinLaunch& b, cudaStream_t s) {
     cudaError_t e;
     b.keys_in = ctx->bin_keys_in; b.vals_in = ctx->bin_vals_in; b.ranks = ctx->bin_ranks; b.pair_cap = ctx->bin_pair_cap;
     if ((e = launch_bin_emit(b, s)) != cudaSuccess) return cuda_fail(ctx, e, "tile-list pairs");
-    // the number of pairs and the horizon travel together
-    if ((e = cudaMemcpyAsync(ctx->bin_result_host, ctx->bin_zero, sizeof(BinResult), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        return cuda_fail(ctx, e, "tile-list pair count read-back");
-    return RGX_OK;
+    return RGX_OK;                 // the number of pairs and the horizon are left in bin_result_host
 }
 
 // ... and the view's one host round trip: the sort needs the number of pairs.  A view whose pairs did not fit is
@@ -1068,7 +1066,8 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
         }
         if (e != cudaSuccess) return cuda_fail(ctx, e, "forward march");
         if (recorded) {
-            cudaMemcpyAsync(ctx->tape_used_host, ctx->tape_used, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+            L.tape_used_host = ctx->tape_used_host;
+            if (L.hz_phase != 3 && (e = launch_report(L, s)) != cudaSuccess) return cuda_fail(ctx, e, "forward march");
             ctx->tape_valid = true;
             ctx->tape_rgba_serial = ctx->rgba_serial;
             ctx->tape_build_id = ctx->build_id;
@@ -1100,12 +1099,12 @@ static int forward_impl(rgx_ctx* ctx, const rgx_scene* scene, const rgx_camera* 
     L.hz_phase = 3; L.horizon = ctx->lists_horizon; L.tile_more = ctx->tile_more;
     L.hz_count = reinterpret_cast<unsigned int*>(ctx->hz_scalars + 1);
     L.hz_rays = ctx->hz_rays;
+    L.hz_count_host = ctx->beyond_host;
     if ((e = cudaMemsetAsync(ctx->hz_scalars + 1, 0, sizeof(unsigned long long), s)) != cudaSuccess)
         return cuda_fail(ctx, e, "horizon counter");
     if ((rc = march_once())) return rc;
     if ((rc = run_colors_if_beyond(ctx, scene, cam->eye, L.hz_count, s))) return rc;
     if ((e = launch_march_forward_listed_rays(L, ctx->sm_count * 4, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(ctx->beyond_host, ctx->hz_scalars + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaEventRecord(ctx->ev_beyond, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "rays beyond the horizon");
     ctx->beyond_pending = true;

@@ -698,7 +698,13 @@ __global__ void __launch_bounds__(kLayoutThreads) bin_layout_kernel(BinLaunch b,
     if ((t & 31) == 0) { atomicMax(&s_longest, longest); if (many) atomicAdd(&s_many, many); }
     __syncthreads();
     longest = s_longest;
-    if (t == 0) { b.result->longest = (unsigned)longest; b.result->long_tiles = (unsigned)s_many; }
+    if (t == 0) {
+        // to the host without a copy behind this kernel: the host waits for it, and a copy takes ten microseconds to get going
+        BinResult r = *b.result;
+        r.longest = (unsigned)longest;
+        r.long_tiles = (unsigned)s_many;
+        *b.result_host = r;
+    }
     // Buckets by length, the longest first; bucket boundaries put every list of more than kSortShort pairs before all others.
     auto bucket = [&](int n) {
         if (n > kSortShort) return 127 - (int)((long long)(n - kSortShort) * 127 / max(longest - kSortShort, 1));

@@ -101,9 +101,21 @@ __global__ void __launch_bounds__(kWarps * 32) march_forward_kernel(const __grid
 // holds their numbers, *L.hz_count how many.  They are marched again from the start by searching the hierarchy,
 // which needs no lists: same hits, met in slot order instead of list order, so the colour equals that of complete
 // lists to summation rounding.  Launched after every such march; returns at once when there are none.
+// The counts of the march that has just finished, to the host's pinned memory (a copy each would hold up the stream for ten
+// microseconds and more).
+__device__ __forceinline__ void report(const MarchLaunch& L) {
+    if (L.tape_used_host && L.tape_used) *L.tape_used_host = *L.tape_used;
+    if (L.hz_count_host) *L.hz_count_host = *L.hz_count;
+}
+__global__ void report_kernel(const __grid_constant__ MarchLaunch L) {
+    after_previous();
+    report(L);
+}
+
 __global__ void __launch_bounds__(kWarps * 32) march_forward_listed_rays_kernel(const __grid_constant__ MarchLaunch L) {
     __shared__ WarpShared shared[kWarps];
     const unsigned int n = *L.hz_count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) report(L);
     if (n == 0u) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float eps = L.m.transmittance_eps;
@@ -201,6 +213,8 @@ cudaError_t launch_march_forward_per_ray(const MarchLaunch& m, cudaStream_t s) {
     else note_launch(), march_forward_kernel<false, false><<<grid, kWarps * 32, 0, s>>>(m);
     return cudaGetLastError();
 }
+
+cudaError_t launch_report(const MarchLaunch& m, cudaStream_t s) { return launch_after(report_kernel, 1, 1, 0, s, m); }
 
 cudaError_t launch_march_forward_listed_rays(const MarchLaunch& m, int ctas, cudaStream_t s) {
     if (m.g.n <= 0 || !m.hz_rays || !m.hz_count) return cudaSuccess;

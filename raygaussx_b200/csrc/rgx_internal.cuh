@@ -152,6 +152,7 @@ struct BinLaunch {
     uint32_t *vals_in, *vals_out;          // [pair capacity] far distance (float bits)
     uint32_t* ranks;                       // [pair capacity] the pair's number among its tile's, in no particular order
     BinResult* result;
+    BinResult* result_host;                // pinned: bin_layout_kernel, the last of the emission, leaves the result there too
     unsigned long long pair_cap;
     int *tile_first, *tile_cnt, *tile_pcnt, *tile_pbegin;   // [tiles + 1]
     int *tile_iota, *tile_cnt_sorted, *tile_order;                      // [tiles]
@@ -207,6 +208,7 @@ struct MarchLaunch {
     const int* tile_more;     // per tile: has pairs that begin beyond the horizon
     int* tile_resume;         // per tile: some ray stopped at the horizon
     unsigned int* hz_count;   // rays that stopped
+    unsigned long long *tape_used_host, *hz_count_host;   // pinned, or null: where the counts of a finished march go
     int* hz_rays;             // hz_phase 3: their numbers, for march_forward_listed_rays_kernel
     float4* grad_rows;    // [grad_copies, n_pad, 4] float4 of accumulated moments, layout in emit_global
     int grad_copies;      // power of two
@@ -304,6 +306,8 @@ cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, c
 float bin_hist_bucket_end(const BinLaunch& b, int bucket);
 cudaError_t launch_march_forward(const MarchLaunch& m, cudaStream_t s);
 // The rays listed in m.hz_rays by a march over lists that stop at a horizon, again by per-ray search (march.cu).
+// The ints that a recording march has used, to pinned memory, where no launch of the above does it.
+cudaError_t launch_report(const MarchLaunch& m, cudaStream_t s);
 cudaError_t launch_march_forward_listed_rays(const MarchLaunch& m, int ctas, cudaStream_t s);
 // The backward in two launches: rays without a recording (searches the lists or the hierarchy), then the replay of
 // the recording, which reads neither lists nor hierarchy.
