@@ -7,6 +7,7 @@
 // hierarchy itself is built inside the OptiX driver.
 #include "rgx_internal.cuh"
 #include "device_math.cuh"
+#include "cluster_sort.cuh"
 #include <cub/device/device_radix_sort.cuh>
 
 namespace rgx {
@@ -220,9 +221,13 @@ cudaError_t launch_build(const BuildLaunch& b, cudaStream_t s) {
     launch_after(bounds_kernel, blocks, tb, 0, s, b);
     if (narrow) launch_after(morton_kernel<uint32_t>, blocks, tb, 0, s, b);
     else launch_after(morton_kernel<uint64_t>, blocks, tb, 0, s, b);
-    size_t temp = b.cub_temp_bytes;
-    cudaError_t e = narrow ? sort_keys<uint32_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s)
-                           : sort_keys<uint64_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s);
+    cudaError_t e = narrow ? cluster_sort((const uint32_t*)b.keys_in, (uint32_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s)
+                           : cluster_sort((const uint64_t*)b.keys_in, (uint64_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s);
+    if (e == cudaErrorNotSupported) {
+        size_t temp = b.cub_temp_bytes;
+        e = narrow ? sort_keys<uint32_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s)
+                   : sort_keys<uint64_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s);
+    }
     if (e != cudaSuccess) return e;
     const int total = b.offset[b.num_levels - 1] + ((b.count[b.num_levels - 1] + kFan - 1) / kFan) * kFan;
     const int slots = b.n_pad + (total - b.offset[1]);

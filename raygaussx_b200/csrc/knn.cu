@@ -18,6 +18,7 @@
 // workspace several ms) for 100 k points (now 0.17, scratch from the caller).
 #include "rgx_internal.cuh"
 #include "device_math.cuh"
+#include "cluster_sort.cuh"
 #include <cub/device/device_radix_sort.cuh>
 #include <algorithm>
 
@@ -302,7 +303,9 @@ cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaS
     launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 592), tb, 0, s, points, n, w.bounds);
     if (wide_keys(n)) launch_after(knn_keys_kernel<uint64_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
     else launch_after(knn_keys_kernel<uint32_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
-    e = sort_points(w, n, s);
+    e = wide_keys(n) ? cluster_sort((const uint64_t*)w.keys_in, (uint64_t*)w.keys_out, w.vals_in, w.vals_out, n, 48, s)
+                     : cluster_sort((const uint32_t*)w.keys_in, (uint32_t*)w.keys_out, w.vals_in, w.vals_out, n, 30, s);
+    if (e == cudaErrorNotSupported) e = sort_points(w, n, s);
     if (e != cudaSuccess) return e;
     launch_after(knn_gather_kernel, w.tree.mid.count, 1024, 0, s, points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
     launch_after(knn_upper_kernel, (w.tree.top.count + 7) / 8, 256, 0, s, w.tree.mid, w.tree.top);
