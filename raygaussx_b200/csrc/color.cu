@@ -80,15 +80,10 @@ __device__ __forceinline__ void load_row(const float* p, int K, float* out) {
     }
 }
 
-__global__ void __launch_bounds__(128) colors_kernel(ColorLaunch c) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
+__host__ __device__ inline int color_slots(const ColorLaunch& c) { return c.perm ? ((c.sc.n + 31) / 32) * 32 : c.sc.n; }
+
+__device__ __forceinline__ void gaussian_color(const ColorLaunch& c, int j) {
     const int n = c.sc.n;
-    const int n_slots = c.perm ? ((n + 31) / 32) * 32 : n;
-    if (j >= n_slots) return;
-    if (c.only_if) {                     // the colours of all Gaussians after all: some ray went beyond the lists' horizon
-        if (*c.only_if == 0u) return;
-        if (c.listed_out) c.listed_out[j] = j < n ? 1 : 0;
-    }
     if (j >= n) {
         c.rgba[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c.listed_code) c.listed_out[j] = 0;
@@ -131,6 +126,21 @@ __global__ void __launch_bounds__(128) colors_kernel(ColorLaunch c) {
         c.rgba[j] = ok ? make_float4(rgb[0] * dens, rgb[1] * dens, rgb[2] * dens, dens) : make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
         c.rgb_out[3 * i] = rgb[0]; c.rgb_out[3 * i + 1] = rgb[1]; c.rgb_out[3 * i + 2] = rgb[2];
+    }
+}
+
+__global__ void __launch_bounds__(128) colors_kernel(ColorLaunch c) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < color_slots(c)) gaussian_color(c, j);
+}
+
+// The colours of all Gaussians after all, where some ray went beyond the lists' horizon.  As a rule none has, and what there is to wait
+// for are the blocks: eight per SM and not one per 128 Gaussians (11 us of a 3 M view).
+__global__ void __launch_bounds__(128) colors_if_beyond_kernel(ColorLaunch c) {
+    if (*c.only_if == 0u) return;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < color_slots(c); j += gridDim.x * blockDim.x) {
+        if (c.listed_out) c.listed_out[j] = j < c.sc.n ? 1 : 0;
+        gaussian_color(c, j);
     }
 }
 
@@ -304,9 +314,10 @@ __global__ void __launch_bounds__(128) clear_kernel(const __grid_constant__ Clea
 }  // namespace
 
 cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s) {
-    int slots = c.perm ? ((c.sc.n + 31) / 32) * 32 : c.sc.n;
+    const int slots = color_slots(c), blocks = (slots + 127) / 128;
     if (slots == 0) return cudaSuccess;
-    note_launch(), colors_kernel<<<(slots + 127) / 128, 128, 0, s>>>(c);
+    if (c.only_if) note_launch(), colors_if_beyond_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 128, 0, s>>>(c);
+    else note_launch(), colors_kernel<<<blocks, 128, 0, s>>>(c);
     return cudaGetLastError();
 }
 
