@@ -412,8 +412,8 @@ void near_begin(rgx_ctx* ctx, int budget_per_ray) {
     ctx->near_lowered = false;
 }
 
-// The number of rays that went beyond the horizon in the latest march over lists that stop at one was copied to the
-// host behind that march; whoever needs it waits for the copy here (by then long done).  A view in which it is not
+// The number of rays that went beyond the horizon in the latest march over lists that stop at one is stored in pinned
+// host memory by the kernel behind that march; whoever needs it waits for that here (by then long done).  A view in which it is not
 // zero makes the lists of the views to come deeper -- unless its own lists had fallen short of the budget:
 // then the estimate was off, and has been corrected already.
 void settle_beyond(rgx_ctx* ctx) {

@@ -468,15 +468,15 @@ __device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq,
 // entries are tested, lane group h tests entry e + h for all the rays; while hits are evaluated, lane h of a ray holds the samples
 // P i + h of its slab, 32 / P samples times four sums in registers.  Hits are evaluated only in the parts of the slab that some ray's
 // stretch inside the Gaussian reaches.
-//   What bounds it: instruction issue (67 % of the slots on 2 M Gaussians at 628x414, 63 % on the 300 k object at 400x400; the rest
-// waits on dependent chains at sixteen warps per SM) and, recording, the 512 bytes of sums per ray and slab.  With P = 1 the sums of a slab would be 128 registers and eight
+//   What bounds it: instruction issue (66 % of the slots on 2 M Gaussians at 628x414, 63 % on the 300 k object at 400x400; the rest
+// waits on dependent chains at sixteen warps per SM; 12 warp instructions per hit, 16 before the tests were culled by the rays' windows) and, recording, the 512 bytes of sums per ray and slab.  With P = 1 the sums of a slab would be 128 registers and eight
 // warps would fill an SM; P = 2 halves them at the price of one exchange per sample in the compositing.
 //   Tests of a group of entries come before their evaluation, through shared memory: the loops are short (a unit of tests and the
 // evaluation of both halves in one body missed the instruction cache) and the evaluation runs over entries that were hit only.
 //   Slabs of the rays are taken in steps: the ray that is furthest behind leads, and every ray whose slab begins before the
 // leader's ends marches with it.  The list is walked once per step over the union of the windows.
-//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.3 -> 3.6, 300 k object 9.3 -> 3.3 (7.8 -> 2.9
-// without recording), 7 M needles 14.6 -> 5.65 (two depths), 1 M at 640x360 1.83 -> 0.81.
+//   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.3 -> 2.8, 300 k object 9.3 -> 2.6 (7.8 -> 2.3
+// without recording), 7 M needles 14.6 -> 3.85 (two depths), 1 M at 640x360 1.83 -> 0.56.
 //
 // HZ: the two-depth variant for forward-only views whose rays end early (binning.cu).  In its first phase
 // (L.hz_phase == 1) the tile lists hold only the pairs that begin before L.horizon; a ray that would need more
@@ -925,7 +925,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
 // patch's rays; a lane walks the samples that lie inside that Gaussian on its ray (a handful of the 32) and keeps the four
 // moment sums in registers.  The thirteen sums of the Gaussian's gradient row are then added up over the rays in shared memory and
 // leave the SM as one coalesced reduction of 52 bytes, where a reduction per ray and hit kept the L2 and the L1 data pipe busy.
-// Bound by instruction issue (78 % of the slots).  Against a warp per ray: 3 M-Gaussian view 7.7 -> 2.7 ms, 300 k object 4.7 -> 2.15 ms.
+// Bound by instruction issue (76 % of the slots) and the FMA pipe.  Against a warp per ray: 3 M-Gaussian view 7.7 -> 2.55 ms, 300 k object 4.7 -> 1.87 ms.
 template <int P>
 struct ReplayShared {
     Staged<kFan> st;
