@@ -319,7 +319,7 @@ __device__ __forceinline__ void patch_cone(const rgx_camera& c, int x0, int y0, 
 
 // Walks the entries of the list that can matter to rays whose windows lie within [wlo, whi]: 32 block summaries per step,
 // the blocks that overlap, their entries filtered by range and by the patch's cone; what is left is staged, and handed to
-// process(first, count) in list order, three groups or more at a time and whatever remains at the end.  `cursor`: first block that
+// process(first, count) in list order, four groups or more at a time and whatever remains at the end.  `cursor`: first block that
 // may still matter to a ray of the patch that has got as far as `wall`; it only moves forward.  whi may shrink while walking (closest hit).
 // One loop with one place that processes: the code that follows is long, and a second copy of it did not fit the instruction
 // cache beside the first (a third of all stalls on the 300 k object).  Fetching a block ahead with asynchronous copies was no
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kPatchWarps * 32, forward_ctas<COUNT>()) march
                 __syncwarp();
             }
             float whi = warp_max_pos(fmaxf(tmax, 0.0f));
-            walk_list<COUNT>(L, tv, sh.cone, wall, warp_min_pos(tmin), whi, cursor, st, 3 * kGroup, lane, tl, [&](int first, int count) {
+            walk_list<COUNT>(L, tv, sh.cone, wall, warp_min_pos(tmin), whi, cursor, st, 4 * kGroup, lane, tl, [&](int first, int count) {
 #pragma unroll 1
                 for (int base = 0; base < count; base += kGroup) {
                     const int f = (first + base) & (kStaged - 1), n = min(count - base, kGroup), nhit0 = nhit;   // a group does not wrap around the ring
