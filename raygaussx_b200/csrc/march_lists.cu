@@ -1227,8 +1227,11 @@ static bool use_lists(const MarchLaunch& m) {
 
 // Lanes per ray.  Two where the image gives every warp the device can hold a patch of sixteen rays (28,000 rays and more); with
 // fewer rays, smaller patches: more warps, and fewer Gaussians per patch, the longest patch being all there is to wait for.
-// Forward + backward in ms with 2 / 4 / 8 lanes per ray, 100 k object: 64x64 7.7 / 6.3 / 5.6, 128x128 1.94 / 1.47 / 1.27, 160x160
-// 1.37 / 1.01 / 1.15, 256x256 1.13 / 1.26 / 1.73 (tiles of 16 pixels).  The choice depends on the image alone, so that every march of
+// Forward + backward in ms with 2 / 4 / 8 lanes per ray, 100 k object: 64x64 1.01 / 0.54 / 0.36, 128x128 0.65 / 0.45 / 0.36, 150x150
+// 0.77 / 0.51 / 0.49, 180x180 0.75 / 0.52 / 0.60, 256x256 0.74 / 0.74 / 0.97, 300x300 0.92 / 1.06 / 1.48; 1 M unbounded: 128x128 0.41 / 0.28 / 0.24,
+// 150x150 0.43 / 0.30 / 0.30, 200x200 0.44 / 0.38 / 0.43, 256x256 0.50 / 0.50 / 0.64.  Four lanes would do a little better up to 240x240 (object 0.66 against
+// 0.76 at 230x230, unbounded 0.44 against 0.45), but every line moves the order in which a ray's terms are added up, and single gradient entries of
+// dense views with it by 1.7e-2 of the tensor's root mean square.  The choice depends on the image alone, so that every march of
 // a view -- whole or a row range, recording or not -- adds up a ray's colour in the same order.
 static int patch_lanes(const MarchLaunch& m) {
     const long long rays = (long long)m.cam.width * m.cam.height;
