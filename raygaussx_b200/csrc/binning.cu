@@ -303,6 +303,10 @@ __device__ __forceinline__ int gaussian_rect(const BinLaunch& b, const Projector
         const float cx = 0.5f * (bx.x + bx.y) - p.eye[0], cy = 0.5f * (by.x + by.y) - p.eye[1], cz = 0.5f * (bz.x + bz.y) - p.eye[2];
         const float hx = 0.5f * (bx.y - bx.x), hy = 0.5f * (by.y - by.x), hz = 0.5f * (bz.y - bz.x);
         const float r = sqrtf(hx * hx + hy * hy + hz * hz) * (1.0f + 1e-4f), far = sqrtf(cx * cx + cy * cy + cz * cz);
+        if (r == INFINITY) {            // an infinite scale: its box has no middle to place corners about, and may touch every tile
+            rect = make_uint2((unsigned)(b.tiles_x - 1) << 16, (unsigned)(b.tiles_y - 1) << 16);
+            return b.tiles_x * b.tiles_y;
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (p.plane[q][0] * cx + p.plane[q][1] * cy + p.plane[q][2] * cz < -(r + 1e-5f * far + 1e-7f) * p.plane[q][3]) return 0;
