@@ -900,7 +900,7 @@ static int forward_two_depth(rgx_ctx* ctx, const rgx_scene* scene, const rgx_cam
     }
     const HorizonPick pk = ctx->bin_result_host->pick;
     if (b.pick) learn_ratio(ctx, ctx->hz_ratio, total);
-    if (!b.pick || pk.cut == kAllBuckets || total == 0) {          // one depth is enough: these are the complete lists
+    if (!b.pick || pk.cut == kAllBuckets) {                        // one depth is enough: these are the complete lists
         lists_now_valid(ctx, cam, m, total, b.pick != nullptr);
         return RGX_OK;
     }
