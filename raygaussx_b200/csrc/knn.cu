@@ -98,20 +98,23 @@ __device__ __forceinline__ void warp_box(float (&lo)[3], float (&hi)[3]) {
 }
 
 // Sorted copies of the points, padded to a multiple of 32 with points at infinity, their boxes and, a block of 1,024 points
-// being one node of the level above, that node's.
+// being one node of the level above, that node's.  A point of which a coordinate is no number goes to infinity, where it is nobody's
+// neighbour, and into no box: the reference's comparisons pass by it too.
 __global__ void __launch_bounds__(1024) knn_gather_kernel(const float* __restrict__ pts, int n, const unsigned* __restrict__ order,
                                                           float4* sorted, KnnLevel leaf, KnnLevel mid) {
     after_previous();
     __shared__ float s_lo[32][3], s_hi[32][3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * 1024 + threadIdx.x, b = blockIdx.x * 32 + warp;
-    float4 p = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < n) {
         const size_t s = order[i];
         p = make_float4(pts[3 * s], pts[3 * s + 1], pts[3 * s + 2], 0.f);
     }
+    const bool is = i < n && p.x == p.x && p.y == p.y && p.z == p.z;
+    if (!is) p = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     if (b < leaf.count) sorted[i] = p;
-    float lo[3] = {p.x, p.y, p.z}, hi[3] = {i < n ? p.x : -INFINITY, i < n ? p.y : -INFINITY, i < n ? p.z : -INFINITY};
+    float lo[3] = {p.x, p.y, p.z}, hi[3] = {is ? p.x : -INFINITY, is ? p.y : -INFINITY, is ? p.z : -INFINITY};
     warp_box(lo, hi);
     if (lane == 0) {
         if (b < leaf.count) {
