@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256) refit_kernel(BuildLaunch b) {
         float2 x = make_float2(FLT_MAX, -FLT_MAX), y = x, z = x;
         if (c < b.count[level]) {
             int idx = b.offset[level] + c;
-            x = __ldcg(&b.bx[idx]); y = __ldcg(&b.by[idx]); z = __ldcg(&b.bz[idx]);
+            x = load_from_l2(&b.bx[idx]); y = load_from_l2(&b.by[idx]); z = load_from_l2(&b.bz[idx]);
         }
         x.x = warp_min(x.x); x.y = warp_max(x.y);
         y.x = warp_min(y.x); y.y = warp_max(y.y);

@@ -66,17 +66,24 @@ __device__ __forceinline__ void sh_basis_grad(float x, float y, float z, int K, 
     }
 }
 
-__device__ __forceinline__ void load_row(const float* p, int K, float* out) {
+struct ReadOnly {                      // not for kernels that are set up early, see after_previous
+    template <class T> __device__ __forceinline__ T operator()(const T* p) const { return __ldg(p); }
+};
+struct Plain {
+    template <class T> __device__ __forceinline__ T operator()(const T* p) const { return *p; }
+};
+template <class Load>
+__device__ __forceinline__ void load_row(const float* p, int K, float* out, Load load) {
     if (K == 16) {
         const float4* p4 = reinterpret_cast<const float4*>(p);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            float4 v = __ldg(p4 + t);
+            const float4 v = load(p4 + t);
             out[4 * t] = v.x; out[4 * t + 1] = v.y; out[4 * t + 2] = v.z; out[4 * t + 3] = v.w;
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) out[k] = k < K ? __ldg(p + k) : 0.f;
+        for (int k = 0; k < 16; ++k) out[k] = k < K ? load(p + k) : 0.f;
     }
 }
 
@@ -113,7 +120,7 @@ __device__ __forceinline__ void gaussian_color(const ColorLaunch& c, int j) {
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) {
         float row[16];
-        load_row(c.sc.color_features + ((size_t)i * 3 + ch) * K, K, row);
+        load_row(c.sc.color_features + ((size_t)i * 3 + ch) * K, K, row, ReadOnly{});
         float acc = rgb[ch];
 #pragma unroll
         for (int k = 0; k < 16; ++k)
@@ -241,7 +248,7 @@ __global__ void __launch_bounds__(128) finalize_kernel(FinalizeLaunch f) {
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) {
             float row[16];
-            load_row(f.sc.color_features + ((size_t)i * 3 + ch) * K, K, row);
+            load_row(f.sc.color_features + ((size_t)i * 3 + ch) * K, K, row, Plain{});
             float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
             for (int k = 0; k < 16; ++k)

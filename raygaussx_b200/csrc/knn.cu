@@ -31,7 +31,7 @@ constexpr int kKnnWarps = 8;
 constexpr int kFilterWarps = 148 * 64;     // as many warps as the device holds at once (303 k points), see knn_query_kernel
 
 // bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
-__global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pts, int n, unsigned* bounds) {
+__global__ void __launch_bounds__(256) knn_bounds_kernel(const float* pts, int n, unsigned* bounds) {
     after_previous();
     __shared__ unsigned s_max[6];
     if (threadIdx.x < 6) s_max[threadIdx.x] = 0u;
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict
 // sorting 64-bit keys costs 0.02 to 0.07 ms (100 k on surfaces 0.153 -> 0.177, 1 M 0.446 -> 0.509).  The extent cannot be told without
 // waiting for the device, so the line is the count from which the loss outweighs that price.
 template <class Key>
-__global__ void __launch_bounds__(256) knn_keys_kernel(const float* __restrict__ pts, int n, const unsigned* bounds,
+__global__ void __launch_bounds__(256) knn_keys_kernel(const float* pts, int n, const unsigned* bounds,
                                                        Key* keys, unsigned* vals) {
     after_previous();
     constexpr int kBits = sizeof(Key) == 8 ? 16 : 10;
@@ -100,7 +100,7 @@ __device__ __forceinline__ void warp_box(float (&lo)[3], float (&hi)[3]) {
 // Sorted copies of the points, padded to a multiple of 32 with points at infinity, their boxes and, a block of 1,024 points
 // being one node of the level above, that node's.  A point of which a coordinate is no number goes to infinity, where it is nobody's
 // neighbour, and into no box: the reference's comparisons pass by it too.
-__global__ void __launch_bounds__(1024) knn_gather_kernel(const float* __restrict__ pts, int n, const unsigned* __restrict__ order,
+__global__ void __launch_bounds__(1024) knn_gather_kernel(const float* pts, int n, const unsigned* order,
                                                           float4* sorted, KnnLevel leaf, KnnLevel mid) {
     after_previous();
     __shared__ float s_lo[32][3], s_hi[32][3];
@@ -165,8 +165,8 @@ struct KnnTree {
 // 1,424 -> 1,271 us, 1 M of an object 539 -> 489, 1 M on surfaces 493 -> 483); with fewer warps than the device holds the vote is one more
 // thing to wait for (30 k points 225 -> 235 us, 100 k 176 -> 178).
 template <bool FILTER>
-__global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* sorted, const unsigned* __restrict__ order,
-                                                                   int n, KnnTree tree, float* __restrict__ out) {
+__global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* sorted, const unsigned* order,
+                                                                   int n, KnnTree tree, float* out) {
     after_previous();
     __shared__ float s_pts[kKnnWarps][3][32];
     const int warp = blockIdx.x * kKnnWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;

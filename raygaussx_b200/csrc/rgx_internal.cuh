@@ -269,14 +269,30 @@ void note_launch();
 
 // Kernels that follow one another on a stream are set up while the one before still runs (programmatic dependent launch): a gap of
 // one to three microseconds less between any two.  A kernel launched by launch_after begins with after_previous(): it lets the
-// next one be set up, and waits until everything before it is done and visible.  It must not load through the read-only path (__ldg, const
-// __restrict__) what another such kernel of the same chain writes.  Iterations of 4 k Gaussians at 64x64 0.390 -> 0.376 ms, of 30 k at
+// next one be set up, and waits until everything before it is done and visible.  What it reads may have just been written by the kernel
+// before it -- the caller's points and parameters, too, by Adam -- and a load through the read-only path (__ldg, const __restrict__), or by an
+// intrinsic with a cache hint, is bound to nothing and may be moved above that wait: such kernels use plain loads and the two below.  Iterations of 4 k Gaussians at 64x64 0.390 -> 0.376 ms, of 30 k at
 // 399x301 0.751 -> 0.721, RGB + alpha + depth of 1 M at 640x360 1.058 -> 1.039, neighbour distances of 30 k points 0.227 -> 0.218.
 //   Not for the march and the colours: blocks that are set up early live with the division between shared memory and L1 cache that
 // the kernel before them asked for (colours behind the sort of the tile lists 33 -> 104 us, march of the 300 k object +3 %).
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ float load_streaming(const float* p) {
+    float v;
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ float4 load_streaming(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ float2 load_from_l2(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(__cvta_generic_to_global(p)) : "memory");
+    return v;
 }
 template <class... Params, class... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {

@@ -29,8 +29,8 @@ __global__ void __launch_bounds__(256) activate_kernel(rgx_activation a) {
             const size_t row = i >> 2;
             const int k = (int)(i & 3) * 4;
             const float* sh = a.sh + row * 15 + k - 1;
-            const float first = k == 0 ? __ldcs(a.rgb + row) : __ldcs(sh);
-            reinterpret_cast<float4*>(a.color)[i] = make_float4(first, __ldcs(sh + 1), __ldcs(sh + 2), __ldcs(sh + 3));
+            const float first = k == 0 ? load_streaming(a.rgb + row) : load_streaming(sh);
+            reinterpret_cast<float4*>(a.color)[i] = make_float4(first, load_streaming(sh + 1), load_streaming(sh + 2), load_streaming(sh + 3));
         }
     } else if (i < (size_t)a.n * 3 * k_all) {
         const size_t row = i / k_all;
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) activate_backward_kernel(rgx_activation a
         if (g.color && i < (size_t)a.n * 12) {
             const size_t row = i >> 2;
             const int k = (int)(i & 3) * 4;
-            const float4 v = __ldcs(reinterpret_cast<const float4*>(g.color) + i);
+            const float4 v = load_streaming(reinterpret_cast<const float4*>(g.color) + i);
             if (k != 0) { if (g.sh) g.sh[row * 15 + k - 1] = v.x; }
             else if (g.rgb) g.rgb[row] = v.x;
             if (g.sh) {
@@ -136,10 +136,10 @@ struct LossArgs {
 // pixel (x, y) of channel c: the mean of its rays; zero outside, as the blur's padding
 __device__ __forceinline__ float pixel_of(const LossArgs& a, int c, int x, int y) {
     const size_t W = (size_t)a.w * a.fx;
-    if (a.fx == 1 && a.fy == 1) return __ldg(&a.rays[((size_t)y * W + x) * 3 + c]);
+    if (a.fx == 1 && a.fy == 1) return a.rays[((size_t)y * W + x) * 3 + c];
     float sum = 0.f;
     for (int j = 0; j < a.fy; ++j)
-        for (int i = 0; i < a.fx; ++i) sum += __ldg(&a.rays[(((size_t)y * a.fy + j) * W + (size_t)x * a.fx + i) * 3 + c]);
+        for (int i = 0; i < a.fx; ++i) sum += a.rays[(((size_t)y * a.fy + j) * W + (size_t)x * a.fx + i) * 3 + c];
     return sum / (float)(a.fx * a.fy);
 }
 
@@ -158,7 +158,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // A block takes a tile of 32x32 pixels of one channel: both images with a rim of five pixels into shared memory, the five blurred
 // moments along x, then along y, all without leaving the SM.  Per pixel the derivative of SSIM with respect to the blurred
 // image, its blurred square and the blurred product (maps, three planes), which is what the backward needs to blur.
-// About 190 arithmetic instructions per pixel and channel; 1256x828: 66 us and 51 us for the backward, where framework operators took 1.9 ms for both.
+// About 190 arithmetic instructions per pixel and channel; 1256x828: 63 us and 50 us for the backward, where framework operators took 1.9 ms for both.
 template <bool SSIM>
 __global__ void __launch_bounds__(kTile * kRows) image_loss_kernel(LossArgs a, float* maps, float2* partial) {
     after_previous();
@@ -169,12 +169,21 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_kernel(LossArgs a, f
     const size_t plane = (size_t)a.w * a.h;
     float l1 = 0.f, ss = 0.f;
     if (SSIM) {
-        for (int j = ty; j < kSpan; j += kRows)
+        for (int j = ty; j < kSpan; j += 2 * kRows)
+#pragma unroll
             for (int i = tx; i < kSpan; i += kTile) {
-                const int x = x0 + i - kRad, y = y0 + j - kRad;
-                const bool in = x >= 0 && y >= 0 && x < a.w && y < a.h;
-                s_x[j][i] = in ? pixel_of(a, c, x, y) : 0.f;
-                s_y[j][i] = in ? __ldg(&a.target[c * plane + (size_t)y * a.w + x]) : 0.f;
+                // two rows at a time, or each pair of loads would wait for the stores of the one before
+                float u[2], v[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int x = x0 + i - kRad, y = y0 + j + k * kRows - kRad;
+                    const bool in = j + k * kRows < kSpan && x >= 0 && y >= 0 && x < a.w && y < a.h;
+                    u[k] = in ? pixel_of(a, c, x, y) : 0.f;
+                    v[k] = in ? a.target[c * plane + (size_t)y * a.w + x] : 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (j + k * kRows < kSpan) { s_x[j + k * kRows][i] = u[k]; s_y[j + k * kRows][i] = v[k]; }
             }
         __syncthreads();
         for (int j = ty; j < kSpan; j += kRows) {
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_kernel(LossArgs a, f
         const int x = x0 + tx, y = y0 + j;
         if (x >= a.w || y >= a.h) continue;
         if (!SSIM) {
-            l1 += fabsf(pixel_of(a, c, x, y) - __ldg(&a.target[c * plane + (size_t)y * a.w + x]));
+            l1 += fabsf(pixel_of(a, c, x, y) - a.target[c * plane + (size_t)y * a.w + x]);
             continue;
         }
         l1 += fabsf(s_x[j + kRad][tx + kRad] - s_y[j + kRad][tx + kRad]);
@@ -271,7 +280,7 @@ __global__ void __launch_bounds__(kTile * kRows) image_loss_backward_kernel(Loss
     for (int j = ty; j < kTile; j += kRows) {
         const int x = x0 + tx, y = y0 + j;
         if (x >= a.w || y >= a.h) continue;
-        const float u = pixel_of(a, c, x, y), t = __ldg(&a.target[c * plane + (size_t)y * a.w + x]);
+        const float u = pixel_of(a, c, x, y), t = a.target[c * plane + (size_t)y * a.w + x];
         float g = (1.0f - a.lambda) * (u > t ? 1.0f : u < t ? -1.0f : 0.0f);
         if (SSIM) {
             float v[3] = {0.f, 0.f, 0.f};
@@ -347,7 +356,7 @@ __global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamT
 #pragma unroll 2
         for (size_t i = begin + 4 * threadIdx.x; i < whole; i += 4 * 256) {
             float4 p = *reinterpret_cast<float4*>(t.param + i), m = *reinterpret_cast<float4*>(t.exp_avg + i), v = *reinterpret_cast<float4*>(t.exp_avg_sq + i);
-            const float4 g = __ldcs(reinterpret_cast<const float4*>(t.grad + i));
+            const float4 g = load_streaming(reinterpret_cast<const float4*>(t.grad + i));
             adam_value(p.x, g.x, m.x, v.x, a.rest1, a.beta2, a.rest2, t.step_size, t.inv_root, a.eps);
             adam_value(p.y, g.y, m.y, v.y, a.rest1, a.beta2, a.rest2, t.step_size, t.inv_root, a.eps);
             adam_value(p.z, g.z, m.z, v.z, a.rest1, a.beta2, a.rest2, t.step_size, t.inv_root, a.eps);

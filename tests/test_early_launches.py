@@ -1,0 +1,54 @@
+"""Kernels that are set up while the kernel before them runs (`launch_after`): they wait before their first access, and they load nothing
+through the read-only path or by an intrinsic with a cache hint, which the compiler may move above that wait.  Read from the sources: no
+run shows a load moved."""
+import glob
+import os
+import re
+
+from tests.conftest import ROOT
+
+CSRC = os.path.join(ROOT, "raygaussx_b200", "csrc")
+DEFINITION = re.compile(r"__(global|device)__([^;{}]*?)\b(\w+)\(((?:[^(){};]|\([^()]*\))*)\)\s*(?:const\s*)?\{")
+
+
+def functions():
+    """name -> (kernel?, parameters, body) of every kernel and device function; bodies of one name in several places are joined."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+        for m in DEFINITION.finditer(text):
+            depth, end = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            kernel, params, body = out.get(m.group(3), (False, "", ""))
+            out[m.group(3)] = (kernel or m.group(1) == "global", params + m.group(4), body + text[m.end():end])
+    return out
+
+
+def launched_early():
+    text = "".join(open(p).read() for p in glob.glob(os.path.join(CSRC, "*.cu*")))
+    return set(re.findall(r"launch_after\(\(?(\w+_kernel)\b", text))
+
+
+def test_early_kernels_wait_first():
+    found, early = functions(), launched_early()
+    assert len(early) > 25
+    for name in early:
+        kernel, _, body = found[name]
+        assert kernel and re.match(r"\s*after_previous\(\);", body), name
+
+
+def test_early_kernels_load_nothing_that_may_be_moved():
+    found = functions()
+    for name in launched_early():
+        todo, seen = [name], set()
+        while todo:
+            f = todo.pop()
+            if f in seen or f not in found:
+                continue
+            seen.add(f)
+            _, params, body = found[f]
+            assert "__restrict__" not in params, (name, f)
+            assert not re.search(r"__ld\w+\(|\bReadOnly\b|global\.nc\b|asm\s*\(\s*\"ld\b", body), (name, f)
+            todo += re.findall(r"\b(\w+)\s*(?:<[^;{}()]*>)?\(", body)
