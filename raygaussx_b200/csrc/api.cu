@@ -383,6 +383,7 @@ int run_colors_if_beyond(rgx_ctx* ctx, const rgx_scene* sc, const float eye[3], 
     c.rgba = ctx->rgba;
     c.sigma_threshold = ctx->sigma_threshold;
     c.only_if = count;
+    c.sm_count = ctx->sm_count;
     c.listed_out = ctx->listed_serial == ctx->rgba_serial ? ctx->listed : nullptr;
     cudaError_t e = launch_colors(c, s);
     return e == cudaSuccess ? RGX_OK : cuda_fail(ctx, e, "colour kernel");
@@ -466,8 +467,11 @@ int rgx_create(int device, rgx_ctx** out) {
     rgx_ctx* ctx = new (std::nothrow) rgx_ctx();
     if (!ctx) return RGX_E_INVALID;
     ctx->device = device;
-    if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || ctx->sm_count <= 0)
-        ctx->sm_count = 148;
+    if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || ctx->sm_count <= 0) {
+        (void)cudaGetLastError();
+        delete ctx;
+        return RGX_E_CUDA;
+    }
     *out = ctx;
     return RGX_OK;
 }

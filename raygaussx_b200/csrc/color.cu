@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(128) clear_kernel(const __grid_constant__ Clea
 cudaError_t launch_colors(const ColorLaunch& c, cudaStream_t s) {
     const int slots = color_slots(c), blocks = (slots + 127) / 128;
     if (slots == 0) return cudaSuccess;
-    if (c.only_if) note_launch(), colors_if_beyond_kernel<<<blocks < 148 * 8 ? blocks : 148 * 8, 128, 0, s>>>(c);
+    if (c.only_if) note_launch(), colors_if_beyond_kernel<<<blocks < c.sm_count * 8 ? blocks : c.sm_count * 8, 128, 0, s>>>(c);
     else note_launch(), colors_kernel<<<blocks, 128, 0, s>>>(c);
     return cudaGetLastError();
 }

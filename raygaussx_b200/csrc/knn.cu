@@ -28,7 +28,6 @@ namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kKnnWarps = 8;
-constexpr int kFilterWarps = 148 * 64;     // as many warps as the device holds at once (303 k points), see knn_query_kernel
 
 // bounds: [0, 3) largest coordinates, [3, 6) largest negated coordinates, as ordered integers that start at zero
 __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* pts, int n, unsigned* bounds) {
@@ -162,8 +161,8 @@ struct KnnTree {
 
 // FILTER: eight points at a time are passed by where none of them is nearer to its query than what a lane has.  Of the points opened
 // few are, so that saves most of the bookkeeping where the kernel is bound by arithmetic (whole call, 3 M points of a core and a shell
-// 1,424 -> 1,271 us, 1 M of an object 539 -> 489, 1 M on surfaces 493 -> 483); with fewer warps than the device holds the vote is one more
-// thing to wait for (30 k points 225 -> 235 us, 100 k 176 -> 178).
+// 1,424 -> 1,271 us, 1 M of an object 539 -> 489, 1 M on surfaces 493 -> 483); with fewer warps than the device holds, 64 on each SM (303 k
+// points on 148), the vote is one more thing to wait for (30 k points 225 -> 235 us, 100 k 176 -> 178).
 template <bool FILTER>
 __global__ void __launch_bounds__(kKnnWarps * 32) knn_query_kernel(const float4* sorted, const unsigned* order,
                                                                    int n, KnnTree tree, float* out) {
@@ -299,11 +298,14 @@ cudaError_t plan_scratch(int n, unsigned char* base, KnnScratch& w) {
     return e;
 }
 
-cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaStream_t s) {
+cudaError_t run_knn(int device, const float* points, int n, float* out, KnnScratch& w, cudaStream_t s) {
     const int tb = 256;
-    cudaError_t e = cudaMemsetAsync(w.bounds, 0, 6 * sizeof(unsigned), s);
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 592), tb, 0, s, points, n, w.bounds);
+    e = cudaMemsetAsync(w.bounds, 0, 6 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 4 * sms), tb, 0, s, points, n, w.bounds);
     if (wide_keys(n)) launch_after(knn_keys_kernel<uint64_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
     else launch_after(knn_keys_kernel<uint32_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
     e = wide_keys(n) ? cluster_sort((const uint64_t*)w.keys_in, (uint64_t*)w.keys_out, w.vals_in, w.vals_out, n, 48, s)
@@ -313,7 +315,7 @@ cudaError_t run_knn(const float* points, int n, float* out, KnnScratch& w, cudaS
     launch_after(knn_gather_kernel, w.tree.mid.count, 1024, 0, s, points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
     launch_after(knn_upper_kernel, (w.tree.top.count + 7) / 8, 256, 0, s, w.tree.mid, w.tree.top);
     const int blocks = (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps;
-    if (w.tree.leaf.count > kFilterWarps) launch_after(knn_query_kernel<true>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
+    if (w.tree.leaf.count > 64 * sms) launch_after(knn_query_kernel<true>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
     else launch_after(knn_query_kernel<false>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
     return cudaGetLastError();
 }
@@ -339,7 +341,7 @@ extern "C" RGX_API int rgx_knn_mean_dist2_scratch(int device, const float* point
     KnnScratch w;
     cudaError_t e = plan_scratch(n, (unsigned char*)scratch, w);
     if (e == cudaSuccess && w.bytes > scratch_bytes) return RGX_E_INVALID;
-    if (e == cudaSuccess) e = run_knn(points, n, mean_dist2, w, (cudaStream_t)stream);
+    if (e == cudaSuccess) e = run_knn(device, points, n, mean_dist2, w, (cudaStream_t)stream);
     if (e != cudaSuccess) { (void)cudaGetLastError(); return RGX_E_CUDA; }
     return RGX_OK;
 }

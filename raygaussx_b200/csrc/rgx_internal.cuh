@@ -227,6 +227,7 @@ struct ColorLaunch {
     unsigned int listed_cut;
     unsigned char* listed_out;   // [n_pad] 1 where the Gaussian is on some list of the view (written with listed_code)
     const unsigned int* only_if; // not null: the kernel does nothing when this counter is zero
+    int sm_count;                // wanted with only_if
 };
 
 struct FinalizeLaunch {

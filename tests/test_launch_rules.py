@@ -1,6 +1,8 @@
-"""Kernels that are set up while the kernel before them runs (`launch_after`): they wait before their first access, and they load nothing
-through the read-only path or by an intrinsic with a cache hint, which the compiler may move above that wait.  Read from the sources: no
-run shows a load moved."""
+"""Rules of the launches that the kernels' sources have to keep and that no run shows broken.
+
+Kernels that are set up while the kernel before them runs (`launch_after`) wait before their first access, and load nothing through the
+read-only path or by an intrinsic with a cache hint, which the compiler may move above that wait.  Grids are sized by the number of SMs that
+the device has, not by one written out."""
 import glob
 import os
 import re
@@ -52,3 +54,9 @@ def test_early_kernels_load_nothing_that_may_be_moved():
             assert "__restrict__" not in params, (name, f)
             assert not re.search(r"__ld\w+\(|\bReadOnly\b|global\.nc\b|asm\s*\(\s*\"ld\b", body), (name, f)
             todo += re.findall(r"\b(\w+)\s*(?:<[^;{}()]*>)?\(", body)
+
+
+def test_the_number_of_sms_is_asked_for():
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+        assert not re.search(r"\b(148|296|592|1184|9472)\b", text), path
