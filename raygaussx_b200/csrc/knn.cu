@@ -133,8 +133,15 @@ __global__ void __launch_bounds__(1024) knn_gather_kernel(const float* pts, int 
     }
 }
 
+// LATE: the query is set up when the gathering is done, not beside it.  Where it has few blocks they crowd otherwise on the SMs without a
+// block of knn_gather_kernel: with 3,125 warps, 391 blocks of eight, beside 98 of those, on 50 SMs.  Up to four blocks per SM (151 k points
+// on 148); whole call, us, beside it and behind it: 40 k points of an object 122.7 and 116.1, 65 k 152.6 and 141.4, 80 k on surfaces 161.1
+// and 148.3, 100 k 182.5 and 174.1, 130 k 187.8 and 182.5, 150 k 193.2 and 192.6; beyond that either may be the faster (180 k on surfaces
+// 206.9 and 200.1, 230 k 214.3 and 221.3).
+template <bool LATE>
 __global__ void __launch_bounds__(256) knn_upper_kernel(KnnLevel below, KnnLevel level) {
-    after_previous();
+    if (LATE) after_previous_then_next();
+    else after_previous();
     const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (node >= level.count) return;
     const int b = node * 32 + lane;
@@ -313,8 +320,9 @@ cudaError_t run_knn(int device, const float* points, int n, float* out, KnnScrat
     if (e == cudaErrorNotSupported) e = sort_points(w, n, s);
     if (e != cudaSuccess) return e;
     launch_after(knn_gather_kernel, w.tree.mid.count, 1024, 0, s, points, n, w.vals_out, w.sorted, w.tree.leaf, w.tree.mid);
-    launch_after(knn_upper_kernel, (w.tree.top.count + 7) / 8, 256, 0, s, w.tree.mid, w.tree.top);
-    const int blocks = (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps;
+    const int blocks = (w.tree.leaf.count + kKnnWarps - 1) / kKnnWarps, upper = (w.tree.top.count + 7) / 8;
+    if (blocks <= 4 * sms) launch_after(knn_upper_kernel<true>, upper, 256, 0, s, w.tree.mid, w.tree.top);
+    else launch_after(knn_upper_kernel<false>, upper, 256, 0, s, w.tree.mid, w.tree.top);
     if (w.tree.leaf.count > 64 * sms) launch_after(knn_query_kernel<true>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
     else launch_after(knn_query_kernel<false>, blocks, kKnnWarps * 32, 0, s, w.sorted, w.vals_out, n, w.tree, out);
     return cudaGetLastError();

@@ -280,6 +280,12 @@ __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The other way round: the next kernel is set up only when everything before this one is done.  For a short kernel that is followed by one
+// of a few blocks per SM: set up beside the kernel before last, those would all go to the SMs that it leaves free.
+__device__ __forceinline__ void after_previous_then_next() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
 __device__ __forceinline__ float load_streaming(const float* p) {
     float v;
     asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));

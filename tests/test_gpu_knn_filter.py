@@ -1,12 +1,13 @@
-"""Neighbour distances on either side of the count from which the query passes points by eight at a time (`-m gpu`): against brute
-force in float64 for a part of the points, with clusters, duplicates and far points among them."""
+"""Neighbour distances on either side of the counts from which the query is set up beside the gathering (four blocks of 256 queries on each
+of 148 SMs) and from which it passes points by eight at a time (`-m gpu`): against brute force in float64 for a part of the points, with
+clusters, duplicates and far points among them."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [32 * 9472, 32 * 9472 + 1, 500_009])
+@pytest.mark.parametrize("n", [4 * 148 * 256, 4 * 148 * 256 + 1, 32 * 9472, 32 * 9472 + 1, 500_009])
 def test_large_clouds_are_exact(n):
     if not torch.cuda.is_available():
         pytest.fail("GPU tests need a CUDA device: there is no CPU path")

@@ -38,7 +38,7 @@ def test_early_kernels_wait_first():
     assert len(early) > 25
     for name in early:
         kernel, _, body = found[name]
-        assert kernel and re.match(r"\s*after_previous\(\);", body), name
+        assert kernel and re.match(r"\s*(after_previous\(\);|if \(LATE\) after_previous_then_next\(\);\s*else after_previous\(\);)", body), name
 
 
 def test_early_kernels_load_nothing_that_may_be_moved():
