@@ -291,8 +291,9 @@ __device__ __forceinline__ bool patch_misses(const float4* cone, float4 g0, floa
     const float3 P = make_float3(fmaf(t, de.x, Oe.x), fmaf(t, de.y, Oe.y), fmaf(t, de.z, Oe.z));
     const float rho = fmaf(__fmul_rn(far, c.w), sqrt_approx(fmaxf(dot3(dp, dp), dot3(dq, dq))), 1.0f);
     const float room = fmaf(__fmul_rn(rho, rho), 1.0005f, 1e-5f) - dot3(P, P);
-    const float h = sqrt_approx(fmaxf(room, 0.0f) * inv_a) * 1.01f;
-    return room < 0.0f || t - h > fmaf(p.w, whi, whi) || t + h < fmaf(-p.w, wlo, wlo);       // false for NaN: kept
+    // (no number where room is none -- a Gaussian without end may have an endless range and no width across the cone --, and then kept)
+    const float h = sqrt_approx(room * inv_a) * 1.01f;
+    return room < 0.0f || t - h > fmaf(p.w, whi, whi) || t + h < fmaf(-p.w, wlo, wlo);
 }
 
 // The cone of a patch: the unit direction of its middle ray with the scale of the diagonals, and the two half diagonals.
