@@ -164,7 +164,7 @@ struct PairGeom {
 // the box and the ellipsoid grown by that much.
 // A ray whose closest approach lies behind the eye misses, even from inside (ellipsoid_stretch in march_common.cuh): for M the whitening
 // map and Oe = M (eye - centre), if -Oe . M d < 0.  `away` = |M^T Oe|, so for a ray of the tile that is at most the central ray's plus
-// chord * away; `slack` is ten times what rounding can make of it.  Such pairs are those of Gaussians that hold the eye and lie
+// chord * away; `slack` covers what rounding makes of it here and in the march (make_pair_geom).  Such pairs are those of Gaussians that hold the eye and lie
 // behind it: a third of the entries that the march of 30 k large Gaussians about the camera tested, a seventh of 1 M
 // (forward of the former at 399x301 0.278 -> 0.229 ms, of the latter at 628x414 0.907 -> 0.851, four views of 3 M 14.47 -> 14.02).
 __device__ __forceinline__ bool pair_range(const float* eye, float4 td, const PairGeom& g, float& tn, float& tf) {
@@ -281,7 +281,10 @@ __device__ __forceinline__ PairGeom make_pair_geom(const float* eye, float2 bx, 
     const float3 r0 = make_float3(g0.w, g1.x, g1.y), r1 = make_float3(g1.z, g1.w, g2.x), r2 = make_float3(g2.y, g2.z, g2.w);
     const float3 Oe = make_float3(dot3(r0, O), dot3(r1, O), dot3(r2, O)), v = r0 * Oe.x + r1 * Oe.y + r2 * Oe.z;
     g.away = sqrtf(dot3(v, v));
-    g.slack = 1e-5f * sqrtf(dot3(Oe, Oe) * (dot3(r0, r0) + dot3(r1, r1) + dot3(r2, r2)));
+    // Oe is good to 3.5 rounding errors of |M| |O|, which is more than |Oe| by up to the ratio of the Gaussian's axes, M d to as many of
+    // |M|, the product to three more of |Oe| |M|; here and in the march: 4.2e-7 |M|^2 |O| and 7.8e-7 |Oe| |M| together
+    const float M2 = dot3(r0, r0) + dot3(r1, r1) + dot3(r2, r2);
+    g.slack = 1e-5f * sqrtf(dot3(Oe, Oe) * M2) + 1e-6f * M2 * sqrtf(dot3(O, O));
     return g;
 }
 

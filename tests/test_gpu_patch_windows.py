@@ -49,3 +49,42 @@ def test_nothing_that_is_met_is_left_out(shape, fov, width, height, inside):
     for a, b, tol, most in zip(got["lists"][:3], got["per_ray"][:3], (1e-5, 1e-5, 1e-4), (rim, rim, 10 * rim)):
         d = (a - b).abs()
         assert d.max().item() < most and (d > tol).float().mean().item() < 1e-3
+
+
+@pytest.mark.parametrize("thin", [[1.0, 1e-3, 1e-3], [1.0, 1.0, 1e-3], [1.0, 0.1, 3e-4]])
+def test_gaussians_nearest_at_the_eye_are_not_taken_to_lie_behind_it(thin):
+    """Needles and discs of a thousand to one that hold the eye and are closest to the ray right there: whether that is in front or behind is
+    decided by rounding, and has to be decided by the march, not by the lists."""
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device: there is no CPU path")
+    from raygaussx_b200 import render_optix as ro
+    dev = torch.device("cuda")
+    n = 1500
+    sc = scenes.tiny_scene(n=n, width=1, height=1, seed=11)
+    g = torch.Generator().manual_seed(5)
+    q = torch.randn(n, 4, generator=g)
+    sc.quaternions = q / q.norm(dim=1, keepdim=True)
+    sc.scales = torch.tensor(thin).repeat(n, 1) * torch.exp(0.3 * torch.randn(n, 1, generator=g))
+    sc.densities = torch.full((n,), 0.3)
+    w, x, y, z = sc.quaternions.double().unbind(1)
+    rows = [1 - 2 * (y * y + z * z), 2 * (x * y - w * z), 2 * (x * z + w * y), 2 * (x * y + w * z), 1 - 2 * (x * x + z * z), 2 * (y * z - w * x),
+            2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)]
+    turn, s = torch.stack(rows, 1).reshape(n, 3, 3), sc.scales.double()
+    along = turn[:, 0, :] / s                                  # the ray's direction (1, 0, 0), in the frame of the Gaussian
+    off = torch.randn(n, 3, generator=g).double()
+    off = off - (off * along).sum(1, keepdim=True) / (along * along).sum(1, keepdim=True) * along
+    off = 0.9 * off / off.norm(dim=1, keepdim=True)            # the eye there: at right angles to the ray
+    sc.positions = -(turn @ (off * s)[:, :, None])[:, :, 0].float()
+    cam = scenes.SimpleCamera((0.0, 0.0, 0.0), target=(1.0, 0.0, 0.0), width=1, height=1).to(dev)
+    cs = ro.camera_struct(cam)
+    tens = [t.to(dev).contiguous() for t in sc.tensors()]
+    r = ro.Renderer(dev)
+    r.build(*tens[:4])
+    got = []
+    for flags in (0, _lib.FLAG_PER_RAY_SEARCH):
+        r.reset_counters()
+        r.forward(*tens, cs, r._march(0.01, False, 4096, False, 1e-3, None, 1, flags | _lib.FLAG_COUNT_WORK))
+        got.append(r.read_counters())
+    assert got[0]["hits"] > n // 4
+    for k in ("rays", "slabs", "slabs_hit", "closest_queries", "hits", "hits_hash", "overflow_slabs"):
+        assert got[0][k] == got[1][k], k
