@@ -218,11 +218,11 @@ cudaError_t launch_build(const BuildLaunch& b, cudaStream_t s) {
     const int n = b.sc.n;
     const int tb = 256, blocks = (n + tb - 1) / tb;
     const bool narrow = 3 * b.morton_bits <= 32;
-    launch_after(bounds_kernel, blocks, tb, 0, s, b);
-    if (narrow) launch_after(morton_kernel<uint32_t>, blocks, tb, 0, s, b);
-    else launch_after(morton_kernel<uint64_t>, blocks, tb, 0, s, b);
-    cudaError_t e = narrow ? cluster_sort((const uint32_t*)b.keys_in, (uint32_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s)
-                           : cluster_sort((const uint64_t*)b.keys_in, (uint64_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s);
+    cudaError_t e;
+    if ((e = launch_after(bounds_kernel, blocks, tb, 0, s, b)) != cudaSuccess) return e;
+    if ((e = launch_after(narrow ? morton_kernel<uint32_t> : morton_kernel<uint64_t>, blocks, tb, 0, s, b)) != cudaSuccess) return e;
+    e = narrow ? cluster_sort((const uint32_t*)b.keys_in, (uint32_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s)
+               : cluster_sort((const uint64_t*)b.keys_in, (uint64_t*)b.keys_out, b.vals_in, b.vals_out, n, 3 * b.morton_bits, s);
     if (e == cudaErrorNotSupported) {
         size_t temp = b.cub_temp_bytes;
         e = narrow ? sort_keys<uint32_t>(b, b.cub_temp, temp, n, 3 * b.morton_bits, s)

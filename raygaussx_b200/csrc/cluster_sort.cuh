@@ -114,7 +114,14 @@ __global__ void __launch_bounds__(kClusterThreads) cluster_sort_kernel(const Key
     }
 }
 
-// cudaErrorNotSupported, and nothing enqueued, where there are too few or too many pairs or the device does not take the cluster.
+// What says that this device, or what is left of it, does not take the cluster.  Any other error is no reason to go on.
+inline bool cluster_refused(cudaError_t e) {
+    return e == cudaErrorInvalidClusterSize || e == cudaErrorInvalidConfiguration || e == cudaErrorInvalidValue || e == cudaErrorLaunchOutOfResources ||
+           e == cudaErrorNotSupported;
+}
+
+// cudaErrorNotSupported, and nothing enqueued, where there are too few or too many pairs or the device does not take the cluster.  Clears
+// that error: the caller has looked at the results of its launches before.
 template <class Key>
 cudaError_t cluster_sort(const Key* keys_in, Key* keys_out, const unsigned* vals_in, unsigned* vals_out, int n, int bits, cudaStream_t s) {
     if (n < kClusterSortFrom || n > kClusterSortTo) return cudaErrorNotSupported;
@@ -134,10 +141,9 @@ cudaError_t cluster_sort(const Key* keys_in, Key* keys_out, const unsigned* vals
         c.stream = s;
         c.attrs = &cluster;
         c.numAttrs = 1;
-        note_launch();
-        e = cudaLaunchKernelEx(&c, cluster_sort_kernel<Key>, keys_in, keys_out, vals_in, vals_out, n, bits, piece);
+        if ((e = cudaLaunchKernelEx(&c, cluster_sort_kernel<Key>, keys_in, keys_out, vals_in, vals_out, n, bits, piece)) == cudaSuccess) note_launch();
     }
-    if (e == cudaSuccess) return e;
+    if (!cluster_refused(e)) return e;
     (void)cudaGetLastError();
     return cudaErrorNotSupported;
 }

@@ -312,9 +312,10 @@ cudaError_t run_knn(int device, const float* points, int n, float* out, KnnScrat
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(w.bounds, 0, 6 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
-    launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 4 * sms), tb, 0, s, points, n, w.bounds);
-    if (wide_keys(n)) launch_after(knn_keys_kernel<uint64_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
-    else launch_after(knn_keys_kernel<uint32_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
+    if ((e = launch_after(knn_bounds_kernel, std::min((n + tb - 1) / tb, 4 * sms), tb, 0, s, points, n, w.bounds)) != cudaSuccess) return e;
+    if (wide_keys(n)) e = launch_after(knn_keys_kernel<uint64_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint64_t*)w.keys_in, w.vals_in);
+    else e = launch_after(knn_keys_kernel<uint32_t>, (n + tb - 1) / tb, tb, 0, s, points, n, w.bounds, (uint32_t*)w.keys_in, w.vals_in);
+    if (e != cudaSuccess) return e;
     e = wide_keys(n) ? cluster_sort((const uint64_t*)w.keys_in, (uint64_t*)w.keys_out, w.vals_in, w.vals_out, n, 48, s)
                      : cluster_sort((const uint32_t*)w.keys_in, (uint32_t*)w.keys_out, w.vals_in, w.vals_out, n, 30, s);
     if (e == cudaErrorNotSupported) e = sort_points(w, n, s);

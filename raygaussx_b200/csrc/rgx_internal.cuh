@@ -303,7 +303,6 @@ __device__ __forceinline__ float2 load_from_l2(const float2* p) {
 }
 template <class... Params, class... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
-    note_launch();
     cudaLaunchAttribute early = {};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -314,7 +313,9 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block
     c.stream = s;
     c.attrs = &early;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<Args&&>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<Args&&>(args)...);
+    if (e == cudaSuccess) note_launch();
+    return e;
 }
 
 // host launchers (each returns the cudaError_t of its last launch)

@@ -32,6 +32,18 @@ def test_every_point_gets_its_own_distance(n):
     assert torch.isfinite(got).all() and (got > 0).all()
 
 
+@pytest.mark.parametrize("n,cluster", [(4096, False), (4097, True), (65535, True), (65536, True), (81920, True), (81921, False)])
+def test_the_cluster_sorts_what_it_is_for(n, cluster):
+    """Own kernels of a call: bounds, keys, gather, upper boxes, query, and the cluster's sort; those of the library are not counted."""
+    dev = gpu()
+    from raygaussx_b200 import _lib
+    from simple_knn._C import distCUDA2
+    pts = torch.randn(n, 3, generator=torch.Generator().manual_seed(n)).to(dev)
+    before = _lib.lib().rgx_kernel_launches()
+    distCUDA2(pts)
+    assert _lib.lib().rgx_kernel_launches() - before == 5 + cluster
+
+
 @pytest.mark.parametrize("n,bits", [(4097, 10), (30_000, 10), (30_000, 20), (70_001, 10), (81_920, 10), (81_920, 20)])
 def test_same_image_and_gradients_as_with_the_library(n, bits):
     dev = gpu()

@@ -10,21 +10,21 @@ import re
 from tests.conftest import ROOT
 
 CSRC = os.path.join(ROOT, "raygaussx_b200", "csrc")
-DEFINITION = re.compile(r"__(global|device)__([^;{}]*?)\b(\w+)\(((?:[^(){};]|\([^()]*\))*)\)\s*(?:const\s*)?\{")
+DEFINITION = r"(%s)([^;{}]*?)\b(\w+)\(((?:[^(){};]|\([^()]*\))*)\)\s*(?:const\s*)?\{"
 
 
-def functions():
-    """name -> (kernel?, parameters, body) of every kernel and device function; bodies of one name in several places are joined."""
+def functions(begin=r"__(?:global|device)__"):
+    """name -> (kernel?, parameters, body) of every function declared so; bodies of one name in several places are joined."""
     out = {}
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
         text = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
-        for m in DEFINITION.finditer(text):
+        for m in re.finditer(DEFINITION % begin, text):
             depth, end = 1, m.end()
             while depth:
                 depth += {"{": 1, "}": -1}.get(text[end], 0)
                 end += 1
             kernel, params, body = out.get(m.group(3), (False, "", ""))
-            out[m.group(3)] = (kernel or m.group(1) == "global", params + m.group(4), body + text[m.end():end])
+            out[m.group(3)] = (kernel or m.group(1) == "__global__", params + m.group(4), body + text[m.end():end])
     return out
 
 
@@ -54,6 +54,23 @@ def test_early_kernels_load_nothing_that_may_be_moved():
             assert "__restrict__" not in params, (name, f)
             assert not re.search(r"__ld\w+\(|\bReadOnly\b|global\.nc\b|asm\s*\(\s*\"ld\b", body), (name, f)
             todo += re.findall(r"\b(\w+)\s*(?:<[^;{}()]*>)?\(", body)
+
+
+def test_launches_before_a_sort_by_cluster_are_looked_at():
+    """cluster_sort clears the error of a cluster that the device does not take; an error from before would go with it."""
+    callers = [body for name, (_, _, body) in functions(r"cudaError_t").items() if "cluster_sort(" in body and name != "cluster_sort"]
+    assert len(callers) == 2
+    for body in callers:
+        before = body[:body.index("cluster_sort(")]
+        assert len(re.findall(r"\blaunch_after\(", before)) == len(re.findall(r"\be = launch_after\(", before)) >= 2
+        assert len(re.findall(r"if \(e != cudaSuccess\) return e;|\) != cudaSuccess\) return e;", before)) >= 2
+
+
+def test_only_launched_kernels_are_counted():
+    body = functions(r"inline cudaError_t")["launch_after"][2]
+    assert body.index("cudaLaunchKernelEx(") < body.index("if (e == cudaSuccess) note_launch();")
+    body = functions(r"cudaError_t")["cluster_sort"][2]
+    assert re.search(r"cudaLaunchKernelEx\([^;]*== cudaSuccess\) note_launch\(\);", body)
 
 
 def test_the_number_of_sms_is_asked_for():
