@@ -1,11 +1,11 @@
-// Stable sort of a few thousand to 82 thousand (key, 32-bit value) pairs by one cluster of sixteen blocks.
+// Stable sort of a few thousand to some 80 thousand (key, 32-bit value) pairs by one cluster of sixteen blocks.
 //
 // The pairs stay in the shared memory of the cluster from the first pass to the last.  Per pass of eight bits every warp counts the
 // digits of its share and numbers its pairs among those of the same digit, the counts are added up over the warps of a block
 // and over the blocks, and every pair goes to its place in the blocks' other buffers.  Bound by latency (three barriers and a dozen
 // rounds of votes a pass); one launch, where the library's sort takes a histogram, a scan and, per pass, a clear and a kernel, each
 // with microseconds until it gets going.  30-bit / 48-bit keys, us, library and here: 4 k 14 and 21 / 74 and 31, 8 k 60 and 23, 30 k 66
-// and 31 / 86 and 47, 66 k 69 and 50 / 93 and 75, 100 k 74 and 75 / 100 and 113: hence the limits.  (Votes on the bits of a digit: with
+// and 31 / 86 and 47, 66 k 69 and 50 / 93 and 75, 100 k 74 and 75 / 100 and 113.  (Votes on the bits of a digit: with
 // __match_any_sync, which takes as long as there are digits, 30 k took 41 us.)
 #pragma once
 #include "rgx_internal.cuh"
@@ -16,8 +16,17 @@ namespace {
 
 constexpr int kSortCluster = 16, kClusterThreads = 1024, kClusterWarps = kClusterThreads / 32, kDigits = 256;
 
-constexpr int kClusterPiece = 5 * kClusterThreads;                             // pairs a block holds at most; a call deals its pairs out in equal pieces
-constexpr int kClusterSortFrom = 4097, kClusterSortTo = kSortCluster * kClusterPiece;
+// Pairs a block holds at most.  A call deals its pairs out in pieces of a multiple of 1,024, the last blocks get what is left or nothing;
+// where the pieces grow the time does, by 4 to 12 us: builds with 30-bit / 60-bit keys of 16,384 and 16,385 Gaussians 35.2 and 41.3 / 55.6 and
+// 67.9 us, of 32,768 and 32,769 43.4 and 51.6 / 76.0 and 86.3 (with the library 70.3 to 76.2 / 114 to 124).
+constexpr int kClusterPiece = 5 * kClusterThreads;
+// From and to how many pairs the cluster is the faster, by the width of the keys (whole calls, us, library and here).  Up to 4,864 short keys
+// are one block's work for the library: builds of 4,864 Gaussians 25 and 32, distances of as many points 46 and 54, of 4,865 65 and 31, 86 and
+// 54.  Long keys take six or eight passes: builds with 60-bit keys of 76,000 130 and 123, of 78,000 131 and 129, of 81,920 131 and
+// 135; distances (48 bits) of 76,000 points 136 and 130, of 78,000 144 and 140, of 81,920 144 and 145.  Short keys end with the memory of the
+// blocks: builds of 81,920 84 and 77.
+template <class Key> constexpr int kClusterSortFrom = sizeof(Key) == 4 ? 4865 : 4097;
+template <class Key> constexpr int kClusterSortTo = sizeof(Key) == 4 ? kSortCluster * kClusterPiece : 78000;
 template <class Key>
 size_t cluster_sort_smem(int piece) { return 2 * (size_t)piece * (sizeof(Key) + sizeof(unsigned) + 1) + sizeof(unsigned) * (kClusterWarps + 2) * kDigits; }
 
@@ -124,7 +133,7 @@ inline bool cluster_refused(cudaError_t e) {
 // that error: the caller has looked at the results of its launches before.
 template <class Key>
 cudaError_t cluster_sort(const Key* keys_in, Key* keys_out, const unsigned* vals_in, unsigned* vals_out, int n, int bits, cudaStream_t s) {
-    if (n < kClusterSortFrom || n > kClusterSortTo) return cudaErrorNotSupported;
+    if (n < kClusterSortFrom<Key> || n > kClusterSortTo<Key>) return cudaErrorNotSupported;
     const int per_block = (n + kSortCluster - 1) / kSortCluster, piece = (per_block + kClusterThreads - 1) / kClusterThreads * kClusterThreads;
     const size_t smem = cluster_sort_smem<Key>(piece);
     cudaError_t e;

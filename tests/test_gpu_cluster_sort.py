@@ -1,6 +1,6 @@
 """Sets of the sizes that one cluster of blocks sorts, and on either side of them (`-m gpu`).  Neighbour distances against brute force
 (every point gets its own), and the march: a set together with Gaussians below the threshold, which take no part, is sorted by the library once
-it has more than 82 thousand members, and must give the same image, bit for bit where the lists' keys have as many bits, and the same gradients."""
+it has more than some 80 thousand members, and must give the same image, bit for bit where the lists' keys have as many bits, and the same gradients."""
 import pytest
 import torch
 
@@ -15,7 +15,7 @@ def gpu():
     return torch.device("cuda")
 
 
-@pytest.mark.parametrize("n", [4096, 4097, 16384, 16385, 65535, 65536, 81920, 81921])
+@pytest.mark.parametrize("n", [4096, 4097, 4864, 4865, 16384, 16385, 65535, 65536, 78000, 78001, 81920, 81921])
 def test_every_point_gets_its_own_distance(n):
     dev = gpu()
     from simple_knn._C import distCUDA2
@@ -32,7 +32,7 @@ def test_every_point_gets_its_own_distance(n):
     assert torch.isfinite(got).all() and (got > 0).all()
 
 
-@pytest.mark.parametrize("n,cluster", [(4096, False), (4097, True), (65535, True), (65536, True), (81920, True), (81921, False)])
+@pytest.mark.parametrize("n,cluster", [(4096, False), (4864, False), (4865, True), (65535, True), (65536, True), (78000, True), (78001, False)])
 def test_the_cluster_sorts_what_it_is_for(n, cluster):
     """Own kernels of a call: bounds, keys, gather, upper boxes, query, and the cluster's sort; those of the library are not counted."""
     dev = gpu()
@@ -44,7 +44,21 @@ def test_the_cluster_sorts_what_it_is_for(n, cluster):
     assert _lib.lib().rgx_kernel_launches() - before == 5 + cluster
 
 
-@pytest.mark.parametrize("n,bits", [(4097, 10), (30_000, 10), (30_000, 20), (70_001, 10), (81_920, 10), (81_920, 20)])
+@pytest.mark.parametrize("n,bits,cluster", [(4864, 10, False), (4865, 10, True), (81_920, 10, True), (81_921, 10, False),
+                                            (4096, 20, False), (4097, 20, True), (78_000, 20, True), (78_001, 20, False)])
+def test_the_cluster_sorts_what_it_is_for_in_a_build(n, bits, cluster):
+    """Own kernels of a build: bounds, keys, gather, refit, and the cluster's sort."""
+    dev = gpu()
+    from raygaussx_b200 import _lib
+    from raygaussx_b200 import render_optix as ro
+    tens = [t.to(dev).contiguous() for t in scenes.tiny_scene(n=n, width=8, height=8, seed=n).tensors()]
+    r = ro.Renderer(dev)
+    before = _lib.lib().rgx_kernel_launches()
+    r.build(*tens[:4], morton_bits=bits)
+    assert _lib.lib().rgx_kernel_launches() - before == 4 + cluster
+
+
+@pytest.mark.parametrize("n,bits", [(4097, 10), (4097, 20), (4865, 10), (30_000, 10), (30_000, 20), (70_001, 10), (78_000, 20), (81_920, 10), (81_920, 20)])
 def test_same_image_and_gradients_as_with_the_library(n, bits):
     dev = gpu()
     from raygaussx_b200 import render_optix as ro
