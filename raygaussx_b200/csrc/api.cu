@@ -73,7 +73,7 @@ struct rgx_ctx {
     int* big_slot = nullptr;
     uint2* big_rect = nullptr;
     int big_cap = 0, sm_count = 0;
-    BinResult* bin_result_host = nullptr;              // pinned; the device's copy heads bin_zero
+    BinResult* bin_result_host = nullptr;              // pinned; the device's copy heads bin_zero, but for `longest` and `long_tiles`, which are left here only
     // two-depth lists of forward-only views (binning.cu, march_lists.cu HZ variant)
     int *tile_more = nullptr;      // in bin_zero
     int *tile_resume = nullptr; int hz_tiles_cap = 0;
@@ -121,7 +121,7 @@ struct rgx_ctx {
     // [0] ints of the recording reserved, [4] rays that went beyond the horizon, [8 ...) per tile: some ray of the latest recording
     // forward could not be recorded; cleared by one memset
     unsigned long long* tape_used = nullptr; long long tape_used_cap = 0;
-    unsigned long long* tape_used_host = nullptr;   // pinned; refreshed asynchronously after every recording forward
+    unsigned long long* tape_used_host = nullptr;   // pinned; stored by the kernel behind every recording forward
     long long* patch_heads = nullptr;               // first chunk of every patch, then a byte per ray: not recorded
     long long patch_head_cap = 0;
     bool tape_valid = false;

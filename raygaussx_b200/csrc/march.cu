@@ -97,10 +97,6 @@ __global__ void __launch_bounds__(kWarps * 32) march_forward_kernel(const __grid
     if (COUNT) flush_tally(L, tl, lane);
 }
 
-// The rays a list march left unfinished because its lists stop at a horizon (march_lists.cu, HZ = 2): L.hz_rays
-// holds their numbers, *L.hz_count how many.  They are marched again from the start by searching the hierarchy,
-// which needs no lists: same hits, met in slot order instead of list order, so the colour equals that of complete
-// lists to summation rounding.  Launched after every such march; returns at once when there are none.
 // The counts of the march that has just finished, to the host's pinned memory (a copy each would hold up the stream for ten
 // microseconds and more).
 __device__ __forceinline__ void report(const MarchLaunch& L) {
@@ -112,6 +108,10 @@ __global__ void report_kernel(const __grid_constant__ MarchLaunch L) {
     report(L);
 }
 
+// The rays a list march left unfinished because its lists stop at a horizon (march_lists.cu, HZ = 2): L.hz_rays
+// holds their numbers, *L.hz_count how many.  They are marched again from the start by searching the hierarchy,
+// which needs no lists: same hits, met in slot order instead of list order, so the colour equals that of complete
+// lists to summation rounding.  Launched after every such march; returns at once when there are none.
 __global__ void __launch_bounds__(kWarps * 32) march_forward_listed_rays_kernel(const __grid_constant__ MarchLaunch L) {
     __shared__ WarpShared shared[kWarps];
     const unsigned int n = *L.hz_count;

@@ -501,8 +501,8 @@ __device__ __forceinline__ float2 fma2_in_place(float2 a, float2 b, float2 c) {
 }
 
 // Sample numbers plus a half of a lane's pairs with two lanes per ray (the first lane's; the other's are one more).  From constant memory,
-// where an instruction takes them as an operand: as literals they cost two moves per pair of samples (four 3 M views 13.47 -> 13.28 ms,
-// three frames of 7 M needles 13.98 -> 13.73, the object 3.05 -> 3.03).
+// where an instruction takes them as an operand, and not literals (four 3 M views 13.47 -> 13.28 ms, three frames of 7 M needles
+// 13.98 -> 13.73, the object 3.05 -> 3.03).
 __constant__ float2 kPairAt[8] = {{0.5f, 2.5f}, {4.5f, 6.5f}, {8.5f, 10.5f}, {12.5f, 14.5f}, {16.5f, 18.5f}, {20.5f, 22.5f}, {24.5f, 26.5f}, {28.5f, 30.5f}};
 
 // Sum of one value over the P lanes of a ray (P consecutive samples), as a balanced tree; `before`: over the lanes before this one.
@@ -536,10 +536,12 @@ struct SampleTree {
 // one; against CTAs of four warps (12 of 168 registers per SM when recording, 16 of 128 otherwise) the recording forward took 3.52
 // instead of 4.09 ms on the 3 M view and 3.39 instead of 3.73 on the 300 k object.  15 warps are slower (four 3 M views 13.98 against
 // 13.46 ms, the object 3.09 against 3.05), 18 of 112 registers much slower (15.25, 3.89): the sums of a slab alone are 64.
+// All of that with two lanes per ray.  Four and eight, whose sums are 32 and 16 registers, have the same number; more was not tried there.
 template <bool COUNT>
 __host__ __device__ constexpr int forward_ctas() { return COUNT ? 4 : 16; }
 // The replay, of 96 registers and 8.9 KB: 20 warps per SM.  18 are 1.5 to 3 % slower (four 3 M views 10.57 against 10.40 ms, the 300 k
-// object 1.95 against 1.89), 17 another 4 % on the 3 M views, 21 (80 registers) as slow as 18.
+// object 1.95 against 1.89), 17 another 4 % on the 3 M views, 21 (80 registers) as slow as 18.  With two lanes per ray, and taken over for
+// four and eight.
 constexpr int kReplayCtas = 20;
 
 template <int P, bool COUNT, bool SAVE, int HZ>
@@ -1226,8 +1228,8 @@ static bool use_lists(const MarchLaunch& m) {
     return !(m.m.flags & (RGX_FLAG_BRUTE_FORCE | RGX_FLAG_PER_RAY_SEARCH)) && m.lists.ent_id != nullptr && m.g.n > 0;
 }
 
-// Lanes per ray.  Two where the image gives every warp the device can hold a patch of sixteen rays (28,000 rays and more); with
-// fewer rays, smaller patches: more warps, and fewer Gaussians per patch, the longest patch being all there is to wait for.
+// Lanes per ray.  Two where the image gives every warp the device can hold a patch of sixteen rays (at sixteen warps on each of 148 SMs that
+// is 37,888 rays; the line is at 200x200); with fewer rays, smaller patches: more warps, and fewer Gaussians per patch, the longest patch being all there is to wait for.
 // Forward + backward in ms with 2 / 4 / 8 lanes per ray, 100 k object: 64x64 1.01 / 0.54 / 0.36, 128x128 0.65 / 0.45 / 0.36, 150x150
 // 0.77 / 0.51 / 0.49, 180x180 0.75 / 0.52 / 0.60, 256x256 0.74 / 0.74 / 0.97, 300x300 0.92 / 1.06 / 1.48; 1 M unbounded: 128x128 0.41 / 0.28 / 0.24,
 // 150x150 0.43 / 0.30 / 0.30, 200x200 0.44 / 0.38 / 0.43, 256x256 0.50 / 0.50 / 0.64.  Four lanes would do a little better up to 240x240 (object 0.66 against

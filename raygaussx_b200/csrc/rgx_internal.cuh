@@ -329,10 +329,11 @@ cudaError_t launch_bin_emit(const BinLaunch& b, cudaStream_t s);
 cudaError_t launch_bin_fill(const BinLaunch& b, int total, const BinResult& r, cudaStream_t s);
 float bin_hist_bucket_end(const BinLaunch& b, int bucket);
 cudaError_t launch_march_forward(const MarchLaunch& m, cudaStream_t s);
-// The rays listed in m.hz_rays by a march over lists that stop at a horizon, again by per-ray search (march.cu).
+// The rays listed in m.hz_rays by a march over lists that stop at a horizon, again by per-ray search (march.cu); the march's counts go to
+// pinned memory with it.
+cudaError_t launch_march_forward_listed_rays(const MarchLaunch& m, int ctas, cudaStream_t s);
 // The ints that a recording march has used, to pinned memory, where no launch of the above does it.
 cudaError_t launch_report(const MarchLaunch& m, cudaStream_t s);
-cudaError_t launch_march_forward_listed_rays(const MarchLaunch& m, int ctas, cudaStream_t s);
 // The backward in two launches: rays without a recording (searches the lists or the hierarchy), then the replay of
 // the recording, which reads neither lists nor hierarchy.
 cudaError_t launch_march_backward_search(const MarchLaunch& m, cudaStream_t s);
