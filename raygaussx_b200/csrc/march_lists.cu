@@ -477,7 +477,7 @@ __device__ __forceinline__ void tape_append(const MarchLaunch& L, TapeState& tq,
 //   Slabs of the rays are taken in steps: the ray that is furthest behind leads, and every ray whose slab begins before the
 // leader's ends marches with it.  The list is walked once per step over the union of the windows.
 //   Measured against a warp per ray with lanes as samples (forward ms): 3 M-Gaussian view 9.3 -> 2.8, 300 k object 9.3 -> 2.6 (7.8 -> 2.3
-// without recording), 7 M needles 14.6 -> 3.85 (two depths), 1 M at 640x360 1.83 -> 0.56.
+// without recording), 7 M needles 14.6 -> 3.85 (two depths), 1 M at 640x360 1.83 -> 0.48.
 //
 // HZ: the two-depth variant for forward-only views whose rays end early (binning.cu).  In its first phase
 // (L.hz_phase == 1) the tile lists hold only the pairs that begin before L.horizon; a ray that would need more
